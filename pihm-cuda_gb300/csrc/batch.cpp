@@ -690,6 +690,12 @@ int run_round(pihm_batch *B, bool *any) {
   B->rounds++;
   const double *res = (const double *)B->h_down;
   const unsigned int *err = (const unsigned int *)(B->h_down + sizeof(double) * 2 * B->max_sys);
+  // an evaluation whose waits ran out leaves its barrier counters as they were
+  for (Sys *s : part)
+    if (s->rhs_req && (err[s->slot] & pihm::kErrWait)) {
+      if (cudaMemsetAsync(B->A.m.bar, 0, sizeof(unsigned int) * pihm::kBarWords, st) != cudaSuccess) return -1;
+      break;
+    }
   for (Sys *s : part) {
     s->prog.clear();
     if (!s->waiting) continue;  // a finished watershed's last operations
@@ -840,6 +846,7 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
   m.eflux_sub = D(NED);
   m.bank_part = D(8 * NE);
   m.err = dalloc<unsigned int>(1, o);
+  m.bar = dalloc<unsigned int>(pihm::kBarWords, o);
   int32_t *se = I(NE), *sr = I(NR), *sed = I(NED), *sb = I(NE);
   m.sys_elem = se;
   m.sys_riv = sr;
@@ -880,7 +887,7 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
   B->down_bytes = sizeof(double) * 2 * MS + sizeof(unsigned int) * MS;
   B->d_down = (char *)dalloc<char>(B->down_bytes, o);
   if (t_count_bytes) return PIHM_GPU_OK;  // sizes counted, nothing allocated
-  if (!ok || !m.err || !A.sysinfo || !A.tickets || !B->d_up || !B->d_down ||
+  if (!ok || !m.err || !m.bar || !A.sysinfo || !A.tickets || !B->d_up || !B->d_down ||
       cudaMallocHost(&B->h_up, up_bytes) != cudaSuccess ||
       cudaMallocHost(&B->h_down, B->down_bytes) != cudaSuccess)
     return PIHM_GPU_ERR_NOMEM;
@@ -900,6 +907,7 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
            cudaMemset(B->d_up, 0, up_bytes) == cudaSuccess &&
            cudaMemset(m.rivflow, 0, sizeof(double) * NUM_RIVFLX * NR) == cudaSuccess &&
            cudaMemset(m.carry_ovl, 0, sizeof(double) * 2 * NR) == cudaSuccess &&
+           cudaMemset(m.bar, 0, sizeof(unsigned int) * pihm::kBarWords) == cudaSuccess &&
            cudaMemset(A.rhs_in, 0, sizeof(double) * NEQ) == cudaSuccess &&
            cudaDeviceSynchronize() == cudaSuccess;
   if (!z) return PIHM_GPU_ERR_CUDA;

@@ -181,7 +181,7 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
   dbytes += carve_size<double>(8 * NB);       // bank_part
   dbytes += 2 * carve_size<double>(3 * NE) + 2 * carve_size<double>(NE) + carve_size<double>(5 * NE);
   dbytes += 2 * carve_size<double>(c->neq);   // staging
-  dbytes += carve_size<unsigned int>(1);
+  dbytes += carve_size<unsigned int>(1) + carve_size<unsigned int>(kBarWords);
   if (cudaMalloc(&c->d_dyn, dbytes) != cudaSuccess) {
     pihm_gpu_destroy(c);
     return PIHM_GPU_ERR_NOMEM;
@@ -208,6 +208,7 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
   c->d_stage_in = carve<double>(dp, c->neq);
   c->d_stage_out = carve<double>(dp, c->neq);
   m.err = carve<unsigned int>(dp, 1);
+  m.bar = carve<unsigned int>(dp, kBarWords);
   m.diag = 0;
   if (pihm::create_rhs_streams(&c->side) != cudaSuccess) {
     pihm_gpu_destroy(c);
@@ -407,8 +408,10 @@ int pihm_gpu_status(pihm_gpu_ctx *c) {
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
   if (err) {
     cudaMemsetAsync(c->m.err, 0, sizeof(unsigned int), c->stream);
+    // a launch whose waits ran out leaves its barrier counters as they were
+    if (err & kErrWait) cudaMemsetAsync(c->m.bar, 0, sizeof(unsigned int) * kBarWords, c->stream);
     cudaStreamSynchronize(c->stream);
-    return PIHM_GPU_ERR_NAN;
+    return err & kErrWait ? PIHM_GPU_ERR_CUDA : PIHM_GPU_ERR_NAN;
   }
   return PIHM_GPU_OK;
 }

@@ -122,11 +122,17 @@ struct TVal {
   int64_t f;
 };
 
+// Every function below evaluates its result without a branch and returns
+// whether the operands were in range (the result means nothing otherwise), so
+// a caller can run independent ones beside each other and test them together:
+// one power is a chain of dependent products, and a warp alone on its
+// scheduler waits out each one's latency.
+
 // 1024 log2 x = 1024 k + w 2^-53, for x positive and normal with |k| <= 126.
 PIHM_IM_FN bool log2k(double x, int &k, int64_t &w) {
   const uint64_t xb = dbits(x);
   const unsigned top = (unsigned)(xb >> 52);  // sign and biased exponent
-  if (top - 897u >= 253u) return false;       // not positive, or |k| > 126
+  const bool ok = top - 897u < 253u;          // positive, |k| <= 126
   k = (int)top - 1023;
   const uint64_t M = (xb & kFrac) | (1ull << 52);
   const unsigned i = (unsigned)(xb >> 42) & 1023u;
@@ -143,7 +149,7 @@ PIHM_IM_FN bool log2k(double x, int &k, int64_t &w) {
   const int64_t r2 = mulhi(r, r);               // r^2 2^80
   const int64_t lp = r + (mulhi(r2, h) >> 6);   // log1p(r) 2^72
   w = PIHM_IM_LD(kImLogH[i]) + ((mulhi(lp, kImK) + 64) >> 7);
-  return true;
+  return ok;
 }
 
 // t = y (1024 k + w 2^-53) for y normal with exponent in [-20, 29] and
@@ -151,19 +157,20 @@ PIHM_IM_FN bool log2k(double x, int &k, int64_t &w) {
 PIHM_IM_FN bool mul_t(double y, int k, int64_t w, TVal &t) {
   const uint64_t yb = dbits(y);
   const int ey = (int)((yb >> 52) & 2047u) - 1023;
-  if ((unsigned)(ey + 20) >= 50u) return false;
+  const bool ok = (unsigned)(ey + 20) < 50u;
   const int64_t my = (int64_t)((yb & kFrac) | (1ull << 52));
   // Q = My (k 2^63 + w) exactly (|My k| < 2^60, |My w| < 2^116); y =
   // My 2^(ey - 52) and 1024 k + w 2^-53 = (k 2^63 + w) 2^-53, so
   // t 2^64 = Q 2^(ey - 41), a right shift by 12..61
-  i128 Q = (i128)my * w + ((i128)(my * k) << 63);
-  Q >>= 41 - ey;
+  const int64_t mk = (int64_t)((uint64_t)my * (uint64_t)(int64_t)k);
+  i128 Q = (i128)((unsigned __int128)((i128)my * w) + ((unsigned __int128)(i128)mk << 63));
+  Q >>= (41 - ey) & 63;
   if (yb >> 63) Q = -Q;
   const int64_t hi = (int64_t)(Q >> 64);
   const uint64_t lo = (uint64_t)Q;
   t.n = hi + (int64_t)(lo >> 63);  // round(t)
   t.f = (int64_t)lo;               // t - round(t), units of 2^-64
-  return t.n < kNMax && t.n > -kNMax;
+  return ok & (t.n < kNMax) & (t.n > -kNMax);
 }
 
 // 2^(t/1024) for |t| < 1.5 * 2^16: a normal double
@@ -191,7 +198,7 @@ PIHM_IM_FN double exp2k(TVal t) {
     mant >>= 1;
     q += 1;
   }
-  return bitsd(((uint64_t)(q + 1023) << 52) + (mant & kFrac));
+  return bitsd(((uint64_t)(int64_t)(q + 1023) << 52) + (mant & kFrac));
 }
 
 // 1024 log2 q for q = fl(1/x), the correctly rounded reciprocal of x, from
@@ -204,19 +211,18 @@ PIHM_IM_FN double exp2k(TVal t) {
 PIHM_IM_FN bool log2k_recip(double x, double q, int k, int64_t w, int &kq, int64_t &wq) {
   const uint64_t xb = dbits(x), qb = dbits(q);
   const int ex = (int)((xb >> 52) & 2047u), eq = (int)((qb >> 52) & 2047u);
-  if (eq - 1u >= 2046u || (qb >> 63)) return false;
   const int s = 104 - (ex - 1023) - (eq - 1023);  // q x = (Mx Mq) 2^-s
-  if (s != 104 && s != 105) return false;
+  bool ok = (eq - 1u < 2046u) & !(qb >> 63) & ((s == 104) | (s == 105));
   const uint64_t Mx = (xb & kFrac) | (1ull << 52), Mq = (qb & kFrac) | (1ull << 52);
   const int64_t D = (int64_t)(Mx * Mq);  // Mx Mq - 2^s (2^s vanishes mod 2^64)
-  if (D > (1ll << 53) || D < -(1ll << 53)) return false;  // |D| <= 2^52 for a correctly rounded q
+  ok &= (D <= (1ll << 53)) & (D >= -(1ll << 53));  // |D| <= 2^52 for a correctly rounded q
   // (1024/ln 2) D 2^-s in units of 2^-53: mulhi(D 2^8, kImK) is
   // (1024/ln 2) D 2^-4 (kImK = (1024/ln 2) 2^52), rounded by 2^(57 - s)
-  const int sh = s - 57;  // 47 or 48
-  const int64_t c = (mulhi(D * 256, kImK) + (1ll << (sh - 1))) >> sh;
+  const int sh = s == 104 ? 47 : 48;  // s - 57
+  const int64_t c = (mulhi((int64_t)((uint64_t)D * 256u), kImK) + (1ll << (sh - 1))) >> sh;
   kq = -k;
   wq = -w + c;
-  return true;
+  return ok;
 }
 
 // x^y on the integer path; false when x or y is outside its ranges.  +0 to
@@ -226,13 +232,11 @@ PIHM_IM_FN bool pow_i(double x, double y, double &out) {
   int k;
   int64_t w;
   TVal t;
-  if (dbits(x) == 0 && dbits(y) - 1u < 0x7FF0000000000000ull) {
-    out = 0.0;
-    return true;
-  }
-  if (!log2k(x, k, w) || !mul_t(y, k, w, t)) return false;
-  out = exp2k(t);
-  return true;
+  const bool zero = (dbits(x) == 0) & (dbits(y) - 1u < 0x7FF0000000000000ull);
+  const bool in_x = log2k(x, k, w), in_t = mul_t(y, k, w, t);
+  const double r = exp2k(t);
+  out = zero ? 0.0 : r;
+  return zero | (in_x & in_t);
 }
 
 
@@ -320,12 +324,10 @@ PIHM_IM_FN uint64_t seed_fixed(float r) {
 PIHM_IM_FN bool div_i(double a, double b, double &q) {
   const uint64_t ab = dbits(a), bb = dbits(b);
   const unsigned ea = (unsigned)(ab >> 52) & 2047u, eb = (unsigned)(bb >> 52) & 2047u;
-  if (eb - 1u >= 2046u) return false;  // zero, subnormal, inf or nan divisor
-  if (ea - 1u >= 2046u) {
-    if (ab << 1) return false;  // subnormal, inf or nan dividend
-    q = bitsd((ab ^ bb) & (1ull << 63));
-    return true;
-  }
+  // neither a zero, subnormal, inf or nan divisor nor a subnormal, inf or
+  // nan dividend
+  const bool zero = (ab << 1) == 0;
+  const bool ok = (eb - 1u < 2046u) & (zero | (ea - 1u < 2046u));
   const uint64_t Ma = (ab & kFrac) | (1ull << 52), Mb = (bb & kFrac) | (1ull << 52);
   // 1/mb, mb = Mb 2^-52 in [1, 2): R = r 2^63.  Newton's step r <- r (1 + e),
   // e = 1 - mb r, never overshoots 1/mb in exact arithmetic; the first step
@@ -364,20 +366,17 @@ PIHM_IM_FN bool div_i(double a, double b, double &q) {
     ex += 1;
   }
   const int eq = ex + 1023;
-  if (eq < 1 || eq > 2046) return false;
-  q = bitsd((((ab ^ bb) >> 63) << 63) | ((uint64_t)eq << 52) | (mant & kFrac));
-  return true;
+  const uint64_t sign = ((ab ^ bb) >> 63) << 63;
+  q = bitsd(sign | (zero ? 0ull : ((uint64_t)(int64_t)eq << 52) | (mant & kFrac)));
+  return ok & (zero | ((unsigned)(eq - 1) < 2046u));
 }
 
 // sqrt(x) for positive normal x, or a zero
 PIHM_IM_FN bool sqrt_i(double x, double &r) {
   const uint64_t xb = dbits(x);
-  if ((xb << 1) == 0) {  // sqrt(+-0) = +-0
-    r = x;
-    return true;
-  }
+  const bool zero = (xb << 1) == 0;          // sqrt(+-0) = +-0
   const unsigned top = (unsigned)(xb >> 52);  // sign and biased exponent
-  if (top - 1u >= 2046u) return false;       // not positive and normal
+  const bool ok = zero | (top - 1u < 2046u);  // else not positive and normal
   const int ex = (int)top - 1023;
   const int odd = ex & 1;
   // x = m 2^(ex - odd), m = M 2^-52 in [1, 4)
@@ -409,8 +408,8 @@ PIHM_IM_FN bool sqrt_i(double x, double &r) {
     mant >>= 1;
     er += 1;
   }
-  r = bitsd(((uint64_t)(er + 1023) << 52) | (mant & kFrac));
-  return true;
+  r = zero ? x : bitsd(((uint64_t)(int64_t)(er + 1023) << 52) | (mant & kFrac));
+  return ok;
 }
 
 }  // namespace im

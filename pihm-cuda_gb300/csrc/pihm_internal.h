@@ -38,6 +38,11 @@ enum RivFlx {
 // -1 - s for river segment s, kBoundary for the domain edge.
 constexpr int32_t kBoundary = INT32_MIN;
 
+// Bits of an error word: a derivative came out NaN; a wait inside a kernel
+// ran out (the evaluation's results are not valid).
+constexpr unsigned kErrNan = 1u, kErrWait = 2u;
+constexpr int kBarWords = 160;  // unsigned words of DevMesh::bar
+
 // Device view of one watershed, passed by value to the kernels.
 struct DevMesh {
   int32_t ne, nr, nbank;
@@ -105,7 +110,8 @@ struct DevMesh {
   double *d_ovl, *d_sub, *d_infil, *d_rechg, *d_et;  // [3][ne],[3][ne],[ne],[ne],[5][ne]
   int diag;
 
-  unsigned int *err;  // error word
+  unsigned int *err;  // error word: kErrNan, kErrWait
+  unsigned int *bar;  // k_rhs_fused's barrier counters (null: not used)
 
   // Launch extents.  A single-watershed context evaluates every item
   // (ne_run = ne, ...); the batch engine's arena places watersheds in ranges of
@@ -246,12 +252,23 @@ struct Profiler {
 
 enum KernelId { K_PREP = 0, K_GRAD, K_MAIN, K_RIVER, K_FINISH, K_EDGE, K_PERMUTE };
 
+// What k_rhs_fused needs to size its cooperative launch: the SMs, and the
+// blocks of 32, 64, 128 and 256 threads of its two builds that can be
+// resident together (0: the device has no cooperative launch).
+struct FusedPlan {
+  static constexpr int kSizes = 4;
+  int sms = 0;
+  int blocks[2][kSizes] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+};
+cudaError_t fused_plan(FusedPlan *f);
+
 // A second stream on which the river kernel of an evaluation runs beside the
 // element kernels (it needs only k_elem_prep's outputs), joined before
 // k_finish.  Null members: everything on one stream.
 struct RhsStreams {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  FusedPlan fused;
 };
 
 // The river kernel's stream and events.  The stream has the highest
@@ -264,6 +281,7 @@ inline cudaError_t create_rhs_streams(RhsStreams *s) {
   if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, greatest);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = fused_plan(&s->fused);
   return e;
 }
 

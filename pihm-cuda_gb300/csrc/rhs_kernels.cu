@@ -1,10 +1,10 @@
 // FP64 right-hand-side kernels of the PIHM hydrologic model for sm_103a.
 //
 // One evaluation of f(t, y) (the reference ODE(), src/ode.c:4-399) runs as
-// seven launches with no host synchronisation, the two river kernels on a
-// second stream beside k_elem_grad/k_edge/k_elem_main (k_edge is listed at
-// its definition: each interior edge is evaluated once and read with a sign
-// by both elements).  GB300 issues ~2 FP64 lanes per clock per SM, so the
+// seven launches with no host synchronisation, the three river kernels on a
+// second stream beside k_elem_grad/k_edge (k_edge is listed at its
+// definition: each interior edge is evaluated once and read with a sign by
+// both elements).  GB300 issues ~2 FP64 lanes per clock per SM, so the
 // FP64 pipe is the scarce one: the element rows' powers, divisions and
 // square roots run in fixed point on the integer pipe (int_math.cuh; the
 // divisions and roots IEEE-exact), comparisons and sign flips on the
@@ -26,24 +26,28 @@
 //                 OvlFlowElemToElem, BoundFluxElem, src/lat_flow.c:285-382),
 //                 EtExtract (src/hydrol.c:33-97), Infil/Recharge/EffKinf/AvgKv
 //                 (src/vert_flow.c:33-270) and the element rows of ydot
-//                 (src/ode.c:111-209).  Elements with river edges hand their
-//                 partial sums to k_finish, because their river-edge fluxes are
-//                 written by the river kernel of the same evaluation.
+//                 (src/ode.c:111-209), the river banks' with this evaluation's
+//                 river-edge fluxes.
 //   k_riv_geom    per segment: channel area and wetted perimeter at the
 //                 stage (src/river_flow.c:520-583), once per segment.
-//   k_river       per segment: RiverFlow (src/river_flow.c:3-94) and
-//                 RiverToElem (:113-183), ChanLeak, OutletFlux, BoundFluxRiver.
-//   k_finish      per segment: upstream accumulation in reference order
+//   k_river       per segment, in four parts: RiverFlow
+//                 (src/river_flow.c:3-94) and RiverToElem (:113-183), ChanLeak,
+//                 OutletFlux, BoundFluxRiver.
+//   k_river_rows  per segment: upstream accumulation in reference order
 //                 (src/river_flow.c:96-110, a CSR list instead of a serial
-//                 loop) and the river rows of ydot (src/ode.c:228-300); per
-//                 river-bank element: the rest of its element rows.
+//                 loop) and the river rows of ydot (src/ode.c:228-300).
+//
+// The river kernels finish before k_elem_main starts, so the banks' rows need
+// no pass of their own after it: one (k_finish, latency-bound, 20 us of a
+// 355 us evaluation of 1M elements) stood at the end of the critical path.
 //
 // Infil reads the river-edge overland flux of the previous evaluation
 // (src/vert_flow.c:61 runs before src/river_flow.c:159-182 rewrites it); that
-// value is the previous evaluation's LEFT/RIGHT_SURF2CHANL, which k_finish
-// copies to carry_ovl, so k_elem_main can read it while this evaluation's
-// k_river runs.
+// value is the previous evaluation's LEFT/RIGHT_SURF2CHANL in carry_ovl, which
+// the bank element's thread in k_elem_main reads and then replaces.
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 #include "fp64_math.cuh"
 #include "pihm_internal.h"
@@ -71,8 +75,7 @@ __device__ __forceinline__ double avg_h_surf(double diff, double hsurf, double h
 // OverLandFlow, src/lat_flow.c:279-283
 __device__ __forceinline__ double overland_flow(double avg_h, double grad_h, double avg_sf,
                                                 double crossa, double avg_rough) {
-  return crossa * pow_manning(avg_h, kManningSurf) * grad_h /
-         (sqrt(avg_sf) * avg_rough);
+  return div_any(crossa * pow_manning(avg_h, kManningSurf) * grad_h, sqrt_any(avg_sf) * avg_rough);
 }
 
 // KrFunc (src/soil.c:8-13) and Psi (src/vert_flow.c:272-278) of one
@@ -91,9 +94,14 @@ __device__ __forceinline__ double overland_flow(double avg_h, double grad_h, dou
 // the rounded reciprocal fl(1/satn), whose logarithm follows from satn's and
 // the exact residual of the division (im::log2k_recip), within the same
 // 0.502 ulp as a power of its own.
-__device__ __forceinline__ void kr_psi(double satn, double vm, double vg_e, double vg_ib, double alpha,
-                                       double &satkfunc, double &psi, double &sq) {
-  sq = sqrt_any(satn);
+//
+// kr_psi evaluates everything without a branch, so that the root, the
+// reciprocal and the two last powers run beside each other, and asks once at
+// the end whether an operand was out of a range (a NaN state); kr_psi_slow
+// then repeats it operation by operation.
+static __device__ __noinline__ void kr_psi_slow(double satn, double vm, double vg_e, double vg_ib, double alpha,
+                                                double *satkfunc, double *psi, double *sq) {
+  *sq = sqrt_any(satn);
   const double q = div_any(1.0, satn);
   double pm, qm;  // satn^m, (1/satn)^m
   int k, kq;
@@ -108,8 +116,35 @@ __device__ __forceinline__ void kr_psi(double satn, double vm, double vg_e, doub
     qm = pow_any(q, vm);
   }
   const double t = 1.0 - pow_any(1.0 - pm, vg_e);
+  *satkfunc = *sq * t * t;
+  *psi = cmp::neg_if(div_any(pow_any(qm - 1.0, vg_ib), alpha), true);
+}
+__device__ __forceinline__ void kr_psi(double satn, double vm, double vg_e, double vg_ib, double alpha,
+                                       double &satkfunc, double &psi, double &sq) {
+  int k, kq;
+  int64_t w, wq;
+  im::TVal t1, t3;
+  double q, p1, p3, d;
+  bool ok = im::sqrt_i(satn, sq);
+  ok &= im::div_i(1.0, satn, q);
+  ok &= im::log2k(satn, k, w);
+  ok &= im::mul_t(vm, k, w, t1);
+  ok &= im::log2k_recip(satn, q, k, w, kq, wq);
+  ok &= im::mul_t(vm, kq, wq, t3);
+  const double pm = im::exp2k(t1), qm = im::exp2k(t3);  // satn^m, (1/satn)^m
+  ok &= im::pow_i(1.0 - pm, vg_e, p1);
+  ok &= im::pow_i(qm - 1.0, vg_ib, p3);
+  const double t = 1.0 - p1;
   satkfunc = sq * t * t;
-  psi = cmp::neg_if(div_any(pow_any(qm - 1.0, vg_ib), alpha), true);
+  ok &= im::div_i(p3, alpha, d);
+  psi = cmp::neg_if(d, true);
+  if (!ok) {
+    double a, b, c;  // the callers' values stay in registers
+    kr_psi_slow(satn, vm, vg_e, vg_ib, alpha, &a, &b, &c);
+    satkfunc = a;
+    psi = b;
+    sq = c;
+  }
 }
 
 // Batch engine: whether the watershed of item idx sits out this evaluation
@@ -123,8 +158,8 @@ __device__ __forceinline__ bool skip_item(const DevMesh &m, const int32_t *sys_o
   return s < 0 || !m.active[s];
 }
 
-__device__ __forceinline__ void report_err(const DevMesh &m, int sy) {
-  atomicOr(m.err_sys ? &m.err_sys[sy] : m.err, 1u);
+__device__ __forceinline__ void report_err(const DevMesh &m, int sy, unsigned code = kErrNan) {
+  atomicOr(m.err_sys ? &m.err_sys[sy] : m.err, code);
 }
 
 // Slot of the calling thread in a block's shared-memory work queue when take
@@ -148,7 +183,43 @@ __device__ __forceinline__ int queue_slot(int *count, bool take) {
 // ---------------------------------------------------------------------------
 constexpr int kPrepBlock = 256;
 
-//
+// SurfH and EffKh of one element (src/hydrol.c:100-134, src/lat_flow.c:248-277):
+// what needs no root or division is stored here; thin asks for
+// surfh = sqrt(sx), mix for effk = num / den.  EffKh's k1 = kmach*areafv +
+// ksath*(1-areafv) and depth - dmac are formed at load (the reference
+// evaluates both inline with the same operations).
+__device__ __forceinline__ void prep_item(const DevMesh &m, int i, double y_surf, double y_gw, bool &thin, double &sx,
+                                          bool &mix, double &num, double &den) {
+  const double surfeqv = clamp0(y_surf);
+  if (cmp::lt0(surfeqv)) {
+    m.surfh[i] = 0.0;
+    m.head[i] = 0.0 + m.zmax[i];
+  } else if (cmp::le_c(surfeqv, 0.5 * kDeprStg)) {
+    thin = true;
+    sx = 2.0 * kDeprStg * surfeqv;
+  } else {
+    const double sh = kDeprStg + (surfeqv - 0.5 * kDeprStg);
+    m.surfh[i] = sh;
+    m.head[i] = sh + m.zmax[i];
+  }
+  double gw = clamp0(y_gw);
+  gw = cmp::gt0(gw) ? gw : 0.0;
+  const double d_dmac = m.d_dmac[i];
+  if (cmp::gt_v(gw, d_dmac)) {
+    const double d1 = cmp::gt_v(gw, m.depth[i]) ? m.dmac[i] : gw - d_dmac;
+    num = m.kh_k1[i] * d1 + m.ksath[i] * d_dmac;
+    den = d1 + d_dmac;
+    mix = true;
+  } else {
+    m.effk[i] = m.ksath[i];
+  }
+}
+__device__ __forceinline__ void prep_root(const DevMesh &m, int i, double sx) {
+  const double sh = sqrt_any(sx);
+  m.surfh[i] = sh;
+  m.head[i] = sh + m.zmax[i];
+}
+
 // kFromRef: the host-buffer evaluation, where the state arrives in reference
 // order in memory the device reads over the host link.  Thread r then takes
 // reference element r (the link read is contiguous), stores its three values
@@ -195,35 +266,7 @@ __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const doubl
   }
   bool thin = false, mix = false;
   double sx = 0.0, num = 0.0, den = 0.0;
-  if (elem) {
-    // SurfH, src/hydrol.c:100-134
-    const double surfeqv = clamp0(y_surf);
-    if (cmp::lt0(surfeqv)) {
-      m.surfh[i] = 0.0;
-      m.head[i] = 0.0 + m.zmax[i];
-    } else if (cmp::le_c(surfeqv, 0.5 * kDeprStg)) {
-      thin = true;
-      sx = 2.0 * kDeprStg * surfeqv;
-    } else {
-      const double sh = kDeprStg + (surfeqv - 0.5 * kDeprStg);
-      m.surfh[i] = sh;
-      m.head[i] = sh + m.zmax[i];
-    }
-    // EffKh, src/lat_flow.c:248-277, with k1 = kmach*areafv + ksath*(1-areafv)
-    // and depth - dmac formed at load (the reference evaluates both inline
-    // with the same operations)
-    double gw = clamp0(y_gw);
-    gw = cmp::gt0(gw) ? gw : 0.0;
-    const double d_dmac = m.d_dmac[i];
-    if (cmp::gt_v(gw, d_dmac)) {
-      const double d1 = cmp::gt_v(gw, m.depth[i]) ? m.dmac[i] : gw - d_dmac;
-      num = m.kh_k1[i] * d1 + m.ksath[i] * d_dmac;
-      den = d1 + d_dmac;
-      mix = true;
-    } else {
-      m.effk[i] = m.ksath[i];
-    }
-  }
+  if (elem) prep_item(m, i, y_surf, y_gw, thin, sx, mix, num, den);
   const int ss = queue_slot(&qs_n, thin);
   if (thin) {
     qs_i[ss] = i;
@@ -237,44 +280,66 @@ __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const doubl
   }
   __syncthreads();
   const int t = threadIdx.x;
-  if (t < qs_n) {
-    const int e = qs_i[t];
-    const double sh = sqrt_any(qs_x[t]);
-    m.surfh[e] = sh;
-    m.head[e] = sh + m.zmax[e];
-  }
+  if (t < qs_n) prep_root(m, qs_i[t], qs_x[t]);
   if (t < qd_n) m.effk[qd_i[t]] = div_any(qd_num[t], qd_den[t]);
 }
 
 // ---------------------------------------------------------------------------
 // k_elem_grad
 // ---------------------------------------------------------------------------
+// What the gradient reads besides the elements' heads: the element whose head
+// each side takes (its own at a no-flow boundary), or -1 and the head itself
+// (a river's water level, a boundary value); and the geometry.
+struct GradIn {
+  int32_t src[3];
+  double h[3], x[3], y[3], inv_x, inv_y;
+};
+__device__ __forceinline__ GradIn grad_load(const DevMesh &m, const double *y, int i) {
+  const int ne = m.ne;
+  GradIn g;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    g.src[j] = m.nb[j * ne + i];
+    g.x[j] = m.nabr_x[j * ne + i];
+    g.y[j] = m.nabr_y[j * ne + i];
+    g.h[j] = 0.0;
+  }
+  g.inv_x = m.inv_den_x[i];
+  g.inv_y = m.inv_den_y[i];
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+    if (g.src[j] < 0) {
+      if (g.src[j] != kBoundary) {
+        const int s = -1 - g.src[j];
+        const double stage = clamp0(y[3 * ne + s]);
+        g.h[j] = cmp::gt_v(stage, m.r_depth[s]) ? m.r_zbed[s] + stage : m.r_zmax[s];
+        g.src[j] = -1;
+      } else if (m.bctype[j * ne + i] == 0) {
+        g.src[j] = i;
+      } else {
+        g.h[j] = m.elem_bc[j * ne + i];
+        g.src[j] = -1;
+      }
+    }
+  return g;
+}
+__device__ __forceinline__ double grad_value(const DevMesh &m, const GradIn &g) {
+  double h[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) h[j] = g.src[j] >= 0 ? m.head[g.src[j]] : g.h[j];
+  const double y0 = g.y[0], y1 = g.y[1], y2 = g.y[2];
+  const double x0 = g.x[0], x1 = g.x[1], x2 = g.x[2];
+  // DhByDl(nabr_y, nabr_x, h) and DhByDl(nabr_x, nabr_y, h)
+  const double dhdx = -1.0 * (y2 * (h[1] - h[0]) + y1 * (h[0] - h[2]) + y0 * (h[2] - h[1])) * g.inv_x;
+  const double dhdy = -1.0 * (x2 * (h[1] - h[0]) + x1 * (h[0] - h[2]) + x0 * (h[2] - h[1])) * g.inv_y;
+  return sqrt_any(dhdx * dhdx + dhdy * dhdy);
+}
+
 __global__ void __launch_bounds__(256) k_elem_grad(DevMesh m, const double *RESTRICT y) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int sy;
   if (i >= m.ne_run || skip_item(m, m.sys_elem, i, &sy)) return;
-  const int ne = m.ne;
-  double h[3];
-  const double hself = m.head[i];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int32_t nb = m.nb[j * ne + i];
-    if (nb >= 0) {
-      h[j] = m.head[nb];
-    } else if (nb != kBoundary) {
-      const int s = -1 - nb;
-      const double stage = clamp0(y[3 * ne + s]);
-      h[j] = cmp::gt_v(stage, m.r_depth[s]) ? m.r_zbed[s] + stage : m.r_zmax[s];
-    } else {
-      h[j] = (m.bctype[j * ne + i] == 0) ? hself : m.elem_bc[j * ne + i];
-    }
-  }
-  const double y0 = m.nabr_y[i], y1 = m.nabr_y[ne + i], y2 = m.nabr_y[2 * ne + i];
-  const double x0 = m.nabr_x[i], x1 = m.nabr_x[ne + i], x2 = m.nabr_x[2 * ne + i];
-  // DhByDl(nabr_y, nabr_x, h) and DhByDl(nabr_x, nabr_y, h)
-  const double dhdx = -1.0 * (y2 * (h[1] - h[0]) + y1 * (h[0] - h[2]) + y0 * (h[2] - h[1])) * m.inv_den_x[i];
-  const double dhdy = -1.0 * (x2 * (h[1] - h[0]) + x1 * (h[0] - h[2]) + x0 * (h[2] - h[1])) * m.inv_den_y[i];
-  m.gradmag[i] = sqrt_any(dhdx * dhdx + dhdy * dhdy);
+  m.gradmag[i] = grad_value(m, grad_load(m, y, i));
 }
 
 // ---------------------------------------------------------------------------
@@ -298,6 +363,39 @@ __global__ void __launch_bounds__(256) k_elem_grad(DevMesh m, const double *REST
 // ---------------------------------------------------------------------------
 constexpr int kEdgeBlock = 256;
 
+// The Darcy flux of edge e (owner i, neighbour k), stored, and the Manning
+// flux's depth and head difference; false (and a zero flux stored) when the
+// upwind element holds no water above the depression storage.
+__device__ __forceinline__ bool edge_item(const DevMesh &m, const double *y, int e, int i, int k, double &avg_h,
+                                          double &diff_h) {
+  const int ne = m.ne;
+  // Darcy flux between the two groundwater columns,
+  // avg_ksat grad_h avg_h edge = (effk_i + effk_k) diff_h avg_h edge/(2 dist)
+  const double gw_i = clamp0(y[2 * ne + i]), gw_k = clamp0(y[2 * ne + k]);
+  diff_h = (gw_i + m.zmin[i]) - (gw_k + m.zmin[k]);
+  avg_h = avg_h_sub(diff_h, gw_i, gw_k);
+  m.eflux_sub[e] = (m.effk[i] + m.effk[k]) * diff_h * avg_h * m.e_subk[e];
+  // Manning overland flux, crossa h^p grad_h / (sqrt(avg_sf) avg_rough) =
+  // avg_h h^p diff_h / sqrt(avg_sf) edge/(dist avg_rough)
+  const double s_i = m.surfh[i], s_k = m.surfh[k];
+  diff_h = m.surf_mode == kKinematic ? m.zmax[i] - m.zmax[k] : m.head[i] - m.head[k];
+  avg_h = avg_h_surf(diff_h, s_i, s_k);
+  // avg_h == 0 gives crossa == 0: the flux is zero
+  const bool wet = cmp::gt0(avg_h);
+  if (!wet) m.eflux_ovl[e] = 0.0;
+  return wet;
+}
+// the friction slope of edge e
+__device__ __forceinline__ double edge_slope(const DevMesh &m, int e, int i, int k, double diff_h) {
+  if (m.surf_mode == kKinematic) {
+    const double grad_h = diff_h * m.e_invdist[e];
+    return cmp::gt0(grad_h) ? grad_h : kGradMin;
+  }
+  const double avg_sf = 0.5 * (m.gradmag[i] + m.gradmag[k]);
+  return cmp::gt_c(avg_sf, kGradMin) ? avg_sf : kGradMin;
+}
+__device__ __forceinline__ double edge_hp(double h) { return h * pow_manning(h, kManningSurf); }
+
 __global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RESTRICT y) {
   __shared__ int q_e[kEdgeBlock];
   __shared__ double q_h[kEdgeBlock], q_d[kEdgeBlock], q_sf[kEdgeBlock];
@@ -309,31 +407,9 @@ __global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RE
   bool wet = false;
   double avg_h = 0.0, diff_h = 0.0, avg_sf = 0.0;
   if (e < m.nedge_run && !skip_item(m, m.sys_edge, e, &sy)) {
-    const int ne = m.ne;
     const int i = m.e_i[e], k = m.e_k[e];
-    // Darcy flux between the two groundwater columns,
-    // avg_ksat grad_h avg_h edge = (effk_i + effk_k) diff_h avg_h edge/(2 dist)
-    const double gw_i = clamp0(y[2 * ne + i]), gw_k = clamp0(y[2 * ne + k]);
-    diff_h = (gw_i + m.zmin[i]) - (gw_k + m.zmin[k]);
-    avg_h = avg_h_sub(diff_h, gw_i, gw_k);
-    m.eflux_sub[e] = (m.effk[i] + m.effk[k]) * diff_h * avg_h * m.e_subk[e];
-    // Manning overland flux, crossa h^p grad_h / (sqrt(avg_sf) avg_rough) =
-    // avg_h h^p diff_h / sqrt(avg_sf) edge/(dist avg_rough)
-    const double s_i = m.surfh[i], s_k = m.surfh[k];
-    if (m.surf_mode == kKinematic) {
-      diff_h = m.zmax[i] - m.zmax[k];
-      avg_h = avg_h_surf(diff_h, s_i, s_k);
-      const double grad_h = diff_h * m.e_invdist[e];
-      avg_sf = cmp::gt0(grad_h) ? grad_h : kGradMin;
-    } else {
-      diff_h = m.head[i] - m.head[k];
-      avg_h = avg_h_surf(diff_h, s_i, s_k);
-      avg_sf = 0.5 * (m.gradmag[i] + m.gradmag[k]);
-      avg_sf = cmp::gt_c(avg_sf, kGradMin) ? avg_sf : kGradMin;
-    }
-    // avg_h == 0 gives crossa == 0: the flux is zero
-    wet = cmp::gt0(avg_h);
-    if (!wet) m.eflux_ovl[e] = 0.0;
+    wet = edge_item(m, y, e, i, k, avg_h, diff_h);
+    avg_sf = edge_slope(m, e, i, k, diff_h);
   }
   const int slot = queue_slot(&q_n, wet);
   if (wet) {
@@ -346,9 +422,7 @@ __global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RE
   const int t = threadIdx.x;
   if (t < q_n) {
     const int qe = q_e[t];
-    const double h = q_h[t];
-    m.eflux_ovl[qe] = h * pow_manning(h, kManningSurf) * q_d[t] * rsqrt(q_sf[t]) *
-                      m.e_ovlk[qe];
+    m.eflux_ovl[qe] = edge_hp(q_h[t]) * q_d[t] * rsqrt(q_sf[t]) * m.e_ovlk[qe];
   }
 }
 
@@ -380,6 +454,354 @@ __device__ __forceinline__ int elem_class(const DevMesh &m, const double *RESTRI
   const int ponded = cmp::gt_c(m.surfh[i], kDeprStg) ? 1 : 0;
   if (cmp::gt_v(gw, m.d_dinf[i])) return 4 + ponded;
   return 2 * ponded + (cmp::lt_v(gw, m.d_dmac[i]) ? 1 : 0);
+}
+
+// One element's rows, in three parts by what they wait for: the state alone
+// (column_state), k_elem_prep's surface water (column_surface), the lateral
+// fluxes (column_rows).  k_elem_main runs them in a row; k_rhs_fused runs the
+// first two while other blocks work on the lateral fluxes.
+struct Column {
+  double gw, unsat, depth, rechg;                 // rechg: unless in_dinf, then infil's
+  double satn_i, satk_i, psi_i, sq_i;             // Infil's saturation, KrFunc, Psi, its root
+  double surfh, dh_by_dz;
+  double kinf_crack;                              // EffKinf with the cracks partly filled (kCrack)
+  double edir_surf, edir_unsat, edir_gw, ett_unsat, ett_gw;
+  bool in_dinf, full, noah;                       // water table within dinf; no room left; Flux-PIHM
+};
+
+__device__ __forceinline__ void column_state(const DevMesh &m, const double *y, int i, int sy, Column &c) {
+  const int ne = m.ne;
+  const double gw = clamp0(y[2 * ne + i]);
+  const double unsat = clamp0(y[ne + i]);
+  // The saturation's powers first: they are the register-hungry part, and
+  // nothing else of the element is live while they run (with the edge fluxes
+  // and the column's parameters loaded before them, 64 registers spilled
+  // 330 bytes a thread).
+  const double depth = m.depth[i];
+  const bool gw_in_dinf = cmp::gt_v(gw, m.d_dinf[i]);
+  c.noah = m.noah && (!m.sys_noah || m.sys_noah[sy]);
+  c.gw = gw;
+  c.unsat = unsat;
+  c.depth = depth;
+  c.in_dinf = gw_in_dinf;
+  c.full = cmp::gt_v(unsat + gw, depth);
+  // KrFunc(beta, 1) == 1 exactly: pow(1 - pow(1, m), e) == pow(0, e) == 0
+  double satn = 1.0, satkfunc = 1.0, psi_u = 0.0, sq = 1.0;
+  c.rechg = 0.0;
+  if (!gw_in_dinf) {
+    const double deficit = depth - gw;
+    satn = div_any(unsat, deficit);
+    satn = cmp::gt_c(satn, 1.0) ? 1.0 : satn;
+    satn = cmp::lt_c(satn, kSatMin) ? kSatMin : satn;
+    kr_psi(satn, m.vg_m[i], m.vg_e[i], m.vg_ib[i], m.alpha[i], satkfunc, psi_u, sq);
+    // Recharge, src/vert_flow.c:132-170: the denominators add up to depth
+    // ((deficit + gw) and the AvgKv weights d1 + d2 + d3, to an ulp);
+    // multiply by 1/depth instead
+    const double inv_depth = m.inv_depth[i], ksatv = m.ksatv[i], dmac = m.dmac[i];
+    const double dh_by_dz = (0.5 * deficit + psi_u) * (2.0 * inv_depth);
+    // AvgKv, src/vert_flow.c:172-209, arithmetic mean (_ARITH_ is defined at
+    // src/include/pihm_func.h:4)
+    double k1, k2, k3, d1, d2, d3;
+    if (cmp::gt_v(deficit, dmac)) {
+      k1 = satkfunc * ksatv;
+      d1 = dmac;
+      k2 = satkfunc * ksatv;
+      d2 = deficit - dmac;
+      k3 = ksatv;
+      d3 = gw;
+    } else {
+      k1 = satkfunc * ksatv;
+      d1 = deficit;
+      k2 = m.kv2_mac[i];
+      d2 = dmac - deficit;
+      k3 = ksatv;
+      d3 = gw - (dmac - deficit);
+    }
+    const double kavg = (k1 * d1 + k2 * d2 + k3 * d3) * inv_depth;
+    double rechg = kavg * dh_by_dz;
+    rechg = (cmp::gt0(rechg) && cmp::le0(unsat)) ? 0.0 : rechg;
+    rechg = (cmp::lt0(rechg) && cmp::le0(gw)) ? 0.0 : rechg;
+    c.rechg = rechg;
+  }
+  // Infil's saturation: the same one, except in Flux-PIHM, where it is
+  // Noah's top-layer moisture (src/vert_flow.c:94-98) and Recharge keeps
+  // the column's
+  c.satn_i = satn;
+  c.satk_i = satkfunc;
+  c.psi_i = psi_u;
+  c.sq_i = sq;
+  if (c.noah && !gw_in_dinf) {
+    double s = m.noah_satn[i];
+    s = cmp::gt_c(s, 1.0) ? 1.0 : s;
+    s = cmp::lt_c(s, kSatMin) ? kSatMin : s;
+    c.satn_i = s;
+    kr_psi(s, m.vg_m[i], m.vg_e[i], m.vg_ib[i], m.alpha[i], c.satk_i, c.psi_i, c.sq_i);
+  }
+}
+
+// EffKinf's conductivity where the cracks carry part of their flow
+// (src/vert_flow.c:211-270).  KrFunc(2, satn): pow(satn, 2) and pow(., 0.5)
+// are a product and sqrt; the root of the saturation is kr_psi's (1 where it
+// is 1).  The roundings are spelt out: every kernel that inlines this
+// rounds alike.
+__device__ __forceinline__ double crack_kinf(const Column &c, double kinf_mat, double kmac_a) {
+  const double t2 = 1.0 - sqrt_any(fma(-c.satn_i, c.satn_i, 1.0));
+  return fma(kmac_a, __dmul_rn(__dmul_rn(c.sq_i, t2), t2), __dmul_rn(kinf_mat, c.satk_i));
+}
+
+__device__ __forceinline__ void column_surface(const DevMesh &m, int i, Column &c) {
+  const double surfh = m.surfh[i];
+  c.surfh = surfh;
+  // Infil's head gradient, src/vert_flow.c:33-130
+  c.dh_by_dz = 0.0;
+  if (!c.full) {
+    const double zmax = m.zmax[i];
+    const double dinf = m.dinf[i];
+    // the head below the infiltration front: the water table when it lies
+    // within dinf of the surface, else the unsaturated zone's; both
+    // reference branches divide (surfh + zmax - head) by the same
+    // denominator, so one division serves a warp whose lanes take both
+    double h_u = c.gw + m.zmin[i];
+    if (!c.in_dinf) {
+      const double psi_c = cmp::gt_nc(c.psi_i, kPsiMin) ? c.psi_i : kPsiMin;
+      h_u = psi_c + zmax - 0.5 * dinf;
+    }
+    const double dh_by_dz = div_any(surfh + zmax - h_u, 0.5 * (surfh + dinf));
+    c.dh_by_dz = (cmp::le0(surfh) && cmp::gt0(dh_by_dz)) ? 0.0 : dh_by_dz;
+  }
+  // EtExtract, src/hydrol.c:33-97
+  const double edir = m.edir[i], ett = m.ett[i];
+  c.edir_surf = c.edir_unsat = c.edir_gw = c.ett_unsat = c.ett_gw = 0.0;
+  if (c.noah) {
+    // Flux-PIHM (src/hydrol.c:43-55,79-83): no ponded-water source, and the
+    // transpiration split by GwTransp (noah/lsm_func.c:163-185) over the
+    // Noah layers from the water table down to the root depth
+    if (c.in_dinf) c.edir_gw = edir;
+    else c.edir_unsat = edir;
+    double gwet = 0.0;
+    if (cmp::gt0(ett) && m.noah_wtin[i]) {
+      gwet = div_any(m.noah_etgw[i], ett);
+      gwet = cmp::gt_c(gwet, 1.0) ? 1.0 : gwet;
+      gwet = cmp::lt0(gwet) ? 0.0 : gwet;
+    }
+    c.ett_unsat = (1.0 - gwet) * ett;
+    c.ett_gw = gwet * ett;
+  } else {
+    if (cmp::ge_c(surfh, kDeprStg)) c.edir_surf = edir;
+    else if (c.in_dinf) c.edir_gw = edir;
+    else c.edir_unsat = edir;
+    if (cmp::gt_v(c.gw, m.d_rzd[i])) c.ett_gw = ett;
+    else c.ett_unsat = ett;
+  }
+}
+
+// The element's parameters that the rows read, and where its lateral fluxes
+// are.  riv[j]: the river segment of side j, or -1; right[j]: its right bank.
+// ovl[j]: on river edges the previous evaluation's flux, which Infil sees.
+struct RowsIn {
+  int32_t code[3], riv[3];
+  bool right[3];
+  double ovl[3];
+  double inv_area, inv_por, pcpdrp, ws0, kinf_mat, kmac_a, areafh, kinfv;
+};
+__device__ __forceinline__ void rows_load(const DevMesh &m, int i, RowsIn &r) {
+  const int ne = m.ne;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    r.code[j] = m.emap[j * ne + i];
+    r.riv[j] = -1;
+    r.right[j] = false;
+    r.ovl[j] = 0.0;
+  }
+  r.inv_area = m.inv_area[i];
+  r.inv_por = m.inv_por[i];
+  r.pcpdrp = m.pcpdrp[i];
+  r.ws0 = m.ws0_surf[i];
+  r.kinf_mat = m.kinf_mat[i];
+  r.kmac_a = m.kmac_a[i];
+  r.areafh = m.areafh[i];
+  r.kinfv = m.kinfv[i];
+  if (r.code[0] == 0 || r.code[1] == 0 || r.code[2] == 0) {
+    int32_t nb[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) nb[j] = m.nb[j * ne + i];
+#pragma unroll
+    for (int j = 0; j < 3; j++) r.riv[j] = (r.code[j] == 0 && nb[j] < 0 && nb[j] != kBoundary) ? -1 - nb[j] : -1;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (r.riv[j] >= 0) r.right[j] = m.left[r.riv[j]] != i;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (r.riv[j] >= 0) r.ovl[j] = -m.carry_ovl[(r.right[j] ? m.nr : 0) + r.riv[j]];
+  }
+}
+
+// kBanks: this evaluation's river fluxes are done, so an element with river
+// edges finishes its rows here; otherwise it hands its partial sums to
+// k_bank_rows.
+template <bool kBanks>
+__device__ __forceinline__ void column_rows(const DevMesh &m, double *ydot, int i, int sy, const Column &c,
+                                            const RowsIn &r) {
+  const int ne = m.ne;
+  const double surfh = c.surfh, inv_area = r.inv_area, pcpdrp = r.pcpdrp;
+  // edge fluxes, with the sign seen from this element (a negative code: the
+  // flux was computed from the neighbour's side); 0 on domain boundaries
+  // (BoundFluxElem)
+  double ovl[3], sub[3], f[3][3];
+  bool riv[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const int32_t code = r.code[j];
+    riv[j] = r.riv[j] >= 0;
+    ovl[j] = r.ovl[j];
+    sub[j] = 0.0;
+    if (code != 0) ovl[j] = cmp::neg_if(m.eflux_ovl[(code > 0 ? code : -code) - 1], code < 0);
+    // (kBanks: every load of this side now, so that they are in flight together)
+    if (kBanks && code != 0) sub[j] = m.eflux_sub[(code > 0 ? code : -code) - 1];
+  }
+  if (kBanks && (riv[0] || riv[1] || riv[2])) {
+    const double *F = m.rivflow;
+    const int nr = m.nr;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (riv[j]) {
+        f[j][0] = F[(r.right[j] ? RIGHT_SURF2CHANL : LEFT_SURF2CHANL) * nr + r.riv[j]];
+        f[j][1] = F[(r.right[j] ? RIGHT_AQUIF2CHANL : LEFT_AQUIF2CHANL) * nr + r.riv[j]];
+        f[j][2] = F[(r.right[j] ? RIGHT_AQUIF2AQUIF : LEFT_AQUIF2AQUIF) * nr + r.riv[j]];
+      }
+  }
+  const double edir_surf = c.edir_surf, edir_unsat = c.edir_unsat, edir_gw = c.edir_gw;
+  const double ett_unsat = c.ett_unsat, ett_gw = c.ett_gw;
+
+  // Infil, src/vert_flow.c:33-130
+  double infil;
+  if (c.full) {
+    infil = 0.0;
+  } else {
+    const double dh_by_dz = c.dh_by_dz;
+    double applrate = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; j++) applrate += -ovl[j] * inv_area;
+    applrate = cmp::gt0(applrate) ? applrate : 0.0;
+    applrate += pcpdrp;
+    double wetfrac = surfh * (1.0 / kDeprStg);
+    wetfrac = cmp::gt0(wetfrac) ? wetfrac : 0.0;
+    wetfrac = cmp::lt_c(wetfrac, 1.0) ? wetfrac : 1.0;
+    // EffKinf, src/vert_flow.c:211-270 (its roundings spelt out, as in
+    // crack_kinf)
+    const double mat = __dmul_rn(r.kinf_mat, c.satk_i);
+    const double both = __dadd_rn(mat, r.kmac_a);
+    double kinf;
+    if (cmp::eq0(r.areafh)) {
+      kinf = r.kinfv * c.satk_i;
+    } else if (cmp::gt_c(surfh, kDeprStg)) {
+      kinf = fma(r.kinf_mat, c.satk_i, r.kmac_a);
+    } else if (cmp::le_v(applrate, dh_by_dz * r.kinfv * c.satk_i)) {
+      kinf = r.kinfv * c.satk_i;
+    } else if (cmp::lt_v(applrate, dh_by_dz * both)) {
+      kinf = kBanks ? c.kinf_crack : crack_kinf(c, r.kinf_mat, r.kmac_a);
+    } else {
+      kinf = both;
+    }
+    infil = kinf * dh_by_dz;
+    if (!c.in_dinf) infil = cmp::gt0(infil) ? infil : 0.0;
+    const double ws0 = r.ws0;
+    const double inv_dt = m.sys_inv_dt ? m.sys_inv_dt[sy] : m.inv_dt;
+    const double infil_max = applrate + (cmp::gt0(ws0) ? ws0 * inv_dt : 0.0);
+    infil = cmp::gt_v(infil, infil_max) ? infil_max : infil;
+    infil *= wetfrac;
+  }
+  if (c.noah) infil *= m.noah_fcr[i];  // frozen top soil, src/vert_flow.c:16-19
+  const double rechg = c.in_dinf ? infil : c.rechg;
+
+  // groundwater fluxes
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const int32_t code = r.code[j];
+    if (code != 0) {
+      sub[j] = cmp::neg_if(kBanks ? sub[j] : m.eflux_sub[(code > 0 ? code : -code) - 1], code < 0);
+    } else if (!riv[j]) {
+      // BoundFluxElem, src/lat_flow.c:340-382
+      const int bct = m.bctype[j * ne + i];
+      if (bct > 0) {
+        const double bc = m.elem_bc[j * ne + i], zmin = m.zmin[i];
+        const double diff_h = c.gw + zmin - bc;
+        const double avg_h = avg_h_sub(diff_h, c.gw, bc - zmin);
+        const double grad_h = div_any(diff_h, m.nabrdist[j * ne + i]);
+        sub[j] = m.effk[i] * grad_h * avg_h * m.edge[j * ne + i];
+      } else if (bct < 0) {
+        sub[j] = -m.elem_bc[j * ne + i];
+      }
+    }
+  }
+
+  if (m.diag) {
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      if (!riv[j]) {
+        m.d_ovl[j * ne + i] = ovl[j];
+        m.d_sub[j * ne + i] = sub[j];
+      }
+    }
+    m.d_infil[i] = infil;
+    m.d_rechg[i] = rechg;
+    m.d_et[i] = edir_surf;
+    m.d_et[ne + i] = edir_unsat;
+    m.d_et[2 * ne + i] = edir_gw;
+    m.d_et[3 * ne + i] = ett_unsat;
+    m.d_et[4 * ne + i] = ett_gw;
+  }
+
+  // river edges: this evaluation's fluxes, and the overland one kept for the
+  // next evaluation's Infil.  A bank's slot of carry_ovl is read in rows_load
+  // and written here by its own element's thread alone.
+  if (kBanks && (riv[0] || riv[1] || riv[2])) {
+    const int nr = m.nr;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (riv[j]) {
+        ovl[j] = -f[j][0];
+        sub[j] = -(f[j][1] + f[j][2]);
+        m.carry_ovl[(r.right[j] ? nr : 0) + r.riv[j]] = f[j][0];
+        if (m.diag) {
+          m.d_ovl[j * ne + i] = ovl[j];
+          m.d_sub[j * ne + i] = sub[j];
+        }
+      }
+  }
+
+  // element rows of ydot, src/ode.c:111-209
+  const double inv_por = r.inv_por;
+  const double base_surf = pcpdrp - infil - edir_surf;
+  const double base_gw = rechg - edir_gw - ett_gw;
+  const double du = (infil - rechg - edir_unsat - ett_unsat) * inv_por;
+  ydot[ne + i] = du;
+  unsigned int bad = cmp::isnan_(du);
+  if (!kBanks && (riv[0] || riv[1] || riv[2])) {
+    const int b = m.bank_slot[i];
+    const int nbk = m.nbank;
+    double *bp = m.bank_part;
+    bp[b] = base_surf;
+    bp[nbk + b] = base_gw;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      bp[(2 + j) * nbk + b] = ovl[j];
+      bp[(5 + j) * nbk + b] = sub[j];
+    }
+    if (bad) report_err(m, sy);
+    return;
+  }
+  double ds = base_surf, dg = base_gw;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    ds -= ovl[j] * inv_area;
+    dg -= sub[j] * inv_area;
+  }
+  dg *= inv_por;
+  ydot[i] = ds;
+  ydot[2 * ne + i] = dg;
+  bad |= cmp::isnan_(ds) | cmp::isnan_(dg);
+  if (bad) report_err(m, sy);
 }
 
 template <int BLOCK, int MINB>
@@ -434,240 +856,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_elem_main(DevMesh m, const doub
   const int i = blockIdx.x * BLOCK + s_order[threadIdx.x];
   int sy;
   if (i >= m.ne_run || skip_item(m, m.sys_elem, i, &sy)) return;
-  const int ne = m.ne;
-  const double gw = clamp0(y[2 * ne + i]);
-  const double unsat = clamp0(y[ne + i]);
-  const double surfh = m.surfh[i];
-  const double zmin = m.zmin[i];
-  const double inv_area = m.inv_area[i];
-  const double gwhead = gw + zmin;
-
-  double ovl[3], sub[3];
-  bool riv[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int32_t code = m.emap[j * ne + i];
-    riv[j] = false;
-    if (code != 0) {
-      // the edge's flux with the sign seen from this element (a negative
-      // code: the flux was computed from the neighbour's side)
-      const int e = (code > 0 ? code : -code) - 1;
-      ovl[j] = cmp::neg_if(m.eflux_ovl[e], code < 0);
-      sub[j] = cmp::neg_if(m.eflux_sub[e], code < 0);
-    } else {
-      const int32_t nb = m.nb[j * ne + i];
-      if (nb != kBoundary) {
-        // river edge: Infil sees the previous evaluation's value
-        const int s = -1 - nb;
-        ovl[j] = -m.carry_ovl[(m.left[s] == i ? 0 : 1) * m.nr + s];
-        sub[j] = 0.0;
-        riv[j] = true;
-      } else {
-        // BoundFluxElem, src/lat_flow.c:340-382
-        const int bct = m.bctype[j * ne + i];
-        ovl[j] = 0.0;
-        if (bct == 0) {
-          sub[j] = 0.0;
-        } else if (bct > 0) {
-          const double bc = m.elem_bc[j * ne + i];
-          const double diff_h = gwhead - bc;
-          const double avg_h = avg_h_sub(diff_h, gw, bc - zmin);
-          const double grad_h = diff_h / m.nabrdist[j * ne + i];
-          sub[j] = m.effk[i] * grad_h * avg_h * m.edge[j * ne + i];
-        } else {
-          sub[j] = -m.elem_bc[j * ne + i];
-        }
-      }
-    }
-  }
-
-  // EtExtract, src/hydrol.c:33-97
-  const double depth = m.depth[i];
-  const double d_dinf = m.d_dinf[i];
-  const double edir = m.edir[i], ett = m.ett[i];
-  double edir_surf = 0.0, edir_unsat = 0.0, edir_gw = 0.0, ett_unsat = 0.0, ett_gw = 0.0;
-  const bool gw_in_dinf = cmp::gt_v(gw, d_dinf);
-  const bool noah = m.noah && (!m.sys_noah || m.sys_noah[sy]);
-  if (noah) {
-    // Flux-PIHM (src/hydrol.c:43-55,79-83): no ponded-water source, and the
-    // transpiration split by GwTransp (noah/lsm_func.c:163-185) over the
-    // Noah layers from the water table down to the root depth
-    if (gw_in_dinf) edir_gw = edir;
-    else edir_unsat = edir;
-    double gwet = 0.0;
-    if (cmp::gt0(ett) && m.noah_wtin[i]) {
-      gwet = div_any(m.noah_etgw[i], ett);
-      gwet = cmp::gt_c(gwet, 1.0) ? 1.0 : gwet;
-      gwet = cmp::lt0(gwet) ? 0.0 : gwet;
-    }
-    ett_unsat = (1.0 - gwet) * ett;
-    ett_gw = gwet * ett;
-  } else {
-    if (cmp::ge_c(surfh, kDeprStg)) edir_surf = edir;
-    else if (gw_in_dinf) edir_gw = edir;
-    else edir_unsat = edir;
-    if (cmp::gt_v(gw, m.d_rzd[i])) ett_gw = ett;
-    else ett_unsat = ett;
-  }
-
-  // Infil, src/vert_flow.c:33-130, and Recharge, :132-170, sharing KrFunc and
-  // Psi of the same saturation
-  const double kinf_mat = m.kinf_mat[i], kmac_a = m.kmac_a[i], areafh = m.areafh[i];
-  const double kinfv = m.kinfv[i], ksatv = m.ksatv[i], dmac = m.dmac[i];
-  const double pcpdrp = m.pcpdrp[i];
-  const double zmax = m.zmax[i];
-  const double dinf = m.dinf[i];
-  double satn = 1.0, satkfunc = 1.0, psi_u = 0.0, sq = 1.0;
-  if (!gw_in_dinf) {
-    const double deficit = depth - gw;
-    satn = div_any(unsat, deficit);
-    satn = cmp::gt_c(satn, 1.0) ? 1.0 : satn;
-    satn = cmp::lt_c(satn, kSatMin) ? kSatMin : satn;
-    kr_psi(satn, m.vg_m[i], m.vg_e[i], m.vg_ib[i], m.alpha[i], satkfunc, psi_u, sq);
-  }
-  // Infil's saturation: the same one, except in Flux-PIHM, where it is
-  // Noah's top-layer moisture (src/vert_flow.c:94-98) and Recharge keeps
-  // the column's
-  double satn_i = satn, satkfunc_i = satkfunc, psi_i = psi_u, sq_i = sq;
-  if (noah && !gw_in_dinf) {
-    double s = m.noah_satn[i];
-    s = cmp::gt_c(s, 1.0) ? 1.0 : s;
-    s = cmp::lt_c(s, kSatMin) ? kSatMin : s;
-    satn_i = s;
-    kr_psi(s, m.vg_m[i], m.vg_e[i], m.vg_ib[i], m.alpha[i], satkfunc_i, psi_i, sq_i);
-  }
-  // KrFunc(beta, 1) == 1 exactly: pow(1 - pow(1, m), e) == pow(0, e) == 0
-  double infil;
-  if (cmp::gt_v(unsat + gw, depth)) {
-    infil = 0.0;
-  } else {
-    double applrate = 0.0;
-#pragma unroll
-    for (int j = 0; j < 3; j++) applrate += -ovl[j] * inv_area;
-    applrate = cmp::gt0(applrate) ? applrate : 0.0;
-    applrate += pcpdrp;
-    double wetfrac = surfh * (1.0 / kDeprStg);
-    wetfrac = cmp::gt0(wetfrac) ? wetfrac : 0.0;
-    wetfrac = cmp::lt_c(wetfrac, 1.0) ? wetfrac : 1.0;
-    // the head below the infiltration front: the water table when it lies
-    // within dinf of the surface, else the unsaturated zone's; both
-    // reference branches divide (surfh + zmax - head) by the same
-    // denominator, so one division serves a warp whose lanes take both
-    double h_u = gwhead;
-    double esatn = 1.0;
-    if (!gw_in_dinf) {
-      const double psi_c = cmp::gt_nc(psi_i, kPsiMin) ? psi_i : kPsiMin;
-      h_u = psi_c + zmax - 0.5 * dinf;
-      esatn = satn_i;
-    }
-    double dh_by_dz = div_any(surfh + zmax - h_u, 0.5 * (surfh + dinf));
-    dh_by_dz = (cmp::le0(surfh) && cmp::gt0(dh_by_dz)) ? 0.0 : dh_by_dz;
-    // EffKinf, src/vert_flow.c:211-270
-    double kinf;
-    if (cmp::eq0(areafh)) {
-      kinf = kinfv * satkfunc_i;
-    } else if (cmp::gt_c(surfh, kDeprStg)) {
-      kinf = kinf_mat * satkfunc_i + kmac_a;
-    } else if (cmp::le_v(applrate, dh_by_dz * kinfv * satkfunc_i)) {
-      kinf = kinfv * satkfunc_i;
-    } else if (cmp::lt_v(applrate, dh_by_dz * (kmac_a + kinf_mat * satkfunc_i))) {
-      // KrFunc(2, satn): pow(satn, 2) and pow(., 0.5) are a product and
-      // sqrt; sqrt(esatn) is kr_psi's (1 when esatn is 1)
-      const double t2 = 1.0 - sqrt_any(1.0 - esatn * esatn);
-      kinf = kinf_mat * satkfunc_i + kmac_a * (sq_i * t2 * t2);
-    } else {
-      kinf = kinf_mat * satkfunc_i + kmac_a;
-    }
-    infil = kinf * dh_by_dz;
-    if (!gw_in_dinf) infil = cmp::gt0(infil) ? infil : 0.0;
-    const double ws0 = m.ws0_surf[i];
-    const double inv_dt = m.sys_inv_dt ? m.sys_inv_dt[sy] : m.inv_dt;
-    const double infil_max = applrate + (cmp::gt0(ws0) ? ws0 * inv_dt : 0.0);
-    infil = cmp::gt_v(infil, infil_max) ? infil_max : infil;
-    infil *= wetfrac;
-  }
-  if (noah) infil *= m.noah_fcr[i];  // frozen top soil, src/vert_flow.c:16-19
-  double rechg;
-  if (gw_in_dinf) {
-    rechg = infil;
-  } else {
-    const double deficit = depth - gw;
-    // the denominators of Recharge add up to depth: (deficit + gw) and the
-    // AvgKv weights d1 + d2 + d3 (to an ulp); multiply by 1/depth instead
-    const double inv_depth = m.inv_depth[i];
-    const double dh_by_dz = (0.5 * deficit + psi_u) * (2.0 * inv_depth);
-    // AvgKv, src/vert_flow.c:172-209, arithmetic mean (_ARITH_ is defined at
-    // src/include/pihm_func.h:4)
-    double k1, k2, k3, d1, d2, d3;
-    if (cmp::gt_v(deficit, dmac)) {
-      k1 = satkfunc * ksatv;
-      d1 = dmac;
-      k2 = satkfunc * ksatv;
-      d2 = deficit - dmac;
-      k3 = ksatv;
-      d3 = gw;
-    } else {
-      k1 = satkfunc * ksatv;
-      d1 = deficit;
-      k2 = m.kv2_mac[i];
-      d2 = dmac - deficit;
-      k3 = ksatv;
-      d3 = gw - (dmac - deficit);
-    }
-    const double kavg = (k1 * d1 + k2 * d2 + k3 * d3) * inv_depth;
-    rechg = kavg * dh_by_dz;
-    rechg = (cmp::gt0(rechg) && cmp::le0(unsat)) ? 0.0 : rechg;
-    rechg = (cmp::lt0(rechg) && cmp::le0(gw)) ? 0.0 : rechg;
-  }
-
-  if (m.diag) {
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      if (!riv[j]) {
-        m.d_ovl[j * ne + i] = ovl[j];
-        m.d_sub[j * ne + i] = sub[j];
-      }
-    }
-    m.d_infil[i] = infil;
-    m.d_rechg[i] = rechg;
-    m.d_et[i] = edir_surf;
-    m.d_et[ne + i] = edir_unsat;
-    m.d_et[2 * ne + i] = edir_gw;
-    m.d_et[3 * ne + i] = ett_unsat;
-    m.d_et[4 * ne + i] = ett_gw;
-  }
-
-  // element rows of ydot, src/ode.c:111-209
-  const double inv_por = m.inv_por[i];
-  const double base_surf = pcpdrp - infil - edir_surf;
-  const double base_gw = rechg - edir_gw - ett_gw;
-  const double du = (infil - rechg - edir_unsat - ett_unsat) * inv_por;
-  ydot[ne + i] = du;
-  unsigned int bad = cmp::isnan_(du);
-  if (riv[0] || riv[1] || riv[2]) {
-    const int b = m.bank_slot[i];
-    const int nbk = m.nbank;
-    double *bp = m.bank_part;
-    bp[b] = base_surf;
-    bp[nbk + b] = base_gw;
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      bp[(2 + j) * nbk + b] = ovl[j];
-      bp[(5 + j) * nbk + b] = sub[j];
-    }
-  } else {
-    double ds = base_surf, dg = base_gw;
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      ds -= ovl[j] * inv_area;
-      dg -= sub[j] * inv_area;
-    }
-    dg *= inv_por;
-    ydot[i] = ds;
-    ydot[2 * ne + i] = dg;
-    bad |= cmp::isnan_(ds) | cmp::isnan_(dg);
-  }
-  if (bad) report_err(m, sy);
+  Column c;
+  column_state(m, y, i, sy, c);
+  column_surface(m, i, c);
+  RowsIn r;
+  rows_load(m, i, r);
+  column_rows<false>(m, ydot, i, sy, c, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -690,10 +884,7 @@ __device__ __forceinline__ double log_of(double x) {
   return log_dd_fast(x, sh, lo) ? sh + lo : log(x);
 }
 
-__global__ void __launch_bounds__(128) k_riv_geom(DevMesh m, const double *RESTRICT y) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int sy;
-  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+__device__ __forceinline__ void geom_item(const DevMesh &m, const double *y, int s) {
   double d = y[3 * m.ne + s];
   d = cmp::gt0(d) ? d : 0.0;
   const double g0 = m.r_geo0[s];
@@ -707,21 +898,29 @@ __global__ void __launch_bounds__(128) k_riv_geom(DevMesh m, const double *RESTR
       area = d * d * g0;
       perim = d * m.r_geo1[s];
       break;
-    case kQuadratic: {
-      const double sd = sqrt(d), w = 1.0 + m.r_geo1[s] * d;
-      area = g0 * d * sd;
-      perim = sqrt(d * w * m.r_geo2[s]) + log_of(m.r_geo4[s] * sd + sqrt(w)) * m.r_geo3[s];
-      break;
-    }
+    case kQuadratic:
     case kCubic: {
-      const double sd = sqrt(d), w = 1.0 + m.r_geo1[s] * d;
-      area = g0 * pow_fast(d, 4.0 / 3.0);
-      perim = 2.0 * (sqrt(d * w) * (1.0 / 3.0) + log_of(m.r_geo2[s] * sd + sqrt(w)) * m.r_geo3[s]);
+      // one path for both shapes, so that a warp with segments of both runs
+      // the roots and the logarithm once
+      const bool cub = m.intrpl_ord[s] == kCubic;
+      const double sd = sqrt_any(d), w = 1.0 + m.r_geo1[s] * d;
+      const double g2 = m.r_geo2[s], dw = d * w;
+      const double root = sqrt_any(cub ? dw : dw * g2);
+      const double lg = log_of((cub ? g2 : m.r_geo4[s]) * sd + sqrt_any(w));
+      area = cub ? g0 * pow_fast(d, 4.0 / 3.0) : g0 * d * sd;
+      perim = cub ? 2.0 * (root * (1.0 / 3.0) + lg * m.r_geo3[s]) : root + lg * m.r_geo3[s];
       break;
     }
   }
   m.r_perim[s] = perim;
   m.r_crossa[s] = area;
+}
+
+__global__ void __launch_bounds__(128) k_riv_geom(DevMesh m, const double *RESTRICT y) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  int sy;
+  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  geom_item(m, y, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -751,17 +950,16 @@ __device__ __forceinline__ double ovl_elem_to_river(double e_zmax, double e_surf
   const double zbank = cmp::gt_v(r.zmax, e_zmax) ? r.zmax : e_zmax;
   const double elem_h = e_zmax + e_surfh;
   const double rivseg_h = r.zbed + r.stage;
-  if (cmp::gt_v(rivseg_h, elem_h)) {
-    if (cmp::gt_v(elem_h, zbank)) return coef * sqrt(rivseg_h - elem_h) * (rivseg_h - zbank);
-    if (cmp::lt_v(zbank, rivseg_h)) return coef * sqrt(rivseg_h - zbank) * (rivseg_h - zbank);
-    return 0.0;
-  }
-  if (cmp::gt_c(e_surfh, kDeprStg)) {
-    if (cmp::gt_v(rivseg_h, zbank)) return -coef * sqrt(elem_h - rivseg_h) * (elem_h - zbank);
-    if (cmp::lt_v(zbank, elem_h)) return -coef * sqrt(elem_h - zbank) * (elem_h - zbank);
-    return 0.0;
-  }
-  return 0.0;
+  // the four cases differ in the head under the root and the head over the
+  // bank: one root and one product serve a warp whose lanes take them all
+  const bool out = cmp::gt_v(rivseg_h, elem_h);
+  if (!out && !cmp::gt_c(e_surfh, kDeprStg)) return 0.0;
+  const double high = out ? rivseg_h : elem_h, low = out ? elem_h : rivseg_h;
+  const bool drowned = cmp::gt_v(low, zbank);  // the lower side stands above the bank too
+  if (!drowned && !cmp::lt_v(zbank, high)) return 0.0;
+  const double over = high - zbank;
+  const double root = sqrt_any(drowned ? high - low : over);
+  return (out ? coef : -coef) * root * over;
 }
 
 // ChanFlowElemToRiver, src/river_flow.c:429-460
@@ -794,41 +992,41 @@ __device__ __forceinline__ double sub_elem_to_river(double e_gw, double e_zmin, 
   return r.length * avg_ksat * grad_h * avg_h;
 }
 
-__global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT y) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int sy;
-  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+// A segment's fluxes in four parts that share no result: the channel flux,
+// the two banks, and the bed's.  One thread per part: a segment's fluxes are a
+// chain of FP64 divisions, roots and a power (18 us for 100 segments or
+// 12,000 with one thread per segment), and the parts run beside each other.
+enum RivPart { PART_CHAN = 0, PART_LEFT, PART_RIGHT, PART_BED, kRivParts };
+
+__device__ __forceinline__ void river_part(const DevMesh &m, const double *y, int s, int part) {
   const int nr = m.nr, ne = m.ne;
+  double *F = m.rivflow;
   const RivState r = load_riv(m, y, s);
-  const int down = m.down[s];
-  double f[NUM_RIVFLX];
-  f[UP_CHANL2CHANL] = 0.0;
-  f[UP_AQUIF2AQUIF] = 0.0;
-  const int L = m.left[s], R = m.right[s];
-  const double effk_l = m.effk[L], effk_r = m.effk[R];
-  if (down > 0) {
-    const int bct = m.bctype_riv[s];
-    if (bct != 0) {
-      // BoundFluxRiver, src/river_flow.c:392-427
-      double flux = 0.0;
-      const double bc = m.river_bc[s];
-      if (bct > 0) {
-        const double total_h = r.stage + r.zbed;
-        const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
-        const double avg_perim = m.r_perim[s];
-        const double crossa = m.r_crossa[s];
-        const double avg_h = cmp::eq0(avg_perim) ? 0.0 : (crossa / avg_perim);
-        flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-      } else {
-        flux = -bc;
+  if (part == PART_CHAN) {
+    const int down = m.down[s];
+    double up = 0.0, dnf;
+    if (down > 0) {
+      const int bct = m.bctype_riv[s];
+      if (bct != 0) {
+        // BoundFluxRiver, src/river_flow.c:392-427
+        double flux = 0.0;
+        const double bc = m.river_bc[s];
+        if (bct > 0) {
+          const double total_h = r.stage + r.zbed;
+          const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
+          const double avg_perim = m.r_perim[s];
+          const double crossa = m.r_crossa[s];
+          const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
+          flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+        } else {
+          flux = -bc;
+        }
+        up += flux;
       }
-      f[UP_CHANL2CHANL] += flux;
-    }
-    const int d = down - 1;
-    const RivState dn = load_riv(m, y, d);
-    const double inv_dist_down = m.r_inv_dist_down[s];
-    // ChanFlowRiverToRiver, src/river_flow.c:257-300
-    {
+      const int d = down - 1;
+      const RivState dn = load_riv(m, y, d);
+      const double inv_dist_down = m.r_inv_dist_down[s];
+      // ChanFlowRiverToRiver, src/river_flow.c:257-300
       const double total_h = r.stage + r.zbed;
       const double perim = m.r_perim[s];
       const double total_h_down = dn.stage + dn.zbed;
@@ -841,11 +1039,46 @@ __global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT
       const double crossa = m.r_crossa[s];
       const double crossa_down = m.r_crossa[d];
       const double avg_crossa = 0.5 * (crossa + crossa_down);
-      const double avg_h = cmp::eq0(avg_perim) ? 0.0 : (avg_crossa / avg_perim);
-      f[DOWN_CHANL2CHANL] = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
+      const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(avg_crossa, avg_perim);
+      dnf = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
+    } else {
+      // OutletFlux, src/river_flow.c:333-390
+      const double depth = m.r_depth[s];
+      const double bc = m.river_bc[s];
+      if (down == kDirichlet) {
+        const double total_h = r.stage + r.zbed;
+        const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
+        const double avg_perim = m.r_perim[s];
+        const double crossa = m.r_crossa[s];
+        const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
+        dnf = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+      } else if (down == kNeumann) {
+        dnf = -bc;
+      } else if (down == kZeroDpthGrad) {
+        const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
+        const double avg_perim = m.r_perim[s];
+        const double crossa = m.r_crossa[s];
+        dnf = sqrt(grad_h) * crossa *
+              (cmp::gt0(avg_perim) ? pow_manning(crossa / avg_perim, kManningRiv) : 0.0) /
+              r.rough;
+      } else {  // kCritDpth (other values are rejected at load)
+        const double crossa = m.r_crossa[s];
+        dnf = crossa * sqrt(kGrav * r.stage);
+      }
     }
-    // SubFlowRiverToRiver, src/river_flow.c:302-331 (arithmetic mean)
-    {
+    F[UP_CHANL2CHANL * nr + s] = up;
+    F[DOWN_CHANL2CHANL * nr + s] = dnf;
+    return;
+  }
+  const int L = m.left[s], R = m.right[s];
+  const double effk_l = m.effk[L], effk_r = m.effk[R];
+  if (part == PART_BED) {
+    const int down = m.down[s];
+    double aq = 0.0;
+    if (down > 0) {
+      // SubFlowRiverToRiver, src/river_flow.c:302-331 (arithmetic mean)
+      const int d = down - 1;
+      const RivState dn = load_riv(m, y, d);
       const double effk = 0.5 * (effk_l + effk_r);
       const double effk_nabr = 0.5 * (m.effk[m.left[d]] + m.effk[m.right[d]]);
       const double total_h = r.gw + r.zmin;
@@ -853,106 +1086,109 @@ __global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT
       const double avg_wid = (r.width + dn.width) / 2.0;
       const double diff_h = total_h - total_h_down;
       const double avg_h = avg_h_sub(diff_h, r.gw, dn.gw);
-      const double grad_h = diff_h * inv_dist_down;
+      const double grad_h = diff_h * m.r_inv_dist_down[s];
       const double avg_ksat = 0.5 * (effk + effk_nabr);
-      f[DOWN_AQUIF2AQUIF] = avg_ksat * grad_h * avg_h * avg_wid;
+      aq = avg_ksat * grad_h * avg_h * avg_wid;
     }
-  } else {
-    // OutletFlux, src/river_flow.c:333-390
-    const double depth = m.r_depth[s];
-    const double bc = m.river_bc[s];
-    double q = 0.0;
-    if (down == kDirichlet) {
-      const double total_h = r.stage + r.zbed;
-      const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
-      const double avg_perim = m.r_perim[s];
-      const double crossa = m.r_crossa[s];
-      const double avg_h = cmp::eq0(avg_perim) ? 0.0 : (crossa / avg_perim);
-      q = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-    } else if (down == kNeumann) {
-      q = -bc;
-    } else if (down == kZeroDpthGrad) {
-      const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
-      const double avg_perim = m.r_perim[s];
-      const double crossa = m.r_crossa[s];
-      q = sqrt(grad_h) * crossa *
-          (cmp::gt0(avg_perim) ? pow_manning(crossa / avg_perim, kManningRiv) : 0.0) /
-          r.rough;
-    } else {  // kCritDpth (other values are rejected at load)
-      const double crossa = m.r_crossa[s];
-      q = crossa * sqrt(kGrav * r.stage);
-    }
-    f[DOWN_CHANL2CHANL] = q;
-    f[DOWN_AQUIF2AQUIF] = 0.0;
-  }
-  // RiverToElem, src/river_flow.c:113-183
-  const double coef = m.r_ovl_coef[s];
-  const double gw_l = clamp0(y[2 * ne + L]), gw_r = clamp0(y[2 * ne + R]);
-  const double zmin_l = m.zmin[L], zmin_r = m.zmin[R];
-  f[LEFT_SURF2CHANL] = ovl_elem_to_river(m.zmax[L], m.surfh[L], r, coef);
-  f[RIGHT_SURF2CHANL] = ovl_elem_to_river(m.zmax[R], m.surfh[R], r, coef);
-  const double r_ksath = m.r_ksath[s];
-  const double inv_dl = m.r_inv_dist_left[s], inv_dr = m.r_inv_dist_right[s];
-  f[LEFT_AQUIF2CHANL] = chan_elem_to_river(gw_l, zmin_l, effk_l, r, r_ksath, inv_dl);
-  f[RIGHT_AQUIF2CHANL] = chan_elem_to_river(gw_r, zmin_r, effk_r, r, r_ksath, inv_dr);
-  const double effk_avg = 0.5 * (effk_l + effk_r);
-  f[LEFT_AQUIF2AQUIF] = sub_elem_to_river(gw_l, zmin_l, effk_l, r, effk_avg, inv_dl);
-  f[RIGHT_AQUIF2AQUIF] = sub_elem_to_river(gw_r, zmin_r, effk_r, r, effk_avg, inv_dr);
-  // ChanLeak, src/river_flow.c:500-518
-  {
+    F[DOWN_AQUIF2AQUIF * nr + s] = aq;
+    F[UP_AQUIF2AQUIF * nr + s] = 0.0;
+    // ChanLeak, src/river_flow.c:500-518
     double diff_h;
     if (cmp::gt0(r.zbed - (r.gw + r.zmin))) diff_h = r.stage;
     else diff_h = r.stage + r.zbed - (r.gw + r.zmin);
     const double grad_h = diff_h * m.r_inv_bedthick[s];
-    f[CHANL_LKG] = m.r_ksatv[s] * r.width * r.length * grad_h;
+    F[CHANL_LKG * nr + s] = m.r_ksatv[s] * r.width * r.length * grad_h;
+    return;
   }
-#pragma unroll
-  for (int k = 0; k < NUM_RIVFLX; k++) m.rivflow[k * nr + s] = f[k];
+  // RiverToElem, src/river_flow.c:113-183, one bank
+  const bool left = part == PART_LEFT;
+  const int e = left ? L : R;
+  const double effk_e = left ? effk_l : effk_r;
+  const double inv_d = left ? m.r_inv_dist_left[s] : m.r_inv_dist_right[s];
+  const double gw_e = clamp0(y[2 * ne + e]), zmin_e = m.zmin[e];
+  F[(left ? LEFT_SURF2CHANL : RIGHT_SURF2CHANL) * nr + s] =
+      ovl_elem_to_river(m.zmax[e], m.surfh[e], r, m.r_ovl_coef[s]);
+  F[(left ? LEFT_AQUIF2CHANL : RIGHT_AQUIF2CHANL) * nr + s] =
+      chan_elem_to_river(gw_e, zmin_e, effk_e, r, m.r_ksath[s], inv_d);
+  const double effk_avg = 0.5 * (effk_l + effk_r);
+  F[(left ? LEFT_AQUIF2AQUIF : RIGHT_AQUIF2AQUIF) * nr + s] =
+      sub_elem_to_river(gw_e, zmin_e, effk_e, r, effk_avg, inv_d);
+}
+
+// part-major, each part's segments padded to whole warps
+__global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT y) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int pad = (m.nr_run + 31) & ~31;
+  const int part = t / pad, s = t - part * pad;
+  int sy;
+  if (part >= kRivParts || s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  river_part(m, y, s, part);
 }
 
 // ---------------------------------------------------------------------------
-// k_finish
+// k_river_rows: upstream sums and the river rows of ydot
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_finish(DevMesh m, double *RESTRICT ydot) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// the quotients of a row, beside each other
+__device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, int s, int sy) {
   const int nr = m.nr, ne = m.ne;
   const double *F = m.rivflow;
-  int sy;
-  if (t < m.nr_run) {
-    const int s = t;
-    if (skip_item(m, m.sys_riv, s, &sy)) return;
-    double up_c = F[UP_CHANL2CHANL * nr + s];
-    double up_a = 0.0;
-    for (int k = m.up_ptr[s]; k < m.up_end[s]; k++) {
-      const int u = m.up_idx[k];
-      up_c -= F[DOWN_CHANL2CHANL * nr + u];
-      up_a -= F[DOWN_AQUIF2AQUIF * nr + u];
-    }
-    const double area = m.r_area[s];
-    double ds = 0.0;
-    ds -= up_c / area;
+  double f[7];
+  f[0] = F[UP_CHANL2CHANL * nr + s];
 #pragma unroll
-    for (int j = 1; j <= 6; j++) ds -= F[j * nr + s] / area;
-    double dg = -F[LEFT_AQUIF2AQUIF * nr + s] - F[RIGHT_AQUIF2AQUIF * nr + s] -
-                F[DOWN_AQUIF2AQUIF * nr + s] - up_a + F[CHANL_LKG * nr + s];
-    dg /= m.r_porosity[s] * area;
-    ydot[3 * ne + s] = ds;
-    ydot[3 * ne + nr + s] = dg;
-    if (m.diag) {
-      m.rivflow[UP_CHANL2CHANL * nr + s] = up_c;
-      m.rivflow[UP_AQUIF2AQUIF * nr + s] = up_a;
-    }
-    if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
-    // the next evaluation's Infil reads this evaluation's river-edge
-    // overland flux (src/vert_flow.c:61 before src/river_flow.c:159-182)
-    m.carry_ovl[s] = F[LEFT_SURF2CHANL * nr + s];
-    m.carry_ovl[nr + s] = F[RIGHT_SURF2CHANL * nr + s];
-    return;
+  for (int j = 1; j <= 6; j++) f[j] = F[j * nr + s];
+  const double aq_l = F[LEFT_AQUIF2AQUIF * nr + s], aq_r = F[RIGHT_AQUIF2AQUIF * nr + s];
+  const double aq_d = F[DOWN_AQUIF2AQUIF * nr + s];
+  const double area = m.r_area[s], por_area = m.r_porosity[s] * area;
+  double up_c = f[0];
+  double up_a = 0.0;
+  for (int k = m.up_ptr[s]; k < m.up_end[s]; k++) {
+    const int u = m.up_idx[k];
+    up_c -= F[DOWN_CHANL2CHANL * nr + u];
+    up_a -= F[DOWN_AQUIF2AQUIF * nr + u];
   }
-  const int b = t - m.nr_run;
+  f[0] = up_c;
+  double dg = -aq_l - aq_r - aq_d - up_a + f[CHANL_LKG];
+  double q[7], qg;
+  bool ok = im::div_i(dg, por_area, qg);
+#pragma unroll
+  for (int j = 0; j <= 6; j++) ok &= im::div_i(f[j], area, q[j]);
+  if (!ok) {
+    qg = div_any(dg, por_area);
+#pragma unroll
+    for (int j = 0; j <= 6; j++) q[j] = div_any(f[j], area);
+  }
+  dg = qg;
+  double ds = 0.0;
+#pragma unroll
+  for (int j = 0; j <= 6; j++) ds -= q[j];
+  ydot[3 * ne + s] = ds;
+  ydot[3 * ne + nr + s] = dg;
+  if (m.diag) {
+    m.rivflow[UP_CHANL2CHANL * nr + s] = up_c;
+    m.rivflow[UP_AQUIF2AQUIF * nr + s] = up_a;
+  }
+  if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
+}
+
+__global__ void __launch_bounds__(128) k_river_rows(DevMesh m, double *RESTRICT ydot) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  int sy;
+  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  river_rows_item(m, ydot, s, sy);
+}
+
+// ---------------------------------------------------------------------------
+// k_bank_rows: the rows of elements with river edges, from k_elem_main's
+// partial sums and the river kernels' fluxes, and the overland flux kept for
+// the next evaluation's Infil.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_bank_rows(DevMesh m, double *RESTRICT ydot) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  int sy;
   if (b >= m.nbank_run || skip_item(m, m.sys_bank, b, &sy)) return;
+  const int nr = m.nr, ne = m.ne, nbk = m.nbank;
+  const double *F = m.rivflow;
   const int i = m.bank_elem[b];
-  const int nbk = m.nbank;
   const double *bp = m.bank_part;
   double ds = bp[b], dg = bp[nbk + b];
   const double inv_area = m.inv_area[i];
@@ -965,9 +1201,11 @@ __global__ void __launch_bounds__(128) k_finish(DevMesh m, double *RESTRICT ydot
       if (m.left[s] == i) {
         o = -F[LEFT_SURF2CHANL * nr + s];
         u = -(F[LEFT_AQUIF2CHANL * nr + s] + F[LEFT_AQUIF2AQUIF * nr + s]);
+        m.carry_ovl[s] = F[LEFT_SURF2CHANL * nr + s];
       } else {
         o = -F[RIGHT_SURF2CHANL * nr + s];
         u = -(F[RIGHT_AQUIF2CHANL * nr + s] + F[RIGHT_AQUIF2AQUIF * nr + s]);
+        m.carry_ovl[nr + s] = F[RIGHT_SURF2CHANL * nr + s];
       }
       if (m.diag) {
         m.d_ovl[j * ne + i] = o;
@@ -984,6 +1222,215 @@ __global__ void __launch_bounds__(128) k_finish(DevMesh m, double *RESTRICT ydot
   ydot[i] = ds;
   ydot[2 * ne + i] = dg;
   if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
+}
+
+// ---------------------------------------------------------------------------
+// k_rhs_fused: the whole evaluation in one cooperative launch, for meshes
+// whose evaluation is the latency of dependent kernels.  The arithmetic of
+// the kernels above, cut by what it depends on and given to four kinds of
+// blocks that run beside each other:
+//
+//   elements  prep -> | A, heads -> gradient -> | B
+//   edges             | A, Darcy flux, h^p ---- | B, slope -> flux | C
+//   rivers    area, perimeter | R, channel flux ------------------- | C, rows
+//   banks     | A, fluxes with the elements ----------------------- (to C)
+//   columns   saturation, powers, recharge | A, infiltration's head | C, rows
+//
+// Everything a block can do without the others' results stands before its
+// wait: an evaluation then takes the chain prep, gradient, slope, rows and
+// three barriers, instead of seven kernels each with its own launch, loads
+// and powers.  Each item's arithmetic is that of the separate kernels, so the
+// results are the same bits.
+//
+// A, B, C, R are counters in device memory that the blocks before them raise
+// once (C: edges, rivers and banks).  The
+// last block through C zeroes them -- elements and edges have raised C or
+// what C waits for by then -- so a captured launch can be replayed.  Cooperative launch makes the blocks
+// resident together; a wait gives up after kBarPolls polls, and the blocks
+// then report kErrWait instead of results.
+// ---------------------------------------------------------------------------
+constexpr int kBarPolls = 1 << 22;  // a few seconds
+constexpr int kBarStride = 32;      // counters on cache lines of their own
+
+__device__ __forceinline__ void bar_arrive(unsigned *cnt) {
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+}
+// false when the wait ran out; the same answer in every thread of the block
+__device__ __forceinline__ bool bar_wait(unsigned *cnt, unsigned blocks, int *s_ok) {
+  if (threadIdx.x == 0) {
+    unsigned v = 0;
+    for (int k = 0; k < kBarPolls; k++) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+      if (v >= blocks) break;
+    }
+    *s_ok = v >= blocks;
+  }
+  __syncthreads();
+  const bool ok = *s_ok != 0;
+  __syncthreads();
+  return ok;
+}
+
+// a block is past its last wait: the last of `blocks` zeroes the counters
+__device__ __forceinline__ void bar_leave(unsigned *bar, unsigned blocks) {
+  if (threadIdx.x == 0 && atomicAdd(bar + 4 * kBarStride, 1u) == blocks - 1)
+    for (int k = 0; k < 5; k++) bar[k * kBarStride] = 0u;
+}
+
+// what a block whose wait ran out leaves: the error word of its items
+__device__ __noinline__ void report_wait(const DevMesh &m, const int32_t *sys_of, int first, int n, int step) {
+  int sy;
+  for (int k = first; k < n; k += step)
+    if (!skip_item(m, sys_of, k, &sy)) report_err(m, sy, kErrWait);
+}
+
+constexpr int kFusedThreads = 256;  // most threads per block
+
+// blocks of each kind, in this order of block index
+struct FusedGrid {
+  int elem, edge, river, col;
+};
+
+template <bool kFromRef, int kMinBlocks>
+__global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
+    k_rhs_fused(const __grid_constant__ DevMesh m, const double *y, double *ydot, const double *y_ref, double *y_int,
+                const int32_t *iperm, const FusedGrid g) {
+  __shared__ int s_ok;
+  unsigned *const A = m.bar, *const B = m.bar + kBarStride, *const C = m.bar + 2 * kBarStride,
+                  *const R = m.bar + 3 * kBarStride;
+  const bool grad = m.surf_mode == kDiffWave;
+  const int ne = m.ne;
+  int blk = blockIdx.x;
+  int sy;
+  if (blk < g.elem) {
+    // ---- elements ----
+    const int first = blk * blockDim.x + threadIdx.x, step = g.elem * blockDim.x;
+    const int n = kFromRef ? ne + 2 * m.nr : m.ne_run;
+    for (int t = first; t < n; t += step) {
+      int i = t;
+      double y_surf, y_gw;
+      if (kFromRef) {
+        if (t >= ne) {  // stage and river gw, same order
+          y_int[2 * ne + t] = y_ref[2 * ne + t];
+          continue;
+        }
+        i = iperm[t];
+        y_surf = y_ref[t];
+        const double u = y_ref[ne + t];
+        y_gw = y_ref[2 * ne + t];
+        y_int[i] = y_surf;
+        y_int[ne + i] = u;
+        y_int[2 * ne + i] = y_gw;
+      } else {
+        if (skip_item(m, m.sys_elem, i, &sy)) continue;
+        y_surf = y[i];
+        y_gw = y[2 * ne + i];
+      }
+      bool thin = false, mix = false;
+      double sx, num, den;
+      prep_item(m, i, y_surf, y_gw, thin, sx, mix, num, den);
+      if (thin) prep_root(m, i, sx);
+      if (mix) m.effk[i] = div_any(num, den);
+    }
+    bar_arrive(A);
+    if (!grad) return;
+    // kFromRef: the river stages grad_load reads are other blocks' copies
+    const bool one = !kFromRef && step >= m.ne_run;  // one element a thread: its geometry before the wait
+    const bool on = one && first < m.ne_run && !skip_item(m, m.sys_elem, first, &sy);
+    GradIn in;
+    if (on) in = grad_load(m, y, first);
+    if (!bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (on) m.gradmag[first] = grad_value(m, in);
+    for (int i = first; !one && i < m.ne_run; i += step)
+      if (!skip_item(m, m.sys_elem, i, &sy)) m.gradmag[i] = grad_value(m, grad_load(m, y, i));
+    bar_arrive(B);
+    return;
+  }
+  blk -= g.elem;
+  if (blk < g.edge) {
+    // ---- edges ----
+    const int first = blk * blockDim.x + threadIdx.x, step = g.edge * blockDim.x;
+    if (!bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
+    bool waited = !grad;
+    // whole blocks go round together: the wait is the block's
+    for (int e = first; e - (int)threadIdx.x < m.nedge_run; e += step) {
+      int i = 0, k = 0;
+      double avg_h = 0.0, diff_h = 0.0, hp = 0.0;
+      bool wet = false;
+      if (e < m.nedge_run && !skip_item(m, m.sys_edge, e, &sy)) {
+        i = m.e_i[e];
+        k = m.e_k[e];
+        wet = edge_item(m, y, e, i, k, avg_h, diff_h);
+        if (wet) hp = edge_hp(avg_h);
+      }
+      if (!waited) {
+        waited = true;
+        if (!bar_wait(B, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
+      }
+      if (wet) m.eflux_ovl[e] = hp * diff_h * rsqrt(edge_slope(m, e, i, k, diff_h)) * m.e_ovlk[e];
+    }
+    bar_arrive(C);
+    return;
+  }
+  blk -= g.edge;
+  const unsigned lateral = g.edge + g.river;
+  if (blk < g.river) {
+    // ---- rivers: the same number of blocks for each part ----
+    const int per = g.river / kRivParts, part = blk / per;
+    const int first = (blk - part * per) * blockDim.x + threadIdx.x, step = per * blockDim.x;
+    bool ok;
+    if (part == PART_CHAN) {
+      // the state alone; kFromRef: river values stand in the same order
+      const double *yr = kFromRef ? y_ref : y;
+      for (int s = first; s < m.nr_run; s += step)
+        if (!skip_item(m, m.sys_riv, s, &sy)) geom_item(m, yr, s);
+      bar_arrive(R);
+      ok = bar_wait(R, per, &s_ok);
+      for (int s = first; ok && s < m.nr_run; s += step)
+        if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, yr, s, PART_CHAN);
+    } else {
+      ok = bar_wait(A, g.elem, &s_ok);
+      for (int s = first; ok && s < m.nr_run; s += step)
+        if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, y, s, part);
+    }
+    if (ok) {
+      bar_arrive(C);
+      if (part != PART_CHAN) return;
+      ok = bar_wait(C, lateral, &s_ok);
+    }
+    if (!ok) return report_wait(m, m.sys_riv, first, m.nr_run, step);
+    bar_leave(m.bar, per + g.col);
+    for (int s = first; s < m.nr_run; s += step)
+      if (!skip_item(m, m.sys_riv, s, &sy)) river_rows_item(m, ydot, s, sy);
+    return;
+  }
+  blk -= g.river;
+  // ---- columns ----
+  const int first = blk * blockDim.x + threadIdx.x, step = g.col * blockDim.x;
+  bool met = false;  // the block has been through A and C
+  for (int i = first; i - (int)threadIdx.x < m.ne_run || !met; i += step) {
+    const bool on = i < m.ne_run && !skip_item(m, m.sys_elem, i, &sy);
+    Column c;
+    RowsIn r;
+    // kFromRef: the state in internal order is the element blocks' to write
+    if (kFromRef && !met && !bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (on) {
+      column_state(m, y, i, sy, c);
+      rows_load(m, i, r);
+    }
+    if (!kFromRef && !met && !bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (on) {
+      column_surface(m, i, c);
+      c.kinf_crack = crack_kinf(c, r.kinf_mat, r.kmac_a);
+    }
+    if (!met) {
+      met = true;
+      if (!bar_wait(C, lateral, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+      bar_leave(m.bar, g.river / kRivParts + g.col);
+    }
+    if (on) column_rows<true>(m, ydot, i, sy, c, r);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1063,14 +1510,84 @@ static void prof_end(Profiler *p, bool on, cudaStream_t st) {
   if (on) cudaEventRecord(p->recs[p->nrec - 1].b, st);
 }
 
+// k_rhs_fused at 128 registers (2 x 256 threads per SM: the powers of a
+// column overlap) and at 64 (4 x 256: twice as many items at once).
+static const void *fused_kernel(int dense, bool from_ref) {
+  if (dense) return from_ref ? (const void *)k_rhs_fused<true, 4> : (const void *)k_rhs_fused<false, 4>;
+  return from_ref ? (const void *)k_rhs_fused<true, 2> : (const void *)k_rhs_fused<false, 2>;
+}
+
+// k_rhs_fused's resident blocks per launch, for 32, 64, 128 and 256 threads.
+cudaError_t fused_plan(FusedPlan *f) {
+  int dev = 0, sms = 0, coop = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  for (int d = 0; d < 2; d++)
+    for (int k = 0; k < FusedPlan::kSizes && e == cudaSuccess; k++) {
+      int a = 0, b = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fused_kernel(d, false), 32 << k, 0);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fused_kernel(d, true), 32 << k, 0);
+      f->blocks[d][k] = coop ? sms * std::min(a, b) : 0;
+    }
+  f->sms = sms;
+  return e;
+}
+
+// How k_rhs_fused would run this evaluation: blocks as small as leave every
+// SM a few warps, so that a small mesh spreads over the chip (the FP64 pipe
+// retires two lanes a clock on each SM), one item a thread.  False when the
+// items are more than can be resident together: the blocks of one kind would
+// then take turns while the others wait, and the separate kernels are faster.
+struct FusedLaunch {
+  FusedGrid g;
+  int dense, threads;
+};
+static bool fused_fits(const DevMesh &m, const FusedPlan &f, bool from_ref, FusedLaunch *l) {
+  const long long elems = from_ref ? m.ne + 2LL * m.nr : m.ne_run;
+  const long long all = elems + m.nedge_run + (long long)kRivParts * m.nr_run + m.ne_run;
+  if (!m.bar || m.ne_run <= 0 || all > 2048LL * f.sms) return false;
+  int k = 0;
+  while (k + 1 < FusedPlan::kSizes && all > (32LL << k) * f.sms) k++;
+  l->threads = 32 << k;
+  l->g = FusedGrid{(int)blocks_for(elems, l->threads), (int)blocks_for(m.nedge_run, l->threads),
+                   kRivParts * (int)blocks_for(m.nr_run, l->threads), (int)blocks_for(m.ne_run, l->threads)};
+  const int want = l->g.elem + l->g.edge + l->g.river + l->g.col;
+  l->dense = want > f.blocks[0][k];
+  return want <= f.blocks[l->dense][k];
+}
+static cudaError_t launch_fused(const DevMesh &m, FusedLaunch &l, const double *y, double *ydot, cudaStream_t st,
+                                const double *y_ref, const int32_t *iperm) {
+  double *y_int = const_cast<double *>(y);  // y_ref: the internal-order buffer the kernel fills
+  void *args[] = {(void *)&m, (void *)&y, &ydot, (void *)&y_ref, &y_int, (void *)&iperm, &l.g};
+  return cudaLaunchCooperativeKernel(fused_kernel(l.dense, y_ref != nullptr),
+                                     dim3(l.g.elem + l.g.edge + l.g.river + l.g.col), dim3(l.threads), args, 0, st);
+}
+
 cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStream_t st,
                        long long *launches, Profiler *prof, const RhsStreams *side, const double *y_ref,
                        const int32_t *iperm) {
   bool on;
-  // the river kernel reads only k_elem_prep's outputs, the state and static
-  // data, so with a side stream it runs beside grad/edge/main (per-kernel
+  // a small mesh in one launch (per-kernel timing keeps the separate kernels):
+  // one evaluation of 1,000 / 20,000 / 40,000 elements takes 18 / 24 / 33 us
+  // instead of 41 / 46 / 54
+  FusedLaunch fl;
+  if (side && !prof && fused_fits(m, side->fused, y_ref != nullptr, &fl)) {
+    ++*launches;
+    return launch_fused(m, fl, y, ydot, st, y_ref, iperm);
+  }
+  // the river kernels read only k_elem_prep's outputs, the state and static
+  // data, so with a side stream they run beside grad/edge/main (per-kernel
   // timing keeps one stream)
   const bool fork = side && side->side && !prof && m.ne_run > 0 && m.nr_run > 0;
+  const auto river = [&](cudaStream_t rs) {
+    on = prof_begin(prof, K_RIVER, rs);
+    k_riv_geom<<<blocks_for(m.nr_run, 128), 128, 0, rs>>>(m, y);
+    k_river<<<blocks_for(kRivParts * ((m.nr_run + 31LL) & ~31LL), 128), 128, 0, rs>>>(m, y);
+    k_river_rows<<<blocks_for(m.nr_run, 128), 128, 0, rs>>>(m, ydot);
+    prof_end(prof, on, rs);
+    *launches += 3;
+  };
   if (m.ne_run > 0) {
     on = prof_begin(prof, K_PREP, st);
     if (y_ref)  // y is the internal-order buffer the kernel fills
@@ -1083,9 +1600,7 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
     if (fork) {
       if (cudaEventRecord(side->fork, st) != cudaSuccess) return cudaErrorUnknown;
       if (cudaStreamWaitEvent(side->side, side->fork, 0) != cudaSuccess) return cudaErrorUnknown;
-      k_riv_geom<<<blocks_for(m.nr_run, 128), 128, 0, side->side>>>(m, y);
-      k_river<<<blocks_for(m.nr_run, 128), 128, 0, side->side>>>(m, y);
-      *launches += 2;
+      river(side->side);
       if (cudaEventRecord(side->join, side->side) != cudaSuccess) return cudaErrorUnknown;
     }
     if (m.surf_mode == kDiffWave) {
@@ -1112,15 +1627,11 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
   if (fork) {
     if (cudaStreamWaitEvent(st, side->join, 0) != cudaSuccess) return cudaErrorUnknown;
   } else if (m.nr_run > 0) {
-    on = prof_begin(prof, K_RIVER, st);  // both river kernels
-    k_riv_geom<<<blocks_for(m.nr_run, 128), 128, 0, st>>>(m, y);
-    k_river<<<blocks_for(m.nr_run, 128), 128, 0, st>>>(m, y);
-    prof_end(prof, on, st);
-    *launches += 2;
+    river(st);
   }
-  if (m.nr_run + m.nbank_run > 0) {
+  if (m.nbank_run > 0) {
     on = prof_begin(prof, K_FINISH, st);
-    k_finish<<<blocks_for((long long)m.nr_run + m.nbank_run, 128), 128, 0, st>>>(m, ydot);
+    k_bank_rows<<<blocks_for(m.nbank_run, 128), 128, 0, st>>>(m, ydot);
     prof_end(prof, on, st);
     ++*launches;
   }
