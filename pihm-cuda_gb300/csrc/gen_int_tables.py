@@ -73,9 +73,21 @@ def main():
         "kImE120": rnd(D(2) ** 62 / 120), "kImE24": rnd(D(2) ** 62 / 24), "kImE6": rnd(D(2) ** 62 / 6),
         "kImE2": 2 ** 61,
     }
+    # exp and log of doubles: 1024 / ln 2 at scale 2^53 and its next 64 bits,
+    # ln 2 and log10 2 at scale 2^64
+    big = D(N) / LN2 * D(2) ** 53
+    kh = int(big)
+    unsigned = {"kImKh": kh, "kImKl": rnd((big - kh) * D(2) ** 64), "kImCLn2": rnd(LN2 * D(2) ** 64),
+                "kImCLog10": rnd(D(2).log10() * D(2) ** 64),
+                # log10(e) at scale 2^64, and 1/j at scale 2^62 for log1p's series
+                "kImLog10E": rnd(D(1).exp().log10() * D(2) ** 64),
+                **{f"kImInv{j}": rnd(D(2) ** 62 / j) for j in range(3, 12)}}
     for k, v in consts.items():
         assert -(2 ** 63) <= v < 2 ** 63
         out.append(f"static constexpr int64_t {k} = {v}ll;")
+    for k, v in unsigned.items():
+        assert 0 <= v < 2 ** 64
+        out.append(f"static constexpr uint64_t {k} = {v}ull;")
     print("\n".join(out))
 
 

@@ -240,6 +240,105 @@ PIHM_IM_FN bool pow_i(double x, double y, double &out) {
 }
 
 
+PIHM_IM_FN uint64_t umulhi(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umul64hi(a, b);
+#else
+  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+PIHM_IM_FN int clz64(uint64_t a) {
+#if defined(__CUDA_ARCH__)
+  return __clzll((long long)a);
+#else
+  return a ? __builtin_clzll(a) : 64;
+#endif
+}
+
+// e^x for |x| < 66.5: t = x (1024 / ln 2) from the 53-bit mantissa times 128
+// bits of the constant (kImKh, kImKl), so the error of t stays below 2^-60 of
+// the result and the exponential is within 0.502 ulp.
+PIHM_IM_FN bool exp_i(double x, double &out) {
+  const uint64_t xb = dbits(x);
+  const int ex = (int)((xb >> 52) & 2047u) - 1023;
+  const uint64_t M = (xb & kFrac) | (1ull << 52);
+  unsigned __int128 Q = (unsigned __int128)M * kImKh + umulhi(M, kImKl);  // |t| 2^(105 - ex)
+  const int sh = 41 - ex;  // to units of 2^-64; beyond 2^-60 of a unit of x the result is 1
+  Q = sh < 127 ? Q >> (sh & 127) : 0;
+  const i128 T = (xb >> 63) ? -(i128)Q : (i128)Q;
+  TVal t;
+  t.n = (int64_t)(T >> 64) + (int64_t)((uint64_t)T >> 63);
+  t.f = (int64_t)(uint64_t)T;
+  out = exp2k(t);
+  return (ex < 7) & (t.n < kNMax) & (t.n > -kNMax);
+}
+
+// log x to the base whose log of 2 is C 2^-64 (kImCLn2, kImCLog10), for x
+// positive and normal with |k| <= 126 and |log2 x| above about 2^-7 (w's
+// error of two units of 2^-53 is then below 0.2 ulp, and within 0.502 ulp of
+// the exact logarithm where |log2 x| > 1/2).
+PIHM_IM_FN bool log_i(double x, uint64_t C, double &out) {
+  int k;
+  int64_t w;
+  const bool ok = log2k(x, k, w);
+  const i128 T = (i128)((unsigned __int128)(i128)k << 63) + w;  // 1024 log2 x in units of 2^-53
+  const unsigned __int128 a = (unsigned __int128)(T < 0 ? -T : T);
+  const uint64_t hi = (uint64_t)(a >> 64), lo = (uint64_t)a;
+  const int sh = hi ? 64 - clz64(hi) : -clz64(lo);              // a = m 2^sh, m in [2^63, 2^64)
+  const uint64_t m = hi ? (uint64_t)(a >> (sh & 63)) : lo << (-sh & 63);
+  const unsigned __int128 p = (unsigned __int128)m * C;         // log x = (p 2^-64) 2^(sh - 63)
+  const int z = clz64((uint64_t)(p >> 64));                     // 0..2
+  const uint64_t q = (uint64_t)((p << (z & 63)) >> 64);
+  const uint64_t mant = (q >> 11) + ((q >> 10) & 1u);           // 53 bits (a carry moves the exponent)
+  const uint64_t bits = ((uint64_t)(int64_t)(sh - z + 1022) << 52) + mant;
+  out = bitsd((T < 0 ? 1ull << 63 : 0ull) | bits);
+  return ok & ((hi | (lo >> 56)) != 0);
+}
+
+// log x for x within 2^-6 of one (where log2k's absolute error is too much of
+// a small logarithm): d = x - 1 is exact, log1p(d) = d P(d), P the series
+// 1 - d/2 + d^2/3 - ... to d^10 (the next term is below 2^-69), its inner
+// half in 32-bit fixed point; within 0.502 ulp.  ten: the logarithm to base 10.
+PIHM_IM_FN bool log_near1_i(double x, bool ten, double &out) {
+  // x - 1 in units of 2^-63 (53 bits of x are at most 2^10 units)
+  const uint64_t xb = dbits(x);
+  const int ex = (int)(xb >> 52) - 1023;  // 0 or -1
+  const uint64_t M = (xb & kFrac) | (1ull << 52);
+  const int64_t d = (int64_t)((ex == 0 ? M << 11 : M << 10) - (1ull << 63));
+  const bool ok = ((ex == 0) | (ex == -1)) & (d < (1ll << 57)) & (d > -(1ll << 57));
+  const int32_t d32 = (int32_t)(d >> 31);  // d 2^32
+  // Horner from 1/11; 2^31 units while the rest multiplies by d^5 or more
+  int32_t h = (int32_t)(kImInv11 >> 31);
+  h = (int32_t)(kImInv10 >> 31) - mulhi32(h, d32);
+  h = (int32_t)(kImInv9 >> 31) - mulhi32(h, d32);
+  h = (int32_t)(kImInv8 >> 31) - mulhi32(h, d32);
+  h = (int32_t)(kImInv7 >> 31) - mulhi32(h, d32);
+  int64_t p = (int64_t)kImInv6 - mulhi((int64_t)h << 31, d << 1);
+  p = (int64_t)kImInv5 - mulhi(p, d << 1);
+  p = (1ll << 60) - mulhi(p, d << 1);            // 1/4
+  p = (int64_t)kImInv3 - mulhi(p, d << 1);
+  p = (1ll << 61) - mulhi(p, d << 1);            // 1/2
+  p = (1ll << 62) - mulhi(p, d << 1);            // P 2^62, in (0.99, 1.01) 2^62
+  const uint64_t a = (uint64_t)(d < 0 ? -d : d);
+  const int z = clz64(a) & 63;
+  const unsigned __int128 v = (unsigned __int128)(a << z) * (uint64_t)p;  // |log x| 2^(63 + 62 + z)
+  // normalise to 64 bits
+  const int y = clz64((uint64_t)(v >> 64));
+  uint64_t q = (uint64_t)((v << (y & 63)) >> 64);  // q 2^(64 - y) = v
+  int e = 63 + 64 - y - (63 + 62 + z);             // |log x| = q 2^(e - 63)
+  if (ten) {
+    const unsigned __int128 t = (unsigned __int128)q * kImLog10E;
+    const int u = clz64((uint64_t)(t >> 64));
+    q = (uint64_t)((t << (u & 63)) >> 64);
+    e -= u;
+  }
+  const uint64_t mant = (q >> 11) + ((q >> 10) & 1u);
+  const uint64_t bits = ((uint64_t)(int64_t)(e + 1022) << 52) + mant;
+  out = a == 0 ? 0.0 : bitsd((d < 0 ? 1ull << 63 : 0ull) | bits);
+  return ok;
+}
+
 // ---------------------------------------------------------------------------
 // Division and square root, correctly rounded (round to nearest even), on
 // the integer pipe.  A single-precision reciprocal (or reciprocal square
@@ -280,14 +379,6 @@ PIHM_IM_FN uint32_t umulhi32(uint32_t a, uint32_t b) {
   return __umulhi(a, b);
 #else
   return (uint32_t)(((uint64_t)a * b) >> 32);
-#endif
-}
-
-PIHM_IM_FN uint64_t umulhi(uint64_t a, uint64_t b) {
-#if defined(__CUDA_ARCH__)
-  return __umul64hi(a, b);
-#else
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
 #endif
 }
 

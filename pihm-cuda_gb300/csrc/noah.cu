@@ -9,11 +9,11 @@
 //                 runoff2, FindWaterTable, CalcLatFlx, src/update.c:34-41)
 //                 and NoahHydrol (FindWaterTable, the moisture clamps, SmFlx,
 //                 src/noah/noah.c:57-97)
-//   k_noah_inputs what the Flux-PIHM right-hand side reads: GwTransp's layer
-//                 sum (noah/lsm_func.c:163-185) and whether the water table
-//                 lies within the root zone, Infil's top-layer saturation
-//                 (src/vert_flow.c:94-98), the frozen-soil factor, and the
-//                 right-hand side's edir, ett and pcpdrp planes
+// and both end with what the Flux-PIHM right-hand side reads (write_inputs;
+// k_noah_inputs after a state is set): GwTransp's layer sum
+// (noah/lsm_func.c:163-185) and whether the water table lies within the root
+// zone, Infil's top-layer saturation (src/vert_flow.c:94-98), the frozen-soil
+// factor, and the right-hand side's edir, ett and pcpdrp planes.
 // Every plane is in the context's internal element order; per-layer planes
 // are [layer][ne].  The state never leaves the device between steps.
 #include <cmath>
@@ -62,28 +62,28 @@ struct NoahPlanes {
 
 namespace {
 
-using noah::Col;
-using noah::L;
+using noah::Real;
+constexpr int L = noah::kMaxLayers;
 
+// What a land-surface step reads of a column.
+template <class Col>
 __device__ void load_col(const NoahPlanes &P, int i, Col &c) {
   const int ne = P.ne;
   c.nsoil = P.i[NI_NSOIL][i];
   c.nroot = P.i[NI_NROOT][i];
   c.isurban = P.i[NI_ISURBAN][i];
   c.nwtbl = P.i[NI_NWTBL][i];
-  for (int k = 0; k < L; k++) {
-    const bool in = k < c.nsoil;
-    c.sldpth[k] = in ? P.l[NL_SLDPTH][k * ne + i] : 0.0;
-    c.zsoil[k] = in ? P.l[NL_ZSOIL][k * ne + i] : 0.0;
-    c.rtdis[k] = in ? P.l[NL_RTDIS][k * ne + i] : 0.0;
-    c.smc[k] = in ? P.l[NL_SMC][k * ne + i] : 0.0;
-    c.sh2o[k] = in ? P.l[NL_SH2O][k * ne + i] : 0.0;
-    c.stc[k] = in ? P.l[NL_STC][k * ne + i] : 0.0;
-    c.et[k] = in ? P.l[NL_ET][k * ne + i] : 0.0;
-    c.runoff2_lyr[k] = in ? P.l[NL_RUNOFF2_LYR][k * ne + i] : 0.0;
-    c.smflxv[k] = in ? P.l[NL_SMFLXV][k * ne + i] : 0.0;
-    c.satdpth[k] = 0.0;
-  }
+#pragma unroll
+  for (int k = 0; k < Col::L; k++)
+    if (k < c.nsoil) {
+      c.sldpth[k] = P.l[NL_SLDPTH][k * ne + i];
+      c.zsoil[k] = P.l[NL_ZSOIL][k * ne + i];
+      c.rtdis[k] = P.l[NL_RTDIS][k * ne + i];
+      c.smc[k] = P.l[NL_SMC][k * ne + i];
+      c.sh2o[k] = P.l[NL_SH2O][k * ne + i];
+      c.stc[k] = P.l[NL_STC][k * ne + i];
+      c.et[k] = P.l[NL_ET][k * ne + i];
+    }
   const double *const *s = P.s;
   c.smcmax = s[NS_SMCMAX][i]; c.smcmin = s[NS_SMCMIN][i]; c.smcref = s[NS_SMCREF][i];
   c.smcwlt = s[NS_SMCWLT][i]; c.smcdry = s[NS_SMCDRY][i]; c.quartz = s[NS_QUARTZ][i];
@@ -106,74 +106,97 @@ __device__ void load_col(const NoahPlanes &P, int i, Col &c) {
   c.fcr = s[NS_FCR][i];
   c.edir = s[NS_EDIR][i]; c.ec = s[NS_EC][i]; c.ett = s[NS_ETT][i]; c.esnow = s[NS_ESNOW][i];
   c.etp = s[NS_ETP][i]; c.drip = s[NS_DRIP][i]; c.pcpdrp = s[NS_PCPDRP][i]; c.snomlt = s[NS_SNOMLT][i];
-  c.ssoil = s[NS_SSOIL][i]; c.sheat = s[NS_SHEAT][i]; c.runoff2 = s[NS_RUNOFF2][i];
-  c.runoff3 = s[NS_RUNOFF3][i]; c.infil = s[NS_INFIL][i]; c.sncovr = s[NS_SNCOVR][i];
+  c.ssoil = s[NS_SSOIL][i]; c.sheat = s[NS_SHEAT][i]; c.sncovr = s[NS_SNCOVR][i];
   c.beta_s = s[NS_BETA_S][i]; c.eta = s[NS_ETA][i]; c.soilm = s[NS_SOILM][i];
   c.etns = s[NS_ETNS][i];
 }
 
 // What a step changes: the state, the outputs and -- for urban land, where
 // SFlx overrides them for good (src/noah/noah.c:201-212) -- the parameters.
+template <class Col>
 __device__ void store_col(const NoahPlanes &P, int i, const Col &c) {
   const int ne = P.ne;
-  for (int k = 0; k < c.nsoil; k++) {
-    P.l[NL_SMC][k * ne + i] = c.smc[k];
-    P.l[NL_SH2O][k * ne + i] = c.sh2o[k];
-    P.l[NL_STC][k * ne + i] = c.stc[k];
-    P.l[NL_ET][k * ne + i] = c.et[k];
-    P.l[NL_RUNOFF2_LYR][k * ne + i] = c.runoff2_lyr[k];
-    P.l[NL_SMFLXV][k * ne + i] = c.smflxv[k];
+#pragma unroll
+  for (int k = 0; k < Col::L; k++) {
+    if (k >= c.nsoil) break;
+    P.l[NL_SMC][k * ne + i] = c.smc[k].v;
+    P.l[NL_SH2O][k * ne + i] = c.sh2o[k].v;
+    P.l[NL_STC][k * ne + i] = c.stc[k].v;
+    P.l[NL_ET][k * ne + i] = c.et[k].v;
   }
-  P.i[NI_NWTBL][i] = c.nwtbl;
   double *const *s = P.s;
   if (c.isurban) {
-    s[NS_SHDFAC][i] = c.shdfac; s[NS_RSMIN][i] = c.rsmin; s[NS_SMCMAX][i] = c.smcmax;
-    s[NS_SMCMIN][i] = c.smcmin; s[NS_SMCREF][i] = c.smcref; s[NS_SMCWLT][i] = c.smcwlt;
-    s[NS_SMCDRY][i] = c.smcdry;
+    s[NS_SHDFAC][i] = c.shdfac.v; s[NS_RSMIN][i] = c.rsmin.v; s[NS_SMCMAX][i] = c.smcmax.v;
+    s[NS_SMCMIN][i] = c.smcmin.v; s[NS_SMCREF][i] = c.smcref.v; s[NS_SMCWLT][i] = c.smcwlt.v;
+    s[NS_SMCDRY][i] = c.smcdry.v;
   }
-  s[NS_T1][i] = c.t1; s[NS_CMC][i] = c.cmc; s[NS_SNEQV][i] = c.sneqv; s[NS_SNOWH][i] = c.snowh;
-  s[NS_SNDENS][i] = c.sndens; s[NS_CH][i] = c.ch; s[NS_CM][i] = c.cm; s[NS_SNOTIME1][i] = c.snotime1;
-  s[NS_ALBEDO][i] = c.albedo; s[NS_EMISSI][i] = c.emissi; s[NS_Q1][i] = c.q1; s[NS_RIBB][i] = c.ribb;
-  s[NS_FCR][i] = c.fcr;
-  s[NS_EDIR][i] = c.edir; s[NS_EC][i] = c.ec; s[NS_ETT][i] = c.ett; s[NS_ESNOW][i] = c.esnow;
-  s[NS_ETP][i] = c.etp; s[NS_DRIP][i] = c.drip; s[NS_PCPDRP][i] = c.pcpdrp; s[NS_SNOMLT][i] = c.snomlt;
-  s[NS_SSOIL][i] = c.ssoil; s[NS_SHEAT][i] = c.sheat; s[NS_RUNOFF2][i] = c.runoff2;
-  s[NS_RUNOFF3][i] = c.runoff3; s[NS_INFIL][i] = c.infil; s[NS_SNCOVR][i] = c.sncovr;
-  s[NS_BETA_S][i] = c.beta_s; s[NS_ETA][i] = c.eta; s[NS_SOILM][i] = c.soilm;
-  s[NS_ETNS][i] = c.etns;
+  s[NS_T1][i] = c.t1.v; s[NS_CMC][i] = c.cmc.v; s[NS_SNEQV][i] = c.sneqv.v; s[NS_SNOWH][i] = c.snowh.v;
+  s[NS_SNDENS][i] = c.sndens.v; s[NS_CH][i] = c.ch.v; s[NS_CM][i] = c.cm.v; s[NS_SNOTIME1][i] = c.snotime1.v;
+  s[NS_ALBEDO][i] = c.albedo.v; s[NS_EMISSI][i] = c.emissi.v; s[NS_Q1][i] = c.q1.v;
+  s[NS_EDIR][i] = c.edir.v; s[NS_EC][i] = c.ec.v; s[NS_ETT][i] = c.ett.v; s[NS_ESNOW][i] = c.esnow.v;
+  s[NS_ETP][i] = c.etp.v; s[NS_DRIP][i] = c.drip.v; s[NS_PCPDRP][i] = c.pcpdrp.v; s[NS_SNOMLT][i] = c.snomlt.v;
+  s[NS_SSOIL][i] = c.ssoil.v; s[NS_SHEAT][i] = c.sheat.v; s[NS_SNCOVR][i] = c.sncovr.v;
+  s[NS_BETA_S][i] = c.beta_s.v; s[NS_ETA][i] = c.eta.v; s[NS_SOILM][i] = c.soilm.v;
+  s[NS_ETNS][i] = c.etns.v;
+}
+
+// The Flux-PIHM right-hand side's inputs from a column's state and outputs.
+template <class Col>
+__device__ __forceinline__ void write_inputs(const NoahTargets &o, int i, const Col &c) {
+  Real g = 0.0;
+  if (c.nwtbl <= c.nroot)
+    for (int j = (c.nwtbl <= 0 ? 0 : c.nwtbl - 1); j < c.nroot; j++) g += c.et[j];
+  o.etgw[i] = g.v;
+  o.wtin[i] = c.nwtbl <= c.nroot;
+  o.satn[i] = ((c.sh2o[0] - c.smcmin) / (c.smcmax - c.smcmin)).v;
+  o.fcr[i] = c.fcr.v;
+  o.edir[i] = c.edir.v;
+  o.ett[i] = c.ett.v;
+  o.pcpdrp[i] = c.pcpdrp.v;
 }
 
 constexpr int kNoahBlock = 128;
-constexpr int kNoahClasses = 8;
+constexpr int kNoahClasses = 32;
 
 // The branch class of an element's next Noah() step: whether it will run the
 // snowpack path (snow on the ground, or precipitation that may fall as snow
-// or freezing rain), whether a soil layer or the skin is frozen (the
-// iterative frozen-water solution of FrH2O), whether it has vegetation (the
-// canopy resistance and transpiration).  Noah() is one thread per element and
-// GB300 retires 2 FP64 lanes per clock per SM, so a warp whose lanes take
+// or freezing rain), whether the surface layer is unstable (SfcDifOff's
+// logarithms and arctangents), how many layers hold ice or frost (each runs
+// FrH2O's iterations, up to 7 told apart).  Noah() is one thread per element
+// and GB300 retires 2 FP64 lanes per clock per SM, so a warp whose lanes take
 // different paths runs each path for all of them; grouping elements by class
 // keeps warps on one path.  Only the order of work changes: every element's
 // arithmetic, and so every result, is the same.
 __device__ __forceinline__ int noah_class(const NoahPlanes &P, int i) {
   const double tf = 273.15;
-  const bool snow = P.s[NS_SNEQV][i] > 0.0 || (P.s[NS_PRCP][i] > 0.0 && P.s[NS_SFCTMP][i] <= tf + 1.0);
-  bool frozen = P.s[NS_T1][i] < tf;
+  const double sfctmp = P.s[NS_SFCTMP][i], t1 = P.s[NS_T1][i];
+  const bool snow = P.s[NS_SNEQV][i] > 0.0 || (P.s[NS_PRCP][i] > 0.0 && sfctmp <= tf + 1.0);
   const int nsoil = P.i[NI_NSOIL][i];
-  for (int k = 0; k < nsoil; k++) frozen = frozen || P.l[NL_STC][k * P.ne + i] < tf;
-  const bool veg = P.s[NS_SHDFAC][i] > 0.0;
-  return (snow ? 4 : 0) + (frozen ? 2 : 0) + (veg ? 1 : 0);
+  int frozen = t1 < tf;
+  for (int k = 0; k < nsoil; k++)
+    frozen += P.l[NL_STC][k * P.ne + i] < tf || P.l[NL_SMC][k * P.ne + i] > P.l[NL_SH2O][k * P.ne + i];
+  const bool unstable = t1 > sfctmp + 0.0098 * P.s[NS_ZLVL][i];
+  return (frozen < 7 ? frozen : 7) * 4 + (snow ? 2 : 0) + (unstable ? 1 : 0);
 }
 
-// class sizes (cls[0..7]; the caller zeroed cls)
+// class sizes (the caller zeroed cls): counted per block in shared
+// memory, one global addition per class and block (one per element onto eight
+// addresses took 60 us for 200,000 elements)
 __global__ void __launch_bounds__(256) k_noah_count(NoahPlanes P) {
+  __shared__ int n[kNoahClasses];
+  if (threadIdx.x < kNoahClasses) n[threadIdx.x] = 0;
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P.ne) return;
-  atomicAdd(&P.cls[noah_class(P, i)], 1);
+  const int c = i < P.ne ? noah_class(P, i) : kNoahClasses;
+  const unsigned mask = __match_any_sync(0xffffffffu, c);
+  if (c < kNoahClasses && (int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&n[c], __popc(mask));
+  __syncthreads();
+  if (threadIdx.x < kNoahClasses && n[threadIdx.x]) atomicAdd(&P.cls[threadIdx.x], n[threadIdx.x]);
 }
 
-// each element's place: its class's start (the sizes summed in class order)
-// plus a cursor; lanes of a warp in one class take consecutive places
+// each element's place: its class's start (the sizes of the classes after it,
+// so that the longest columns, snow and frost, start first) plus a cursor;
+// lanes of a warp in one class take consecutive places
 __global__ void __launch_bounds__(256) k_noah_place(NoahPlanes P) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = i < P.ne;
@@ -185,46 +208,73 @@ __global__ void __launch_bounds__(256) k_noah_place(NoahPlanes P) {
   if (lane == lead) base = atomicAdd(&P.cls[kNoahClasses + c], __popc(mask));
   base = __shfl_sync(mask, base, lead);
   int start = 0;
-  for (int k = 0; k < c; k++) start += P.cls[k];
+  for (int k = kNoahClasses - 1; k > c; k--) start += P.cls[k];
   P.order[start + base + __popc(mask & ((1u << lane) - 1u))] = i;
 }
 
-__global__ void __launch_bounds__(kNoahBlock) k_noah_step(NoahPlanes P, double dt, unsigned int *err) {
+// kLayers: the most layers any column has (4, the usual Noah column, or 11):
+// a column's layer arrays stand in local memory, 1 KB instead of 2.4.
+template <int kLayers>
+__global__ void __launch_bounds__(kNoahBlock, 4) k_noah_step(NoahPlanes P, NoahTargets o, double dt,
+                                                             unsigned int *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P.ne) return;
   const int i = P.order[t];
-  Col c;
+  noah::Layers<kLayers> layers;
+  noah::ColT<kLayers> c(layers);
   load_col(P, i, c);
-  noah::noah_step(c, dt);
+  noah::noah_step(c, Real(dt));
   // the reference exits when the snow density exceeds one (SFlx) or a
   // state turns NaN; here the context's error word records it
   if (c.sneqv > 1.0e-7 && !(c.sndens <= 1.0)) atomicOr(err, 1u);
   if (c.t1 != c.t1 || c.edir != c.edir || c.ett != c.ett) atomicOr(err, 1u);
   store_col(P, i, c);
+  write_inputs(o, i, c);
 }
 
 // y: the model state after the step (internal order); first: no previous
-// state yet, ws0 is taken from y
-__global__ void __launch_bounds__(kNoahBlock) k_noah_post(NoahPlanes P, NoahTargets o, const double *y, double dt,
-                                                          int first) {
+// state yet, ws0 is taken from y.  Only what the soil moisture needs of a
+// column moves: 23 scalars and 7 layer planes in, 9 and 4 out, of the 85 and 9
+// of a land-surface step.  200,000 elements: 0.33 ms instead of 0.72, the FP64
+// pipe 62 % busy with the layers' additions and products.
+template <int kLayers>
+__global__ void __launch_bounds__(kNoahBlock, 4) k_noah_post(NoahPlanes P, NoahTargets o, const double *y, double dt,
+                                                             int first) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.ne) return;
   const int ne = P.ne;
-  Col c;
-  load_col(P, i, c);
+  double *const *s = P.s;
+  noah::Layers<kLayers> layers;
+  noah::ColT<kLayers> c(layers);
+  c.nsoil = P.i[NI_NSOIL][i];
+  c.nroot = P.i[NI_NROOT][i];
+#pragma unroll
+  for (int k = 0; k < kLayers; k++)
+    if (k < c.nsoil) {
+      c.sldpth[k] = P.l[NL_SLDPTH][k * ne + i];
+      c.zsoil[k] = P.l[NL_ZSOIL][k * ne + i];
+      c.smc[k] = P.l[NL_SMC][k * ne + i];
+      c.sh2o[k] = P.l[NL_SH2O][k * ne + i];
+      c.et[k] = P.l[NL_ET][k * ne + i];
+      c.runoff2_lyr[k] = P.l[NL_RUNOFF2_LYR][k * ne + i];
+    }
+  c.smcmax = s[NS_SMCMAX][i]; c.smcmin = s[NS_SMCMIN][i]; c.alpha = s[NS_ALPHA][i]; c.beta = s[NS_BETA][i];
+  c.ksatv = s[NS_KSATV][i]; c.porosity = s[NS_POROSITY][i]; c.depth = s[NS_DEPTH][i]; c.area = s[NS_AREA][i];
+  c.frzx = s[NS_FRZX][i]; c.fcr = s[NS_FCR][i];
+  c.edir = s[NS_EDIR][i]; c.ett = s[NS_ETT][i]; c.pcpdrp = s[NS_PCPDRP][i];
   // Summary, src/update.c:3-48: the element state from y, then MassBalance
-  const double unsat = y[ne + i], gw = y[2 * ne + i];
-  const double gw0 = first ? gw : P.s[NS_GW0][i];
-  const double unsat0 = first ? unsat : P.s[NS_UNSAT0][i];
-  double soilw0 = gw0 + unsat0;
+  const Real unsat = y[ne + i], gw = y[2 * ne + i];
+  const Real gw0 = first ? gw : Real(s[NS_GW0][i]);
+  const Real unsat0 = first ? unsat : Real(s[NS_UNSAT0][i]);
+  Real soilw0 = gw0 + unsat0;
   soilw0 = (soilw0 > c.depth) ? c.depth : soilw0;
   soilw0 = (soilw0 < 0.0) ? 0.0 : soilw0;
-  double soilw1 = gw + unsat;
+  Real soilw1 = gw + unsat;
   soilw1 = (soilw1 > c.depth) ? c.depth : soilw1;
   soilw1 = (soilw1 < 0.0) ? 0.0 : soilw1;
-  double subrunoff = 0.0;
+  Real subrunoff = 0.0;
   const int64_t ds = o.stride;
-  for (int j = 0; j < 3; j++) subrunoff += o.d_sub[j * ds + i] / c.area;
+  for (int j = 0; j < 3; j++) subrunoff += Real(o.d_sub[j * ds + i]) / c.area;
   // the last evaluation's ET split: edir_unsat, edir_gw, ett_unsat, ett_gw
   c.infil = (soilw1 - soilw0) * c.porosity / dt + subrunoff + o.d_et[ds + i] + o.d_et[2 * ds + i] +
             o.d_et[3 * ds + i] + o.d_et[4 * ds + i];
@@ -233,13 +283,32 @@ __global__ void __launch_bounds__(kNoahBlock) k_noah_post(NoahPlanes P, NoahTarg
     c.infil = 0.0;
   }
   c.runoff2 = subrunoff;
-  c.nwtbl = noah::find_water_table(c.sldpth, c.nsoil, gw, c.satdpth);
+  c.nwtbl = noah::find_water_table<kLayers>(c.sldpth, c.nsoil, gw, c.satdpth);
   noah::calc_lat_flx(c);
-  P.s[NS_GW0][i] = gw;
-  P.s[NS_UNSAT0][i] = unsat;
+  s[NS_GW0][i] = gw.v;
+  s[NS_UNSAT0][i] = unsat.v;
   // NoahHydrol
-  noah::noah_hydrol(c, gw, dt);
-  store_col(P, i, c);
+  noah::noah_hydrol(c, Real(dt));
+#pragma unroll
+  for (int k = 0; k < kLayers; k++) {
+    if (k >= c.nsoil) break;
+    P.l[NL_SMC][k * ne + i] = c.smc[k].v;
+    P.l[NL_SH2O][k * ne + i] = c.sh2o[k].v;
+    P.l[NL_RUNOFF2_LYR][k * ne + i] = c.runoff2_lyr[k].v;
+  }
+  P.i[NI_NWTBL][i] = c.nwtbl;
+  s[NS_INFIL][i] = c.infil.v;
+  s[NS_RUNOFF2][i] = c.runoff2.v;
+  if (c.nwtbl != 0) {  // else SmFlx only saturated the column
+#pragma unroll
+    for (int k = 0; k < kLayers; k++) {
+      if (k >= c.nsoil) break;
+      P.l[NL_SMFLXV][k * ne + i] = c.smflxv[k].v;
+    }
+    s[NS_FCR][i] = c.fcr.v;
+    s[NS_RUNOFF3][i] = c.runoff3.v;
+  }
+  write_inputs(o, i, c);
 }
 
 // ws0 from the state a run starts from
@@ -289,9 +358,9 @@ int upload(const int32_t *perm, int ne, const double *src, int per, double *cons
 }
 
 int upload_layers(const int32_t *perm, int ne, const double *src, double *plane, cudaStream_t st) {
-  double *dst[noah::L];
-  for (int k = 0; k < noah::L; k++) dst[k] = plane + (size_t)k * ne;
-  return upload(perm, ne, src, noah::L, dst, st);
+  double *dst[noah::kMaxLayers];
+  for (int k = 0; k < noah::kMaxLayers; k++) dst[k] = plane + (size_t)k * ne;
+  return upload(perm, ne, src, noah::kMaxLayers, dst, st);
 }
 
 int upload_int(const int32_t *perm, int ne, const int32_t *src, int32_t *dst) {
@@ -332,10 +401,12 @@ int noah_set_state(NoahInstance &n, const pihm_noah_state *s, const int32_t *per
 int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_t *perm, int ne,
                const NoahTargets &tg, cudaStream_t st, NoahInstance *out) {
   if (!p || !s || !out || p->nelem != ne || !p->nsoil || !p->sldpth || !p->nroot || !p->rtdis) return PIHM_GPU_ERR_ARG;
+  int layers = 0;
   for (int r = 0; r < ne; r++) {
     // HRT and SRT read the second layer: at least two
-    if (p->nsoil[r] < 2 || p->nsoil[r] > noah::L || p->nroot[r] < 1 || p->nroot[r] > p->nsoil[r])
+    if (p->nsoil[r] < 2 || p->nsoil[r] > noah::kMaxLayers || p->nroot[r] < 1 || p->nroot[r] > p->nsoil[r])
       return PIHM_GPU_ERR_ARG;
+    if (p->nsoil[r] > layers) layers = p->nsoil[r];
   }
   const double *params[] = {p->smcmax, p->smcmin, p->smcref, p->smcwlt, p->smcdry, p->quartz, p->csoil,
                             p->alpha, p->beta, p->ksatv, p->porosity, p->depth, p->area, p->shdfac,
@@ -351,7 +422,7 @@ int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_
       !s->cm || !s->snotime1 || !s->albedo || !s->emissi || !s->q1 || !s->ribb || !s->fcr)
     return PIHM_GPU_ERR_ARG;
   const size_t NE = ne;
-  const size_t bytes = NS_COUNT * padded<double>(NE) + NL_COUNT * padded<double>(noah::L * NE) +
+  const size_t bytes = NS_COUNT * padded<double>(NE) + NL_COUNT * padded<double>(noah::kMaxLayers * NE) +
                        NI_COUNT * padded<int32_t>(NE) + padded<int32_t>(NE) + padded<int32_t>(2 * kNoahClasses);
   NoahInstance n;
   if (cudaMalloc(&n.alloc, bytes) != cudaSuccess) return PIHM_GPU_ERR_NOMEM;
@@ -359,6 +430,7 @@ int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_
   n.tg = tg;
   n.ne = ne;
   n.first = 1;
+  n.layers = layers;
   if (cudaMemset(n.alloc, 0, bytes) != cudaSuccess) {
     noah_release(n);
     return PIHM_GPU_ERR_CUDA;
@@ -372,7 +444,7 @@ int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_
   }
   for (int k = 0; k < NL_COUNT; k++) {
     P.l[k] = (double *)cur;
-    cur += padded<double>(noah::L * NE);
+    cur += padded<double>(noah::kMaxLayers * NE);
   }
   for (int k = 0; k < NI_COUNT; k++) {
     P.i[k] = (int32_t *)cur;
@@ -384,10 +456,10 @@ int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_
   int rc = PIHM_GPU_OK;
   for (int k = 0; k < kParams && !rc; k++) rc = upload_scalar(perm, ne, params[k], P.s[k], st);
   // layer depths below the surface (DefSldpth, noah/lsm_func.c:152-156)
-  std::vector<double> zsoil((size_t)noah::L * ne, 0.0);
+  std::vector<double> zsoil((size_t)noah::kMaxLayers * ne, 0.0);
   for (int r = 0; r < ne; r++) {
-    const double *sl = p->sldpth + (size_t)noah::L * r;
-    double *z = zsoil.data() + (size_t)noah::L * r;
+    const double *sl = p->sldpth + (size_t)noah::kMaxLayers * r;
+    double *z = zsoil.data() + (size_t)noah::kMaxLayers * r;
     z[0] = -sl[0];
     for (int k = 1; k < p->nsoil[r]; k++) z[k] = -sl[k] + z[k - 1];
   }
@@ -427,9 +499,11 @@ int noah_launch_step(NoahInstance &n, double dt, unsigned int *err, cudaStream_t
   if (cudaMemsetAsync(n.P->cls, 0, sizeof(int32_t) * 2 * kNoahClasses, st) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
   k_noah_count<<<(n.ne + 255) / 256, 256, 0, st>>>(*n.P);
   k_noah_place<<<(n.ne + 255) / 256, 256, 0, st>>>(*n.P);
-  k_noah_step<<<(n.ne + kNoahBlock - 1) / kNoahBlock, kNoahBlock, 0, st>>>(*n.P, dt, err);
+  const int blocks = (n.ne + kNoahBlock - 1) / kNoahBlock;
+  if (n.layers <= 4) k_noah_step<4><<<blocks, kNoahBlock, 0, st>>>(*n.P, n.tg, dt, err);
+  else k_noah_step<L><<<blocks, kNoahBlock, 0, st>>>(*n.P, n.tg, dt, err);
   *launches += 3;
-  return cuda_rc(cudaGetLastError()) ?: launch_inputs(n, st, launches);
+  return cuda_rc(cudaGetLastError());
 }
 
 int noah_launch_begin(NoahInstance &n, const double *y0, cudaStream_t st, int64_t *launches) {
@@ -442,10 +516,12 @@ int noah_launch_begin(NoahInstance &n, const double *y0, cudaStream_t st, int64_
 
 int noah_launch_post(NoahInstance &n, const double *y, double dt, cudaStream_t st, int64_t *launches) {
   if (!n.alloc || !y || !(dt > 0.0)) return PIHM_GPU_ERR_ARG;
-  k_noah_post<<<(n.ne + kNoahBlock - 1) / kNoahBlock, kNoahBlock, 0, st>>>(*n.P, n.tg, y, dt, n.first);
+  const int blocks = (n.ne + kNoahBlock - 1) / kNoahBlock;
+  if (n.layers <= 4) k_noah_post<4><<<blocks, kNoahBlock, 0, st>>>(*n.P, n.tg, y, dt, n.first);
+  else k_noah_post<L><<<blocks, kNoahBlock, 0, st>>>(*n.P, n.tg, y, dt, n.first);
   n.first = 0;
   ++*launches;
-  return cuda_rc(cudaGetLastError()) ?: launch_inputs(n, st, launches);
+  return cuda_rc(cudaGetLastError());
 }
 
 int noah_get(NoahInstance &n, int field, const int32_t *perm, cudaStream_t st, double *out) {
@@ -455,11 +531,11 @@ int noah_get(NoahInstance &n, int field, const int32_t *perm, cudaStream_t st, d
   if (cudaStreamSynchronize(st) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
   static const int layer_of[] = {NL_SMC, NL_SH2O, NL_STC, NL_ET, NL_RUNOFF2_LYR, NL_SMFLXV};
   if (field < 6) {
-    std::vector<double> h((size_t)noah::L * ne);
+    std::vector<double> h((size_t)noah::kMaxLayers * ne);
     if (cudaMemcpy(h.data(), P.l[layer_of[field]], sizeof(double) * h.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
       return PIHM_GPU_ERR_CUDA;
-    for (int k = 0; k < noah::L; k++)
-      for (int i = 0; i < ne; i++) out[(size_t)noah::L * perm[i] + k] = h[(size_t)k * ne + i];
+    for (int k = 0; k < noah::kMaxLayers; k++)
+      for (int i = 0; i < ne; i++) out[(size_t)noah::kMaxLayers * perm[i] + k] = h[(size_t)k * ne + i];
     return PIHM_GPU_OK;
   }
   static const int scalar_of[] = {NS_T1, NS_CMC, NS_SNEQV, NS_SNOWH, NS_SNDENS, NS_CH, NS_CM, NS_ALBEDO,

@@ -223,6 +223,7 @@ struct NoahInstance {
   NoahTargets tg{};
   int ne = 0;
   int first = 1;
+  int layers = 0;  // the most soil layers a column has
 };
 // pihm_gpu_noah_init's work for any targets (perm[internal] = reference element)
 int noah_build(const pihm_noah_params *p, const pihm_noah_state *s, const int32_t *perm, int ne,
