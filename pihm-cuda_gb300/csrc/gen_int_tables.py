@@ -22,6 +22,8 @@ decimal.getcontext().prec = 60
 
 N = 1024
 LN2 = D(2).ln()
+# pi by Machin's formula, 16 atan(1/5) - 4 atan(1/239)
+PI = sum((D(-1) ** k / (2 * k + 1)) * (16 / D(5) ** (2 * k + 1) - 4 / D(239) ** (2 * k + 1)) for k in range(60))
 
 
 def rnd(v: D) -> int:
@@ -81,7 +83,10 @@ def main():
                 "kImCLog10": rnd(D(2).log10() * D(2) ** 64),
                 # log10(e) at scale 2^64, and 1/j at scale 2^62 for log1p's series
                 "kImLog10E": rnd(D(1).exp().log10() * D(2) ** 64),
-                **{f"kImInv{j}": rnd(D(2) ** 62 / j) for j in range(3, 12)}}
+                **{f"kImInv{j}": rnd(D(2) ** 62 / j) for j in range(3, 12)},
+                # pi / 2 at scale 2^62, and 1 / (2k (2k + 1)) at scale 2^64 for the sine's series
+                "kImHalfPi": rnd(PI / 2 * D(2) ** 62),
+                **{f"kImSin{k}": rnd(D(2) ** 64 / (2 * k * (2 * k + 1))) for k in range(1, 12)}}
     for k, v in consts.items():
         assert -(2 ** 63) <= v < 2 ** 63
         out.append(f"static constexpr int64_t {k} = {v}ll;")

@@ -339,6 +339,37 @@ PIHM_IM_FN bool log_near1_i(double x, bool ten, double &out) {
   return ok;
 }
 
+// cos x for 0 <= x < 3.15, as -sin(x - pi/2) in fixed point: the sine's
+// series to the 23rd power (the next term is below 2^-66), absolute error
+// below 2^-60.  Next to the zero at pi/2 that is more of the result than of a
+// cosine that is accurate relatively; a caller that adds it to one (the
+// soil-moisture factor 1 - cos) does not see the difference.
+PIHM_IM_FN bool cos_i(double x, double &out) {
+  const uint64_t xb = dbits(x);
+  const int ex = (int)(xb >> 52) - 1023;  // (a sign bit makes it large)
+  const uint64_t M = (xb & kFrac) | (1ull << 52);
+  const bool ok = ex <= 1 && (ex < 1 || M < 7093169413108531ull);  // 3.15
+  const uint64_t X = ex >= -10 ? M << ((10 + ex) & 63) : (ex > -73 ? M >> ((-10 - ex) & 63) : 0);  // x 2^62
+  const int64_t Y = (int64_t)(X - kImHalfPi);                      // y = x - pi/2 in units of 2^-62
+  const uint64_t z = (uint64_t)((unsigned __int128)((i128)Y * Y) >> 63);  // y^2 2^61
+  // sin y = y (1 - z/(2 3) (1 - z/(4 5) (1 - ...)))
+  const uint64_t f[11] = {kImSin11, kImSin10, kImSin9, kImSin8, kImSin7, kImSin6,
+                          kImSin5,  kImSin4,  kImSin3, kImSin2, kImSin1};
+  uint64_t p = 1ull << 62;
+#if defined(__CUDACC__)
+#pragma unroll
+#endif
+  for (int k = 0; k < 11; k++) p = (1ull << 62) - umulhi((uint64_t)(((unsigned __int128)p * z) >> 61), f[k]);
+  const int64_t S = (int64_t)(((i128)Y * (int64_t)p) >> 62);                // sin y 2^62
+  const uint64_t a = (uint64_t)(S < 0 ? -S : S);
+  const int c = clz64(a) & 63;
+  const uint64_t q = a << c;
+  const uint64_t mant = (q >> 11) + ((q >> 10) & 1u);
+  const uint64_t bits = ((uint64_t)(int64_t)(1023 - c) << 52) + mant;  // a 2^-62 = q 2^(1 - c - 63)
+  out = a == 0 ? 0.0 : bitsd((S < 0 ? 0ull : 1ull << 63) | bits);      // -sin
+  return ok;
+}
+
 // ---------------------------------------------------------------------------
 // Division and square root, correctly rounded (round to nearest even), on
 // the integer pipe.  A single-precision reciprocal (or reciprocal square

@@ -5,12 +5,13 @@
 //
 // Numerics.  This file is compiled without multiply-add contraction
 // (-fmad=false), so every product and sum rounds where the reference's C
-// rounds; divisions and square roots are IEEE.  exp, log and pow go through
-// the table-driven double-double routines of fp64_math.cuh (about 0.51 ulp,
-// almost always the correctly rounded value the C library returns too);
-// pow(x, 2) is x * x, the correctly rounded square; cos is CUDA's.  So the
-// step reproduces the reference's values to the last bit on nearly every
-// element, and within a few ulps of the affected terms elsewhere.
+// rounds; divisions and square roots are IEEE.  exp, log and pow are the
+// fixed-point functions of int_math.cuh (0.502 ulp, almost always the
+// correctly rounded value the C library returns too), cos there has an
+// absolute error of 2^-60 beside its rounding; pow(x, 2) is x * x, the
+// correctly rounded square.  So the step reproduces the reference's values to
+// the last bit on nearly every element, and within a few ulps of the affected
+// terms elsewhere.
 //
 // Work is split by what it depends on: k_land_station interpolates each
 // station's record and forms everything that depends on it alone (vapour
@@ -43,15 +44,29 @@ constexpr double kTSnow = -3.0, kTRain = 1.0, kT0 = 0.0;
 constexpr double kCp = 1004.0, kLvH2O = 2.501e6, kSigma = 5.67e-8, kRd = 287.04, kRv = 461.5;
 
 constexpr int kLandBlock = 256;
+constexpr int kStepBlock = 128;
 
+// The elementary functions and comparisons stay off the FP64 pipe, which was
+// 74 % busy with them; the FP64 versions, for arguments out of the ranges,
+// are out of line.
+static __device__ __noinline__ double exp_slow(double x) { return exp(x); }
+static __device__ __noinline__ double log_slow(double x) { return log(x); }
+static __device__ __noinline__ double cos_slow(double x) { return cos(x); }
 __device__ __forceinline__ double exp_l(double x) {
   double r;
-  return exp_dd_checked(x, 0.0, r) ? r : exp(x);
+  return im::exp_i(x, r) ? r : exp_slow(x);
 }
 __device__ __forceinline__ double log_l(double x) {
-  double sh, lo;
-  return log_dd_fast(x, sh, lo) ? sh + lo : log(x);
+  double r;
+  return im::log_i(x, kImCLn2, r) ? r : log_slow(x);
 }
+__device__ __forceinline__ double cos_l(double x) {
+  double r;
+  return im::cos_i(x, r) ? r : cos_slow(x);
+}
+__device__ __forceinline__ double at_least(double x, double c) { return cmp::lt_c(x, c) ? c : x; }  // c > 0
+__device__ __forceinline__ double at_most(double x, double c) { return cmp::gt_c(x, c) ? c : x; }   // c > 0
+__device__ __forceinline__ double not_neg(double x) { return cmp::lt0(x) ? 0.0 : x; }
 
 // IntrplForc's bisection (src/forcing.c:503-528): the knot `middle` with
 // T[middle-1] <= t <= T[middle], or -1.  The host has checked that t lies in
@@ -101,6 +116,8 @@ enum StationVal {
 // IntrplForc and the station-only sub-expressions of IntcpSnowEt
 // (src/is_sm_et.c:49-56, 70-77, 97-100, 149-150), in the reference's order.
 __global__ void k_land_station(LandDev L, int64_t t, int month) {
+  // the step's blocks may start now; they wait for this grid's end
+  asm volatile("griddepcontrol.launch_dependents;");
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
   if (k < L.nmeteo) {
@@ -138,7 +155,7 @@ __global__ void k_land_station(LandDev L, int64_t t, int month) {
     o[SV_GAMMAS] = gammas;
     o[SV_FRAC_SNOW] = frac_snow;
     o[SV_MELT] = melt;
-    o[SV_CGAMMA] = 4.0 * 0.7 * kSigma * kRd / kCp * pow_fast(tk, 4.0);
+    o[SV_CGAMMA] = 4.0 * 0.7 * kSigma * kRd / kCp * pow_any(tk, 4.0);
     o[SV_CDELTA] = kLvH2O * kLvH2O * 0.622 / kRv / kCp / (tk * tk);
   } else if (k < L.nmeteo + L.nlai) {
     const int s = k - L.nmeteo;
@@ -156,13 +173,34 @@ __global__ void __launch_bounds__(kLandBlock) k_land_month(LandDev L, int ne, in
   if (i >= ne) return;
   const double z0 = g_monthly_rl[(__ldg(&L.lc[i]) - 1) * 12 + month];
   const double zlvl = __ldg(&L.zlvl[i]);
-  L.ra_num[i] = log_l(zlvl / z0) * log_l(10.0 * zlvl / z0);
+  L.ra_num[i] = log_l(div_any(zlvl, z0)) * log_l(div_any(10.0 * zlvl, z0));
 }
 
-__global__ void __launch_bounds__(kLandBlock) k_land_step(LandDev L, const double *__restrict__ y, int ne,
-                                                          int month, double dt) {
-  const int i = blockIdx.x * kLandBlock + threadIdx.x;
+// Bound by the FP64 pipe (62 % busy: 125 additions and products a warp, 80 us
+// of the 130 for 400,000 elements; with the FP64 power, exponential, cosine
+// and comparisons 170, and 150 us).  128 x 8 per SM: 256-thread blocks ran 3.4
+// waves, and the time hardly depends on the warps in flight (4 to 10 blocks:
+// 133 to 129 us).
+__global__ void __launch_bounds__(kStepBlock, 8) k_land_step(LandDev L, const double *__restrict__ y, int ne,
+                                                             int month, double dt) {
+  const int i = blockIdx.x * kStepBlock + threadIdx.x;
   if (i >= ne) return;
+  // what no station value enters, before the wait for k_land_station: the
+  // soil-moisture factor of the soil evaporation
+  const double depth = __ldg(&L.depth[i]);
+  const double unsat = y[ne + i], gw = y[2 * ne + i];
+  double satn;
+  const double deficit = depth - gw;
+  if (cmp::lt_v(deficit, __ldg(&L.rzd[i]))) {
+    satn = 1.0;
+  } else {
+    const double r = div_any(unsat, deficit);
+    satn = cmp::gt_c(r, 1.0) ? 1.0 : (cmp::lt0(r) ? 0.0 : 0.5 * (1.0 - cos_l(3.14 * r)));
+  }
+  double betas = div_any(satn * __ldg(&L.porosity[i]) + __ldg(&L.smcmin[i]) - __ldg(&L.smcwlt[i]), __ldg(&L.dsmc[i]));
+  betas = at_most(at_least(betas, 0.0001), 1.0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
   const double *sv = L.station + (size_t)(__ldg(&L.meteo[i]) - 1) * kStationVals;
   const int lc = __ldg(&L.lc[i]) - 1;
   const int lt = __ldg(&L.lai_type[i]);
@@ -182,7 +220,7 @@ __global__ void __launch_bounds__(kLandBlock) k_land_step(LandDev L, const doubl
   double sneqv = L.sneqv[i];
   sneqv += frac_snow * prcp * dt;
   double melt_rate = sv[SV_MELT];
-  if (sneqv > melt_rate * dt) {
+  if (cmp::gt_v(sneqv, melt_rate * dt)) {
     sneqv -= melt_rate * dt;
   } else {
     melt_rate = div_any(sneqv, dt);
@@ -199,72 +237,61 @@ __global__ void __launch_bounds__(kLandBlock) k_land_step(LandDev L, const doubl
                              1000.0 * kLvH2O * (delta + gamma));
 
   // soil evaporation
-  const double depth = __ldg(&L.depth[i]);
-  const double unsat = y[ne + i], gw = y[2 * ne + i];
-  double satn;
-  if (depth - gw < __ldg(&L.rzd[i])) {
-    satn = 1.0;
-  } else {
-    const double r = div_any(unsat, depth - gw);
-    satn = (r > 1.0) ? 1.0 : ((r < 0.0) ? 0.0 : 0.5 * (1.0 - cos(3.14 * r)));
-  }
-  double betas = div_any(satn * __ldg(&L.porosity[i]) + __ldg(&L.smcmin[i]) - __ldg(&L.smcwlt[i]), __ldg(&L.dsmc[i]));
-  betas = (betas < 0.0001) ? 0.0001 : ((betas > 1.0) ? 1.0 : betas);
   double edir = (1.0 - shdfac) * (betas * betas) * etp;
   edir *= L.cal_edir;
-  edir = (edir < 0.0) ? 0.0 : edir;
+  edir = not_neg(edir);
 
   // canopy evaporation, transpiration and drip
   double cmc = L.cmc[i];
   double ec, ett, drip;
-  if (lai > 0.0) {
+  if (cmp::gt0(lai)) {
     const double cfactr = __ldg(&L.cfactr[i]);
-    const double cm = (cmc < 0.0) ? 0.0 : ((cmc > intcp_max) ? intcp_max : cmc);
+    const double cm = cmp::lt0(cmc) ? 0.0 : (cmp::gt_v(cmc, intcp_max) ? intcp_max : cmc);
     // ec divides the clamped storage by intcp_max; ett's expression divides
     // only the unclamped branch (src/is_sm_et.c:128-131, 164-168)
     const double base_ec = div_any(cm, intcp_max);
-    const double base_ett = (cmc < 0.0) ? 0.0 : base_ec;
-    const double pw_ec = pow_fast(base_ec, cfactr);
+    const double base_ett = cmp::lt0(cmc) ? 0.0 : base_ec;
+    const double pw_ec = pow_any(base_ec, cfactr);
     const double pw_ett = (__double_as_longlong(base_ett) == __double_as_longlong(base_ec)) ? pw_ec
-                                                                                           : pow_fast(base_ett, cfactr);
+                                                                                           : pow_any(base_ett, cfactr);
     ec = shdfac * pw_ec * etp;
     ec *= L.cal_ec;
-    ec = (ec < 0.0) ? 0.0 : ec;
+    ec = not_neg(ec);
 
     double fr = div_any(1.1 * radnet, __ldg(&L.rgl[i]) * lai);
-    fr = (fr < 0.0) ? 0.0 : fr;
+    fr = not_neg(fr);
     double alphar = div_any(1.0 + fr, fr + __ldg(&L.rs_ratio[i]));
-    alphar = (alphar > 10000.0) ? 10000.0 : alphar;
+    alphar = at_most(alphar, 10000.0);
     const double dtopt = __ldg(&L.topt_c[i]) - sfctmp;
     double etas = 1.0 - 0.0016 * (dtopt * dtopt);
-    etas = (etas < 0.0001) ? 0.0001 : etas;
+    etas = at_least(etas, 0.0001);
     const double gammas = sv[SV_GAMMAS];
     const double rsmax = __ldg(&L.rsmax[i]);
     double rs = div_any(__ldg(&L.rsmin[i]) * alphar, betas * lai * etas * gammas);
-    rs = (rs > rsmax) ? rsmax : rs;
+    rs = cmp::gt_v(rs, rsmax) ? rsmax : rs;
     const double dg = div_any(delta, gamma);  // the reference forms it twice
     const double pc = div_any(1.0 + dg, 1.0 + div_any(rs, ra) + dg);
     ett = shdfac * pc * (1.0 - pw_ett) * etp;
     ett *= L.cal_ett;
-    ett = (ett < 0.0) ? 0.0 : ett;
-    ett = ((gw < __ldg(&L.d_rzd[i])) && unsat <= 0.0) ? 0.0 : ett;
+    ett = not_neg(ett);
+    ett = (cmp::lt_v(gw, __ldg(&L.d_rzd[i])) && cmp::le0(unsat)) ? 0.0 : ett;
     // Rutter and Morton (1977): D0 = 6.52e-7 m s-1
-    drip = (cmc <= 0.0) ? 0.0 : 6.52E-7 * intcp_max * exp_l(div_any(3.89 * cmc, intcp_max));
+    drip = cmp::le0(cmc) ? 0.0 : 6.52E-7 * intcp_max * exp_l(div_any(3.89 * cmc, intcp_max));
   } else {
     ett = 0.0;
     ec = 0.0;
     drip = 0.0;
   }
-  if (drip < 0.0) drip = 0.0;
-  if (drip * dt > cmc) drip = div_any(cmc, dt);
+  drip = not_neg(drip);
+  if (cmp::gt_v(drip * dt, cmc)) drip = div_any(cmc, dt);
 
   const double isval = cmc + (1.0 - frac_snow) * prcp * shdfac * dt - ec * dt - drip * dt;
-  if (isval > intcp_max) {
+  if (cmp::gt_v(isval, intcp_max)) {
     cmc = intcp_max;
     drip += div_any(isval - intcp_max, dt);
-  } else if (isval < 0.0) {
+  } else if (cmp::lt0(isval)) {
     cmc = 0.0;
-    if (ec + drip > 0.0) {
+    if (cmp::gt0(ec + drip)) {
       ec = div_any(ec, ec + drip) * (cmc + (1.0 - frac_snow) * prcp * shdfac * dt);
       drip = div_any(drip, ec + drip) * (cmc + (1.0 - frac_snow) * prcp * shdfac * dt);
     }
@@ -503,9 +530,21 @@ int land_launch(LandInstance &li, int64_t t, double stepsize, const double *y_de
   }
   const int nser = li.L.nmeteo + li.L.nlai;
   k_land_station<<<(nser + 127) / 128, 128, 0, st>>>(li.L, t, tm.tm_mon);
-  k_land_step<<<grid, kLandBlock, 0, st>>>(li.L, y_dev, ne, tm.tm_mon, stepsize);
   *launches += 2;
-  return cuda_rc(cudaGetLastError());
+  if (cudaGetLastError() != cudaSuccess) return PIHM_GPU_ERR_CUDA;
+  // a programmatic dependent launch: the step's blocks start beside
+  // k_land_station (a chain of 8 us on one SM) and wait for it where they
+  // first need a station's values
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((ne + kStepBlock - 1) / kStepBlock));
+  cfg.blockDim = dim3(kStepBlock);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cuda_rc(cudaLaunchKernelEx(&cfg, k_land_step, li.L, y_dev, ne, (int)tm.tm_mon, stepsize));
 }
 
 void land_release(LandInstance &li) {

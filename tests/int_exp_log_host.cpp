@@ -18,4 +18,8 @@ void im_log(const double *x, double *out, int32_t *ok, int64_t n, int32_t ten) {
 void im_log_near1(const double *x, double *out, int32_t *ok, int64_t n, int32_t ten) {
   for (int64_t i = 0; i < n; i++) ok[i] = pihm::im::log_near1_i(x[i], ten != 0, out[i]) ? 1 : 0;
 }
+// cos x for 0 <= x < 3.15
+void im_cos(const double *x, double *out, int32_t *ok, int64_t n) {
+  for (int64_t i = 0; i < n; i++) ok[i] = pihm::im::cos_i(x[i], out[i]) ? 1 : 0;
+}
 }

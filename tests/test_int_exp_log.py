@@ -90,3 +90,28 @@ def test_logarithm_next_to_one(lib, ten):
             assert ulps(g, D(float(v)).log10() if ten else D(float(v)).ln()) < 0.502, v
     _, ok = call(lib.im_log_near1, [1.02, 0.98, 2.0, 0.5, 0.0, -1.0, np.inf, np.nan], ctypes.c_int32(ten))
     assert not ok.any()
+
+
+def cos_ref(x):
+    """cos x to 50 digits by its series."""
+    x = D(float(x))
+    term = s = D(1)
+    for k in range(1, 45):
+        term *= -x * x / ((2 * k - 1) * (2 * k))
+        s += term
+    return s
+
+
+def test_cosine(lib):
+    decimal.getcontext().prec = 60
+    rng = np.random.default_rng(6)
+    x = np.concatenate([3.14 * rng.uniform(0.0, 1.0, 1500), 2.0 ** rng.uniform(-80.0, 0.0, 300),
+                        np.pi / 2 + rng.uniform(-1e-3, 1e-3, 200), [0.0, 3.14, 3.1499]])
+    got, ok = call(lib.im_cos, x)
+    assert ok.all()
+    want = [cos_ref(v) for v in x]
+    # the absolute error 2^-60 beside the rounding of the result
+    for g, w in zip(got, want):
+        assert abs(D(float(g)) - w) <= D(math.ulp(float(w))) * D("0.5") + D(2) ** -60, float(w)
+    _, ok = call(lib.im_cos, [3.2, 4.0, -1.0, -1e-300, np.inf, np.nan])
+    assert not ok.any()
