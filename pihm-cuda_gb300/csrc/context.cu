@@ -9,6 +9,7 @@
 
 #include <type_traits>
 
+#include "host_flag.h"
 #include "mesh_image.h"
 #include "pihm_internal.h"
 
@@ -83,6 +84,8 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
   c->nan_check_deferred = 0;
   c->prof = nullptr;
   c->d_noah = nullptr;
+  c->h_status = nullptr;
+  c->status_seq = 0;
   c->host_path = 0;
   c->last_direct = 0;
   {
@@ -210,6 +213,12 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
   m.err = carve<unsigned int>(dp, 1);
   m.bar = carve<unsigned int>(dp, kBarWords);
   m.diag = 0;
+  if (cudaMallocHost((void **)&c->h_status, 2 * sizeof(uint64_t)) != cudaSuccess) {
+    c->h_status = nullptr;
+    pihm_gpu_destroy(c);
+    return PIHM_GPU_ERR_NOMEM;
+  }
+  c->h_status[0] = c->h_status[1] = 0;
   if (pihm::create_rhs_streams(&c->side) != cudaSuccess) {
     pihm_gpu_destroy(c);
     return PIHM_GPU_ERR_CUDA;
@@ -235,6 +244,7 @@ void pihm_gpu_destroy(pihm_gpu_ctx *c) {
   if (c->d_static) cudaFree(c->d_static);
   if (c->d_dyn) cudaFree(c->d_dyn);
   if (c->d_noah) cudaFree(c->d_noah);
+  if (c->h_status) cudaFreeHost(c->h_status);
   pihm::land_release(c->land);
   pihm::noah_release(c->noahlsm);
   if (c->side.fork) cudaEventDestroy(c->side.fork);
@@ -400,12 +410,19 @@ int pihm_gpu_rhs(pihm_gpu_ctx *c, double t, const double *y, double *ydot) {
   return cuda_fail(launch_rhs(c->m, y, ydot, c->stream, &c->launches, c->prof, &c->side));
 }
 
+// the error word to the host, behind everything queued on the stream
+__global__ static void k_status(const unsigned int *err, uint64_t *host, uint64_t seq) {
+  host[0] = *err;
+  pihm::host_flag_set(host + 1, seq);
+}
+
 int pihm_gpu_status(pihm_gpu_ctx *c) {
   if (!c) return PIHM_GPU_ERR_ARG;
-  unsigned int err = 0;
-  if (cudaMemcpyAsync(&err, c->m.err, sizeof(err), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
+  const uint64_t seq = ++c->status_seq;
+  k_status<<<1, 1, 0, c->stream>>>(c->m.err, c->h_status, seq);
+  if (cudaGetLastError() != cudaSuccess || !pihm::host_flag_wait(c->h_status + 1, seq, c->stream))
     return PIHM_GPU_ERR_CUDA;
-  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
+  const unsigned int err = (unsigned int)c->h_status[0];
   if (err) {
     cudaMemsetAsync(c->m.err, 0, sizeof(unsigned int), c->stream);
     // a launch whose waits ran out leaves its barrier counters as they were

@@ -21,7 +21,14 @@ __device__ __forceinline__ Pair red_identity() {
 
 template <int OP>
 __device__ __forceinline__ Pair red_combine(Pair p, Pair q) {
-  if (OP == R_MAXABS) return {fmax(p.v, q.v), 0.0};
+  if (OP == R_MAXABS) {
+    // fmax of values that are not negative (a NaN loses, as in fmax), by
+    // their bit patterns
+    const unsigned long long a = (unsigned long long)__double_as_longlong(p.v);
+    const unsigned long long b = (unsigned long long)__double_as_longlong(q.v);
+    const unsigned long long inf = 0x7FF0000000000000ull;
+    return {__longlong_as_double((long long)((a > inf || (b <= inf && b > a)) ? b : a)), 0.0};
+  }
   if (OP == R_MIN || OP == R_MINQ) return {fmin(p.v, q.v), fmax(p.f, q.f)};
   if (OP == R_INVTEST || OP == R_CONSTR) return {0.0, fmax(p.f, q.f)};
   return {__dadd_rn(p.v, q.v), 0.0};

@@ -23,6 +23,7 @@
 #include <map>
 #include <mutex>
 
+#include "host_flag.h"
 #include "pihm_nvector.h"
 #include "nv_ops.cuh"
 
@@ -35,13 +36,18 @@ struct Scratch {
   unsigned int *ticket = nullptr;
   double *result = nullptr;     // [2] value, flag
   double *slots = nullptr;      // [2 * PIHM_NV_SLOTS] value, flag per slot
-  double *host = nullptr;       // pinned [2 + 2 * PIHM_NV_SLOTS + 1]
+  // pinned, written by the kernels: [0..1] a reduction's value and flag, then
+  // the slots' values, a device word, and the sequence number of the last
+  // write (host_flag.h)
+  double *host = nullptr;
+  uint64_t seq = 0;
+  uint64_t *seq_word() const { return (uint64_t *)(host + 2 + PIHM_NV_SLOTS + 1); }
 };
 
 // Scratch layout: partial values [kMaxBlocks], partial flags [kMaxBlocks],
 // result [2], ticket, one spare, slots [2 * PIHM_NV_SLOTS].
 constexpr size_t kScratchDoubles = 2 * kMaxBlocks + 4 + 2 * PIHM_NV_SLOTS;
-constexpr size_t kHostDoubles = 2 + 2 * PIHM_NV_SLOTS + 1;
+constexpr size_t kHostDoubles = 2 + PIHM_NV_SLOTS + 2;
 
 static int scratch_alloc(Scratch &s) {
   void *p = nullptr;
@@ -53,6 +59,7 @@ static int scratch_alloc(Scratch &s) {
   s.slots = (double *)(c + sizeof(double) * (2 * kMaxBlocks + 4));
   if (cudaMemset(p, 0, sizeof(double) * kScratchDoubles) != cudaSuccess) return -1;
   if (cudaMallocHost(&s.host, sizeof(double) * kHostDoubles) != cudaSuccess) return -1;
+  std::memset(s.host, 0, sizeof(double) * kHostDoubles);
   return 0;
 }
 
@@ -147,7 +154,8 @@ __global__ void __launch_bounds__(kThreads) k_red(long long n, const double *__r
                                                   const double *__restrict__ y, double *__restrict__ z,
                                                   double *partials, double *partials_f,
                                                   unsigned int *ticket, double *result,
-                                                  long long wrms_n) {
+                                                  long long wrms_n, double *host, uint64_t *host_seq,
+                                                  uint64_t seq) {
   __shared__ Pair sh[kThreads / 32];
   __shared__ bool last;
   Pair acc = red_identity<OP>();
@@ -219,7 +227,22 @@ __global__ void __launch_bounds__(kThreads) k_red(long long n, const double *__r
     result[0] = wrms_n > 0 ? __dsqrt_rn(__ddiv_rn(v.v, (double)wrms_n)) : v.v;
     result[1] = v.f;
     *ticket = 0u;
+    if (host) {
+      host[0] = result[0];
+      host[1] = v.f;
+      pihm::host_flag_set(host_seq, seq);
+    }
   }
+}
+
+// slots 0..count-1 and a device word to the host
+__global__ void k_fetch(const double *slots, int count, const unsigned int *word, double *host, uint64_t *host_seq,
+                        uint64_t seq) {
+  if ((int)threadIdx.x < count) host[2 + threadIdx.x] = slots[2 * threadIdx.x];
+  if (threadIdx.x == 0 && word) *(unsigned int *)(host + 2 + PIHM_NV_SLOTS) = *word;
+  __threadfence_system();
+  __syncwarp();
+  if (threadIdx.x == 0) pihm::host_flag_set(host_seq, seq);
 }
 
 // z = a*x + b*y with a and b formed from device-resident slots: one thread
@@ -277,19 +300,20 @@ namespace pihm_nv {
 // carved from the caller's buffer), leave the result in result_dev[0..1].
 template <int OP>
 static int red_launch(long long n, const double *x, const double *y, double *z, double *partials,
-                      unsigned int *ticket, double *result_dev, cudaStream_t st, long long wrms_n = 0) {
+                      unsigned int *ticket, double *result_dev, cudaStream_t st, long long wrms_n = 0,
+                      double *host = nullptr, uint64_t *host_seq = nullptr, uint64_t seq = 0) {
   const unsigned g = red_grid_for(n);
-  k_red<OP><<<g, kThreads, 0, st>>>(n, x, y, z, partials, partials + kMaxBlocks, ticket, result_dev, wrms_n);
+  k_red<OP><<<g, kThreads, 0, st>>>(n, x, y, z, partials, partials + kMaxBlocks, ticket, result_dev, wrms_n,
+                                    host, host_seq, seq);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 template <int OP>
 static int red_family(Family *f, long long n, const double *x, const double *y, double *z, double out[2]) {
   Scratch &s = f->scratch;
-  if (red_launch<OP>(n, x, y, z, s.partials, s.ticket, s.result, f->stream)) return -2;
-  if (cudaMemcpyAsync(s.host, s.result, sizeof(double) * 2, cudaMemcpyDeviceToHost, f->stream) != cudaSuccess)
-    return -2;
-  if (cudaStreamSynchronize(f->stream) != cudaSuccess) return -2;
+  const uint64_t seq = ++s.seq;
+  if (red_launch<OP>(n, x, y, z, s.partials, s.ticket, s.result, f->stream, 0, s.host, s.seq_word(), seq)) return -2;
+  if (!pihm::host_flag_wait(s.seq_word(), seq, f->stream)) return -2;
   out[0] = s.host[0];
   out[1] = s.host[1];
   return 0;
@@ -561,16 +585,11 @@ int N_VFetchSlots_PihmGpu(N_Vector v, int count, double *out, const unsigned int
                           unsigned int *word_out) {
   if (!v || count < 0 || count > PIHM_NV_SLOTS || (count > 0 && !out) || (dev_word && !word_out)) return -1;
   Scratch &s = C(v)->fam->scratch;
-  double *h = s.host + 2;  // after the reductions' own result pair
-  if (count > 0 &&
-      cudaMemcpyAsync(h, s.slots, sizeof(double) * 2 * count, cudaMemcpyDeviceToHost, S(v)) != cudaSuccess)
-    return -2;
-  unsigned int *hw = (unsigned int *)(h + 2 * PIHM_NV_SLOTS);
-  if (dev_word && cudaMemcpyAsync(hw, dev_word, sizeof(unsigned int), cudaMemcpyDeviceToHost, S(v)) != cudaSuccess)
-    return -2;
-  if (cudaStreamSynchronize(S(v)) != cudaSuccess) return -2;
-  for (int i = 0; i < count; i++) out[i] = h[2 * i];
-  if (dev_word) *word_out = *hw;
+  const uint64_t seq = ++s.seq;
+  k_fetch<<<1, 32, 0, S(v)>>>(s.slots, count, dev_word, s.host, s.seq_word(), seq);
+  if (cudaGetLastError() != cudaSuccess || !pihm::host_flag_wait(s.seq_word(), seq, S(v))) return -2;
+  for (int i = 0; i < count; i++) out[i] = s.host[2 + i];
+  if (dev_word) *word_out = *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS);
   return 0;
 }
 

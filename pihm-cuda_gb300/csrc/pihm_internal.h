@@ -323,6 +323,8 @@ struct pihm_gpu_ctx {
   int host_path;                      // 0 direct where possible, 1 always copy
   int last_direct;                    // the last rhs_host accessed host memory directly
   int32_t *h_perm, *h_iperm;          // host copies (perm, inverse)
+  uint64_t *h_status;      // pinned [2]: the error word as k_status read it, and its sequence number
+  uint64_t status_seq;
   int diag;
   int nan_check_deferred;  // 1: pihm_gpu_ode does not synchronise to read the error word
   long long launches;      // kernels launched by this context so far
