@@ -2,14 +2,19 @@
 // bdf_core.h over any SUNDIALS 2.7 N_Vector, driven through the vector's own
 // operations table -- the device N_Vector of this library on the GPU, a host
 // serial vector in the tests -- with the right-hand side called through a
-// CVRhsFn.  Every operation completes when it is issued, so each call into
-// the integrator runs its coroutines straight through; the sequence of
-// vector operations and right-hand-side evaluations is the one CVODE makes
+// CVRhsFn.  Every operation completes when it is issued or waits in a queue
+// that is emptied before anything else can see its result (nv_queue.h), so
+// each call into the integrator runs its coroutines straight through; the
+// sequence of vector operations and right-hand-side evaluations is the one
+// CVODE makes
 // (and therefore so is the river-edge flux the PIHM right-hand side carries
 // from one evaluation to the next).
 #include <chrono>
+#include <cmath>
+#include <utility>
 
 #include "bdf_core.h"
+#include "nv_queue.h"
 #include "pihm_bdf.h"
 #include "pihm_gpu.h"
 #include "pihm_nvector.h"
@@ -62,70 +67,105 @@ struct NVectorOps {
   Vec slot_vec = nullptr;
   double host_slots[PIHM_NV_SLOTS] = {0};
 
+  // Device vectors' operations wait here for the next value that is read
+  // back, right-hand side or return to the caller (nv_queue.h).
+  pihm_nv::NvQueue queue;
+  void flush() { (void)queue.flush(); }
+
   Vec clone(Vec w) { return w->ops->nvclone(w); }
   void destroy(Vec v) {
+    flush();
     if (v) v->ops->nvdestroy(v);
   }
   bool valid(Vec v) const { return v != nullptr; }
 
   pihm::ReadyVoid linear_sum(double a, Vec x, double b, Vec y, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.linear_sum(a, x, b, y, z)) return {};
+    flush();
     z->ops->nvlinearsum(a, x, b, y, z);
     return {};
   }
   pihm::ReadyVoid const_(double c, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_CONST, c, 0, nullptr, nullptr, z)) return {};
+    flush();
     z->ops->nvconst(c, z);
     return {};
   }
   pihm::ReadyVoid scale(double c, Vec x, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.scale(c, x, z)) return {};
+    flush();
     z->ops->nvscale(c, x, z);
     return {};
   }
   pihm::ReadyVoid abs_(Vec x, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_ABS, 0, 0, x, nullptr, z)) return {};
+    flush();
     z->ops->nvabs(x, z);
     return {};
   }
   pihm::ReadyVoid inv(Vec x, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_INV, 0, 0, x, nullptr, z)) return {};
+    flush();
     z->ops->nvinv(x, z);
     return {};
   }
   pihm::ReadyVoid div(Vec x, Vec y, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_DIV, 0, 0, x, y, z)) return {};
+    flush();
     z->ops->nvdiv(x, y, z);
     return {};
   }
   pihm::ReadyVoid prod(Vec x, Vec y, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_PROD, 0, 0, x, y, z)) return {};
+    flush();
     z->ops->nvprod(x, y, z);
     return {};
   }
   pihm::ReadyVoid addconst(Vec x, double b, Vec z) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (queue.ew(pihm_nv::EW_ADDCONST, 0, b, x, nullptr, z)) return {};
+    flush();
     z->ops->nvaddconst(x, b, z);
     return {};
   }
   pihm::Ready<double> dot(Vec x, Vec y) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    double v;
+    if (queue.reduce(pihm_nv::R_DOT, x, y, &v)) return {v};
+    flush();
     return {x->ops->nvdotprod(x, y)};
   }
   pihm::Ready<double> maxnorm(Vec x) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    double v;
+    if (queue.reduce(pihm_nv::R_MAXABS, x, nullptr, &v)) return {v};
+    flush();
     return {x->ops->nvmaxnorm(x)};
   }
   pihm::Ready<double> wrms(Vec x, Vec w) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    double v;
+    if (queue.reduce(pihm_nv::R_WSQ, x, w, &v)) return {std::sqrt(v / (double)N_VGetLength_PihmGpu(x))};
+    flush();
     return {x->ops->nvwrmsnorm(x, w)};
   }
   pihm::Ready<double> vmin(Vec x) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    double v;
+    if (queue.reduce(pihm_nv::R_MIN, x, nullptr, &v)) return {v};
+    flush();
     return {x->ops->nvmin(x)};
   }
   pihm::Ready<int> rhs(double t, Vec y, Vec ydot) {
     Scope sc(timer, PIHM_BDF_OPT_RHS);
+    flush();
     return {f(t, y, ydot, user_data)};
   }
 
@@ -154,12 +194,16 @@ struct NVectorOps {
   }
   pihm::ReadyVoid dot_slot(Vec x, Vec y, int slot) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (mode == 2 && queue.reduce_slot(pihm_nv::R_DOT, x, y, slot)) return {};
+    flush();
     if (mode == 2) N_VDotProdSlot_PihmGpu(x, y, slot);
     else host_slots[slot] = x->ops->nvdotprod(x, y);
     return {};
   }
   pihm::ReadyVoid wrms_slot(Vec x, Vec w, int slot) {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
+    if (mode == 2 && queue.reduce_slot(pihm_nv::R_WSQ, x, w, slot)) return {};
+    flush();
     if (mode == 2) N_VWrmsNormSlot_PihmGpu(x, w, slot);
     else host_slots[slot] = x->ops->nvwrmsnorm(x, w);
     return {};
@@ -168,14 +212,18 @@ struct NVectorOps {
     Scope sc(timer, PIHM_BDF_OPT_ELEMENTWISE);
     if (mode == 2) {
       const pihm_nv_coef ca = {a.kind, a.slot, a.value}, cb = {b.kind, b.slot, b.value};
+      if (queue.linear_sum_coef(ca, x, cb, y, z)) return {};
+      flush();
       N_VLinearSumCoef_PihmGpu(&ca, x, &cb, y, z);
     } else {
+      flush();
       z->ops->nvlinearsum(host_coef_value(a), x, host_coef_value(b), y, z);
     }
     return {};
   }
   pihm::Ready<int> rhs_deferred(double t, Vec y, Vec ydot) {
     Scope sc(timer, PIHM_BDF_OPT_RHS);
+    flush();
     if (!rhs_deferrable) return {f(t, y, ydot, user_data)};
     const int rc = pihm_gpu_ode_launch(t, y, ydot, user_data);
     rhs_pending = rc == 0;
@@ -192,7 +240,12 @@ struct NVectorOps {
     const bool pending = rhs_pending;
     rhs_pending = false;
     const unsigned int *dev_word = pending ? pihm_gpu_error_word((pihm_gpu_ctx *)user_data) : nullptr;
-    if (N_VFetchSlots_PihmGpu(slot_vec, count, out, dev_word, &word) != 0) return {-1};
+    int rc = 0;
+    if (!queue.fetch(slot_vec, count, out, dev_word, &word, &rc)) {
+      flush();
+      rc = N_VFetchSlots_PihmGpu(slot_vec, count, out, dev_word, &word);
+    }
+    if (rc != 0) return {-1};
     if (word != 0) {
       (void)pihm_gpu_status((pihm_gpu_ctx *)user_data);  // reads and clears the word
       return {-1};
@@ -205,6 +258,13 @@ struct NVectorOps {
 
 struct pihm_bdf : pihm::bdf::BdfCore<NVectorOps> {};
 
+// A call into the integrator leaves nothing queued.
+static int run(pihm_bdf *m, pihm::Task<int> task) {
+  const int rc = pihm::run_sync(std::move(task));
+  m->ops.flush();
+  return rc;
+}
+
 extern "C" {
 
 pihm_bdf *pihm_bdf_create(void) { return new pihm_bdf(); }
@@ -213,12 +273,12 @@ int pihm_bdf_init(pihm_bdf *m, pihm_bdf_rhs_fn f, double t0, N_Vector y0) {
   if (!m || !f || !y0) return PIHM_BDF_ILL_INPUT;
   m->ops.f = f;
   m->ops.mode = -1;
-  return pihm::run_sync(m->init(t0, y0));
+  return run(m, m->init(t0, y0));
 }
 
 int pihm_bdf_reinit(pihm_bdf *m, double t0, N_Vector y0) {
   if (!m || !m->alloc_done || !y0) return PIHM_BDF_ILL_INPUT;
-  return pihm::run_sync(m->init(t0, y0));
+  return run(m, m->init(t0, y0));
 }
 
 int pihm_bdf_ss_tolerances(pihm_bdf *m, double reltol, double abstol) {
@@ -294,7 +354,7 @@ int pihm_bdf_set_stop_time(pihm_bdf *m, double tstop) {
 
 int pihm_bdf_solve(pihm_bdf *m, double tout, N_Vector yout, double *tret) {
   if (!m || !yout || !tret) return PIHM_BDF_ILL_INPUT;
-  return pihm::run_sync(m->solve(tout, yout, tret));
+  return run(m, m->solve(tout, yout, tret));
 }
 
 int pihm_bdf_get_stats(const pihm_bdf *m, pihm_bdf_stats *s) {

@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "host_flag.h"
+#include "nv_queue.h"
 #include "pihm_nvector.h"
 #include "nv_ops.cuh"
 
@@ -32,7 +33,7 @@ namespace pihm_nv {
 constexpr double kBigReal = DBL_MAX;
 
 struct Scratch {
-  double *partials = nullptr;   // [kMaxBlocks]
+  double *partials = nullptr;   // [kPartials]
   unsigned int *ticket = nullptr;
   double *result = nullptr;     // [2] value, flag
   double *slots = nullptr;      // [2 * PIHM_NV_SLOTS] value, flag per slot
@@ -44,9 +45,13 @@ struct Scratch {
   uint64_t *seq_word() const { return (uint64_t *)(host + 2 + PIHM_NV_SLOTS + 1); }
 };
 
-// Scratch layout: partial values [kMaxBlocks], partial flags [kMaxBlocks],
+// Scratch layout: partial values and flags (kMaxBlocks each, or the eight
+// warps of kSeqSpread blocks for two reductions of a sequence, nv_queue.h),
 // result [2], ticket, one spare, slots [2 * PIHM_NV_SLOTS].
-constexpr size_t kScratchDoubles = 2 * kMaxBlocks + 4 + 2 * PIHM_NV_SLOTS;
+constexpr int kSeqSpread = 128;
+constexpr size_t kPartials = 16 * kSeqSpread;
+static_assert(kPartials >= 2 * kMaxBlocks, "reduction partials");
+constexpr size_t kScratchDoubles = kPartials + 4 + 2 * PIHM_NV_SLOTS;
 constexpr size_t kHostDoubles = 2 + PIHM_NV_SLOTS + 2;
 
 static int scratch_alloc(Scratch &s) {
@@ -54,9 +59,9 @@ static int scratch_alloc(Scratch &s) {
   if (cudaMalloc(&p, sizeof(double) * kScratchDoubles) != cudaSuccess) return -1;
   char *c = (char *)p;
   s.partials = (double *)c;
-  s.result = (double *)(c + sizeof(double) * 2 * kMaxBlocks);
-  s.ticket = (unsigned int *)(c + sizeof(double) * (2 * kMaxBlocks + 2));
-  s.slots = (double *)(c + sizeof(double) * (2 * kMaxBlocks + 4));
+  s.result = (double *)(c + sizeof(double) * kPartials);
+  s.ticket = (unsigned int *)(c + sizeof(double) * (kPartials + 2));
+  s.slots = (double *)(c + sizeof(double) * (kPartials + 4));
   if (cudaMemset(p, 0, sizeof(double) * kScratchDoubles) != cudaSuccess) return -1;
   if (cudaMallocHost(&s.host, sizeof(double) * kHostDoubles) != cudaSuccess) return -1;
   std::memset(s.host, 0, sizeof(double) * kHostDoubles);
@@ -317,6 +322,314 @@ static int red_family(Family *f, long long n, const double *x, const double *y, 
   out[0] = s.host[0];
   out[1] = s.host[1];
   return 0;
+}
+
+// ---------------------------------------------------------------------------
+// sequences: element-wise operations and the reduction that ends them
+// ---------------------------------------------------------------------------
+// r = OP(a, b, x, y, z) for a run-time operation code
+template <int U>
+__device__ __forceinline__ void seq_eval(int op, double a, double b, const double (&x)[U], const double (&y)[U],
+                                         const double (&z)[U], double (&r)[U]) {
+#define PIHM_SEQ_CASE(OP)                                                  \
+  case OP:                                                                 \
+    _Pragma("unroll") for (int u = 0; u < U; u++) r[u] = ew_eval<OP>(a, b, x[u], y[u], z[u]); \
+    break;
+  switch (op) {
+    PIHM_SEQ_CASE(EW_LIN)
+    PIHM_SEQ_CASE(EW_LIN1)
+    PIHM_SEQ_CASE(EW_LIN2)
+    PIHM_SEQ_CASE(EW_SUM)
+    PIHM_SEQ_CASE(EW_DIFF)
+    PIHM_SEQ_CASE(EW_SCALESUM)
+    PIHM_SEQ_CASE(EW_SCALEDIFF)
+    PIHM_SEQ_CASE(EW_AXPY)
+    PIHM_SEQ_CASE(EW_AXPY1)
+    PIHM_SEQ_CASE(EW_AXPYM1)
+    PIHM_SEQ_CASE(EW_CONST)
+    PIHM_SEQ_CASE(EW_PROD)
+    PIHM_SEQ_CASE(EW_DIV)
+    PIHM_SEQ_CASE(EW_SCALE)
+    PIHM_SEQ_CASE(EW_COPY)
+    PIHM_SEQ_CASE(EW_NEG)
+    PIHM_SEQ_CASE(EW_ABS)
+    PIHM_SEQ_CASE(EW_INV)
+    PIHM_SEQ_CASE(EW_ADDCONST)
+    default: break;
+  }
+#undef PIHM_SEQ_CASE
+}
+
+// An operation as a block runs it: coefficients from slots resolved.
+struct SeqHead {
+  double a, b;
+  const double *x, *y;
+  double *z;
+  int op, fwd;
+};
+
+template <int U>
+__device__ __forceinline__ void seq_load(const SeqHead &h, const long long (&i)[U], const bool (&on)[U],
+                                         const double (&prev)[U], double (&x)[U], double (&y)[U], double (&z)[U]) {
+  const bool lx = ew_reads_x(h.op) && !(h.fwd & SEQ_X), ly = ew_reads_y(h.op) && !(h.fwd & SEQ_Y),
+             lz = ew_reads_z(h.op) && !(h.fwd & SEQ_Z);
+  __builtin_assume(__isGlobal(h.x));
+  __builtin_assume(__isGlobal(h.y));
+  __builtin_assume(__isGlobal(h.z));
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    x[u] = lx && on[u] ? h.x[i[u]] : prev[u];
+    y[u] = ly && on[u] ? h.y[i[u]] : prev[u];
+    z[u] = lz && on[u] ? h.z[i[u]] : prev[u];
+  }
+}
+
+// p combined with the identity, as the first step of a sum or of a tree over
+// fewer values than lanes: of the sums only -0 changes.
+template <int RED>
+__device__ __forceinline__ Pair red_first(Pair p) {
+  if (RED == R_DOT || RED == R_WSQ) {
+    const long long b = __double_as_longlong(p.v);
+    return {__longlong_as_double(b == (long long)0x8000000000000000ull ? 0 : b), 0.0};
+  }
+  return red_combine<RED>(red_identity<RED>(), p);
+}
+
+// The shuffle tree of one warp, and the tree over a block's eight warp
+// values, as red_block makes them.
+template <int RED>
+__device__ __forceinline__ double warp_tree(double x) {
+  Pair v = {x, 0.0};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const Pair q = {__shfl_down_sync(0xffffffffu, v.v, o), 0.0};
+    v = red_combine<RED>(v, q);
+  }
+  return v.v;
+}
+template <int RED>
+__device__ __forceinline__ double eight_tree(const volatile double *w) {
+  Pair v[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) v[k] = red_first<RED>({w[k], 0.0});
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; k++) v[k] = red_combine<RED>(v[k], v[k + o]);
+  return v[0].v;
+}
+
+// One reduction over the blocks of k_seq; r picks the shared and global
+// words.  kSpread: `part` has a value per warp of the reduction order.
+template <int RED, bool kSpread, int kT>
+__device__ __forceinline__ void seq_tail_block(double acc, int vwarp, bool writer, double *part, double *sh) {
+  const double v = warp_tree<RED>(acc);
+  if (writer) {
+    if (kSpread) part[vwarp] = v;
+    else sh[threadIdx.x >> 5] = v;
+  }
+}
+template <int RED, bool kSpread, int kT>
+__device__ __forceinline__ void seq_tail_last(int nblk, const double *part, double *sh) {
+  const int lane = threadIdx.x & 31;
+  for (int vw = threadIdx.x >> 5; vw < 8; vw += kT / 32) {
+    double v = red_identity<RED>().v;
+    if (vw * 32 < nblk) {
+      for (int b = vw * 32 + lane, k = 0; b < nblk; b += kThreads, k++) {
+        const Pair t = {kSpread ? eight_tree<RED>(part + 8 * b) : ((const volatile double *)part)[b], 0.0};
+        v = k == 0 ? red_first<RED>(t).v : red_combine<RED>({v, 0.0}, t).v;
+      }
+      v = warp_tree<RED>(v);
+    }
+    if (lane == 0) sh[vw] = v;
+  }
+}
+
+// A sequence over a vector: element-wise operations in order, then nothing
+// (RA < 0), one reduction (RA) or two (RA, RB).  An operation on a vector the
+// one before wrote takes the value from registers, and a result that is
+// overwritten unread is not stored.
+//
+// What it saves: a separate kernel costs about 4 us an operation in front of
+// a reduction (four operations and a dot product over 6,200 entries: 27.4 us
+// until the value is on the host, 12.9 here; a dot product alone 11.5, an
+// empty kernel 7.0), and each passes over the vectors.
+//
+// kSpread (short vectors, one pass): a warp has one FP64 instruction in
+// flight, 69 clocks, whatever its threads do beside it, and an SM takes one
+// every 20, so work is spread over warps rather than over a thread's
+// registers.  The four entries a thread of the reduction order accumulates go
+// to four warps of a block, one per scheduler, and a block carries one warp
+// of that order, whose tree's value it leaves in partials[8 * block + warp];
+// the last block finishes the trees of the order's blocks.  Eight linear sums
+// and a dot product over 6,200 entries: 13.7 us, with four entries a thread
+// 18.0.  Long vectors fill the SMs with four entries a thread (k_red's
+// layout) and are bound by the FP64 pipe; the spread form's tail grows with
+// the blocks (eight operations and a dot product, spread / four a thread:
+// 17.4 / 21.5 us over 90,000 entries, 22.3 / 21.3 over 150,000).
+template <int RA, int RB, bool kSpread, int kT>
+__global__ void __launch_bounds__(kT, 4) k_seq(const __grid_constant__ Seq q) {
+  constexpr int R0 = RA < 0 ? 0 : RA, R1 = RB < 0 ? 0 : RB, U = kSpread ? 1 : 4;
+  __shared__ SeqHead s_op[kSeqOps];
+  __shared__ double sh[2][8];
+  __shared__ double s_term[kSpread ? 2 : 1][kSpread ? kT : 1];
+  __shared__ bool last;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const long long n = q.n;
+  const int nblk = (int)red_grid_for(n);
+  const long long stride = (long long)nblk * kThreads;
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+  if (tid < q.nops) {
+    const SeqOp &o = q.op[tid];
+    SeqHead h = {o.a, o.b, o.x, o.y, o.z, o.code, o.fwd};
+    if (o.code == EW_COUNT) {
+      const double a = coef_value(o.ka, o.a, o.ka == COEF_HOST ? 0.0 : q.slots[2 * o.sa]);
+      const double b = coef_value(o.kb, o.b, o.kb == COEF_HOST ? 0.0 : q.slots[2 * o.sb]);
+      const EwCall<int> c = select_linear_sum<int>(a, 0, b, 1, o.ztag);
+      const int fx = (o.fwd & SEQ_X) ? 1 : 0, fy = (o.fwd & SEQ_Y) ? 1 : 0;
+      h.op = c.op;
+      h.a = c.a;
+      h.b = c.b;
+      h.x = c.x == 0 ? o.x : o.y;
+      h.y = c.y == 0 ? o.x : o.y;
+      h.fwd = (o.fwd & (SEQ_Z | SEQ_DEAD)) | ((c.x == 0 ? fx : fy) ? SEQ_X : 0) | ((c.y == 0 ? fx : fy) ? SEQ_Y : 0);
+    }
+    s_op[tid] = h;
+  }
+  __syncthreads();
+  Pair acc[2] = {red_identity<R0>(), red_identity<R1>()};
+  const int nops = q.nops;
+  const int vwarp = kSpread ? blockIdx.x : blockIdx.x * (kT / 32) + wid;
+  for (long long i0 = (long long)vwarp * 32 + lane + (kSpread ? wid * stride : 0); i0 < n; i0 += 4 * stride) {
+    double prev[U], x[U], y[U], z[U];
+    long long i[U];
+    bool on[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      prev[u] = 0.0;
+      i[u] = i0 + u * stride;
+      on[u] = i[u] < n;
+    }
+    for (int p = 0; p < nops; p++) {
+      const SeqHead h = s_op[p];
+      seq_load<U>(h, i, on, prev, x, y, z);
+      seq_eval<U>(h.op, h.a, h.b, x, y, z, prev);
+      if (!(h.fwd & SEQ_DEAD)) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (on[u]) h.z[i[u]] = prev[u];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < (RA < 0 ? 0 : (RB < 0 ? 1 : 2)); r++) {
+      const SeqRed &d = q.red[r];
+      const bool two = (r == 0 ? R0 : R1) == R_DOT || (r == 0 ? R0 : R1) == R_WSQ;
+      Pair t[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        x[u] = (d.fwd & SEQ_X) || !on[u] ? prev[u] : d.x[i[u]];
+        y[u] = !two ? 0.0 : ((d.fwd & SEQ_Y) || !on[u] ? prev[u] : d.y[i[u]]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) t[u] = r == 0 ? red_term<R0>(x[u], y[u]) : red_term<R1>(x[u], y[u]);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (kSpread) s_term[r][tid] = t[u].v;
+        else if (on[u]) acc[r] = r == 0 ? red_combine<R0>(acc[r], t[u]) : red_combine<R1>(acc[r], t[u]);
+      }
+    }
+  }
+  if (RA < 0) return;
+
+  double *part[2] = {q.partials, q.partials + (kSpread ? 8 * kSeqSpread : kMaxBlocks)};
+  if (kSpread) {
+    __syncthreads();
+    // the second reduction's warps follow the first's
+    const int r = wid;
+    if (wid < (RB < 0 ? 1 : 2)) {
+      const long long i0 = (long long)vwarp * 32 + lane;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (i0 + u * stride < n) {
+          const Pair t = {s_term[RB < 0 ? 0 : r][u * 32 + lane], 0.0};
+          if (u == 0) acc[0] = r == 0 ? red_first<R0>(t) : red_first<R1>(t);
+          else acc[0] = r == 0 ? red_combine<R0>(acc[0], t) : red_combine<R1>(acc[0], t);
+        }
+      if (r == 0) seq_tail_block<R0, true, kT>(acc[0].v, vwarp, lane == 0, part[0], sh[0]);
+      else seq_tail_block<R1, true, kT>(i0 < n ? acc[0].v : red_identity<R1>().v, vwarp, lane == 0, part[1], sh[1]);
+    }
+  } else {
+    seq_tail_block<R0, false, kT>(acc[0].v, vwarp, lane == 0, part[0], sh[0]);
+    if (RB >= 0) seq_tail_block<R1, false, kT>(acc[1].v, vwarp, lane == 0, part[1], sh[1]);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    if (!kSpread) {
+      part[0][blockIdx.x] = eight_tree<R0>(sh[0]);
+      if (RB >= 0) part[1][blockIdx.x] = eight_tree<R1>(sh[1]);
+      __threadfence();
+    }
+    last = atomicAdd(q.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // the last block combines the blocks' values in a fixed order
+  seq_tail_last<R0, kSpread, kT>(nblk, part[0], sh[0]);
+  if (RB >= 0) seq_tail_last<R1, kSpread, kT>(nblk, part[1], sh[1]);
+  __syncthreads();
+  if (wid == 0 && lane < (RB < 0 ? 1 : 2)) {
+    const SeqRed &d = q.red[lane];
+    double v = lane == 0 ? eight_tree<R0>(sh[0]) : eight_tree<R1>(sh[1]);
+    // the WRMS norm itself, sqrt(sum / n), as N_VWrmsNorm forms it
+    if (d.wrms_n > 0) v = __dsqrt_rn(__ddiv_rn(v, (double)d.wrms_n));
+    d.out[0] = v;
+    d.out[1] = 0.0;
+    if (q.host_seq && q.fetch < 0) q.host[lane] = v;
+  }
+  if (tid == 0) *q.ticket = 0u;
+  if (q.host_seq == nullptr) return;
+  __syncthreads();
+  for (int k = tid; k < q.fetch; k += kT) q.host[2 + k] = ((const volatile double *)q.slots)[2 * k];
+  if (tid == 0 && q.word) *(unsigned int *)(q.host + 2 + PIHM_NV_SLOTS) = *q.word;
+  __threadfence_system();
+  __syncthreads();
+  if (tid == 0) pihm::host_flag_set(q.host_seq, q.seq);
+}
+
+template <int RA, int RB, bool kSpread, int kT>
+static int seq_launch_t(const Seq &q, unsigned grid, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kT);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k_seq<RA, RB, kSpread, kT>, q) == cudaSuccess) return 0;
+  (void)cudaGetLastError();
+  return -2;
+}
+
+template <int RA, int RB>
+static int seq_launch_r(const Seq &q, cudaStream_t st) {
+  // 131,072 entries and fewer spread: see k_seq
+  const unsigned g = red_grid_for(q.n);
+  if (g <= kSeqSpread) return seq_launch_t<RA, RB, true, 128>(q, g * (kThreads / 32), st);
+  return seq_launch_t<RA, RB, false, kThreads>(q, g, st);
+}
+
+static int seq_launch(const Seq &q, cudaStream_t st) {
+  switch (q.nred ? q.red[0].op : -1) {
+    case R_DOT: return q.nred == 2 ? seq_launch_r<R_DOT, R_DOT>(q, st) : seq_launch_r<R_DOT, -1>(q, st);
+    case R_WSQ: return seq_launch_r<R_WSQ, -1>(q, st);
+    case R_MAXABS: return seq_launch_r<R_MAXABS, -1>(q, st);
+    case R_MIN: return q.nred == 2 ? seq_launch_r<R_MIN, R_WSQ>(q, st) : seq_launch_r<R_MIN, -1>(q, st);
+    default: return seq_launch_r<-1, -1>(q, st);
+  }
 }
 
 }  // namespace pihm_nv
@@ -638,3 +951,164 @@ int pihm_gpu_nv_dot_prod(const double *x, const double *y, int64_t n, void *stre
 }
 
 }  // extern "C"
+
+// ---------------------------------------------------------------------------
+// the queue (nv_queue.h)
+// ---------------------------------------------------------------------------
+namespace pihm_nv {
+
+// whether the vectors (null: not an operand) are the queue's, adopting z's
+// family and length when nothing is queued
+bool NvQueue::take(N_Vector z, N_Vector x, N_Vector y) {
+  if (z->ops->nvgetvectorid != N_VGetVectorID_PihmGpu || L(z) <= 0) return false;
+  if (empty()) {
+    fam = C(z)->fam;
+    q.n = L(z);
+  }
+  for (N_Vector v : {z, x, y})
+    if (v && (v->ops->nvgetvectorid != N_VGetVectorID_PihmGpu || C(v)->fam != fam || L(v) != q.n)) return false;
+  return true;
+}
+
+void NvQueue::push(const SeqOp &o) {
+  if (q.nred > 0 || q.nops == kSeqOps) {
+    flush();
+  }
+  SeqOp &d = q.op[q.nops];
+  d = o;
+  if (q.nops > 0) {
+    const double *pz = q.op[q.nops - 1].z;
+    d.fwd = (uint8_t)((o.x == pz ? SEQ_X : 0) | (o.y == pz ? SEQ_Y : 0) | (o.z == pz ? SEQ_Z : 0));
+  }
+  q.nops++;
+}
+
+void NvQueue::push_red(const SeqRed &r) {
+  if (q.nred == 2 || (q.nred == 1 && !(r.op == R_DOT && q.red[0].op == R_DOT))) {
+    flush();
+  }
+  SeqRed &d = q.red[q.nred++];
+  d = r;
+  if (q.nops > 0) {
+    const double *pz = q.op[q.nops - 1].z;
+    d.fwd = (uint8_t)((r.x == pz ? SEQ_X : 0) | (r.y == pz ? SEQ_Y : 0));
+  }
+}
+
+int NvQueue::launch() {
+  // results that nothing reads before they are overwritten
+  for (int p = 0; p < q.nops; p++) {
+    const double *z = q.op[p].z;
+    for (int r = p + 1; r < q.nops; r++) {
+      const SeqOp &o = q.op[r];
+      const bool sum = o.code == EW_COUNT, prev = r == p + 1;
+      if (!prev && (((sum || ew_reads_x(o.code)) && o.x == z) || ((sum || ew_reads_y(o.code)) && o.y == z) ||
+                    ((sum || ew_reads_z(o.code)) && o.z == z)))
+        break;
+      if (o.z == z) {
+        q.op[p].fwd |= SEQ_DEAD;
+        break;
+      }
+    }
+  }
+  q.partials = fam->scratch.partials;
+  q.slots = fam->scratch.slots;
+  q.ticket = fam->scratch.ticket;
+  const int r = seq_launch(q, fam->stream);
+  q.nops = q.nred = 0;
+  return r;
+}
+
+int NvQueue::flush() {
+  if (empty()) return 0;
+  q.host_seq = nullptr;
+  q.fetch = -1;
+  return launch();
+}
+
+bool NvQueue::linear_sum(double a, N_Vector x, double b, N_Vector y, N_Vector z) {
+  if (z->ops->nvlinearsum != N_VLinearSum_PihmGpu || !take(z, x, y)) return false;
+  const EwCall<const double *> c = select_linear_sum<const double *>(a, D(x), b, D(y), D(z));
+  push({c.x, c.y, D(z), c.a, c.b, (uint8_t)c.op});
+  return true;
+}
+
+bool NvQueue::linear_sum_coef(const pihm_nv_coef &a, N_Vector x, const pihm_nv_coef &b, N_Vector y, N_Vector z) {
+  if (a.kind == PIHM_NV_COEF_HOST && b.kind == PIHM_NV_COEF_HOST) return linear_sum(a.value, x, b.value, y, z);
+  if (!take(z, x, y)) return false;
+  const uint8_t ztag = D(z) == D(x) ? 0 : (D(z) == D(y) ? 1 : 2);
+  push({D(x), D(y), D(z), a.value, b.value, EW_COUNT, 0, (uint8_t)a.kind, (uint8_t)a.slot, (uint8_t)b.kind,
+        (uint8_t)b.slot, ztag});
+  return true;
+}
+
+bool NvQueue::scale(double c, N_Vector x, N_Vector z) {
+  if (z->ops->nvscale != N_VScale_PihmGpu || !take(z, x, nullptr)) return false;
+  const EwCall<const double *> e = select_scale<const double *>(c, D(x), D(z));
+  push({e.x, e.x, D(z), e.a, e.b, (uint8_t)e.op});
+  return true;
+}
+
+bool NvQueue::ew(int op, double a, double b, N_Vector x, N_Vector y, N_Vector z) {
+  const _generic_N_Vector_Ops *o = z->ops;
+  bool own = false;
+  switch (op) {
+    case EW_CONST: own = o->nvconst == N_VConst_PihmGpu; break;
+    case EW_ABS: own = o->nvabs == N_VAbs_PihmGpu; break;
+    case EW_INV: own = o->nvinv == N_VInv_PihmGpu; break;
+    case EW_DIV: own = o->nvdiv == N_VDiv_PihmGpu; break;
+    case EW_PROD: own = o->nvprod == N_VProd_PihmGpu; break;
+    case EW_ADDCONST: own = o->nvaddconst == N_VAddConst_PihmGpu; break;
+    default: break;
+  }
+  if (!own || !take(z, x, y)) return false;
+  push({x ? D(x) : nullptr, y ? D(y) : nullptr, D(z), a, b, (uint8_t)op});
+  return true;
+}
+
+bool NvQueue::reduce(int op, N_Vector x, N_Vector y, double *value) {
+  const _generic_N_Vector_Ops *o = x->ops;
+  const bool own = op == R_DOT      ? o->nvdotprod == N_VDotProd_PihmGpu
+                   : op == R_WSQ    ? o->nvwrmsnorm == N_VWrmsNorm_PihmGpu
+                   : op == R_MAXABS ? o->nvmaxnorm == N_VMaxNorm_PihmGpu
+                                    : o->nvmin == N_VMin_PihmGpu;
+  // with nothing queued the vector's own kernel is the shorter one
+  if (!own || empty() || !take(x, y, nullptr)) return false;
+  if (q.nred > 0) {  // its value is the first one's
+    flush();
+  }
+  Scratch &s = fam->scratch;
+  push_red({D(x), y ? D(y) : nullptr, s.result, 0, op, 0});
+  q.host = s.host;
+  q.host_seq = s.seq_word();
+  q.seq = ++s.seq;
+  q.fetch = -1;
+  const bool ok = launch() == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  *value = ok ? s.host[0] : NAN;
+  return true;
+}
+
+bool NvQueue::reduce_slot(int op, N_Vector x, N_Vector y, int slot) {
+  if (slot < 0 || slot >= PIHM_NV_SLOTS || !take(x, y, nullptr)) return false;
+  push_red({D(x), D(y), fam->scratch.slots + 2 * slot, op == R_WSQ ? q.n : 0, op, 0});
+  return true;
+}
+
+bool NvQueue::fetch(N_Vector v, int count, double *out, const unsigned int *dev_word, unsigned int *word_out,
+                    int *rc) {
+  if (q.nred == 0 || count < 0 || count > PIHM_NV_SLOTS || !take(v, nullptr, nullptr)) return false;
+  Scratch &s = fam->scratch;
+  q.host = s.host;
+  q.host_seq = s.seq_word();
+  q.seq = ++s.seq;
+  q.fetch = count;
+  q.word = dev_word;
+  *rc = -2;
+  if (launch() || !pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream)) return true;
+  for (int i = 0; i < count; i++) out[i] = s.host[2 + i];
+  if (dev_word) *word_out = *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS);
+  *rc = 0;
+  return true;
+}
+
+}  // namespace pihm_nv
