@@ -17,6 +17,7 @@
 #include "nv_queue.h"
 #include "pihm_bdf.h"
 #include "pihm_gpu.h"
+#include "pihm_internal.h"
 #include "pihm_nvector.h"
 
 namespace {
@@ -64,6 +65,7 @@ struct NVectorOps {
   int mode = -1;
   bool rhs_deferrable = false;  // the right-hand side's status joins the slot read-back
   bool rhs_pending = false;
+  bool rhs_bad = false;
   Vec slot_vec = nullptr;
   double host_slots[PIHM_NV_SLOTS] = {0};
 
@@ -167,6 +169,41 @@ struct NVectorOps {
     Scope sc(timer, PIHM_BDF_OPT_RHS);
     flush();
     return {f(t, y, ydot, user_data)};
+  }
+
+  // ---- two values of one pass (bdf_core.h) ----
+  bool joined(Vec v) const { return queue.accepts(v); }
+  // the minimum of m, and the WRMS norm of x by w
+  pihm::Ready<std::pair<double, double>> min_wrms(Vec m, Vec x, Vec w) {
+    Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    double mn, sum;
+    if (queue.min_wsq(m, x, w, &mn, &sum, nullptr, nullptr))
+      return {{mn, std::sqrt(sum / (double)N_VGetLength_PihmGpu(x))}};
+    flush();
+    mn = m->ops->nvmin(m);
+    return {{mn, x->ops->nvwrmsnorm(x, w)}};
+  }
+  // the WRMS norm of x by w and its sum of squares (NAN: not known), with the status of a
+  // right-hand side left pending (rhs_failed)
+  pihm::Ready<std::pair<double, double>> wrms_sum(Vec x, Vec w) {
+    Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
+    unsigned int word = 0;
+    const unsigned int *dev_word = rhs_pending ? pihm_gpu_error_word((pihm_gpu_ctx *)user_data) : nullptr;
+    rhs_pending = false;
+    double sum = NAN;
+    if (!queue.min_wsq(nullptr, x, w, nullptr, &sum, dev_word, &word)) {
+      flush();
+      rhs_bad = dev_word && pihm_gpu_status((pihm_gpu_ctx *)user_data) != PIHM_GPU_OK;
+      return {{x->ops->nvwrmsnorm(x, w), NAN}};
+    }
+    rhs_bad = word != 0;
+    if (rhs_bad) (void)pihm_gpu_status((pihm_gpu_ctx *)user_data);  // reads and clears the word
+    return {{std::sqrt(sum / (double)N_VGetLength_PihmGpu(x)), sum}};
+  }
+  bool rhs_failed() const { return rhs_bad; }
+  // a Newton iteration's right-hand side may leave its status to wrms_sum
+  bool rhs_status_joins(Vec v) const {
+    return rhs_deferrable && joined(v) && !((const pihm_gpu_ctx *)user_data)->nan_check_deferred;
   }
 
   // ---- device-resident GMRES scalars (bdf_core.h atimes_gs_deferred) ----

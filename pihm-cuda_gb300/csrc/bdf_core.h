@@ -212,6 +212,31 @@ struct BdfCore {
   }
 
   // ---------------------------------------------------------------- weights
+  // Ops that can give two values of one pass: `joined` says whether they do
+  // for these vectors.
+  static constexpr bool kJoinedOps = requires(Ops &o, Vec v) { o.joined(v); };
+  bool joined(Vec v) {
+    if constexpr (kJoinedOps) return ops.joined(v);
+    else return false;
+  }
+
+  // ewt_set of zn[0] and the WRMS norm of zn[0] by the new weights together.
+  // The weights are formed before the minimum is known to be positive: a
+  // failure leaves infinite ones, and every use of them is behind the next
+  // call's own ewt_set.
+  Task<int> ewt_set_norm(double *nrm) {
+    if constexpr (kJoinedOps) {
+      co_await ops.abs_(zn[0], tempv);
+      co_await ops.scale(reltol, tempv, tempv);
+      co_await ops.addconst(tempv, abstol, tempv);
+      co_await ops.inv(tempv, ewt);
+      const auto r = co_await ops.min_wrms(tempv, zn[0], ewt);
+      *nrm = r.second;
+      co_return (r.first <= ZERO) ? -1 : 0;
+    }
+    co_return -1;
+  }
+
   Task<int> ewt_set(Vec ycur_, Vec weight) {
     co_await ops.abs_(ycur_, tempv);
     co_await ops.scale(reltol, tempv, tempv);
@@ -612,7 +637,9 @@ struct BdfCore {
 
   // SpgmrSolve with x = 0 initially, s1 = s2 = weight, no preconditioning and
   // no restarts.  The solution is left in xsol.
-  Task<int> spgmr(Vec b, Vec weight, double delta, int *nli_inc) {
+  // bsum: the sum of squares of weight * b where lsolve's norm came with it
+  // (the same products in the same order as the dot product of V[0]).
+  Task<int> spgmr(Vec b, Vec weight, double delta, const double *bsum, int *nli_inc) {
     const int l_max = maxl;
     const bool deferred = deferred_scalars();
     int l_plus_1 = 0, krydim = 0;
@@ -624,8 +651,11 @@ struct BdfCore {
     // stubs) before scaling, V[0] = s2 r0; the copies change no value and
     // vtemp is written before it is next read, so only the product is made.
     co_await ops.prod(weight, b, V[0]);
-    double r_norm, beta, rho;
-    r_norm = beta = sun_sqrt(co_await ops.dot(V[0], V[0]));
+    // (an `if`: both branches of a conditional expression with a co_await run)
+    double r_norm, beta, rho, vv;
+    if (bsum) vv = *bsum;
+    else vv = co_await ops.dot(V[0], V[0]);
+    r_norm = beta = sun_sqrt(vv);
     if (r_norm <= delta) co_return SPGMR_SUCCESS;
     rho = beta;
     co_await ops.const_(ZERO, xcor);
@@ -679,7 +709,18 @@ struct BdfCore {
   // CVSpgmrSolve, cvode_spgmr.c:366-420: solve (I - gamma J) x = b in place
   Task<int> lsolve(Vec b, Vec weight, Vec ynow, Vec fnow) {
     const double deltar = eplifac * tq[4];
-    const double bnorm = co_await ops.wrms(b, weight);
+    double bnorm, bsum;
+    const bool with_sum = joined(b);
+    if constexpr (kJoinedOps) {
+      if (with_sum) {
+        const auto r = co_await ops.wrms_sum(b, weight);
+        // a right-hand side whose status came with the norm
+        if (ops.rhs_failed()) co_return RHSFUNC_FAIL;
+        bnorm = r.first;
+        bsum = r.second;
+      }
+    }
+    if (!with_sum) bnorm = co_await ops.wrms(b, weight);
     if (bnorm <= deltar) {
       if (mnewt > 0) co_await ops.const_(ZERO, b);
       co_return 0;
@@ -689,7 +730,7 @@ struct BdfCore {
     const double delta = deltar * sqrtN;
     co_await ops.const_(ZERO, xsol);
     int nli_inc = 0;
-    const int retval = co_await spgmr(b, weight, delta, &nli_inc);
+    const int retval = co_await spgmr(b, weight, delta, with_sum && bsum == bsum ? &bsum : nullptr, &nli_inc);
     co_await ops.scale(ONE, xsol, b);
     nli += nli_inc;
     if (retval != SPGMR_SUCCESS) ncfl++;
@@ -712,6 +753,7 @@ struct BdfCore {
       co_await ops.linear_sum(rl1, zn[1], ONE, acor, tempv);
       co_await ops.linear_sum(gamma, ftemp, -ONE, tempv, tempv);
       const int retval = co_await lsolve(tempv, ewt, y, ftemp);
+      if (retval == RHSFUNC_FAIL) co_return RHSFUNC_FAIL;
       nni++;
       if (retval < 0) co_return LSOLVE_FAIL;
       if (retval > 0) co_return CONV_FAIL;
@@ -721,22 +763,33 @@ struct BdfCore {
       if (m_it > 0) crate = sun_max(CRDOWN * crate, del / delp);
       const double dcon = del * sun_min(ONE, crate) / tq[4];
       if (dcon <= ONE) {
-        acnrm = (m_it == 0) ? del : co_await ops.wrms(acor, ewt);
+        acnrm = del;
+        if (m_it > 0) acnrm = co_await ops.wrms(acor, ewt);
         co_return SUCCESS;
       }
       mnewt = ++m_it;
       if ((m_it == maxcor) || ((m_it >= 2) && (del > RDIV * delp))) co_return CONV_FAIL;
       delp = del;
-      const int rv = co_await ops.rhs(tn, y, ftemp);
+      const int rv = co_await newton_rhs(y);
       nfe++;
       if (rv < 0) co_return RHSFUNC_FAIL;
       if (rv > 0) co_return RHSFUNC_RECVR;
     }
   }
 
+  // ftemp = f(tn, yy) for the Newton iteration.  Where the evaluation's
+  // status can come with the next value read back, lsolve's norm, it does not
+  // wait here.
+  Task<int> newton_rhs(Vec yy) {
+    if constexpr (kDeferredOps) {
+      if (ops.deferred_scalars(zn[0]) && ops.rhs_status_joins(zn[0])) co_return co_await ops.rhs_deferred(tn, yy, ftemp);
+    }
+    co_return co_await ops.rhs(tn, yy, ftemp);
+  }
+
   Task<int> nls_newton() {
     crate = ONE;  // PREC_NONE: no linear-solver setup
-    const int retval = co_await ops.rhs(tn, zn[0], ftemp);
+    const int retval = co_await newton_rhs(zn[0]);
     nfe++;
     if (retval < 0) co_return RHSFUNC_FAIL;
     if (retval > 0) co_return RHSFUNC_RECVR;
@@ -1183,8 +1236,13 @@ struct BdfCore {
     for (;;) {
       next_h = h;
       next_q = q;
+      double nrm = ZERO;
+      const bool with_norm = nst > 0 && joined(zn[0]);
       if (nst > 0) {
-        if ((co_await ewt_set(zn[0], ewt)) != 0) {
+        int bad;
+        if (with_norm) bad = co_await ewt_set_norm(&nrm);
+        else bad = co_await ewt_set(zn[0], ewt);
+        if (bad != 0) {
           istate = ILL_INPUT;
           tretlast = *tret = tn;
           co_await ops.scale(ONE, zn[0], yout);
@@ -1197,7 +1255,7 @@ struct BdfCore {
         co_await ops.scale(ONE, zn[0], yout);
         break;
       }
-      const double nrm = co_await ops.wrms(zn[0], ewt);
+      if (!with_norm) nrm = co_await ops.wrms(zn[0], ewt);
       tolsf = uround * nrm;
       if (tolsf > ONE) {
         istate = TOO_MUCH_ACC;

@@ -69,6 +69,12 @@ class NvQueue {
   // op: R_DOT, R_MAXABS, R_WSQ, R_MIN: queued, run, *value the reduction
   // (NAN when the device failed, as the vector's own operation gives)
   bool reduce(int op, N_Vector x, N_Vector y, double *value);
+  // Whether the queue takes v at all.
+  bool accepts(N_Vector v) const;
+  // min(m) and the sum of squares of x * w after the queued work, or (m
+  // null) the sum alone; dev_word (may be null): a device word read with them
+  bool min_wsq(N_Vector m, N_Vector x, N_Vector w, double *mn, double *sum, const unsigned int *dev_word,
+               unsigned int *word_out);
   // R_DOT, or R_WSQ as the WRMS norm, left in a slot
   bool reduce_slot(int op, N_Vector x, N_Vector y, int slot);
   // N_VFetchSlots_PihmGpu with the queued work ahead of it

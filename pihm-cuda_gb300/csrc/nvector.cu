@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kT, 4) k_seq(const __grid_constant__ Seq q) {
     if (d.wrms_n > 0) v = __dsqrt_rn(__ddiv_rn(v, (double)d.wrms_n));
     d.out[0] = v;
     d.out[1] = 0.0;
-    if (q.host_seq && q.fetch < 0) q.host[lane] = v;
+    if (q.host_seq) q.host[lane] = v;
   }
   if (tid == 0) *q.ticket = 0u;
   if (q.host_seq == nullptr) return;
@@ -984,7 +984,8 @@ void NvQueue::push(const SeqOp &o) {
 }
 
 void NvQueue::push_red(const SeqRed &r) {
-  if (q.nred == 2 || (q.nred == 1 && !(r.op == R_DOT && q.red[0].op == R_DOT))) {
+  if (q.nred == 2 || (q.nred == 1 && !(q.red[0].op == R_DOT && r.op == R_DOT) &&
+                      !(q.red[0].op == R_MIN && r.op == R_WSQ))) {
     flush();
   }
   SeqRed &d = q.red[q.nred++];
@@ -1085,6 +1086,31 @@ bool NvQueue::reduce(int op, N_Vector x, N_Vector y, double *value) {
   q.fetch = -1;
   const bool ok = launch() == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
   *value = ok ? s.host[0] : NAN;
+  return true;
+}
+
+bool NvQueue::accepts(N_Vector v) const {
+  const _generic_N_Vector_Ops *o = v->ops;
+  return o->nvgetvectorid == N_VGetVectorID_PihmGpu && o->nvwrmsnorm == N_VWrmsNorm_PihmGpu &&
+         o->nvdotprod == N_VDotProd_PihmGpu && o->nvmin == N_VMin_PihmGpu && o->nvprod == N_VProd_PihmGpu && L(v) > 0;
+}
+
+bool NvQueue::min_wsq(N_Vector m, N_Vector x, N_Vector w, double *mn, double *sum, const unsigned int *dev_word,
+                      unsigned int *word_out) {
+  if (!take(x, w, m)) return false;
+  if (q.nred > 0) flush();
+  Scratch &s = fam->scratch;
+  if (m) push_red({D(m), nullptr, s.result, 0, R_MIN, 0});
+  push_red({D(x), D(w), s.result, 0, R_WSQ, 0});
+  q.host = s.host;
+  q.host_seq = s.seq_word();
+  q.seq = ++s.seq;
+  q.fetch = dev_word ? 0 : -1;
+  q.word = dev_word;
+  const bool ok = launch() == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  if (m) *mn = ok ? s.host[0] : NAN;
+  *sum = ok ? s.host[m ? 1 : 0] : NAN;
+  if (dev_word) *word_out = ok ? *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS) : ~0u;
   return true;
 }
 
