@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "batch_engine.h"
+#include "host_flag.h"
 #include "pihm_deck.h"
 
 using namespace pihm;
@@ -55,10 +56,17 @@ BatchOps::Ew BatchOps::push(int code, double a, double b, int x, int y, int z, d
   return Ew{s};
 }
 
-BatchOps::Red BatchOps::reduce(int red, int x, int y, bool wrms) {
+void BatchOps::Red2::await_suspend(std::coroutine_handle<> h) const noexcept { s->waiting = h; }
+std::pair<double, double> BatchOps::Red2::await_resume() const noexcept {
+  if (sum) return {std::sqrt(s->red_value / (double)s->neq), s->red_value};
+  return {s->red_value, std::sqrt(s->red_value2 / (double)s->neq)};
+}
+
+BatchOps::Red BatchOps::reduce(int red, int x, int y, bool wrms, int w) {
   s->red = red;
   s->rx = (uint8_t)x;
   s->ry = (uint8_t)y;
+  s->rw = (uint8_t)w;
   s->red_wrms = wrms;
   return Red{s};
 }
@@ -533,9 +541,13 @@ int run_round(pihm_batch *B, bool *any) {
   Op *ops = (Op *)(B->h_up + B->up_ops_off);
   uint8_t *active = (uint8_t *)B->h_up;
   std::memset(active, 0, B->max_sys);
-  int nops = 0, nblocks = 0;
+  int nops = 0, nblocks = 0, most = 0;
   bool rhs = false;
   std::vector<Sys *> forcing;  // watersheds whose programs start a model step with a deck's forcing
+  // the program kernel itself ends the round when every watershed in it ends
+  // in a reduction and nothing follows it
+  bool flagged = true;
+  int top = -1;                // highest slot
   int64_t el_req = 0;          // elements of the watersheds evaluated this round
   // Right-hand-side gating: a watershed that waits for an evaluation is held
   // back while others still have reductions to run, until the waiting ones
@@ -561,12 +573,17 @@ int run_round(pihm_batch *B, bool *any) {
     r.red = waiting ? s->red : -1;
     r.rx = s->rx;
     r.ry = s->ry;
-    r.pad0 = r.pad1 = 0;
+    r.rw = s->rw;
+    r.pad = 0;
+    flagged = flagged && r.red >= 0;
+    top = std::max(top, (int)s->slot);
     r.bstart = nblocks;
     if (s->pending_k >= 0 || s->pending_post) forcing.push_back(s);
     std::memcpy(ops + nops, s->prog.data(), sizeof(Op) * s->prog.size());
     nops += (int)s->prog.size();
-    nblocks += (int)pihm_nv::red_grid_for(s->neq);
+    const int nb = (int)pihm_nv::red_grid_for(s->neq);
+    nblocks += nb;
+    most = std::max(most, nb);
     if (waiting && s->rhs_req) {
       active[s->slot] = 1;
       rhs = true;
@@ -577,12 +594,16 @@ int run_round(pihm_batch *B, bool *any) {
   if (part.empty()) return 0;
   *any = true;
   cudaStream_t st = B->st;
-  const size_t up1 = B->up_round_off + sizeof(RoundSys) * part.size();
-  if (cudaMemcpyAsync(B->d_up, B->h_up, up1, cudaMemcpyHostToDevice, st) != cudaSuccess) return -1;
-  if (nops && cudaMemcpyAsync(B->d_up + B->up_ops_off, B->h_up + B->up_ops_off, sizeof(Op) * nops,
-                              cudaMemcpyHostToDevice, st) != cudaSuccess)
+  uint64_t *seq_word = (uint64_t *)B->h_down;
+  const uint64_t seq = ++B->round_seq;
+  const auto up16 = [](size_t n) { return (n + 15) & ~size_t(15); };
+  // clears the evaluation's error words too, before the program, the
+  // land-surface and Noah steps and the evaluation
+  if (launch_upload(B->h_up, B->d_up, up16(B->up_round_off + sizeof(RoundSys) * part.size()), B->up_ops_off,
+                    up16(sizeof(Op) * nops), B->err_sys, rhs ? B->max_sys : 0, st) != cudaSuccess)
     return -1;
   int variant = B->prog_forced >= 0 ? B->prog_forced : B->prog_variant;
+  if (B->prog_forced < 0 && most <= pihm_nv::kMaxBlocks / 8 && nblocks <= kSpreadBlocks) variant = kProgramSpread;
   const bool tune = B->prog_forced < 0 && B->tuning && nblocks >= pihm_batch::kTuneMinBlocks && B->tev[0];
   if (tune) {
     variant = B->tune_next;
@@ -595,11 +616,13 @@ int run_round(pihm_batch *B, bool *any) {
     if (s->has_bc && stage_bc(B, s, s->start + (int64_t)s->pending_k * (int64_t)s->ctrl.stepsize) != PIHM_GPU_OK)
       return -1;
   if (B->profiling) cudaEventRecord(B->ev[0], st);
-  if (launch_program(B->A, (int)part.size(), nblocks, variant, st) != cudaSuccess) return -1;
-  B->launches++;
+  // (its events must be behind it, so a timed round ends with its own kernel)
+  flagged = flagged && !rhs && !tune && !B->profiling && forcing.empty();
+  if (launch_program(B->A, (int)part.size(), nblocks, variant, flagged ? seq_word : nullptr, seq, st) != cudaSuccess)
+    return -1;
+  B->launches += 2;
   if (B->profiling) cudaEventRecord(B->ev[1], st);
   if (tune) cudaEventRecord(B->tev[1], st);
-  if (rhs && cudaMemsetAsync(B->err_sys, 0, sizeof(unsigned int) * B->max_sys, st) != cudaSuccess) return -1;
   // after the program, which ends the previous model step's state in vector
   // slot 0, and before the evaluation that starts the next step: Flux-PIHM's
   // post-step (Summary's _NOAH_ part and NoahHydrol, src/update.c:34-41,
@@ -641,9 +664,14 @@ int run_round(pihm_batch *B, bool *any) {
     B->rhs_rounds++;
   }
   if (B->profiling) cudaEventRecord(B->ev[2], st);
-  if (cudaMemcpyAsync(B->h_down, B->d_down, B->down_bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
+  const double *res = (const double *)B->h_down + 2;
+  unsigned int *err = (unsigned int *)(B->h_down + sizeof(double) * (2 + 2 * B->max_sys));
+  if (!flagged) {
+    if (launch_round_done(B->err_sys, err, top + 1, seq_word, seq, st) != cudaSuccess) return -1;
+    B->launches++;
+  }
   const auto t_wait = std::chrono::steady_clock::now();
-  if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+  if (!pihm::host_flag_wait(seq_word, seq, st)) return -1;
   const auto t_done = std::chrono::steady_clock::now();
   B->wait_ms += std::chrono::duration<double, std::milli>(t_done - t_wait).count();
   B->host_ms += std::chrono::duration<double, std::milli>(t_wait - t_start).count();
@@ -688,8 +716,6 @@ int run_round(pihm_batch *B, bool *any) {
     B->rhs_ms += b;
   }
   B->rounds++;
-  const double *res = (const double *)B->h_down;
-  const unsigned int *err = (const unsigned int *)(B->h_down + sizeof(double) * 2 * B->max_sys);
   // an evaluation whose waits ran out leaves its barrier counters as they were
   for (Sys *s : part)
     if (s->rhs_req && (err[s->slot] & pihm::kErrWait)) {
@@ -702,6 +728,7 @@ int run_round(pihm_batch *B, bool *any) {
     if (s->red >= 0) {
       const double v = res[2 * s->slot];
       s->red_value = s->red_wrms ? std::sqrt(v / (double)s->neq) : v;
+      s->red_value2 = res[2 * s->slot + 1];
       s->red = -1;
     }
     if (s->rhs_req) {
@@ -883,19 +910,20 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
   B->up_ops_off = B->up_round_off + ((sizeof(RoundSys) * MS + 255) & ~size_t(255));
   const size_t up_bytes = B->up_ops_off + sizeof(Op) * MS * kMaxProgOps;
   B->d_up = (char *)dalloc<char>(up_bytes, o);
-  // download block: results | error words
-  B->down_bytes = sizeof(double) * 2 * MS + sizeof(unsigned int) * MS;
-  B->d_down = (char *)dalloc<char>(B->down_bytes, o);
+  // download block: sequence number | results | error words
+  const size_t down_bytes = sizeof(double) * (2 + 2 * MS) + sizeof(unsigned int) * MS;
+  B->err_sys = dalloc<unsigned int>(MS, o);
+  A.done = dalloc<unsigned int>(1, o);
   if (t_count_bytes) return PIHM_GPU_OK;  // sizes counted, nothing allocated
-  if (!ok || !m.err || !m.bar || !A.sysinfo || !A.tickets || !B->d_up || !B->d_down ||
+  if (!ok || !m.err || !m.bar || !A.sysinfo || !A.tickets || !B->d_up || !B->err_sys || !A.done ||
       cudaMallocHost(&B->h_up, up_bytes) != cudaSuccess ||
-      cudaMallocHost(&B->h_down, B->down_bytes) != cudaSuccess)
+      cudaMallocHost(&B->h_down, down_bytes) != cudaSuccess)
     return PIHM_GPU_ERR_NOMEM;
   m.active = (const uint8_t *)B->d_up;
   A.round = (RoundSys *)(B->d_up + B->up_round_off);
   A.ops = (Op *)(B->d_up + B->up_ops_off);
-  A.results = (double *)B->d_down;
-  B->err_sys = (unsigned int *)(B->d_down + sizeof(double) * 2 * MS);
+  std::memset(B->h_down, 0, down_bytes);
+  A.results = (double *)B->h_down + 2;
   m.err_sys = B->err_sys;
   // everything starts free: owner -1, zero scratch
   bool z = cudaMemset(se, 0xff, sizeof(int32_t) * NE) == cudaSuccess &&
@@ -903,6 +931,8 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
            cudaMemset(sed, 0xff, sizeof(int32_t) * NED) == cudaSuccess &&
            cudaMemset(sb, 0xff, sizeof(int32_t) * NE) == cudaSuccess &&
            cudaMemset(A.tickets, 0, sizeof(unsigned int) * MS) == cudaSuccess &&
+           cudaMemset(A.done, 0, sizeof(unsigned int)) == cudaSuccess &&
+           cudaMemset(B->err_sys, 0, sizeof(unsigned int) * MS) == cudaSuccess &&
            cudaMemset(snoah, 0, sizeof(int32_t) * MS) == cudaSuccess &&
            cudaMemset(B->d_up, 0, up_bytes) == cudaSuccess &&
            cudaMemset(m.rivflow, 0, sizeof(double) * NUM_RIVFLX * NR) == cudaSuccess &&

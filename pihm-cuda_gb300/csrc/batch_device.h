@@ -53,12 +53,15 @@ struct SysInfo {
   int64_t rec_off;               // first entry of its hydrograph record
 };
 
+// Two reductions in one: the minimum of rx, and the sum of squares of ry * rw.
+constexpr int kRedMinWsq = 32;
+
 // One watershed's work in one round.
 struct RoundSys {
   int32_t sys, prog_off, prog_len;
-  int32_t red;      // -1: none, else a pihm_nv::RedOp (R_DOT, R_MAXABS, R_WSQ, R_MIN)
+  int32_t red;      // -1: none, else a pihm_nv::RedOp (R_DOT, R_MAXABS, R_WSQ, R_MIN) or kRedMinWsq
   int32_t bstart;   // first block of the program kernel that works on it
-  uint8_t rx, ry, pad0, pad1;
+  uint8_t rx, ry, rw, pad;
 };
 
 struct DeviceArena {
@@ -69,17 +72,43 @@ struct DeviceArena {
   SysInfo *sysinfo;     // [max_sys]
   double *partials;     // [max_sys][2 * kMaxBlocks]
   unsigned int *tickets;  // [max_sys]
-  double *results;      // [max_sys][2]
+  double *results;      // [max_sys][2], pinned host memory
+  unsigned int *done;   // watersheds of the round whose reduction is finished
   double *rec;          // hydrograph records
   RoundSys *round;      // round list, then the ops, one upload per round
   Op *ops;
   int max_sys;
 };
 
+// A round's upload from pinned host memory by a kernel that the program
+// kernel can start beside (two copies before it and one behind it, with a
+// synchronisation, cost about 10 us of a round's 47): n1 bytes at offset 0 and n2 at
+// offset off2 of both, multiples of 16; zero words are cleared.
+cudaError_t launch_upload(const char *host, char *dev, size_t n1, size_t off2, size_t n2, unsigned int *zero, int nzero,
+                          cudaStream_t st);
+
 // Run one round's programs: nrs watersheds over nblocks blocks in total.
 // variant 0, 1, 2: entries a thread keeps in flight (1, 2, 4); same results.
+// flag: with every watershed of the round ending in a reduction, the last of
+// them hands seq to the host (host_flag.h); null: launch_round_done does.
 constexpr int kProgramVariants = 3;
-cudaError_t launch_program(const DeviceArena &a, int nrs, int nblocks, int variant, cudaStream_t st);
+// A fourth layout, same results: one warp of the reduction order a block, its
+// threads' four entries on four warps.  A warp has one FP64 instruction in
+// flight (69 clocks) and an SM takes one every 20, so a round that leaves the
+// SMs short of warps is bound by that latency: model steps of 8 watersheds of
+// 17,566 elements 7.5 -> 6.2 ms, of 20 of 104,308 (rounds of up to 315
+// blocks) 11.4 -> 10.5 ms.  From about 400 blocks the FP64 pipe is full either
+// way (24 of 187,100: 12.1 ms with rounds up to 400 blocks spread, 12.5 with
+// all or none).  Its partial values need a watershed of kMaxBlocks / 8 blocks
+// or fewer.
+constexpr int kProgramSpread = 3;
+constexpr int kSpreadBlocks = 400;
+cudaError_t launch_program(const DeviceArena &a, int nrs, int nblocks, int variant, uint64_t *flag, uint64_t seq,
+                           cudaStream_t st);
+
+// Behind a round's last kernel: n words to the host, then seq.
+cudaError_t launch_round_done(const unsigned int *words, unsigned int *host, int n, uint64_t *flag, uint64_t seq,
+                              cudaStream_t st);
 
 // One host-to-device copy of a watershed's upload: bytes from src (host
 // memory) to dst (arena).

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "batch_device.h"
@@ -103,7 +104,19 @@ struct BatchOps {
 
   Ew push(int code, double a, double b, int x, int y, int z, double c = 0.0, int i0 = 0, int i1 = 0);
   Ew push(const pihm_nv::EwCall<int> &e) { return push(e.op, e.a, e.b, e.x, e.y, e.z); }
-  Red reduce(int red, int x, int y, bool wrms);
+  Red reduce(int red, int x, int y, bool wrms, int w = 0);
+  // two values of one pass (bdf_core.h)
+  struct Red2 {
+    Sys *s;
+    bool sum;  // the WRMS norm and its sum of squares; else a minimum and a WRMS norm
+    bool await_ready() const noexcept { return false; }
+    void await_suspend(std::coroutine_handle<> h) const noexcept;
+    std::pair<double, double> await_resume() const noexcept;
+  };
+  bool joined(int) const { return true; }
+  Red2 min_wrms(int m, int x, int w) { return Red2{(reduce(kRedMinWsq, m, x, false, w), s), false}; }
+  Red2 wrms_sum(int x, int w) { return Red2{(reduce(pihm_nv::R_WSQ, x, w, false), s), true}; }
+  bool rhs_failed() const { return false; }
 
   Ew linear_sum(double a, int x, double b, int y, int z) {
     return push(pihm_nv::select_linear_sum<int>(a, x, b, y, z));
@@ -147,10 +160,10 @@ struct Sys {
   // the program of the current round
   std::vector<Op> prog;
   int red = -1;
-  uint8_t rx = 0, ry = 0;
+  uint8_t rx = 0, ry = 0, rw = 0;
   bool red_wrms = false, rhs_req = false, rhs_pending_out = false;
   uint8_t rhs_out = 0;
-  double red_value = 0.0;
+  double red_value = 0.0, red_value2 = 0.0;
   int rhs_rc = 0;
   // an input deck's forcing (pihm_batch_job.deck / .land)
   const pihm_deck *deck = nullptr;  // ApplyBc every model step when has_bc
@@ -216,10 +229,10 @@ struct pihm_batch {
   char *h_up = nullptr;
   char *d_up = nullptr;
   size_t up_active_bytes = 0, up_round_off = 0, up_ops_off = 0;
-  // per-round download: results [max_sys][2], then error words [max_sys]
+  // per-round download, written by the kernels: the round's sequence number
+  // (host_flag.h; two doubles), results [max_sys][2], error words [max_sys]
   char *h_down = nullptr;
-  char *d_down = nullptr;
-  size_t down_bytes = 0;
+  uint64_t round_seq = 0;
   unsigned int *err_sys = nullptr;
   // scheduling policy
   double rhs_gate = 1.0;

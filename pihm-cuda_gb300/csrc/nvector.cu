@@ -384,43 +384,8 @@ __device__ __forceinline__ void seq_load(const SeqHead &h, const long long (&i)[
   }
 }
 
-// p combined with the identity, as the first step of a sum or of a tree over
-// fewer values than lanes: of the sums only -0 changes.
-template <int RED>
-__device__ __forceinline__ Pair red_first(Pair p) {
-  if (RED == R_DOT || RED == R_WSQ) {
-    const long long b = __double_as_longlong(p.v);
-    return {__longlong_as_double(b == (long long)0x8000000000000000ull ? 0 : b), 0.0};
-  }
-  return red_combine<RED>(red_identity<RED>(), p);
-}
-
-// The shuffle tree of one warp, and the tree over a block's eight warp
-// values, as red_block makes them.
-template <int RED>
-__device__ __forceinline__ double warp_tree(double x) {
-  Pair v = {x, 0.0};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const Pair q = {__shfl_down_sync(0xffffffffu, v.v, o), 0.0};
-    v = red_combine<RED>(v, q);
-  }
-  return v.v;
-}
-template <int RED>
-__device__ __forceinline__ double eight_tree(const volatile double *w) {
-  Pair v[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) v[k] = red_first<RED>({w[k], 0.0});
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < o; k++) v[k] = red_combine<RED>(v[k], v[k + o]);
-  return v[0].v;
-}
-
-// One reduction over the blocks of k_seq; r picks the shared and global
-// words.  kSpread: `part` has a value per warp of the reduction order.
+// One reduction within a block of k_seq.  kSpread: `part` has a value per
+// warp of the reduction order.
 template <int RED, bool kSpread, int kT>
 __device__ __forceinline__ void seq_tail_block(double acc, int vwarp, bool writer, double *part, double *sh) {
   const double v = warp_tree<RED>(acc);
@@ -429,22 +394,6 @@ __device__ __forceinline__ void seq_tail_block(double acc, int vwarp, bool write
     else sh[threadIdx.x >> 5] = v;
   }
 }
-template <int RED, bool kSpread, int kT>
-__device__ __forceinline__ void seq_tail_last(int nblk, const double *part, double *sh) {
-  const int lane = threadIdx.x & 31;
-  for (int vw = threadIdx.x >> 5; vw < 8; vw += kT / 32) {
-    double v = red_identity<RED>().v;
-    if (vw * 32 < nblk) {
-      for (int b = vw * 32 + lane, k = 0; b < nblk; b += kThreads, k++) {
-        const Pair t = {kSpread ? eight_tree<RED>(part + 8 * b) : ((const volatile double *)part)[b], 0.0};
-        v = k == 0 ? red_first<RED>(t).v : red_combine<RED>({v, 0.0}, t).v;
-      }
-      v = warp_tree<RED>(v);
-    }
-    if (lane == 0) sh[vw] = v;
-  }
-}
-
 // A sequence over a vector: element-wise operations in order, then nothing
 // (RA < 0), one reduction (RA) or two (RA, RB).  An operation on a vector the
 // one before wrote takes the value from registers, and a result that is
@@ -576,8 +525,8 @@ __global__ void __launch_bounds__(kT, 4) k_seq(const __grid_constant__ Seq q) {
   if (!last) return;
   __threadfence();
   // the last block combines the blocks' values in a fixed order
-  seq_tail_last<R0, kSpread, kT>(nblk, part[0], sh[0]);
-  if (RB >= 0) seq_tail_last<R1, kSpread, kT>(nblk, part[1], sh[1]);
+  tree_last<R0, kSpread, kT>(nblk, part[0], sh[0]);
+  if (RB >= 0) tree_last<R1, kSpread, kT>(nblk, part[1], sh[1]);
   __syncthreads();
   if (wid == 0 && lane < (RB < 0 ? 1 : 2)) {
     const SeqRed &d = q.red[lane];
