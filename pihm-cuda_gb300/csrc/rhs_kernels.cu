@@ -992,10 +992,42 @@ __device__ __forceinline__ double sub_elem_to_river(double e_gw, double e_zmin, 
   return r.length * avg_ksat * grad_h * avg_h;
 }
 
+// OutletFlux, src/river_flow.c:333-390
+__device__ __forceinline__ void outlet_flux(const DevMesh &m, const RivState &r, int s, int down) {
+  const int nr = m.nr;
+  double dnf;
+  const double depth = m.r_depth[s];
+  const double bc = m.river_bc[s];
+  if (down == kDirichlet) {
+    const double total_h = r.stage + r.zbed;
+    const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
+    const double avg_perim = m.r_perim[s];
+    const double crossa = m.r_crossa[s];
+    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
+    dnf = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+  } else if (down == kNeumann) {
+    dnf = -bc;
+  } else if (down == kZeroDpthGrad) {
+    const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
+    const double avg_perim = m.r_perim[s];
+    const double crossa = m.r_crossa[s];
+    dnf = div_any(sqrt_any(grad_h) * crossa *
+                      (cmp::gt0(avg_perim) ? pow_manning(div_any(crossa, avg_perim), kManningRiv) : 0.0),
+                  r.rough);
+  } else {  // kCritDpth (other values are rejected at load)
+    const double crossa = m.r_crossa[s];
+    dnf = crossa * sqrt_any(kGrav * r.stage);
+  }
+  m.rivflow[UP_CHANL2CHANL * nr + s] = 0.0;
+  m.rivflow[DOWN_CHANL2CHANL * nr + s] = dnf;
+}
+
 // A segment's fluxes in four parts that share no result: the channel flux,
 // the two banks, and the bed's.  One thread per part: a segment's fluxes are a
 // chain of FP64 divisions, roots and a power (18 us for 100 segments or
 // 12,000 with one thread per segment), and the parts run beside each other.
+// An outlet's channel flux goes with its bed, the shortest part: with the
+// channel fluxes of its warp it took the warp 2 us longer than the others.
 enum RivPart { PART_CHAN = 0, PART_LEFT, PART_RIGHT, PART_BED, kRivParts };
 
 __device__ __forceinline__ void river_part(const DevMesh &m, const double *y, int s, int part) {
@@ -1004,68 +1036,43 @@ __device__ __forceinline__ void river_part(const DevMesh &m, const double *y, in
   const RivState r = load_riv(m, y, s);
   if (part == PART_CHAN) {
     const int down = m.down[s];
-    double up = 0.0, dnf;
-    if (down > 0) {
-      const int bct = m.bctype_riv[s];
-      if (bct != 0) {
-        // BoundFluxRiver, src/river_flow.c:392-427
-        double flux = 0.0;
-        const double bc = m.river_bc[s];
-        if (bct > 0) {
-          const double total_h = r.stage + r.zbed;
-          const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
-          const double avg_perim = m.r_perim[s];
-          const double crossa = m.r_crossa[s];
-          const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
-          flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-        } else {
-          flux = -bc;
-        }
-        up += flux;
-      }
-      const int d = down - 1;
-      const RivState dn = load_riv(m, y, d);
-      const double inv_dist_down = m.r_inv_dist_down[s];
-      // ChanFlowRiverToRiver, src/river_flow.c:257-300
-      const double total_h = r.stage + r.zbed;
-      const double perim = m.r_perim[s];
-      const double total_h_down = dn.stage + dn.zbed;
-      const double perim_down = m.r_perim[d];
-      const double avg_perim = (perim + perim_down) / 2.0;
-      const double avg_rough = (r.rough + dn.rough) / 2.0;
-      const double diff_h = (m.riv_mode == kKinematic) ? (r.zbed - dn.zbed) : (total_h - total_h_down);
-      const double grad_h = diff_h * inv_dist_down;
-      const double avg_sf = cmp::gt0(grad_h) ? grad_h : kRivGradMin;
-      const double crossa = m.r_crossa[s];
-      const double crossa_down = m.r_crossa[d];
-      const double avg_crossa = 0.5 * (crossa + crossa_down);
-      const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(avg_crossa, avg_perim);
-      dnf = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
-    } else {
-      // OutletFlux, src/river_flow.c:333-390
-      const double depth = m.r_depth[s];
+    if (down <= 0) return;  // an outlet: the bed's part
+    double up = 0.0;
+    const int bct = m.bctype_riv[s];
+    if (bct != 0) {
+      // BoundFluxRiver, src/river_flow.c:392-427
+      double flux = 0.0;
       const double bc = m.river_bc[s];
-      if (down == kDirichlet) {
+      if (bct > 0) {
         const double total_h = r.stage + r.zbed;
         const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
         const double avg_perim = m.r_perim[s];
         const double crossa = m.r_crossa[s];
         const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
-        dnf = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-      } else if (down == kNeumann) {
-        dnf = -bc;
-      } else if (down == kZeroDpthGrad) {
-        const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
-        const double avg_perim = m.r_perim[s];
-        const double crossa = m.r_crossa[s];
-        dnf = sqrt(grad_h) * crossa *
-              (cmp::gt0(avg_perim) ? pow_manning(crossa / avg_perim, kManningRiv) : 0.0) /
-              r.rough;
-      } else {  // kCritDpth (other values are rejected at load)
-        const double crossa = m.r_crossa[s];
-        dnf = crossa * sqrt(kGrav * r.stage);
+        flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+      } else {
+        flux = -bc;
       }
+      up += flux;
     }
+    const int d = down - 1;
+    const RivState dn = load_riv(m, y, d);
+    const double inv_dist_down = m.r_inv_dist_down[s];
+    // ChanFlowRiverToRiver, src/river_flow.c:257-300
+    const double total_h = r.stage + r.zbed;
+    const double perim = m.r_perim[s];
+    const double total_h_down = dn.stage + dn.zbed;
+    const double perim_down = m.r_perim[d];
+    const double avg_perim = (perim + perim_down) / 2.0;
+    const double avg_rough = (r.rough + dn.rough) / 2.0;
+    const double diff_h = (m.riv_mode == kKinematic) ? (r.zbed - dn.zbed) : (total_h - total_h_down);
+    const double grad_h = diff_h * inv_dist_down;
+    const double avg_sf = cmp::gt0(grad_h) ? grad_h : kRivGradMin;
+    const double crossa = m.r_crossa[s];
+    const double crossa_down = m.r_crossa[d];
+    const double avg_crossa = 0.5 * (crossa + crossa_down);
+    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(avg_crossa, avg_perim);
+    const double dnf = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
     F[UP_CHANL2CHANL * nr + s] = up;
     F[DOWN_CHANL2CHANL * nr + s] = dnf;
     return;
@@ -1098,6 +1105,7 @@ __device__ __forceinline__ void river_part(const DevMesh &m, const double *y, in
     else diff_h = r.stage + r.zbed - (r.gw + r.zmin);
     const double grad_h = diff_h * m.r_inv_bedthick[s];
     F[CHANL_LKG * nr + s] = m.r_ksatv[s] * r.width * r.length * grad_h;
+    if (down <= 0) outlet_flux(m, r, s, down);
     return;
   }
   // RiverToElem, src/river_flow.c:113-183, one bank
@@ -1128,8 +1136,25 @@ __global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT
 // ---------------------------------------------------------------------------
 // k_river_rows: upstream sums and the river rows of ydot
 // ---------------------------------------------------------------------------
+// What a river row reads of the mesh: the first upstream segments' indices
+// are a chain of loads in front of their fluxes.
+struct RiverRowsIn {
+  double area, porosity;
+  int first, end, up[3];
+};
+__device__ __forceinline__ RiverRowsIn river_rows_load(const DevMesh &m, int s) {
+  RiverRowsIn r;
+  r.area = m.r_area[s];
+  r.porosity = m.r_porosity[s];
+  r.first = m.up_ptr[s];
+  r.end = m.up_end[s];
+#pragma unroll
+  for (int k = 0; k < 3; k++) r.up[k] = r.first + k < r.end ? m.up_idx[r.first + k] : 0;
+  return r;
+}
+
 // the quotients of a row, beside each other
-__device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, int s, int sy) {
+__device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, int s, int sy, const RiverRowsIn &r) {
   const int nr = m.nr, ne = m.ne;
   const double *F = m.rivflow;
   double f[7];
@@ -1138,10 +1163,22 @@ __device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, 
   for (int j = 1; j <= 6; j++) f[j] = F[j * nr + s];
   const double aq_l = F[LEFT_AQUIF2AQUIF * nr + s], aq_r = F[RIGHT_AQUIF2AQUIF * nr + s];
   const double aq_d = F[DOWN_AQUIF2AQUIF * nr + s];
-  const double area = m.r_area[s], por_area = m.r_porosity[s] * area;
+  const double area = r.area, por_area = r.porosity * area;
   double up_c = f[0];
   double up_a = 0.0;
-  for (int k = m.up_ptr[s]; k < m.up_end[s]; k++) {
+  double fc[3], fa[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    fc[k] = F[DOWN_CHANL2CHANL * nr + r.up[k]];
+    fa[k] = F[DOWN_AQUIF2AQUIF * nr + r.up[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (r.first + k < r.end) {
+      up_c -= fc[k];
+      up_a -= fa[k];
+    }
+  for (int k = r.first + 3; k < r.end; k++) {
     const int u = m.up_idx[k];
     up_c -= F[DOWN_CHANL2CHANL * nr + u];
     up_a -= F[DOWN_AQUIF2AQUIF * nr + u];
@@ -1174,7 +1211,7 @@ __global__ void __launch_bounds__(128) k_river_rows(DevMesh m, double *RESTRICT 
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   int sy;
   if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
-  river_rows_item(m, ydot, s, sy);
+  river_rows_item(m, ydot, s, sy, river_rows_load(m, s));
 }
 
 // ---------------------------------------------------------------------------
@@ -1379,30 +1416,39 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     // ---- rivers: the same number of blocks for each part ----
     const int per = g.river / kRivParts, part = blk / per;
     const int first = (blk - part * per) * blockDim.x + threadIdx.x, step = per * blockDim.x;
+    // areas and perimeters need the state alone; kFromRef: river values stand
+    // in the same order.  Every part's blocks take a quarter of their
+    // segments, so that no SM has a block full of them beside its elements
+    // (21,000 elements: 9.5 us until the last with the channel blocks alone)
+    const double *yr = kFromRef ? y_ref : y;
+    const int quarter = blockDim.x / kRivParts;
+    for (int s = first + part * quarter; s < m.nr_run; s += step)
+      if ((int)threadIdx.x < quarter && !skip_item(m, m.sys_riv, s, &sy)) geom_item(m, yr, s);
+    bar_arrive(R);
     bool ok;
     if (part == PART_CHAN) {
-      // the state alone; kFromRef: river values stand in the same order
-      const double *yr = kFromRef ? y_ref : y;
-      for (int s = first; s < m.nr_run; s += step)
-        if (!skip_item(m, m.sys_riv, s, &sy)) geom_item(m, yr, s);
-      bar_arrive(R);
-      ok = bar_wait(R, per, &s_ok);
+      ok = bar_wait(R, g.river, &s_ok);
       for (int s = first; ok && s < m.nr_run; s += step)
         if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, yr, s, PART_CHAN);
     } else {
       ok = bar_wait(A, g.elem, &s_ok);
+      if (ok && part == PART_BED) ok = bar_wait(R, g.river, &s_ok);
       for (int s = first; ok && s < m.nr_run; s += step)
         if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, y, s, part);
     }
     if (ok) {
       bar_arrive(C);
       if (part != PART_CHAN) return;
-      ok = bar_wait(C, lateral, &s_ok);
     }
+    const bool on = first < m.nr_run && !skip_item(m, m.sys_riv, first, &sy);
+    RiverRowsIn in;
+    if (on) in = river_rows_load(m, first);
+    if (ok) ok = bar_wait(C, lateral, &s_ok);
     if (!ok) return report_wait(m, m.sys_riv, first, m.nr_run, step);
     bar_leave(m.bar, per + g.col);
-    for (int s = first; s < m.nr_run; s += step)
-      if (!skip_item(m, m.sys_riv, s, &sy)) river_rows_item(m, ydot, s, sy);
+    if (on) river_rows_item(m, ydot, first, sy, in);
+    for (int s = first + step; s < m.nr_run; s += step)
+      if (!skip_item(m, m.sys_riv, s, &sy)) river_rows_item(m, ydot, s, sy, river_rows_load(m, s));
     return;
   }
   blk -= g.river;
