@@ -658,7 +658,7 @@ int run_round(pihm_batch *B, bool *any) {
   if (rhs) {
     B->A.m.main_shape = shape;
     if (stune) cudaEventRecord(B->sev[0], st);
-    if (launch_rhs(B->A.m, B->A.rhs_in, B->A.rhs_out, st, &B->launches, nullptr, &B->side) != cudaSuccess)
+    if (launch_rhs(B->A.m, B->A.rhs_in, B->A.rhs_out, st, &B->launches, nullptr, &B->fused) != cudaSuccess)
       return -1;
     if (stune) cudaEventRecord(B->sev[1], st);
     B->rhs_rounds++;
@@ -941,7 +941,7 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
            cudaMemset(A.rhs_in, 0, sizeof(double) * NEQ) == cudaSuccess &&
            cudaDeviceSynchronize() == cudaSuccess;
   if (!z) return PIHM_GPU_ERR_CUDA;
-  if (pihm::create_rhs_streams(&B->side) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
+  if (pihm::fused_plan(&B->fused) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
   {
     int dev = 0, pageable = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&

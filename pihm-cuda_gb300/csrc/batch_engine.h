@@ -259,7 +259,7 @@ struct pihm_batch {
   int shape_n[kShapes] = {0};
   cudaEvent_t sev[2] = {nullptr, nullptr};
   int noah_resident = 0;  // Flux-PIHM watersheds resident (the arena's noah and diagnostics switch on)
-  pihm::RhsStreams side;  // river kernel beside the element kernels
+  pihm::FusedPlan fused;  // residency of the one-launch evaluation
   int host_pageable = 0;  // the device can access pageable host memory (uploads by one gather kernel)
   // counters and timing (host: building rounds and running the coroutines;
   // wait: blocked on the device; program/rhs: device time, when profiling)
@@ -278,9 +278,6 @@ struct pihm_batch {
       if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : sev)
       if (e) cudaEventDestroy(e);
-    if (side.fork) cudaEventDestroy(side.fork);
-    if (side.join) cudaEventDestroy(side.join);
-    if (side.side) cudaStreamDestroy(side.side);
     slots.clear();
     for (void *p : owned) cudaFree(p);
     if (h_up) cudaFreeHost(h_up);

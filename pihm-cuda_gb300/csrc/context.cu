@@ -219,7 +219,7 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
     return PIHM_GPU_ERR_NOMEM;
   }
   c->h_status[0] = c->h_status[1] = 0;
-  if (pihm::create_rhs_streams(&c->side) != cudaSuccess) {
+  if (pihm::fused_plan(&c->fused) != cudaSuccess) {
     pihm_gpu_destroy(c);
     return PIHM_GPU_ERR_CUDA;
   }
@@ -247,9 +247,6 @@ void pihm_gpu_destroy(pihm_gpu_ctx *c) {
   if (c->h_status) cudaFreeHost(c->h_status);
   pihm::land_release(c->land);
   pihm::noah_release(c->noahlsm);
-  if (c->side.fork) cudaEventDestroy(c->side.fork);
-  if (c->side.join) cudaEventDestroy(c->side.join);
-  if (c->side.side) cudaStreamDestroy(c->side.side);
   std::free(c->h_perm);
   std::free(c->h_iperm);
   delete c;
@@ -407,7 +404,7 @@ int pihm_gpu_rhs(pihm_gpu_ctx *c, double t, const double *y, double *ydot) {
   (void)t;
   if (!c || !y || !ydot) return PIHM_GPU_ERR_ARG;
   c->m.diag = c->diag;
-  return cuda_fail(launch_rhs(c->m, y, ydot, c->stream, &c->launches, c->prof, &c->side));
+  return cuda_fail(launch_rhs(c->m, y, ydot, c->stream, &c->launches, c->prof, &c->fused));
 }
 
 // the error word to the host, behind everything queued on the stream
@@ -490,7 +487,7 @@ static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_
     // fills y_int itself
     double *y_int = c->d_stage_out, *ydot_int = c->d_stage_in;
     c->m.diag = c->diag;
-    cudaError_t e = launch_rhs(c->m, y_int, ydot_int, c->stream, &c->launches, c->prof, &c->side, y_dev,
+    cudaError_t e = launch_rhs(c->m, y_int, ydot_int, c->stream, &c->launches, c->prof, &c->fused, y_dev,
                                c->d_iperm);
     if (e == cudaSuccess) {
       e = launch_permute_ref(ydot_int, yd_dev, c->d_iperm, c->ne, c->nr, 0, c->stream);
@@ -517,7 +514,7 @@ static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, cp.arrived[s], 0);
   if (e == cudaSuccess) {
     c->m.diag = c->diag;
-    e = launch_rhs(c->m, out, in, c->stream, &c->launches, c->prof, &c->side, in, c->d_iperm);
+    e = launch_rhs(c->m, out, in, c->stream, &c->launches, c->prof, &c->fused, in, c->d_iperm);
   }
   if (e == cudaSuccess) {
     e = launch_permute(in, out, c->d_perm, c->ne, c->nr, 0, c->stream);

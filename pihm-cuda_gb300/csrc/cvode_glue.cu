@@ -39,7 +39,7 @@ static int ode_launch_device(pihm_gpu_ctx *c, N_Vector y, N_Vector ydot) {
   if (N_VGetLength_PihmGpu(y) != c->neq || N_VGetLength_PihmGpu(ydot) != c->neq) return -1;
   c->m.diag = c->diag;
   return pihm::launch_rhs(c->m, N_VGetDeviceArrayPointer_PihmGpu(y), N_VGetDeviceArrayPointer_PihmGpu(ydot),
-                          c->stream, &c->launches, c->prof, &c->side) == cudaSuccess
+                          c->stream, &c->launches, c->prof, &c->fused) == cudaSuccess
              ? 0
              : -1;
 }

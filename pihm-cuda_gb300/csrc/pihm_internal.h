@@ -263,33 +263,10 @@ struct FusedPlan {
 };
 cudaError_t fused_plan(FusedPlan *f);
 
-// A second stream on which the river kernel of an evaluation runs beside the
-// element kernels (it needs only k_elem_prep's outputs), joined before
-// k_finish.  Null members: everything on one stream.
-struct RhsStreams {
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  FusedPlan fused;
-};
-
-// The river kernel's stream and events.  The stream has the highest
-// priority the device offers, so that the few, long-running river blocks are
-// dispatched ahead of the element kernels' many short ones and finish under
-// them instead of after them.
-inline cudaError_t create_rhs_streams(RhsStreams *s) {
-  int least = 0, greatest = 0;
-  cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, greatest);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = fused_plan(&s->fused);
-  return e;
-}
-
 // y_ref, iperm (host-buffer evaluation of a single watershed): the state in
 // reference order, read by k_elem_prep, which fills y (internal order) from it.
 cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStream_t st,
-                       long long *launches, Profiler *prof, const RhsStreams *side = nullptr,
+                       long long *launches, Profiler *prof, const FusedPlan *fused = nullptr,
                        const double *y_ref = nullptr, const int32_t *iperm = nullptr);
 
 }  // namespace pihm
@@ -331,6 +308,6 @@ struct pihm_gpu_ctx {
   pihm::Profiler *prof;    // non-null while profiling is on
   void *d_noah;            // Flux-PIHM input planes, allocated on first use
   pihm::LandInstance land;  // land-surface model (pihm_gpu_land_init); alloc null when absent
-  pihm::RhsStreams side;   // river kernel beside the element kernels
+  pihm::FusedPlan fused;   // residency of the one-launch evaluation
   pihm::NoahInstance noahlsm;   // Noah land-surface model (pihm_gpu_noah_init); alloc null when absent
 };

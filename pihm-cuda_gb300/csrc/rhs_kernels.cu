@@ -1,11 +1,9 @@
 // FP64 right-hand-side kernels of the PIHM hydrologic model for sm_103a.
 //
 // One evaluation of f(t, y) (the reference ODE(), src/ode.c:4-399) runs as
-// seven launches with no host synchronisation, the three river kernels on a
-// second stream beside k_elem_grad/k_edge (k_edge is listed at its
-// definition: each interior edge is evaluated once and read with a sign by
-// both elements).  GB300 issues ~2 FP64 lanes per clock per SM, so the
-// FP64 pipe is the scarce one: the element rows' powers, divisions and
+// one cooperative launch (k_rhs_fused: small meshes) or five programmatic
+// dependent launches, with no host synchronisation.  An SM takes an FP64 warp
+// instruction every 20 clocks, so the FP64 pipe is the scarce one: the element rows' powers, divisions and
 // square roots run in fixed point on the integer pipe (int_math.cuh; the
 // divisions and roots IEEE-exact), comparisons and sign flips on the
 // integer pipe too (fp64_cmp.h), divisions by static quantities are
@@ -26,25 +24,26 @@
 //                 OvlFlowElemToElem, BoundFluxElem, src/lat_flow.c:285-382),
 //                 EtExtract (src/hydrol.c:33-97), Infil/Recharge/EffKinf/AvgKv
 //                 (src/vert_flow.c:33-270) and the element rows of ydot
-//                 (src/ode.c:111-209), the river banks' with this evaluation's
-//                 river-edge fluxes.
+//                 (src/ode.c:111-209) but for the river banks'.
+//   k_edge        per interior edge: the Darcy and Manning fluxes, evaluated
+//                 once and read with a sign by both elements.
 //   k_riv_geom    per segment: channel area and wetted perimeter at the
-//                 stage (src/river_flow.c:520-583), once per segment.
+//                 stage (src/river_flow.c:520-583), once per segment; part
+//                 of k_elem_prep's grid.
 //   k_river       per segment, in four parts: RiverFlow
 //                 (src/river_flow.c:3-94) and RiverToElem (:113-183), ChanLeak,
-//                 OutletFlux, BoundFluxRiver.
+//                 OutletFlux, BoundFluxRiver; part of k_elem_grad's grid.
 //   k_river_rows  per segment: upstream accumulation in reference order
 //                 (src/river_flow.c:96-110, a CSR list instead of a serial
-//                 loop) and the river rows of ydot (src/ode.c:228-300).
-//
-// The river kernels finish before k_elem_main starts, so the banks' rows need
-// no pass of their own after it: one (k_finish, latency-bound, 20 us of a
-// 355 us evaluation of 1M elements) stood at the end of the critical path.
+//                 loop) and the river rows of ydot (src/ode.c:228-300); part
+//                 of k_bank_rows's grid.
+//   k_bank_rows   per element with river edges: its rows of ydot from
+//                 k_elem_main's sums and the river fluxes.
 //
 // Infil reads the river-edge overland flux of the previous evaluation
 // (src/vert_flow.c:61 runs before src/river_flow.c:159-182 rewrites it); that
 // value is the previous evaluation's LEFT/RIGHT_SURF2CHANL in carry_ovl, which
-// the bank element's thread in k_elem_main reads and then replaces.
+// k_elem_main reads and k_bank_rows then replaces.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -147,6 +146,14 @@ __device__ __forceinline__ void kr_psi(double satn, double vm, double vg_e, doub
   }
 }
 
+// The large-mesh kernels are programmatic dependent launches: each waits for
+// the one before it where it first needs its results, and lets the next one's
+// blocks in once all of its own are past that wait -- so the kernel two ahead
+// is always finished.  What stands before a wait reads only what an earlier
+// evaluation or the caller left.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Batch engine: whether the watershed of item idx sits out this evaluation
 // (a free arena slot, or a watershed that did not ask for one).  Always false
 // in a single-watershed context.
@@ -220,6 +227,356 @@ __device__ __forceinline__ void prep_root(const DevMesh &m, int i, double sx) {
   m.head[i] = sh + m.zmax[i];
 }
 
+// ---------------------------------------------------------------------------
+// k_riv_geom: wetted perimeter and cross-section area of every segment at its
+// stage (RivPerim / RivCsArea, src/river_flow.c:520-583), once per segment
+// and evaluation (k_river needs them for the segment and for its downstream
+// neighbour), with the coefficient-only factors formed at load (r_geo*, in
+// the order the shape's formula uses them):
+//   rectangle  area d c,           perimeter 2 d + c
+//   triangle   area d^2 / c,       perimeter 2 d sqrt(1 + c^2) / c
+//   quadratic  area 4 d^1.5 / (3 sqrt c),
+//              perimeter sqrt(d (1 + 4 c d) / c) + ln(2 sqrt(c d) + sqrt(1 + 4 c d)) / (2 c)
+//   cubic      area 3 d^(4/3) / (2 c^(1/3)),
+//              perimeter 2 (sqrt(d (1 + 9 c^(2/3) d)) / 3
+//                           + ln(3 c^(1/3) sqrt(d) + sqrt(1 + 9 c^(2/3) d)) / (9 c^(1/3)))
+// The reference's pow(x, 0.5) is sqrt(x).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double log_of(double x) {
+  double sh, lo;
+  return log_dd_fast(x, sh, lo) ? sh + lo : log(x);
+}
+
+__device__ __forceinline__ void geom_item(const DevMesh &m, const double *y, int s) {
+  double d = y[3 * m.ne + s];
+  d = cmp::gt0(d) ? d : 0.0;
+  const double g0 = m.r_geo0[s];
+  double area = 0.0, perim = 0.0;
+  switch (m.intrpl_ord[s]) {
+    case kRectangle:
+      area = d * g0;
+      perim = 2.0 * d + g0;
+      break;
+    case kTriangle:
+      area = d * d * g0;
+      perim = d * m.r_geo1[s];
+      break;
+    case kQuadratic:
+    case kCubic: {
+      // one path for both shapes, so that a warp with segments of both runs
+      // the roots and the logarithm once
+      const bool cub = m.intrpl_ord[s] == kCubic;
+      const double sd = sqrt_any(d), w = 1.0 + m.r_geo1[s] * d;
+      const double g2 = m.r_geo2[s], dw = d * w;
+      const double root = sqrt_any(cub ? dw : dw * g2);
+      const double lg = log_of((cub ? g2 : m.r_geo4[s]) * sd + sqrt_any(w));
+      area = cub ? g0 * pow_fast(d, 4.0 / 3.0) : g0 * d * sd;
+      perim = cub ? 2.0 * (root * (1.0 / 3.0) + lg * m.r_geo3[s]) : root + lg * m.r_geo3[s];
+      break;
+    }
+  }
+  m.r_perim[s] = perim;
+  m.r_crossa[s] = area;
+}
+
+__global__ void __launch_bounds__(128) k_riv_geom(DevMesh m, const double *RESTRICT y) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  int sy;
+  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  geom_item(m, y, s);
+}
+
+// ---------------------------------------------------------------------------
+// k_river
+// ---------------------------------------------------------------------------
+struct RivState {
+  double stage, gw, zbed, zmin, zmax, length, width, rough;
+};
+
+__device__ __forceinline__ RivState load_riv(const DevMesh &m, const double *y, int s) {
+  RivState r;
+  r.stage = clamp0(y[3 * m.ne + s]);
+  r.gw = clamp0(y[3 * m.ne + m.nr + s]);
+  r.zbed = m.r_zbed[s];
+  r.zmin = m.r_zmin[s];
+  r.zmax = m.r_zmax[s];
+  r.length = m.r_length[s];
+  r.width = m.r_width[s];
+  r.rough = m.r_rough[s];
+  return r;
+}
+
+// OvlFlowElemToRiver, src/river_flow.c:185-255, with the weir coefficient
+// cwr 2 sqrt(2 g) length / 3 formed at load (coef)
+__device__ __forceinline__ double ovl_elem_to_river(double e_zmax, double e_surfh, const RivState &r,
+                                                    double coef) {
+  const double zbank = cmp::gt_v(r.zmax, e_zmax) ? r.zmax : e_zmax;
+  const double elem_h = e_zmax + e_surfh;
+  const double rivseg_h = r.zbed + r.stage;
+  // the four cases differ in the head under the root and the head over the
+  // bank: one root and one product serve a warp whose lanes take them all
+  const bool out = cmp::gt_v(rivseg_h, elem_h);
+  if (!out && !cmp::gt_c(e_surfh, kDeprStg)) return 0.0;
+  const double high = out ? rivseg_h : elem_h, low = out ? elem_h : rivseg_h;
+  const bool drowned = cmp::gt_v(low, zbank);  // the lower side stands above the bank too
+  if (!drowned && !cmp::lt_v(zbank, high)) return 0.0;
+  const double over = high - zbank;
+  const double root = sqrt_any(drowned ? high - low : over);
+  return (out ? coef : -coef) * root * over;
+}
+
+// ChanFlowElemToRiver, src/river_flow.c:429-460
+__device__ __forceinline__ double chan_elem_to_river(double e_gw, double e_zmin, double effk,
+                                                     const RivState &r, double r_ksath,
+                                                     double inv_distance) {
+  const double diff_h = (r.stage + r.zbed) - (e_gw + e_zmin);
+  double avg_h;
+  if (cmp::gt_v(e_zmin, r.zbed)) avg_h = e_gw;
+  else if (cmp::gt_v(e_zmin + e_gw, r.zbed)) avg_h = e_zmin + e_gw - r.zbed;
+  else avg_h = 0.0;
+  avg_h = avg_h_sub(diff_h, r.stage, avg_h);
+  const double grad_h = diff_h * inv_distance;
+  const double avg_ksat = 0.5 * (effk + r_ksath);
+  return r.length * avg_ksat * grad_h * avg_h;
+}
+
+// SubFlowElemToRiver, src/river_flow.c:462-498 (arithmetic mean)
+__device__ __forceinline__ double sub_elem_to_river(double e_gw, double e_zmin, double effk,
+                                                    const RivState &r, double effk_riv,
+                                                    double inv_distance) {
+  const double diff_h = (r.gw + r.zmin) - (e_gw + e_zmin);
+  double avg_h;
+  if (cmp::gt_v(e_zmin, r.zbed)) avg_h = 0.0;
+  else if (cmp::gt_v(e_zmin + e_gw, r.zbed)) avg_h = r.zbed - e_zmin;
+  else avg_h = e_gw;
+  avg_h = avg_h_sub(diff_h, r.gw, avg_h);
+  const double avg_ksat = 0.5 * (effk + effk_riv);
+  const double grad_h = diff_h * inv_distance;
+  return r.length * avg_ksat * grad_h * avg_h;
+}
+
+// OutletFlux, src/river_flow.c:333-390
+__device__ __forceinline__ void outlet_flux(const DevMesh &m, const RivState &r, int s, int down) {
+  const int nr = m.nr;
+  double dnf;
+  const double depth = m.r_depth[s];
+  const double bc = m.river_bc[s];
+  if (down == kDirichlet) {
+    const double total_h = r.stage + r.zbed;
+    const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
+    const double avg_perim = m.r_perim[s];
+    const double crossa = m.r_crossa[s];
+    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
+    dnf = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+  } else if (down == kNeumann) {
+    dnf = -bc;
+  } else if (down == kZeroDpthGrad) {
+    const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
+    const double avg_perim = m.r_perim[s];
+    const double crossa = m.r_crossa[s];
+    dnf = div_any(sqrt_any(grad_h) * crossa *
+                      (cmp::gt0(avg_perim) ? pow_manning(div_any(crossa, avg_perim), kManningRiv) : 0.0),
+                  r.rough);
+  } else {  // kCritDpth (other values are rejected at load)
+    const double crossa = m.r_crossa[s];
+    dnf = crossa * sqrt_any(kGrav * r.stage);
+  }
+  m.rivflow[UP_CHANL2CHANL * nr + s] = 0.0;
+  m.rivflow[DOWN_CHANL2CHANL * nr + s] = dnf;
+}
+
+// A segment's fluxes in four parts that share no result: the channel flux,
+// the two banks, and the bed's.  One thread per part: a segment's fluxes are a
+// chain of FP64 divisions, roots and a power (18 us for 100 segments or
+// 12,000 with one thread per segment), and the parts run beside each other.
+// An outlet's channel flux goes with its bed, the shortest part: with the
+// channel fluxes of its warp it took the warp 2 us longer than the others.
+enum RivPart { PART_CHAN = 0, PART_LEFT, PART_RIGHT, PART_BED, kRivParts };
+
+__device__ __forceinline__ void river_part(const DevMesh &m, const double *y, int s, int part) {
+  const int nr = m.nr, ne = m.ne;
+  double *F = m.rivflow;
+  const RivState r = load_riv(m, y, s);
+  if (part == PART_CHAN) {
+    const int down = m.down[s];
+    if (down <= 0) return;  // an outlet: the bed's part
+    double up = 0.0;
+    const int bct = m.bctype_riv[s];
+    if (bct != 0) {
+      // BoundFluxRiver, src/river_flow.c:392-427
+      double flux = 0.0;
+      const double bc = m.river_bc[s];
+      if (bct > 0) {
+        const double total_h = r.stage + r.zbed;
+        const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
+        const double avg_perim = m.r_perim[s];
+        const double crossa = m.r_crossa[s];
+        const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
+        flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
+      } else {
+        flux = -bc;
+      }
+      up += flux;
+    }
+    const int d = down - 1;
+    const RivState dn = load_riv(m, y, d);
+    const double inv_dist_down = m.r_inv_dist_down[s];
+    // ChanFlowRiverToRiver, src/river_flow.c:257-300
+    const double total_h = r.stage + r.zbed;
+    const double perim = m.r_perim[s];
+    const double total_h_down = dn.stage + dn.zbed;
+    const double perim_down = m.r_perim[d];
+    const double avg_perim = (perim + perim_down) / 2.0;
+    const double avg_rough = (r.rough + dn.rough) / 2.0;
+    const double diff_h = (m.riv_mode == kKinematic) ? (r.zbed - dn.zbed) : (total_h - total_h_down);
+    const double grad_h = diff_h * inv_dist_down;
+    const double avg_sf = cmp::gt0(grad_h) ? grad_h : kRivGradMin;
+    const double crossa = m.r_crossa[s];
+    const double crossa_down = m.r_crossa[d];
+    const double avg_crossa = 0.5 * (crossa + crossa_down);
+    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(avg_crossa, avg_perim);
+    const double dnf = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
+    F[UP_CHANL2CHANL * nr + s] = up;
+    F[DOWN_CHANL2CHANL * nr + s] = dnf;
+    return;
+  }
+  const int L = m.left[s], R = m.right[s];
+  const double effk_l = m.effk[L], effk_r = m.effk[R];
+  if (part == PART_BED) {
+    const int down = m.down[s];
+    double aq = 0.0;
+    if (down > 0) {
+      // SubFlowRiverToRiver, src/river_flow.c:302-331 (arithmetic mean)
+      const int d = down - 1;
+      const RivState dn = load_riv(m, y, d);
+      const double effk = 0.5 * (effk_l + effk_r);
+      const double effk_nabr = 0.5 * (m.effk[m.left[d]] + m.effk[m.right[d]]);
+      const double total_h = r.gw + r.zmin;
+      const double total_h_down = dn.gw + dn.zmin;
+      const double avg_wid = (r.width + dn.width) / 2.0;
+      const double diff_h = total_h - total_h_down;
+      const double avg_h = avg_h_sub(diff_h, r.gw, dn.gw);
+      const double grad_h = diff_h * m.r_inv_dist_down[s];
+      const double avg_ksat = 0.5 * (effk + effk_nabr);
+      aq = avg_ksat * grad_h * avg_h * avg_wid;
+    }
+    F[DOWN_AQUIF2AQUIF * nr + s] = aq;
+    F[UP_AQUIF2AQUIF * nr + s] = 0.0;
+    // ChanLeak, src/river_flow.c:500-518
+    double diff_h;
+    if (cmp::gt0(r.zbed - (r.gw + r.zmin))) diff_h = r.stage;
+    else diff_h = r.stage + r.zbed - (r.gw + r.zmin);
+    const double grad_h = diff_h * m.r_inv_bedthick[s];
+    F[CHANL_LKG * nr + s] = m.r_ksatv[s] * r.width * r.length * grad_h;
+    if (down <= 0) outlet_flux(m, r, s, down);
+    return;
+  }
+  // RiverToElem, src/river_flow.c:113-183, one bank
+  const bool left = part == PART_LEFT;
+  const int e = left ? L : R;
+  const double effk_e = left ? effk_l : effk_r;
+  const double inv_d = left ? m.r_inv_dist_left[s] : m.r_inv_dist_right[s];
+  const double gw_e = clamp0(y[2 * ne + e]), zmin_e = m.zmin[e];
+  F[(left ? LEFT_SURF2CHANL : RIGHT_SURF2CHANL) * nr + s] =
+      ovl_elem_to_river(m.zmax[e], m.surfh[e], r, m.r_ovl_coef[s]);
+  F[(left ? LEFT_AQUIF2CHANL : RIGHT_AQUIF2CHANL) * nr + s] =
+      chan_elem_to_river(gw_e, zmin_e, effk_e, r, m.r_ksath[s], inv_d);
+  const double effk_avg = 0.5 * (effk_l + effk_r);
+  F[(left ? LEFT_AQUIF2AQUIF : RIGHT_AQUIF2AQUIF) * nr + s] =
+      sub_elem_to_river(gw_e, zmin_e, effk_e, r, effk_avg, inv_d);
+}
+
+// part-major, each part's segments padded to whole warps
+__global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT y) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int pad = (m.nr_run + 31) & ~31;
+  const int part = t / pad, s = t - part * pad;
+  int sy;
+  if (part >= kRivParts || s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  river_part(m, y, s, part);
+}
+
+// ---------------------------------------------------------------------------
+// k_river_rows: upstream sums and the river rows of ydot
+// ---------------------------------------------------------------------------
+// What a river row reads of the mesh: the first upstream segments' indices
+// are a chain of loads in front of their fluxes.
+struct RiverRowsIn {
+  double area, porosity;
+  int first, end, up[3];
+};
+__device__ __forceinline__ RiverRowsIn river_rows_load(const DevMesh &m, int s) {
+  RiverRowsIn r;
+  r.area = m.r_area[s];
+  r.porosity = m.r_porosity[s];
+  r.first = m.up_ptr[s];
+  r.end = m.up_end[s];
+#pragma unroll
+  for (int k = 0; k < 3; k++) r.up[k] = r.first + k < r.end ? m.up_idx[r.first + k] : 0;
+  return r;
+}
+
+// the quotients of a row, beside each other
+__device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, int s, int sy, const RiverRowsIn &r) {
+  const int nr = m.nr, ne = m.ne;
+  const double *F = m.rivflow;
+  double f[7];
+  f[0] = F[UP_CHANL2CHANL * nr + s];
+#pragma unroll
+  for (int j = 1; j <= 6; j++) f[j] = F[j * nr + s];
+  const double aq_l = F[LEFT_AQUIF2AQUIF * nr + s], aq_r = F[RIGHT_AQUIF2AQUIF * nr + s];
+  const double aq_d = F[DOWN_AQUIF2AQUIF * nr + s];
+  const double area = r.area, por_area = r.porosity * area;
+  double up_c = f[0];
+  double up_a = 0.0;
+  double fc[3], fa[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    fc[k] = F[DOWN_CHANL2CHANL * nr + r.up[k]];
+    fa[k] = F[DOWN_AQUIF2AQUIF * nr + r.up[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (r.first + k < r.end) {
+      up_c -= fc[k];
+      up_a -= fa[k];
+    }
+  for (int k = r.first + 3; k < r.end; k++) {
+    const int u = m.up_idx[k];
+    up_c -= F[DOWN_CHANL2CHANL * nr + u];
+    up_a -= F[DOWN_AQUIF2AQUIF * nr + u];
+  }
+  f[0] = up_c;
+  double dg = -aq_l - aq_r - aq_d - up_a + f[CHANL_LKG];
+  double q[7], qg;
+  bool ok = im::div_i(dg, por_area, qg);
+#pragma unroll
+  for (int j = 0; j <= 6; j++) ok &= im::div_i(f[j], area, q[j]);
+  if (!ok) {
+    qg = div_any(dg, por_area);
+#pragma unroll
+    for (int j = 0; j <= 6; j++) q[j] = div_any(f[j], area);
+  }
+  dg = qg;
+  double ds = 0.0;
+#pragma unroll
+  for (int j = 0; j <= 6; j++) ds -= q[j];
+  ydot[3 * ne + s] = ds;
+  ydot[3 * ne + nr + s] = dg;
+  if (m.diag) {
+    m.rivflow[UP_CHANL2CHANL * nr + s] = up_c;
+    m.rivflow[UP_AQUIF2AQUIF * nr + s] = up_a;
+  }
+  if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
+}
+
+__global__ void __launch_bounds__(128) k_river_rows(DevMesh m, double *RESTRICT ydot) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  int sy;
+  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
+  river_rows_item(m, ydot, s, sy, river_rows_load(m, s));
+}
+
 // kFromRef: the host-buffer evaluation, where the state arrives in reference
 // order in memory the device reads over the host link.  Thread r then takes
 // reference element r (the link read is contiguous), stores its three values
@@ -229,20 +586,26 @@ __device__ __forceinline__ void prep_root(const DevMesh &m, int i, double sx) {
 template <bool kFromRef>
 __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const double *RESTRICT y,
                                                           const double *RESTRICT y_ref, double *RESTRICT y_int,
-                                                          const int32_t *RESTRICT iperm) {
+                                                          const int32_t *RESTRICT iperm, int river_blocks) {
   __shared__ int qs_i[kPrepBlock], qd_i[kPrepBlock];
   __shared__ double qs_x[kPrepBlock], qd_num[kPrepBlock], qd_den[kPrepBlock];
   __shared__ int qs_n, qd_n;
+  int sy = 0;
+  next_may_start();
+  if ((int)blockIdx.x < river_blocks) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < m.nr_run && !skip_item(m, m.sys_riv, s, &sy)) geom_item(m, kFromRef ? y_ref : y, s);
+    return;
+  }
   if (threadIdx.x == 0) {
     qs_n = 0;
     qd_n = 0;
   }
   __syncthreads();
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t0 = (blockIdx.x - river_blocks) * blockDim.x + threadIdx.x;
   int i = t0;
   double y_surf = 0.0, y_gw = 0.0;
   bool elem;
-  int sy = 0;
   if (kFromRef) {
     const int ne = m.ne;
     elem = t0 < ne;
@@ -335,11 +698,27 @@ __device__ __forceinline__ double grad_value(const DevMesh &m, const GradIn &g) 
   return sqrt_any(dhdx * dhdx + dhdy * dhdy);
 }
 
-__global__ void __launch_bounds__(256) k_elem_grad(DevMesh m, const double *RESTRICT y) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// (40 registers, the gradient's own need: the river fluxes' 50 would keep a
+// sixth of the SM's warps out)
+__global__ void __launch_bounds__(256, 6) k_elem_grad(DevMesh m, const double *y, int river_blocks, bool from_ref) {
   int sy;
-  if (i >= m.ne_run || skip_item(m, m.sys_elem, i, &sy)) return;
-  m.gradmag[i] = grad_value(m, grad_load(m, y, i));
+  if ((int)blockIdx.x < river_blocks) {
+    wait_for_previous();
+    next_may_start();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int pad = (m.nr_run + 31) & ~31;
+    const int part = t / pad, s = t - part * pad;
+    if (part < kRivParts && s < m.nr_run && !skip_item(m, m.sys_riv, s, &sy)) river_part(m, y, s, part);
+    return;
+  }
+  const int i = (blockIdx.x - river_blocks) * blockDim.x + threadIdx.x;
+  const bool on = i < m.ne_run && !skip_item(m, m.sys_elem, i, &sy);
+  GradIn g;
+  if (on && !from_ref) g = grad_load(m, y, i);
+  wait_for_previous();
+  next_may_start();
+  if (on && from_ref) g = grad_load(m, y, i);
+  if (on) m.gradmag[i] = grad_value(m, g);
 }
 
 // ---------------------------------------------------------------------------
@@ -396,7 +775,7 @@ __device__ __forceinline__ double edge_slope(const DevMesh &m, int e, int i, int
 }
 __device__ __forceinline__ double edge_hp(double h) { return h * pow_manning(h, kManningSurf); }
 
-__global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RESTRICT y) {
+__global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *y) {
   __shared__ int q_e[kEdgeBlock];
   __shared__ double q_h[kEdgeBlock], q_d[kEdgeBlock], q_sf[kEdgeBlock];
   __shared__ int q_n;
@@ -406,8 +785,15 @@ __global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RE
   int sy;
   bool wet = false;
   double avg_h = 0.0, diff_h = 0.0, avg_sf = 0.0;
-  if (e < m.nedge_run && !skip_item(m, m.sys_edge, e, &sy)) {
-    const int i = m.e_i[e], k = m.e_k[e];
+  int i = 0, k = 0;
+  const bool on = e < m.nedge_run && !skip_item(m, m.sys_edge, e, &sy);
+  if (on) {
+    i = m.e_i[e];
+    k = m.e_k[e];
+  }
+  wait_for_previous();
+  next_may_start();
+  if (on) {
     wet = edge_item(m, y, e, i, k, avg_h, diff_h);
     avg_sf = edge_slope(m, e, i, k, diff_h);
   }
@@ -448,10 +834,10 @@ __global__ void __launch_bounds__(kEdgeBlock) k_edge(DevMesh m, const double *RE
 // watershed without an evaluation) sort last and leave as whole warps.
 constexpr int kElemClasses = 8;
 
-__device__ __forceinline__ int elem_class(const DevMesh &m, const double *RESTRICT y, int i) {
+__device__ __forceinline__ int elem_class(const DevMesh &m, const double *y, int i) {
   const int ne = m.ne;
   const double gw = clamp0(y[2 * ne + i]);
-  const int ponded = cmp::gt_c(m.surfh[i], kDeprStg) ? 1 : 0;
+  const int ponded = cmp::gt_c(clamp0(y[i]), 0.5 * kDeprStg) ? 1 : 0;  // SurfH above the depression storage
   if (cmp::gt_v(gw, m.d_dinf[i])) return 4 + ponded;
   return 2 * ponded + (cmp::lt_v(gw, m.d_dmac[i]) ? 1 : 0);
 }
@@ -805,8 +1191,11 @@ __device__ __forceinline__ void column_rows(const DevMesh &m, double *ydot, int 
 }
 
 template <int BLOCK, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) k_elem_main(DevMesh m, const double *RESTRICT y,
-                                                    double *RESTRICT ydot) {
+__global__ void __launch_bounds__(BLOCK, MINB) k_elem_main(DevMesh m, const double *y, double *RESTRICT ydot,
+                                                           bool from_ref) {
+  // the state itself may be read before the kernels ahead have finished,
+  // unless they wrote it
+  if (from_ref) wait_for_previous();
   // a stable ranking: class-major, then warp, then lane, so each class keeps
   // the block's element order and a warp's elements lie close together
   constexpr int kWarps = BLOCK / 32, kSlots = kElemClasses * kWarps;
@@ -855,9 +1244,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_elem_main(DevMesh m, const doub
   }
   const int i = blockIdx.x * BLOCK + s_order[threadIdx.x];
   int sy;
-  if (i >= m.ne_run || skip_item(m, m.sys_elem, i, &sy)) return;
+  const bool on = i < m.ne_run && !skip_item(m, m.sys_elem, i, &sy);
   Column c;
-  column_state(m, y, i, sy, c);
+  if (on) column_state(m, y, i, sy, c);
+  wait_for_previous();
+  next_may_start();
+  if (!on) return;
   column_surface(m, i, c);
   RowsIn r;
   rows_load(m, i, r);
@@ -865,397 +1257,75 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_elem_main(DevMesh m, const doub
 }
 
 // ---------------------------------------------------------------------------
-// k_riv_geom: wetted perimeter and cross-section area of every segment at its
-// stage (RivPerim / RivCsArea, src/river_flow.c:520-583), once per segment
-// and evaluation (k_river needs them for the segment and for its downstream
-// neighbour), with the coefficient-only factors formed at load (r_geo*, in
-// the order the shape's formula uses them):
-//   rectangle  area d c,           perimeter 2 d + c
-//   triangle   area d^2 / c,       perimeter 2 d sqrt(1 + c^2) / c
-//   quadratic  area 4 d^1.5 / (3 sqrt c),
-//              perimeter sqrt(d (1 + 4 c d) / c) + ln(2 sqrt(c d) + sqrt(1 + 4 c d)) / (2 c)
-//   cubic      area 3 d^(4/3) / (2 c^(1/3)),
-//              perimeter 2 (sqrt(d (1 + 9 c^(2/3) d)) / 3
-//                           + ln(3 c^(1/3) sqrt(d) + sqrt(1 + 9 c^(2/3) d)) / (9 c^(1/3)))
-// The reference's pow(x, 0.5) is sqrt(x).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double log_of(double x) {
-  double sh, lo;
-  return log_dd_fast(x, sh, lo) ? sh + lo : log(x);
-}
-
-__device__ __forceinline__ void geom_item(const DevMesh &m, const double *y, int s) {
-  double d = y[3 * m.ne + s];
-  d = cmp::gt0(d) ? d : 0.0;
-  const double g0 = m.r_geo0[s];
-  double area = 0.0, perim = 0.0;
-  switch (m.intrpl_ord[s]) {
-    case kRectangle:
-      area = d * g0;
-      perim = 2.0 * d + g0;
-      break;
-    case kTriangle:
-      area = d * d * g0;
-      perim = d * m.r_geo1[s];
-      break;
-    case kQuadratic:
-    case kCubic: {
-      // one path for both shapes, so that a warp with segments of both runs
-      // the roots and the logarithm once
-      const bool cub = m.intrpl_ord[s] == kCubic;
-      const double sd = sqrt_any(d), w = 1.0 + m.r_geo1[s] * d;
-      const double g2 = m.r_geo2[s], dw = d * w;
-      const double root = sqrt_any(cub ? dw : dw * g2);
-      const double lg = log_of((cub ? g2 : m.r_geo4[s]) * sd + sqrt_any(w));
-      area = cub ? g0 * pow_fast(d, 4.0 / 3.0) : g0 * d * sd;
-      perim = cub ? 2.0 * (root * (1.0 / 3.0) + lg * m.r_geo3[s]) : root + lg * m.r_geo3[s];
-      break;
-    }
-  }
-  m.r_perim[s] = perim;
-  m.r_crossa[s] = area;
-}
-
-__global__ void __launch_bounds__(128) k_riv_geom(DevMesh m, const double *RESTRICT y) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int sy;
-  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
-  geom_item(m, y, s);
-}
-
-// ---------------------------------------------------------------------------
-// k_river
-// ---------------------------------------------------------------------------
-struct RivState {
-  double stage, gw, zbed, zmin, zmax, length, width, rough;
-};
-
-__device__ __forceinline__ RivState load_riv(const DevMesh &m, const double *y, int s) {
-  RivState r;
-  r.stage = clamp0(y[3 * m.ne + s]);
-  r.gw = clamp0(y[3 * m.ne + m.nr + s]);
-  r.zbed = m.r_zbed[s];
-  r.zmin = m.r_zmin[s];
-  r.zmax = m.r_zmax[s];
-  r.length = m.r_length[s];
-  r.width = m.r_width[s];
-  r.rough = m.r_rough[s];
-  return r;
-}
-
-// OvlFlowElemToRiver, src/river_flow.c:185-255, with the weir coefficient
-// cwr 2 sqrt(2 g) length / 3 formed at load (coef)
-__device__ __forceinline__ double ovl_elem_to_river(double e_zmax, double e_surfh, const RivState &r,
-                                                    double coef) {
-  const double zbank = cmp::gt_v(r.zmax, e_zmax) ? r.zmax : e_zmax;
-  const double elem_h = e_zmax + e_surfh;
-  const double rivseg_h = r.zbed + r.stage;
-  // the four cases differ in the head under the root and the head over the
-  // bank: one root and one product serve a warp whose lanes take them all
-  const bool out = cmp::gt_v(rivseg_h, elem_h);
-  if (!out && !cmp::gt_c(e_surfh, kDeprStg)) return 0.0;
-  const double high = out ? rivseg_h : elem_h, low = out ? elem_h : rivseg_h;
-  const bool drowned = cmp::gt_v(low, zbank);  // the lower side stands above the bank too
-  if (!drowned && !cmp::lt_v(zbank, high)) return 0.0;
-  const double over = high - zbank;
-  const double root = sqrt_any(drowned ? high - low : over);
-  return (out ? coef : -coef) * root * over;
-}
-
-// ChanFlowElemToRiver, src/river_flow.c:429-460
-__device__ __forceinline__ double chan_elem_to_river(double e_gw, double e_zmin, double effk,
-                                                     const RivState &r, double r_ksath,
-                                                     double inv_distance) {
-  const double diff_h = (r.stage + r.zbed) - (e_gw + e_zmin);
-  double avg_h;
-  if (cmp::gt_v(e_zmin, r.zbed)) avg_h = e_gw;
-  else if (cmp::gt_v(e_zmin + e_gw, r.zbed)) avg_h = e_zmin + e_gw - r.zbed;
-  else avg_h = 0.0;
-  avg_h = avg_h_sub(diff_h, r.stage, avg_h);
-  const double grad_h = diff_h * inv_distance;
-  const double avg_ksat = 0.5 * (effk + r_ksath);
-  return r.length * avg_ksat * grad_h * avg_h;
-}
-
-// SubFlowElemToRiver, src/river_flow.c:462-498 (arithmetic mean)
-__device__ __forceinline__ double sub_elem_to_river(double e_gw, double e_zmin, double effk,
-                                                    const RivState &r, double effk_riv,
-                                                    double inv_distance) {
-  const double diff_h = (r.gw + r.zmin) - (e_gw + e_zmin);
-  double avg_h;
-  if (cmp::gt_v(e_zmin, r.zbed)) avg_h = 0.0;
-  else if (cmp::gt_v(e_zmin + e_gw, r.zbed)) avg_h = r.zbed - e_zmin;
-  else avg_h = e_gw;
-  avg_h = avg_h_sub(diff_h, r.gw, avg_h);
-  const double avg_ksat = 0.5 * (effk + effk_riv);
-  const double grad_h = diff_h * inv_distance;
-  return r.length * avg_ksat * grad_h * avg_h;
-}
-
-// OutletFlux, src/river_flow.c:333-390
-__device__ __forceinline__ void outlet_flux(const DevMesh &m, const RivState &r, int s, int down) {
-  const int nr = m.nr;
-  double dnf;
-  const double depth = m.r_depth[s];
-  const double bc = m.river_bc[s];
-  if (down == kDirichlet) {
-    const double total_h = r.stage + r.zbed;
-    const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
-    const double avg_perim = m.r_perim[s];
-    const double crossa = m.r_crossa[s];
-    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
-    dnf = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-  } else if (down == kNeumann) {
-    dnf = -bc;
-  } else if (down == kZeroDpthGrad) {
-    const double grad_h = (r.zbed - (m.r_node_zmax[s] - depth)) * m.r_inv_half_len[s];
-    const double avg_perim = m.r_perim[s];
-    const double crossa = m.r_crossa[s];
-    dnf = div_any(sqrt_any(grad_h) * crossa *
-                      (cmp::gt0(avg_perim) ? pow_manning(div_any(crossa, avg_perim), kManningRiv) : 0.0),
-                  r.rough);
-  } else {  // kCritDpth (other values are rejected at load)
-    const double crossa = m.r_crossa[s];
-    dnf = crossa * sqrt_any(kGrav * r.stage);
-  }
-  m.rivflow[UP_CHANL2CHANL * nr + s] = 0.0;
-  m.rivflow[DOWN_CHANL2CHANL * nr + s] = dnf;
-}
-
-// A segment's fluxes in four parts that share no result: the channel flux,
-// the two banks, and the bed's.  One thread per part: a segment's fluxes are a
-// chain of FP64 divisions, roots and a power (18 us for 100 segments or
-// 12,000 with one thread per segment), and the parts run beside each other.
-// An outlet's channel flux goes with its bed, the shortest part: with the
-// channel fluxes of its warp it took the warp 2 us longer than the others.
-enum RivPart { PART_CHAN = 0, PART_LEFT, PART_RIGHT, PART_BED, kRivParts };
-
-__device__ __forceinline__ void river_part(const DevMesh &m, const double *y, int s, int part) {
-  const int nr = m.nr, ne = m.ne;
-  double *F = m.rivflow;
-  const RivState r = load_riv(m, y, s);
-  if (part == PART_CHAN) {
-    const int down = m.down[s];
-    if (down <= 0) return;  // an outlet: the bed's part
-    double up = 0.0;
-    const int bct = m.bctype_riv[s];
-    if (bct != 0) {
-      // BoundFluxRiver, src/river_flow.c:392-427
-      double flux = 0.0;
-      const double bc = m.river_bc[s];
-      if (bct > 0) {
-        const double total_h = r.stage + r.zbed;
-        const double grad_h = (total_h - bc) * m.r_inv_half_len[s];
-        const double avg_perim = m.r_perim[s];
-        const double crossa = m.r_crossa[s];
-        const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(crossa, avg_perim);
-        flux = overland_flow(avg_h, grad_h, grad_h, crossa, r.rough);
-      } else {
-        flux = -bc;
-      }
-      up += flux;
-    }
-    const int d = down - 1;
-    const RivState dn = load_riv(m, y, d);
-    const double inv_dist_down = m.r_inv_dist_down[s];
-    // ChanFlowRiverToRiver, src/river_flow.c:257-300
-    const double total_h = r.stage + r.zbed;
-    const double perim = m.r_perim[s];
-    const double total_h_down = dn.stage + dn.zbed;
-    const double perim_down = m.r_perim[d];
-    const double avg_perim = (perim + perim_down) / 2.0;
-    const double avg_rough = (r.rough + dn.rough) / 2.0;
-    const double diff_h = (m.riv_mode == kKinematic) ? (r.zbed - dn.zbed) : (total_h - total_h_down);
-    const double grad_h = diff_h * inv_dist_down;
-    const double avg_sf = cmp::gt0(grad_h) ? grad_h : kRivGradMin;
-    const double crossa = m.r_crossa[s];
-    const double crossa_down = m.r_crossa[d];
-    const double avg_crossa = 0.5 * (crossa + crossa_down);
-    const double avg_h = cmp::eq0(avg_perim) ? 0.0 : div_any(avg_crossa, avg_perim);
-    const double dnf = overland_flow(avg_h, grad_h, avg_sf, crossa, avg_rough);
-    F[UP_CHANL2CHANL * nr + s] = up;
-    F[DOWN_CHANL2CHANL * nr + s] = dnf;
-    return;
-  }
-  const int L = m.left[s], R = m.right[s];
-  const double effk_l = m.effk[L], effk_r = m.effk[R];
-  if (part == PART_BED) {
-    const int down = m.down[s];
-    double aq = 0.0;
-    if (down > 0) {
-      // SubFlowRiverToRiver, src/river_flow.c:302-331 (arithmetic mean)
-      const int d = down - 1;
-      const RivState dn = load_riv(m, y, d);
-      const double effk = 0.5 * (effk_l + effk_r);
-      const double effk_nabr = 0.5 * (m.effk[m.left[d]] + m.effk[m.right[d]]);
-      const double total_h = r.gw + r.zmin;
-      const double total_h_down = dn.gw + dn.zmin;
-      const double avg_wid = (r.width + dn.width) / 2.0;
-      const double diff_h = total_h - total_h_down;
-      const double avg_h = avg_h_sub(diff_h, r.gw, dn.gw);
-      const double grad_h = diff_h * m.r_inv_dist_down[s];
-      const double avg_ksat = 0.5 * (effk + effk_nabr);
-      aq = avg_ksat * grad_h * avg_h * avg_wid;
-    }
-    F[DOWN_AQUIF2AQUIF * nr + s] = aq;
-    F[UP_AQUIF2AQUIF * nr + s] = 0.0;
-    // ChanLeak, src/river_flow.c:500-518
-    double diff_h;
-    if (cmp::gt0(r.zbed - (r.gw + r.zmin))) diff_h = r.stage;
-    else diff_h = r.stage + r.zbed - (r.gw + r.zmin);
-    const double grad_h = diff_h * m.r_inv_bedthick[s];
-    F[CHANL_LKG * nr + s] = m.r_ksatv[s] * r.width * r.length * grad_h;
-    if (down <= 0) outlet_flux(m, r, s, down);
-    return;
-  }
-  // RiverToElem, src/river_flow.c:113-183, one bank
-  const bool left = part == PART_LEFT;
-  const int e = left ? L : R;
-  const double effk_e = left ? effk_l : effk_r;
-  const double inv_d = left ? m.r_inv_dist_left[s] : m.r_inv_dist_right[s];
-  const double gw_e = clamp0(y[2 * ne + e]), zmin_e = m.zmin[e];
-  F[(left ? LEFT_SURF2CHANL : RIGHT_SURF2CHANL) * nr + s] =
-      ovl_elem_to_river(m.zmax[e], m.surfh[e], r, m.r_ovl_coef[s]);
-  F[(left ? LEFT_AQUIF2CHANL : RIGHT_AQUIF2CHANL) * nr + s] =
-      chan_elem_to_river(gw_e, zmin_e, effk_e, r, m.r_ksath[s], inv_d);
-  const double effk_avg = 0.5 * (effk_l + effk_r);
-  F[(left ? LEFT_AQUIF2AQUIF : RIGHT_AQUIF2AQUIF) * nr + s] =
-      sub_elem_to_river(gw_e, zmin_e, effk_e, r, effk_avg, inv_d);
-}
-
-// part-major, each part's segments padded to whole warps
-__global__ void __launch_bounds__(128) k_river(DevMesh m, const double *RESTRICT y) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int pad = (m.nr_run + 31) & ~31;
-  const int part = t / pad, s = t - part * pad;
-  int sy;
-  if (part >= kRivParts || s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
-  river_part(m, y, s, part);
-}
-
-// ---------------------------------------------------------------------------
-// k_river_rows: upstream sums and the river rows of ydot
-// ---------------------------------------------------------------------------
-// What a river row reads of the mesh: the first upstream segments' indices
-// are a chain of loads in front of their fluxes.
-struct RiverRowsIn {
-  double area, porosity;
-  int first, end, up[3];
-};
-__device__ __forceinline__ RiverRowsIn river_rows_load(const DevMesh &m, int s) {
-  RiverRowsIn r;
-  r.area = m.r_area[s];
-  r.porosity = m.r_porosity[s];
-  r.first = m.up_ptr[s];
-  r.end = m.up_end[s];
-#pragma unroll
-  for (int k = 0; k < 3; k++) r.up[k] = r.first + k < r.end ? m.up_idx[r.first + k] : 0;
-  return r;
-}
-
-// the quotients of a row, beside each other
-__device__ __forceinline__ void river_rows_item(const DevMesh &m, double *ydot, int s, int sy, const RiverRowsIn &r) {
-  const int nr = m.nr, ne = m.ne;
-  const double *F = m.rivflow;
-  double f[7];
-  f[0] = F[UP_CHANL2CHANL * nr + s];
-#pragma unroll
-  for (int j = 1; j <= 6; j++) f[j] = F[j * nr + s];
-  const double aq_l = F[LEFT_AQUIF2AQUIF * nr + s], aq_r = F[RIGHT_AQUIF2AQUIF * nr + s];
-  const double aq_d = F[DOWN_AQUIF2AQUIF * nr + s];
-  const double area = r.area, por_area = r.porosity * area;
-  double up_c = f[0];
-  double up_a = 0.0;
-  double fc[3], fa[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    fc[k] = F[DOWN_CHANL2CHANL * nr + r.up[k]];
-    fa[k] = F[DOWN_AQUIF2AQUIF * nr + r.up[k]];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (r.first + k < r.end) {
-      up_c -= fc[k];
-      up_a -= fa[k];
-    }
-  for (int k = r.first + 3; k < r.end; k++) {
-    const int u = m.up_idx[k];
-    up_c -= F[DOWN_CHANL2CHANL * nr + u];
-    up_a -= F[DOWN_AQUIF2AQUIF * nr + u];
-  }
-  f[0] = up_c;
-  double dg = -aq_l - aq_r - aq_d - up_a + f[CHANL_LKG];
-  double q[7], qg;
-  bool ok = im::div_i(dg, por_area, qg);
-#pragma unroll
-  for (int j = 0; j <= 6; j++) ok &= im::div_i(f[j], area, q[j]);
-  if (!ok) {
-    qg = div_any(dg, por_area);
-#pragma unroll
-    for (int j = 0; j <= 6; j++) q[j] = div_any(f[j], area);
-  }
-  dg = qg;
-  double ds = 0.0;
-#pragma unroll
-  for (int j = 0; j <= 6; j++) ds -= q[j];
-  ydot[3 * ne + s] = ds;
-  ydot[3 * ne + nr + s] = dg;
-  if (m.diag) {
-    m.rivflow[UP_CHANL2CHANL * nr + s] = up_c;
-    m.rivflow[UP_AQUIF2AQUIF * nr + s] = up_a;
-  }
-  if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
-}
-
-__global__ void __launch_bounds__(128) k_river_rows(DevMesh m, double *RESTRICT ydot) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int sy;
-  if (s >= m.nr_run || skip_item(m, m.sys_riv, s, &sy)) return;
-  river_rows_item(m, ydot, s, sy, river_rows_load(m, s));
-}
-
-// ---------------------------------------------------------------------------
 // k_bank_rows: the rows of elements with river edges, from k_elem_main's
-// partial sums and the river kernels' fluxes, and the overland flux kept for
-// the next evaluation's Infil.
+// partial sums and the river fluxes, and the overland flux kept for the next
+// evaluation's Infil; and the river rows.  A chain of four dependent loads
+// for a few thousand items: the three that lead to the fluxes (the element,
+// its neighbours, the bank's side) are done while k_elem_main ends.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_bank_rows(DevMesh m, double *RESTRICT ydot) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+// (80 registers: its blocks stand in the SMs while k_elem_main ends; at 128 an
+// ensemble of four contexts' 400,000 elements took 1,072 us instead of 1,058)
+__global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRICT ydot, int river_blocks) {
   int sy;
-  if (b >= m.nbank_run || skip_item(m, m.sys_bank, b, &sy)) return;
+  if ((int)blockIdx.x < river_blocks) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = s < m.nr_run && !skip_item(m, m.sys_riv, s, &sy);
+    RiverRowsIn in;
+    if (on) in = river_rows_load(m, s);
+    wait_for_previous();
+    if (on) river_rows_item(m, ydot, s, sy, in);
+    return;
+  }
+  const int b = (blockIdx.x - river_blocks) * blockDim.x + threadIdx.x;
+  const bool on = b < m.nbank_run && !skip_item(m, m.sys_bank, b, &sy);
   const int nr = m.nr, ne = m.ne, nbk = m.nbank;
+  int i = 0, seg[3] = {-1, -1, -1};
+  bool left[3] = {false, false, false};
+  double inv_area = 0.0, inv_por = 0.0;
+  if (on) {
+    i = m.bank_elem[b];
+    inv_area = m.inv_area[i];
+    inv_por = m.inv_por[i];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const int32_t nb = m.nb[j * ne + i];
+      if (nb < 0 && nb != kBoundary) {
+        seg[j] = -1 - nb;
+        left[j] = m.left[seg[j]] == i;
+      }
+    }
+  }
+  wait_for_previous();
+  if (!on) return;
   const double *F = m.rivflow;
-  const int i = m.bank_elem[b];
   const double *bp = m.bank_part;
-  double ds = bp[b], dg = bp[nbk + b];
-  const double inv_area = m.inv_area[i];
+  double ds = bp[b], dg = bp[nbk + b], f[3][3], o[3], u[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const int32_t nb = m.nb[j * ne + i];
-    double o, u;
-    if (nb < 0 && nb != kBoundary) {
-      const int s = -1 - nb;
-      if (m.left[s] == i) {
-        o = -F[LEFT_SURF2CHANL * nr + s];
-        u = -(F[LEFT_AQUIF2CHANL * nr + s] + F[LEFT_AQUIF2AQUIF * nr + s]);
-        m.carry_ovl[s] = F[LEFT_SURF2CHANL * nr + s];
-      } else {
-        o = -F[RIGHT_SURF2CHANL * nr + s];
-        u = -(F[RIGHT_AQUIF2CHANL * nr + s] + F[RIGHT_AQUIF2AQUIF * nr + s]);
-        m.carry_ovl[nr + s] = F[RIGHT_SURF2CHANL * nr + s];
-      }
-      if (m.diag) {
-        m.d_ovl[j * ne + i] = o;
-        m.d_sub[j * ne + i] = u;
-      }
+    if (seg[j] >= 0) {
+      f[j][0] = F[(left[j] ? LEFT_SURF2CHANL : RIGHT_SURF2CHANL) * nr + seg[j]];
+      f[j][1] = F[(left[j] ? LEFT_AQUIF2CHANL : RIGHT_AQUIF2CHANL) * nr + seg[j]];
+      f[j][2] = F[(left[j] ? LEFT_AQUIF2AQUIF : RIGHT_AQUIF2AQUIF) * nr + seg[j]];
     } else {
-      o = bp[(2 + j) * nbk + b];
-      u = bp[(5 + j) * nbk + b];
+      o[j] = bp[(2 + j) * nbk + b];
+      u[j] = bp[(5 + j) * nbk + b];
     }
-    ds -= o * inv_area;
-    dg -= u * inv_area;
   }
-  dg *= m.inv_por[i];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    if (seg[j] >= 0) {
+      o[j] = -f[j][0];
+      u[j] = -(f[j][1] + f[j][2]);
+      m.carry_ovl[(left[j] ? 0 : nr) + seg[j]] = f[j][0];
+      if (m.diag) {
+        m.d_ovl[j * ne + i] = o[j];
+        m.d_sub[j * ne + i] = u[j];
+      }
+    }
+    ds -= o[j] * inv_area;
+    dg -= u[j] * inv_area;
+  }
+  dg *= inv_por;
   ydot[i] = ds;
   ydot[2 * ne + i] = dg;
   if (cmp::isnan_(ds) | cmp::isnan_(dg)) report_err(m, sy);
@@ -1610,78 +1680,94 @@ static cudaError_t launch_fused(const DevMesh &m, FusedLaunch &l, const double *
                                      dim3(l.g.elem + l.g.edge + l.g.river + l.g.col), dim3(l.threads), args, 0, st);
 }
 
+template <class... P, class... A>
+static cudaError_t launch_after(void (*kernel)(P...), unsigned grid, int block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStream_t st,
-                       long long *launches, Profiler *prof, const RhsStreams *side, const double *y_ref,
+                       long long *launches, Profiler *prof, const FusedPlan *fused, const double *y_ref,
                        const int32_t *iperm) {
   bool on;
   // a small mesh in one launch (per-kernel timing keeps the separate kernels):
   // one evaluation of 1,000 / 20,000 / 40,000 elements takes 18 / 24 / 33 us
   // instead of 41 / 46 / 54
   FusedLaunch fl;
-  if (side && !prof && fused_fits(m, side->fused, y_ref != nullptr, &fl)) {
+  if (fused && !prof && fused_fits(m, *fused, y_ref != nullptr, &fl)) {
     ++*launches;
     return launch_fused(m, fl, y, ydot, st, y_ref, iperm);
   }
-  // the river kernels read only k_elem_prep's outputs, the state and static
-  // data, so with a side stream they run beside grad/edge/main (per-kernel
-  // timing keeps one stream)
-  const bool fork = side && side->side && !prof && m.ne_run > 0 && m.nr_run > 0;
-  const auto river = [&](cudaStream_t rs) {
-    on = prof_begin(prof, K_RIVER, rs);
-    k_riv_geom<<<blocks_for(m.nr_run, 128), 128, 0, rs>>>(m, y);
-    k_river<<<blocks_for(kRivParts * ((m.nr_run + 31LL) & ~31LL), 128), 128, 0, rs>>>(m, y);
-    k_river_rows<<<blocks_for(m.nr_run, 128), 128, 0, rs>>>(m, ydot);
-    prof_end(prof, on, rs);
-    *launches += 3;
+  // The river work rides in the element kernels' grids, ahead of the
+  // elements: geometry with k_elem_prep, fluxes with k_elem_grad, rows with
+  // k_bank_rows.  Per-kernel timing, and an arena without elements, keep
+  // them apart.  Against river kernels on a second stream, its two events and
+  // plain launches, with k_bank_rows's 10 us of latency at the end: 60,000
+  // elements 55 -> 43 us, 200,000 103 -> 86, 400,000 171 -> 146, 1,000,000
+  // 345 -> 322.
+  const bool with = !prof && m.ne_run > 0 && m.nr_run > 0;
+  const bool from_ref = y_ref != nullptr;
+  const unsigned rows = m.nr_run > 0 ? blocks_for(m.nr_run, 128) : 0;
+  const unsigned parts = m.nr_run > 0 ? kRivParts * ((m.nr_run + 31u) & ~31u) : 0;
+  cudaError_t err = cudaSuccess;
+  const auto after = [&](auto kernel, unsigned grid, int block, auto... args) {
+    if (err == cudaSuccess) err = launch_after(kernel, grid, block, st, args...);
+    ++*launches;
   };
   if (m.ne_run > 0) {
     on = prof_begin(prof, K_PREP, st);
-    if (y_ref)  // y is the internal-order buffer the kernel fills
-      k_elem_prep<true><<<blocks_for((long long)m.ne + 2LL * m.nr, kPrepBlock), kPrepBlock, 0, st>>>(
-          m, nullptr, y_ref, const_cast<double *>(y), iperm);
+    const unsigned geom = with ? blocks_for(m.nr_run, kPrepBlock) : 0;
+    if (from_ref)  // y is the internal-order buffer the kernel fills
+      k_elem_prep<true><<<geom + blocks_for((long long)m.ne + 2LL * m.nr, kPrepBlock), kPrepBlock, 0, st>>>(
+          m, nullptr, y_ref, const_cast<double *>(y), iperm, (int)geom);
     else
-      k_elem_prep<false><<<blocks_for(m.ne_run, kPrepBlock), kPrepBlock, 0, st>>>(m, y, nullptr, nullptr, nullptr);
+      k_elem_prep<false><<<geom + blocks_for(m.ne_run, kPrepBlock), kPrepBlock, 0, st>>>(m, y, nullptr, nullptr,
+                                                                                      nullptr, (int)geom);
     prof_end(prof, on, st);
     ++*launches;
-    if (fork) {
-      if (cudaEventRecord(side->fork, st) != cudaSuccess) return cudaErrorUnknown;
-      if (cudaStreamWaitEvent(side->side, side->fork, 0) != cudaSuccess) return cudaErrorUnknown;
-      river(side->side);
-      if (cudaEventRecord(side->join, side->side) != cudaSuccess) return cudaErrorUnknown;
-    }
-    if (m.surf_mode == kDiffWave) {
+    const bool grad = m.surf_mode == kDiffWave;
+    if (grad || with) {
       on = prof_begin(prof, K_GRAD, st);
-      k_elem_grad<<<blocks_for(m.ne_run, 256), 256, 0, st>>>(m, y);
+      const unsigned river = with ? blocks_for(parts, 256) : 0;
+      after(k_elem_grad, river + (grad ? blocks_for(m.ne_run, 256) : 0), 256, m, y, (int)river, from_ref);
       prof_end(prof, on, st);
-      ++*launches;
     }
     if (m.nedge_run > 0) {
       on = prof_begin(prof, K_EDGE, st);
-      k_edge<<<blocks_for(m.nedge_run, kEdgeBlock), kEdgeBlock, 0, st>>>(m, y);
+      after(k_edge, blocks_for(m.nedge_run, kEdgeBlock), kEdgeBlock, m, y);
       prof_end(prof, on, st);
-      ++*launches;
     }
     on = prof_begin(prof, K_MAIN, st);
     switch (m.main_shape) {
-      case 1: k_elem_main<256, 4><<<blocks_for(m.ne_run, 256), 256, 0, st>>>(m, y, ydot); break;
-      case 2: k_elem_main<128, 8><<<blocks_for(m.ne_run, 128), 128, 0, st>>>(m, y, ydot); break;
-      default: k_elem_main<512, 2><<<blocks_for(m.ne_run, 512), 512, 0, st>>>(m, y, ydot); break;
+      case 1: after(k_elem_main<256, 4>, blocks_for(m.ne_run, 256), 256, m, y, ydot, from_ref); break;
+      case 2: after(k_elem_main<128, 8>, blocks_for(m.ne_run, 128), 128, m, y, ydot, from_ref); break;
+      default: after(k_elem_main<512, 2>, blocks_for(m.ne_run, 512), 512, m, y, ydot, from_ref); break;
     }
     prof_end(prof, on, st);
-    ++*launches;
   }
-  if (fork) {
-    if (cudaStreamWaitEvent(st, side->join, 0) != cudaSuccess) return cudaErrorUnknown;
-  } else if (m.nr_run > 0) {
-    river(st);
-  }
-  if (m.nbank_run > 0) {
-    on = prof_begin(prof, K_FINISH, st);
-    k_bank_rows<<<blocks_for(m.nbank_run, 128), 128, 0, st>>>(m, ydot);
+  if (!with && m.nr_run > 0) {
+    on = prof_begin(prof, K_RIVER, st);
+    k_riv_geom<<<rows, 128, 0, st>>>(m, y);
+    k_river<<<blocks_for(parts, 128), 128, 0, st>>>(m, y);
+    k_river_rows<<<rows, 128, 0, st>>>(m, ydot);
     prof_end(prof, on, st);
-    ++*launches;
+    *launches += 3;
   }
-  return cudaGetLastError();
+  const unsigned late = with ? rows : 0;
+  if (late > 0 || m.nbank_run > 0) {
+    on = prof_begin(prof, K_FINISH, st);
+    after(k_bank_rows, late + (m.nbank_run > 0 ? blocks_for(m.nbank_run, 128) : 0), 128, m, ydot, (int)late);
+    prof_end(prof, on, st);
+  }
+  return err == cudaSuccess ? cudaGetLastError() : err;
 }
 
 cudaError_t launch_permute(const double *src, double *dst, const int32_t *perm, int ne, int nr,
