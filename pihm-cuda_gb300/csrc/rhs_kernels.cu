@@ -189,6 +189,7 @@ __device__ __forceinline__ int queue_slot(int *count, bool take) {
 // evaluated densely.
 // ---------------------------------------------------------------------------
 constexpr int kPrepBlock = 256;
+constexpr unsigned kPrepWave = 8 * 152;  // blocks the SMs hold at once
 
 // SurfH and EffKh of one element (src/hydrol.c:100-134, src/lat_flow.c:248-277):
 // what needs no root or division is stored here; thin asks for
@@ -591,7 +592,12 @@ __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const doubl
   __shared__ double qs_x[kPrepBlock], qd_num[kPrepBlock], qd_den[kPrepBlock];
   __shared__ int qs_n, qd_n;
   int sy = 0;
-  next_may_start();
+  // With more blocks than the SMs hold at once (8 each), k_elem_grad's would
+  // stand waiting through the last of them: its blocks come when these end.
+  // One stream pays 1 us of 147 for it (400,000 elements), four that fill the
+  // device gain 28 of 1,056.  In one wave the early start gives 4 us of 86.
+  const bool early = gridDim.x <= kPrepWave;
+  if (early || (int)blockIdx.x < river_blocks) next_may_start();
   if ((int)blockIdx.x < river_blocks) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < m.nr_run && !skip_item(m, m.sys_riv, s, &sy)) geom_item(m, kFromRef ? y_ref : y, s);
@@ -630,6 +636,7 @@ __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const doubl
   bool thin = false, mix = false;
   double sx = 0.0, num = 0.0, den = 0.0;
   if (elem) prep_item(m, i, y_surf, y_gw, thin, sx, mix, num, den);
+  if (!early) next_may_start();
   const int ss = queue_slot(&qs_n, thin);
   if (thin) {
     qs_i[ss] = i;
