@@ -1280,6 +1280,7 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
     RiverRowsIn in;
     if (on) in = river_rows_load(m, s);
     wait_for_previous();
+    next_may_start();
     if (on) river_rows_item(m, ydot, s, sy, in);
     return;
   }
@@ -1303,6 +1304,7 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
     }
   }
   wait_for_previous();
+  next_may_start();
   if (!on) return;
   const double *F = m.rivflow;
   const double *bp = m.bank_part;
@@ -1523,6 +1525,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     if (ok) ok = bar_wait(C, lateral, &s_ok);
     if (!ok) return report_wait(m, m.sys_riv, first, m.nr_run, step);
     bar_leave(m.bar, per + g.col);
+    next_may_start();
     if (on) river_rows_item(m, ydot, first, sy, in);
     for (int s = first + step; s < m.nr_run; s += step)
       if (!skip_item(m, m.sys_riv, s, &sy)) river_rows_item(m, ydot, s, sy, river_rows_load(m, s));
@@ -1551,6 +1554,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
       met = true;
       if (!bar_wait(C, lateral, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
       bar_leave(m.bar, g.river / kRivParts + g.col);
+      next_may_start();
     }
     if (on) column_rows<true>(m, ydot, i, sy, c, r);
   }
@@ -1559,38 +1563,33 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
 // ---------------------------------------------------------------------------
 // state reordering between reference and internal order
 // ---------------------------------------------------------------------------
-__global__ void k_permute(const double *RESTRICT src, double *RESTRICT dst, const int32_t *RESTRICT perm,
-                          int ne, int nr, int to_internal) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n_el = 3LL * ne;
-  if (t < n_el) {
-    const int blk = (int)(t / ne);
-    const int i = (int)(t - (long long)blk * ne);
-    const long long ref = (long long)blk * ne + perm[i];
-    if (to_internal) dst[t] = src[ref];
-    else dst[ref] = src[t];
-  } else if (t < n_el + 2LL * nr) {
-    dst[t] = src[t];
-  }
+// blockIdx.y is the plane (surface, unsaturated, groundwater), and the blocks
+// past its elements copy the river values; the index is read before the wait
+// for the evaluation's last kernel (these are dependent launches too).
+__global__ void __launch_bounds__(256) k_permute(const double *src, double *dst, const int32_t *RESTRICT perm, int ne,
+                                                 int nr, int to_internal) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool elem = i < ne;
+  const int r = elem ? perm[i] : 0;
+  wait_for_previous();
+  const long long plane = (long long)blockIdx.y * ne;
+  if (elem) dst[plane + (to_internal ? i : r)] = src[plane + (to_internal ? r : i)];
+  else if (blockIdx.y == 2 && i - ne < 2 * nr) dst[plane + i] = src[plane + i];
 }
 
 // The same reordering walked in reference order (iperm: reference ->
 // internal element index): the reference-order side is read or written
 // contiguously, which is the side in host memory when the host-buffer
 // evaluation accesses it directly.
-__global__ void k_permute_ref(const double *RESTRICT src, double *RESTRICT dst,
-                              const int32_t *RESTRICT iperm, int ne, int nr, int to_internal) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n_el = 3LL * ne;
-  if (t < n_el) {
-    const int blk = (int)(t / ne);
-    const int r = (int)(t - (long long)blk * ne);
-    const long long in = (long long)blk * ne + iperm[r];
-    if (to_internal) dst[in] = src[t];
-    else dst[t] = src[in];
-  } else if (t < n_el + 2LL * nr) {
-    dst[t] = src[t];
-  }
+__global__ void __launch_bounds__(256) k_permute_ref(const double *src, double *dst, const int32_t *RESTRICT iperm,
+                                                     int ne, int nr, int to_internal) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool elem = r < ne;
+  const int i = elem ? iperm[r] : 0;
+  wait_for_previous();
+  const long long plane = (long long)blockIdx.y * ne;
+  if (elem) dst[plane + (to_internal ? i : r)] = src[plane + (to_internal ? r : i)];
+  else if (blockIdx.y == 2 && r - ne < 2 * nr) dst[plane + r] = src[plane + r];
 }
 
 }  // namespace pihm
@@ -1688,9 +1687,9 @@ static cudaError_t launch_fused(const DevMesh &m, FusedLaunch &l, const double *
 }
 
 template <class... P, class... A>
-static cudaError_t launch_after(void (*kernel)(P...), unsigned grid, int block, cudaStream_t st, A... args) {
+static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int block, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.stream = st;
   cudaLaunchAttribute at{};
@@ -1726,7 +1725,7 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
   const unsigned parts = m.nr_run > 0 ? kRivParts * ((m.nr_run + 31u) & ~31u) : 0;
   cudaError_t err = cudaSuccess;
   const auto after = [&](auto kernel, unsigned grid, int block, auto... args) {
-    if (err == cudaSuccess) err = launch_after(kernel, grid, block, st, args...);
+    if (err == cudaSuccess) err = launch_after(kernel, dim3(grid), block, st, args...);
     ++*launches;
   };
   if (m.ne_run > 0) {
@@ -1779,18 +1778,14 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
 
 cudaError_t launch_permute(const double *src, double *dst, const int32_t *perm, int ne, int nr,
                            int to_internal, cudaStream_t st) {
-  const long long n = 3LL * ne + 2LL * nr;
-  if (n == 0) return cudaSuccess;
-  k_permute<<<blocks_for(n, 256), 256, 0, st>>>(src, dst, perm, ne, nr, to_internal);
-  return cudaGetLastError();
+  if (ne + 2LL * nr == 0) return cudaSuccess;
+  return launch_after(k_permute, dim3(blocks_for(ne + 2LL * nr, 256), 3), 256, st, src, dst, perm, ne, nr, to_internal);
 }
 
 cudaError_t launch_permute_ref(const double *src, double *dst, const int32_t *iperm, int ne, int nr,
                                int to_internal, cudaStream_t st) {
-  const long long n = 3LL * ne + 2LL * nr;
-  if (n == 0) return cudaSuccess;
-  k_permute_ref<<<blocks_for(n, 256), 256, 0, st>>>(src, dst, iperm, ne, nr, to_internal);
-  return cudaGetLastError();
+  if (ne + 2LL * nr == 0) return cudaSuccess;
+  return launch_after(k_permute_ref, dim3(blocks_for(ne + 2LL * nr, 256), 3), 256, st, src, dst, iperm, ne, nr, to_internal);
 }
 
 }  // namespace pihm
