@@ -19,6 +19,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <numeric>
 #include <thread>
 #include <vector>
 
@@ -158,128 +159,110 @@ int h2d(T *dst, const T *src, size_t n, cudaStream_t st) {
   return cudaMemcpyAsync(dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, st) == cudaSuccess ? 0 : -1;
 }
 
-// A watershed's uploads: on a device that can access pageable host memory,
-// descriptors for one gather kernel that reads the host arrays directly
-// (one launch instead of about a hundred staged copies); else staged copies.
-// Either way every source must stay valid until flush() has synchronised.
+// Uploads of one or more watersheds: on a device that can access pageable
+// host memory, descriptors for one gather kernel that reads the host arrays
+// directly and moves indices to the watershed's ranges (one launch and one
+// synchronisation instead of about a hundred staged copies a watershed); else
+// staged copies of indices moved here.  Either way every source must stay
+// valid until flush() has synchronised.
 struct Uploader {
   bool direct;
   cudaStream_t st;
   std::vector<CopyDesc> desc;
+  std::vector<std::vector<int32_t>> moved;
   uint64_t max_bytes = 0;
   int rc = 0;
+  void push(void *dst, const void *src, size_t bytes, int op, int64_t a, int64_t b) {
+    if (desc.size() >= 60000) flush();  // the kernel's grid
+    desc.push_back({src, dst, (uint64_t)bytes, op, (int32_t)a, (int32_t)b, 0});
+    max_bytes = std::max<uint64_t>(max_bytes, bytes);
+  }
   template <class T>
   void operator()(T *dst, const T *src, size_t n) {
     if (n == 0) return;
-    if (direct) {
-      desc.push_back({(const void *)src, (void *)dst, (uint64_t)(sizeof(T) * n)});
-      max_bytes = std::max<uint64_t>(max_bytes, sizeof(T) * n);
-    } else {
-      rc |= h2d(dst, src, n, st);
-    }
+    if (direct) push(dst, src, sizeof(T) * n, UP_COPY, 0, 0);
+    else rc |= h2d(dst, src, n, st);
+  }
+  void index(int32_t *dst, const int32_t *src, size_t n, int op, int64_t a, int64_t b = 0) {
+    if (n == 0) return;
+    if (direct) return push(dst, src, sizeof(int32_t) * n, op, a, b);
+    std::vector<int32_t> t(n);
+    for (size_t q = 0; q < n; q++) t[q] = upload_index(op, src ? src[q] : 0, (int32_t)a, (int32_t)b);
+    moved.push_back(std::move(t));
+    rc |= h2d(dst, (const int32_t *)moved.back().data(), n, st);
+  }
+  void zero(double *dst, size_t n) {
+    if (n == 0) return;
+    if (direct) push(dst, nullptr, sizeof(double) * n, UP_FILL, 0, 0);
+    else if (cudaMemsetAsync(dst, 0, sizeof(double) * n, st) != cudaSuccess) rc = -1;
   }
   int flush() {
     if (direct && !desc.empty() && launch_gather_host(desc.data(), (int)desc.size(), max_bytes, st) != cudaSuccess)
       rc = -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+    desc.clear();
+    moved.clear();
+    max_bytes = 0;
     return rc;
   }
 };
 
-// Translate a watershed image's indices to its arena ranges and upload it.
-int place(pihm_batch *B, Sys *s, const Prepared &job) {
+// A watershed image's upload to its arena ranges, queued in `up`; the image
+// and `s` stay until it has been flushed.
+void place(pihm_batch *B, Sys *s, const Prepared &job, Uploader &up) {
   const SystemImage &im = job.im;
   DevMesh &m = B->A.m;
-  cudaStream_t st = B->st;
-  Uploader up{B->host_pageable != 0, st, {}};
   const int ne = im.ne, nr = im.nr;
   const int64_t NE = B->ne_cap, NR = B->nr_cap;
   const int64_t eo = s->eoff, ro = s->roff, edo = s->edoff, bo = s->boff, uo = s->upoff;
-  int rc = 0;
   for (int k = 0; k < EP_COUNT; k++) up((double *)(m.*kElemMember[k]) + eo, im.el[k].data(), ne);
   for (int k = 0; k < XP_COUNT; k++)
     for (int j = 0; j < 3; j++)
       up((double *)(m.*kEdgeMember[k]) + j * NE + eo, im.ed[k].data() + (size_t)j * ne, ne);
-  std::vector<int32_t> t(3 * (size_t)ne);
-  for (size_t q = 0; q < t.size(); q++) {
-    const int32_t v = im.nb[q];
-    t[q] = v >= 0 ? (int32_t)(v + eo) : (v == kBoundary ? v : (int32_t)(-1 - ((-1 - v) + ro)));
-  }
-  for (int j = 0; j < 3; j++) up((int32_t *)m.nb + j * NE + eo, t.data() + (size_t)j * ne, ne);
-  std::vector<int32_t> t2(3 * (size_t)ne);
-  for (size_t q = 0; q < t2.size(); q++) {
-    const int32_t v = im.emap[q];
-    t2[q] = v > 0 ? (int32_t)(v + edo) : (v < 0 ? (int32_t)(v - edo) : 0);
-  }
   for (int j = 0; j < 3; j++) {
-    up((int32_t *)m.emap + j * NE + eo, t2.data() + (size_t)j * ne, ne);
-    up((int32_t *)m.bctype + j * NE + eo, im.bct.data() + (size_t)j * ne, ne);
+    const size_t q = (size_t)j * ne;
+    up.index((int32_t *)m.nb + j * NE + eo, im.nb.data() + q, ne, UP_NABR, eo, ro);
+    up.index((int32_t *)m.emap + j * NE + eo, im.emap.data() + q, ne, UP_EDGE, edo);
+    up((int32_t *)m.bctype + j * NE + eo, im.bct.data() + q, ne);
   }
-  std::vector<int32_t> ei(im.nedge), ek(im.nedge);
-  for (int e = 0; e < im.nedge; e++) {
-    ei[e] = (int32_t)(im.e_i[e] + eo);
-    ek[e] = (int32_t)(im.e_k[e] + eo);
-  }
-  up((int32_t *)m.e_i + edo, ei.data(), im.nedge);
-  up((int32_t *)m.e_k + edo, ek.data(), im.nedge);
+  up.index((int32_t *)m.e_i + edo, im.e_i.data(), im.nedge, UP_ADD, eo);
+  up.index((int32_t *)m.e_k + edo, im.e_k.data(), im.nedge, UP_ADD, eo);
   up((double *)m.e_invdist + edo, im.e_invdist.data(), im.nedge);
   up((double *)m.e_subk + edo, im.e_subk.data(), im.nedge);
   up((double *)m.e_ovlk + edo, im.e_ovlk.data(), im.nedge);
-  std::vector<int32_t> bs(ne), be(im.nbank);
-  for (int i = 0; i < ne; i++) bs[i] = im.bank_slot[i] >= 0 ? (int32_t)(im.bank_slot[i] + bo) : -1;
-  for (int b = 0; b < im.nbank; b++) be[b] = (int32_t)(im.bank_elem[b] + eo);
-  up((int32_t *)m.bank_slot + eo, bs.data(), ne);
-  up((int32_t *)m.bank_elem + bo, be.data(), im.nbank);
-  std::vector<int32_t> dn(nr), lf(nr), rt(nr), ub(nr), ue(nr), ui(im.up_idx.size());
-  for (int r = 0; r < nr; r++) {
-    dn[r] = im.down[r] > 0 ? (int32_t)(im.down[r] + ro) : im.down[r];
-    lf[r] = (int32_t)(im.left[r] + eo);
-    rt[r] = (int32_t)(im.right[r] + eo);
-    ub[r] = (int32_t)(im.up_ptr[r] + uo);
-    ue[r] = (int32_t)(im.up_ptr[r + 1] + uo);
-  }
-  for (size_t q = 0; q < ui.size(); q++) ui[q] = (int32_t)(im.up_idx[q] + ro);
-  up((int32_t *)m.down + ro, dn.data(), nr);
-  up((int32_t *)m.left + ro, lf.data(), nr);
-  up((int32_t *)m.right + ro, rt.data(), nr);
+  up.index((int32_t *)m.bank_slot + eo, im.bank_slot.data(), ne, UP_SLOT, bo);
+  up.index((int32_t *)m.bank_elem + bo, im.bank_elem.data(), im.nbank, UP_ADD, eo);
+  up.index((int32_t *)m.down + ro, im.down.data(), nr, UP_DOWN, ro);
+  up.index((int32_t *)m.left + ro, im.left.data(), nr, UP_ADD, eo);
+  up.index((int32_t *)m.right + ro, im.right.data(), nr, UP_ADD, eo);
   up((int32_t *)m.intrpl_ord + ro, im.ord.data(), nr);
   up((int32_t *)m.bctype_riv + ro, im.rbct.data(), nr);
-  up((int32_t *)m.up_ptr + ro, ub.data(), nr);
-  up((int32_t *)m.up_end + ro, ue.data(), nr);
-  up((int32_t *)m.up_idx + uo, ui.data(), ui.size());
+  up.index((int32_t *)m.up_ptr + ro, im.up_ptr.data(), nr, UP_ADD, uo);
+  up.index((int32_t *)m.up_end + ro, im.up_ptr.data() + 1, nr, UP_ADD, uo);
+  up.index((int32_t *)m.up_idx + uo, im.up_idx.data(), im.up_idx.size(), UP_ADD, ro);
   for (int k = 0; k < RP_COUNT; k++) up((double *)(m.*kRiverMember[k]) + ro, im.rv[k].data(), nr);
-  // boundary conditions (reference order in the job)
-  std::vector<double> bc(3 * (size_t)ne, 0.0);
-  if (!job.elem_bc.empty())
-    for (int j = 0; j < 3; j++)
-      for (int i = 0; i < ne; i++) bc[(size_t)j * ne + i] = job.elem_bc[3 * (size_t)im.perm[i] + j];
-  for (int j = 0; j < 3; j++) up((double *)m.elem_bc + j * NE + eo, bc.data() + (size_t)j * ne, ne);
-  std::vector<double> rbc(nr, 0.0);
-  if (!job.river_bc.empty()) std::copy(job.river_bc.begin(), job.river_bc.end(), rbc.begin());
-  up((double *)m.river_bc + ro, rbc.data(), nr);
+  // boundary conditions
+  for (int j = 0; j < 3; j++) {
+    if (job.elem_bc.empty()) up.zero((double *)m.elem_bc + j * NE + eo, ne);
+    else up((double *)m.elem_bc + j * NE + eo, job.elem_bc.data() + (size_t)j * ne, ne);
+  }
+  if (job.river_bc.empty()) up.zero((double *)m.river_bc + ro, nr);
+  else up((double *)m.river_bc + ro, job.river_bc.data(), nr);
   // a fresh watershed carries no river-edge flux from an earlier evaluation
-  for (int k = 0; k < NUM_RIVFLX; k++)
-    if (nr && cudaMemsetAsync(m.rivflow + k * NR + ro, 0, sizeof(double) * nr, st) != cudaSuccess) rc = -1;
-  for (int k = 0; k < 2; k++)
-    if (nr && cudaMemsetAsync(m.carry_ovl + k * NR + ro, 0, sizeof(double) * nr, st) != cudaSuccess) rc = -1;
+  for (int k = 0; k < NUM_RIVFLX; k++) up.zero(m.rivflow + k * NR + ro, nr);
+  for (int k = 0; k < 2; k++) up.zero(m.carry_ovl + k * NR + ro, nr);
   // owner tables
-  std::vector<int32_t> own(std::max<int64_t>({(int64_t)ne, (int64_t)nr, (int64_t)im.nedge, (int64_t)im.nbank, 1}),
-                           s->slot);
-  up((int32_t *)m.sys_elem + eo, own.data(), ne);
-  up((int32_t *)m.sys_riv + ro, own.data(), nr);
-  up((int32_t *)m.sys_edge + edo, own.data(), im.nedge);
-  up((int32_t *)m.sys_bank + bo, own.data(), im.nbank);
-  const double dt = job.ctrl.stepsize;
-  up((double *)m.sys_dt + s->slot, &dt, 1);
-  const double inv_dt = 1.0 / dt;
-  up((double *)m.sys_inv_dt + s->slot, &inv_dt, 1);
+  up.index((int32_t *)m.sys_elem + eo, nullptr, ne, UP_FILL, s->slot);
+  up.index((int32_t *)m.sys_riv + ro, nullptr, nr, UP_FILL, s->slot);
+  up.index((int32_t *)m.sys_edge + edo, nullptr, im.nedge, UP_FILL, s->slot);
+  up.index((int32_t *)m.sys_bank + bo, nullptr, im.nbank, UP_FILL, s->slot);
+  s->dt = job.ctrl.stepsize;
+  s->inv_dt = 1.0 / s->dt;
+  up((double *)m.sys_dt + s->slot, (const double *)&s->dt, 1);
+  up((double *)m.sys_inv_dt + s->slot, (const double *)&s->inv_dt, 1);
   // initial state, internal order, into vector slot 0
-  std::vector<double> y(s->neq);
-  for (int p = 0; p < 3; p++)
-    for (int i = 0; i < ne; i++) y[(size_t)p * ne + i] = job.y0[(size_t)p * ne + im.perm[i]];
-  for (int64_t q = 3LL * ne; q < s->neq; q++) y[q] = job.y0[q];
-  up(B->A.vec + s->soff, y.data(), s->neq);
-  SysInfo info{};
+  up(B->A.vec + s->soff, job.y0.data(), s->neq);
+  SysInfo &info = s->info;
   info.off = s->soff;
   info.neq = (int32_t)s->neq;
   info.ne = ne;
@@ -288,9 +271,7 @@ int place(pihm_batch *B, Sys *s, const Prepared &job) {
   info.roff = (int32_t)ro;
   info.nblk = (int32_t)pihm_nv::red_grid_for(s->neq);
   info.rec_off = s->recoff;
-  up(B->A.sysinfo + s->slot, &info, 1);
-  rc |= up.flush();
-  return rc ? PIHM_GPU_ERR_CUDA : PIHM_GPU_OK;
+  up(B->A.sysinfo + s->slot, (const SysInfo *)&info, 1);
 }
 
 }  // namespace
@@ -350,8 +331,17 @@ int prepare(const pihm_batch_job *job, int surf_mode, int riv_mode, int order, P
   if (brc != PIHM_GPU_OK) return brc;
   const int ne = p->im.ne, nr = p->im.nr;
   const size_t neq = 3 * (size_t)ne + 2 * (size_t)nr;
-  p->y0.assign(job->y0, job->y0 + neq);
-  if (job->elem_bc) p->elem_bc.assign(job->elem_bc, job->elem_bc + 3 * (size_t)ne);
+  // the state and the boundary values in internal order
+  const int32_t *perm = p->im.perm.data();
+  p->y0.resize(neq);
+  for (int k = 0; k < 3; k++)
+    for (int i = 0; i < ne; i++) p->y0[(size_t)k * ne + i] = job->y0[(size_t)k * ne + perm[i]];
+  std::copy(job->y0 + 3 * (size_t)ne, job->y0 + neq, p->y0.begin() + 3 * (size_t)ne);
+  if (job->elem_bc) {
+    p->elem_bc.resize(3 * (size_t)ne);
+    for (int j = 0; j < 3; j++)
+      for (int i = 0; i < ne; i++) p->elem_bc[(size_t)j * ne + i] = job->elem_bc[3 * (size_t)perm[i] + j];
+  }
   if (job->river_bc) p->river_bc.assign(job->river_bc, job->river_bc + nr);
   if (!job->land && !job->noah) {
     p->pcp.assign(job->pcpdrp, job->pcpdrp + job->nsteps);
@@ -465,7 +455,9 @@ int stage_bc(pihm_batch *B, Sys *s, int64_t t) {
 
 // Reserve arena ranges for a prepared job, upload it and start its model
 // loop.  PIHM_GPU_ERR_NOMEM when it does not fit now.
-int admit(pihm_batch *B, const Prepared &p, int32_t *id) {
+// Ranges, tables and the coroutine of one watershed; its upload is left in
+// `up` unless a deck or Noah needs it in place.
+int admit_queued(pihm_batch *B, const Prepared &p, Uploader &up, int32_t *id) {
   const SystemImage &im = p.im;
   int slot = -1;
   for (int k = 0; k < B->max_sys; k++)
@@ -511,9 +503,12 @@ int admit(pihm_batch *B, const Prepared &p, int32_t *id) {
   s->core.ops.s = s.get();
   Sys *sp = s.get();
   B->slots[slot] = std::move(s);
-  int prc = place(B, sp, p);
+  place(B, sp, p, up);
+  int prc = PIHM_GPU_OK;
+  if ((p.deck || p.land || p.noah) && up.flush()) prc = PIHM_GPU_ERR_CUDA;
   if (prc == PIHM_GPU_OK) prc = attach_deck(B, sp, p);
   if (prc != PIHM_GPU_OK) {
+    (void)up.flush();  // ahead of what frees the ranges
     free_ranges(B, sp);
     B->slots[slot].reset();
     return prc;
@@ -528,6 +523,26 @@ int admit(pihm_batch *B, const Prepared &p, int32_t *id) {
   resume(sp);
   *id = sp->id;
   return PIHM_GPU_OK;
+}
+
+// An admitted watershed whose upload failed.
+void withdraw(pihm_batch *B, int32_t id) {
+  auto it = B->by_id.find(id);
+  if (it == B->by_id.end()) return;
+  Sys *s = it->second;
+  free_ranges(B, s);
+  B->by_id.erase(it);
+  B->slots[s->slot].reset();
+  B->update_extents();
+}
+
+int admit(pihm_batch *B, const Prepared &p, int32_t *id) {
+  Uploader up{B->host_pageable != 0, B->st};
+  const int rc = admit_queued(B, p, up, id);
+  if (rc != PIHM_GPU_OK) return rc;
+  if (up.flush() == 0) return PIHM_GPU_OK;
+  withdraw(B, *id);
+  return PIHM_GPU_ERR_CUDA;
 }
 
 
@@ -1024,32 +1039,42 @@ int pihm_batch_add_many(pihm_batch *B, const pihm_batch_job *jobs, int32_t n, in
   if (!B || !jobs || !ids || n < 0) return PIHM_GPU_ERR_ARG;
   std::vector<Prepared> prep(n);
   std::vector<int> rcs(n, PIHM_GPU_OK);
+  // the largest first, so that the threads end together
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return (jobs[a].mesh ? jobs[a].mesh->nelem : 0) > (jobs[b].mesh ? jobs[b].mesh->nelem : 0);
+  });
   const int nt = std::max(1, std::min<int>(threads, n));
-  std::atomic<int> next{0};
-  auto work = [&] {
-    for (int k; (k = next.fetch_add(1)) < n;)
-      rcs[k] = prepare(&jobs[k], B->A.m.surf_mode, B->A.m.riv_mode, B->order, &prep[k]);
+  const auto on_threads = [&](auto &&one) {
+    std::atomic<int> next{0};
+    const auto work = [&] {
+      for (int k; (k = next.fetch_add(1)) < n;) one(order[k]);
+    };
+    std::vector<std::thread> pool;
+    for (int t = 1; t < nt; t++) pool.emplace_back(work);
+    work();
+    for (auto &t : pool) t.join();
   };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nt; t++) pool.emplace_back(work);
-  work();
-  for (auto &t : pool) t.join();
+  on_threads([&](int k) { rcs[k] = prepare(&jobs[k], B->A.m.surf_mode, B->A.m.riv_mode, B->order, &prep[k]); });
   int rc = PIHM_GPU_OK, count = 0;
+  Uploader up{B->host_pageable != 0, B->st};
   for (int k = 0; k < n; k++) {
     ids[k] = -1;
     if (rc != PIHM_GPU_OK) continue;
-    if (rcs[k] != PIHM_GPU_OK) {
-      rc = rcs[k];
-      continue;
-    }
-    const int arc = admit(B, prep[k], &ids[k]);
-    if (arc != PIHM_GPU_OK) {
-      rc = arc;
-      continue;
-    }
-    count++;
-    prep[k] = Prepared();  // release the host image early
+    rc = rcs[k];
+    if (rc == PIHM_GPU_OK) rc = admit_queued(B, prep[k], up, &ids[k]);
+    if (rc == PIHM_GPU_OK) count++;
   }
+  if (up.flush() != 0) {
+    for (int k = 0; k < n; k++) {
+      if (ids[k] >= 0) withdraw(B, ids[k]);
+      ids[k] = -1;
+    }
+    count = 0;
+    rc = PIHM_GPU_ERR_CUDA;
+  }
+  on_threads([&](int k) { prep[k] = Prepared(); });  // unmapping the images takes as long as a quarter of building them
   if (admitted) *admitted = count;
   return rc;
 }

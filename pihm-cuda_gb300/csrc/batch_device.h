@@ -22,6 +22,7 @@
 
 #include <cstdint>
 
+#include "nv_select.h"
 #include "pihm_internal.h"
 
 namespace pihm {
@@ -110,14 +111,34 @@ cudaError_t launch_program(const DeviceArena &a, int nrs, int nblocks, int varia
 cudaError_t launch_round_done(const unsigned int *words, unsigned int *host, int n, uint64_t *flag, uint64_t seq,
                               cudaStream_t st);
 
-// One host-to-device copy of a watershed's upload: bytes from src (host
-// memory) to dst (arena).
+// One part of a watershed's upload: bytes from src (host memory) to dst
+// (arena), 32-bit indices moved to the watershed's ranges on the way.
+enum UploadOp : int32_t {
+  UP_COPY = 0,
+  UP_FILL,   // a, n times; src unused
+  UP_ADD,    // v + a
+  UP_SLOT,   // -1 stays, else v + a
+  UP_DOWN,   // v > 0: v + a, else v
+  UP_NABR,   // v >= 0: v + a; the boundary stays; a river segment moves by b
+  UP_EDGE    // a signed one-based edge: v > 0: v + a, v < 0: v - a
+};
 struct CopyDesc {
   const void *src;
   void *dst;
   uint64_t bytes;
+  int32_t op, a, b, pad;
 };
-// Copies every descriptor with one kernel that reads the host memory
+PIHM_HD inline int32_t upload_index(int op, int32_t v, int32_t a, int32_t b) {
+  switch (op) {
+    case UP_FILL: return a;
+    case UP_ADD: return v + a;
+    case UP_SLOT: return v < 0 ? v : v + a;
+    case UP_DOWN: return v > 0 ? v + a : v;
+    case UP_NABR: return v >= 0 ? v + a : (v == kBoundary ? v : v - b);
+    default: return v > 0 ? v + a : (v < 0 ? v - a : 0);
+  }
+}
+// Takes every descriptor with one kernel that reads the host memory
 // directly.  Only for a device that can access pageable host memory
 // (cudaDevAttrPageableMemoryAccess): desc and every src may be ordinary
 // host allocations, and they must stay valid until the stream has passed

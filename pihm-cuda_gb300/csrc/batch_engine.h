@@ -148,6 +148,8 @@ struct Sys {
   int32_t ne = 0, nr = 0, nedge = 0, nbank = 0, nup = 0, nrec = 0;
   int64_t neq = 0;
   std::vector<int32_t> perm;
+  SysInfo info{};
+  double dt = 0.0, inv_dt = 0.0;
   // job
   pihm_step_control ctrl{};
   int32_t nsteps = 0, outlet = -1, steps_done = 0;

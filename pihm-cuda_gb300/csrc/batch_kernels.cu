@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kU == 0 ? kSpreadThreads : kThreads, (kU == 0 
 static_assert(sizeof(Op) == 40 && sizeof(Op) % sizeof(double) == 0, "Op is staged as doubles");
 
 // blockIdx.y picks the descriptor, blockIdx.x a kGatherChunk-byte chunk of
-// it; 8-byte words where source, destination and size allow, else 4-byte
+// it; indices word by word, else 8-byte words where source, destination and size allow, else 4-byte
 // words, else bytes
 constexpr uint64_t kGatherChunk = 64 * 1024;
 
@@ -347,6 +347,11 @@ __global__ void __launch_bounds__(256) k_gather_host(const CopyDesc *desc, int n
   const uintptr_t align = (uintptr_t)d.src | (uintptr_t)d.dst | (uintptr_t)d.bytes;
   const char *src = (const char *)d.src;
   char *dst = (char *)d.dst;
+  if (d.op != UP_COPY) {  // 32-bit words
+    for (uint64_t b = lo + 4 * (uint64_t)threadIdx.x; b < hi; b += 4 * (uint64_t)blockDim.x)
+      *(int32_t *)(dst + b) = upload_index(d.op, d.op == UP_FILL ? 0 : *(const int32_t *)(src + b), d.a, d.b);
+    return;
+  }
   if ((align & 7) == 0) {
     for (uint64_t b = lo + 8 * (uint64_t)threadIdx.x; b < hi; b += 8 * (uint64_t)blockDim.x)
       *(uint64_t *)(dst + b) = *(const uint64_t *)(src + b);

@@ -37,15 +37,10 @@ class MeshDesc(ctypes.Structure):
         d = MeshDesc()
         d.nelem = nelem
         d.nriver = nriver
-        keep = []
-        for name in _ORDER:
-            if name in _INTS:
-                a = np.ascontiguousarray(arrays[name], np.int32)
-                setattr(d, name, a.ctypes.data_as(_I32P))
-            else:
-                a = np.ascontiguousarray(arrays[name], np.float64)
-                setattr(d, name, a.ctypes.data_as(_F64P))
-            keep.append(a)
+        keep = [np.ascontiguousarray(arrays[name], np.int32 if name in _INTS else np.float64) for name in _ORDER]
+        # all the pointers at once: a ctypes cast per array took 0.1 ms a mesh
+        at = np.frombuffer(d, np.uint64, len(_ORDER), getattr(MeshDesc, _ORDER[0]).offset)
+        at[:] = [a.__array_interface__["data"][0] for a in keep]
         d._keep = keep
         return d
 
