@@ -1,7 +1,7 @@
 // FP64 logarithm, exponential and power evaluated on the integer pipe.
 //
-// GB300 retires 2 FP64 lanes per clock per SM but 64 integer lanes: a
-// warp-wide FP64 instruction holds the SM's FP64 pipe for 16 cycles, an
+// GB300 retires 1.6 FP64 lanes per clock per SM but 64 integer lanes: a
+// warp-wide FP64 instruction holds the SM's FP64 pipe for 20 cycles, an
 // integer instruction for half a cycle.  The right-hand side's powers
 // (van Genuchten's KrFunc and Psi, Manning's h^0.6666667) therefore run
 // here in 64-bit fixed point with 128-bit products, and only their inputs

@@ -38,7 +38,7 @@ constexpr double kSh2oMin = 0.02;
 constexpr double kBadVal = -999.0;
 
 // A double whose divisions, roots, comparisons, sign changes and elementary
-// functions stay off the FP64 pipe.  GB300 retires 2 FP64 lanes per clock per
+// functions stay off the FP64 pipe.  GB300 retires 1.6 FP64 lanes per clock per
 // SM; a column step is mostly divisions, logarithms, powers and tests, and
 // with the FP64 instructions for them the pipe was busy for 4.9 of the 5.8 ms
 // of a 200,000-element step (15,500 FP64 instructions a warp).  Divisions,

@@ -16,7 +16,7 @@
 // Divisions and reciprocals run on the integer pipe (int_math.cuh: a float
 // seed, two fixed-point Newton steps and an exact midpoint test, the IEEE
 // quotient bit for bit) with the FP64 instruction for zeros, subnormals,
-// infinities and NaN: GB300 retires 2 FP64 lanes per clock per SM, and an
+// infinities and NaN: GB300 retires 1.6 FP64 lanes per clock per SM, and an
 // FP64 division costs about as much pipe time as fifteen additions.
 #pragma once
 

@@ -1657,8 +1657,8 @@ cudaError_t fused_plan(FusedPlan *f) {
 }
 
 // How k_rhs_fused would run this evaluation: blocks as small as leave every
-// SM a few warps, so that a small mesh spreads over the chip (the FP64 pipe
-// retires two lanes a clock on each SM), one item a thread.  False when the
+// SM a few warps, so that a small mesh spreads over the chip (an SM takes an
+// FP64 warp instruction every 20 clocks), one item a thread.  False when the
 // items are more than can be resident together: the blocks of one kind would
 // then take turns while the others wait, and the separate kernels are faster.
 struct FusedLaunch {
