@@ -58,7 +58,7 @@ BatchOps::Ew BatchOps::push(int code, double a, double b, int x, int y, int z, d
 }
 
 void BatchOps::Red2::await_suspend(std::coroutine_handle<> h) const noexcept { s->waiting = h; }
-std::pair<double, double> BatchOps::Red2::await_resume() const noexcept {
+bdf::Two BatchOps::Red2::await_resume() const noexcept {
   if (sum) return {std::sqrt(s->red_value / (double)s->neq), s->red_value};
   return {s->red_value, std::sqrt(s->red_value2 / (double)s->neq)};
 }

@@ -7,7 +7,6 @@
 #include <cstdint>
 #include <map>
 #include <memory>
-#include <utility>
 #include <vector>
 
 #include "batch_device.h"
@@ -111,7 +110,7 @@ struct BatchOps {
     bool sum;  // the WRMS norm and its sum of squares; else a minimum and a WRMS norm
     bool await_ready() const noexcept { return false; }
     void await_suspend(std::coroutine_handle<> h) const noexcept;
-    std::pair<double, double> await_resume() const noexcept;
+    bdf::Two await_resume() const noexcept;
   };
   bool joined(int) const { return true; }
   Red2 min_wrms(int m, int x, int w) { return Red2{(reduce(kRedMinWsq, m, x, false, w), s), false}; }

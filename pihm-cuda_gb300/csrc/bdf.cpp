@@ -174,7 +174,7 @@ struct NVectorOps {
   // ---- two values of one pass (bdf_core.h) ----
   bool joined(Vec v) const { return queue.accepts(v); }
   // the minimum of m, and the WRMS norm of x by w
-  pihm::Ready<std::pair<double, double>> min_wrms(Vec m, Vec x, Vec w) {
+  pihm::Ready<pihm::bdf::Two> min_wrms(Vec m, Vec x, Vec w) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
     double mn, sum;
     if (queue.min_wsq(m, x, w, &mn, &sum, nullptr, nullptr))
@@ -185,7 +185,7 @@ struct NVectorOps {
   }
   // the WRMS norm of x by w and its sum of squares (NAN: not known), with the status of a
   // right-hand side left pending (rhs_failed)
-  pihm::Ready<std::pair<double, double>> wrms_sum(Vec x, Vec w) {
+  pihm::Ready<pihm::bdf::Two> wrms_sum(Vec x, Vec w) {
     Scope sc(timer, PIHM_BDF_OPT_REDUCTION);
     unsigned int word = 0;
     const unsigned int *dev_word = rhs_pending ? pihm_gpu_error_word((pihm_gpu_ctx *)user_data) : nullptr;

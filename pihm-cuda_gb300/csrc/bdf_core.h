@@ -88,6 +88,11 @@ inline double sun_powi(double b, int e) {
 inline double sun_max(double a, double b) { return (a > b) ? a : b; }
 inline double sun_min(double a, double b) { return (a < b) ? a : b; }
 
+// Two values of one pass over the vectors.
+struct Two {
+  double first, second;
+};
+
 // A linear-sum coefficient held as a reduction result on the vectors' side
 // (policies with device-resident scalars): a constant, or -s, 1/s, 1/(1/s),
 // -(1/(1/s)) of slot s.
