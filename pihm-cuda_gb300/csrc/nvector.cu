@@ -99,12 +99,38 @@ static inline unsigned grid_for(long long n) {
   return (unsigned)(b > 0 ? b : 1);
 }
 
+// The kernels here are programmatic dependent launches: a block waits for the
+// kernel before it and reads nothing until then.  An iteration's sixteen
+// operations over 31,337 entries take 68 us instead of 86, over 3.06M 238
+// instead of 258.  A grid of one wave lets the next one's blocks in as it
+// starts; of more, they would hold its own blocks' places (3.06M: 262).
+constexpr unsigned kWave = 8 * 152;
+__device__ __forceinline__ void begin_after_previous() {
+  if (gridDim.x <= kWave) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+static int launch_after(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, P(args)...) == cudaSuccess) return 0;
+  (void)cudaGetLastError();
+  return -2;
+}
+
 // ---------------------------------------------------------------------------
 // element-wise kernels
 // ---------------------------------------------------------------------------
 template <int OP>
-__global__ void k_ew(long long n, double a, double b, const double *__restrict__ x,
-                     const double *__restrict__ y, double *z) {
+__global__ void k_ew(long long n, double a, double b, const double *x, const double *y, double *z) {
+  begin_after_previous();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const double xv = ew_reads_x(OP) ? x[i] : 0.0;
@@ -118,8 +144,7 @@ template <int OP>
 static int ew(long long n, double a, double b, const double *x, const double *y, double *z,
               cudaStream_t st) {
   if (n <= 0) return 0;
-  k_ew<OP><<<grid_for(n), kThreads, 0, st>>>(n, a, b, x, y, z);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_after(k_ew<OP>, grid_for(n), kThreads, st, n, a, b, x, y, z);
 }
 
 // One element-wise call after the serial N_Vector's case analysis.
@@ -155,14 +180,14 @@ static int linear_sum(double a, const double *x, double b, const double *y, doub
 // x, y, w are the operands; m (optional) receives the ConstrMask output and
 // z the InvTest output.
 template <int OP>
-__global__ void __launch_bounds__(kThreads) k_red(long long n, const double *__restrict__ x,
-                                                  const double *__restrict__ y, double *__restrict__ z,
+__global__ void __launch_bounds__(kThreads) k_red(long long n, const double *x, const double *y, double *z,
                                                   double *partials, double *partials_f,
                                                   unsigned int *ticket, double *result,
                                                   long long wrms_n, double *host, uint64_t *host_seq,
                                                   uint64_t seq) {
   __shared__ Pair sh[kThreads / 32];
   __shared__ bool last;
+  begin_after_previous();
   Pair acc = red_identity<OP>();
   const long long stride = (long long)gridDim.x * blockDim.x;
   long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -270,6 +295,7 @@ __global__ void k_lin_coef(long long n, int ka, int sa, double va, int kb, int s
                            const double *x, const double *y, double *z, const double *slots) {
   __shared__ int s_op, s_xt, s_yt;
   __shared__ double s_a, s_b;
+  begin_after_previous();
   if (threadIdx.x == 0) {
     const double a = coef_value(ka, va, ka == COEF_HOST ? 0.0 : slots[2 * sa]);
     const double b = coef_value(kb, vb, kb == COEF_HOST ? 0.0 : slots[2 * sb]);
@@ -308,9 +334,8 @@ static int red_launch(long long n, const double *x, const double *y, double *z, 
                       unsigned int *ticket, double *result_dev, cudaStream_t st, long long wrms_n = 0,
                       double *host = nullptr, uint64_t *host_seq = nullptr, uint64_t seq = 0) {
   const unsigned g = red_grid_for(n);
-  k_red<OP><<<g, kThreads, 0, st>>>(n, x, y, z, partials, partials + kMaxBlocks, ticket, result_dev, wrms_n,
-                                    host, host_seq, seq);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_after(k_red<OP>, g, kThreads, st, n, x, y, z, partials, partials + kMaxBlocks, ticket, result_dev,
+                      wrms_n, host, host_seq, seq);
 }
 
 template <int OP>
@@ -427,7 +452,7 @@ __global__ void __launch_bounds__(kT, 4) k_seq(const __grid_constant__ Seq q) {
   const long long n = q.n;
   const int nblk = (int)red_grid_for(n);
   const long long stride = (long long)nblk * kThreads;
-  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+  begin_after_previous();
   if (tid < q.nops) {
     const SeqOp &o = q.op[tid];
     SeqHead h = {o.a, o.b, o.x, o.y, o.z, o.code, o.fwd};
@@ -549,18 +574,7 @@ __global__ void __launch_bounds__(kT, 4) k_seq(const __grid_constant__ Seq q) {
 
 template <int RA, int RB, bool kSpread, int kT>
 static int seq_launch_t(const Seq &q, unsigned grid, cudaStream_t st) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kT);
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, k_seq<RA, RB, kSpread, kT>, q) == cudaSuccess) return 0;
-  (void)cudaGetLastError();
-  return -2;
+  return launch_after(k_seq<RA, RB, kSpread, kT>, grid, kT, st, q);
 }
 
 template <int RA, int RB>
@@ -838,9 +852,8 @@ int N_VLinearSumCoef_PihmGpu(const pihm_nv_coef *a, N_Vector x, const pihm_nv_co
     return linear_sum(a->value, D(x), b->value, D(y), D(z), n, S(z));
   if (n <= 0) return 0;
   const int ztag = D(z) == D(x) ? 0 : (D(z) == D(y) ? 1 : 2);
-  k_lin_coef<<<grid_for(n), kThreads, 0, S(z)>>>(n, a->kind, a->slot, a->value, b->kind, b->slot, b->value, ztag,
-                                                  D(x), D(y), D(z), C(z)->fam->scratch.slots);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_after(k_lin_coef, grid_for(n), kThreads, S(z), n, a->kind, a->slot, a->value, b->kind, b->slot,
+                      b->value, ztag, D(x), D(y), D(z), C(z)->fam->scratch.slots);
 }
 
 int N_VFetchSlots_PihmGpu(N_Vector v, int count, double *out, const unsigned int *dev_word,
