@@ -75,7 +75,9 @@ int pihm_bdf_set_stop_time(pihm_bdf *mem, double tstop);
  * once, together with the right-hand side's status when that is this
  * library's pihm_gpu_ode on the vectors' stream (pihm_gpu_ode_launch): one
  * host round trip per iteration instead of one per reduction and per
- * evaluation.  setting -1 (default): on for device vectors of this library
+ * evaluation.  A Newton iteration's evaluation leaves its status to the
+ * linear solver's norm in the same way (unless pihm_gpu_set_nan_check defers
+ * it further).  setting -1 (default): on for device vectors of this library
  * integrated with pihm_gpu_ode; 1: on for any vectors (host vectors keep
  * the values on the host; a right-hand side other than pihm_gpu_ode reports
  * at once, and recoverable failures are retried as CVODE retries them);
@@ -87,7 +89,9 @@ int pihm_bdf_set_deferred_scalars(pihm_bdf *mem, int setting);
 int pihm_bdf_get_deferred_scalars(const pihm_bdf *mem);
 /* Host time inside the integrator's vector operations (no CVODE
  * counterpart), accumulated while on (pihm_bdf_set_op_timing resets it):
- * issuing element-wise operations (and reductions left on the device),
+ * issuing element-wise operations (and reductions left on the device; the
+ * device vectors' operations are queued and run with the next reduction or
+ * ahead of the next right-hand side, and none is left queued on return),
  * reductions until their value is back on the host (and slot read-backs),
  * right-hand-side calls until they return.  Wall time outside these is the
  * integrator's own host work plus the device time the calls waited for. */

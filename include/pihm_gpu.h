@@ -275,7 +275,7 @@ int pihm_gpu_launch_count(const pihm_gpu_ctx *ctx, int64_t *count);
 int pihm_gpu_set_profiling(pihm_gpu_ctx *ctx, int on);
 /* Synchronise, then return and reset the accumulated device time (ms) and
  * launch count per kernel: 0 prep, 1 gradient, 2 element, 3 river,
- * 4 finish, 5 edge, 6 permute; n entries are written. */
+ * 4 finish (k_bank_rows), 5 edge, 6 permute; n entries are written. */
 int pihm_gpu_kernel_times(pihm_gpu_ctx *ctx, double *ms, int64_t *calls, int n);
 
 /* Diagnostic: the power of the right-hand-side kernels (the integer-pipe

@@ -147,7 +147,7 @@ int pihm_gpu_nv_dot_prod(const double *x, const double *y, int64_t n, void *stre
  * and the Gram-Schmidt dot products (ModifiedGS, sundials_iterative.c) are
  * only coefficients of the next linear sums until the Hessenberg column is
  * complete.  These entry points keep such values in the vector family's
- * slot array on the device, use them there, and read them back in one copy.
+ * slot array on the device, use them there, and read them back in one round trip.
  * --------------------------------------------------------------------- */
 #define PIHM_NV_SLOTS 16
 /* A linear-sum coefficient: a host constant, or derived from slot s. */
