@@ -6,8 +6,8 @@
 // the current round, and a reduction or a right-hand-side evaluation ends the
 // program and suspends the coroutine.  A round uploads all programs, runs them
 // in one launch of the program kernel (batch_kernels.cu), evaluates the right
-// hand side once over the arena for the watersheds that asked for it, reads
-// back every reduction result and error word in one copy, and resumes the
+// hand side once over the arena for the watersheds that asked for it, finds
+// every reduction result and error word in pinned memory, and resumes the
 // coroutines.  Watersheds therefore proceed independently -- each with its own
 // step size, order, Newton and Krylov iterations, model step and stopping
 // time -- while sharing every launch.

@@ -1351,7 +1351,8 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
 //   elements  prep -> | A, heads -> gradient -> | B
 //   edges             | A, Darcy flux, h^p ---- | B, slope -> flux | C
 //   rivers    area, perimeter | R, channel flux ------------------- | C, rows
-//   banks     | A, fluxes with the elements ----------------------- (to C)
+//   banks     area, perimeter | A, fluxes with the elements -------- (to C)
+//   beds      area, perimeter | A, R, bed fluxes, outlets ---------- (to C)
 //   columns   saturation, powers, recharge | A, infiltration's head | C, rows
 //
 // Everything a block can do without the others' results stands before its
@@ -1361,11 +1362,11 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
 // results are the same bits.
 //
 // A, B, C, R are counters in device memory that the blocks before them raise
-// once (C: edges, rivers and banks).  The
-// last block through C zeroes them -- elements and edges have raised C or
-// what C waits for by then -- so a captured launch can be replayed.  Cooperative launch makes the blocks
-// resident together; a wait gives up after kBarPolls polls, and the blocks
-// then report kErrWait instead of results.
+// once (R: every river block; C: edges, rivers, banks and beds).  The last
+// block through C zeroes them -- every other block has raised C, or what C
+// waits for, behind its own last wait -- so a captured launch can be replayed.
+// Cooperative launch makes the blocks resident together; a wait gives up after
+// kBarPolls polls, and the blocks then report kErrWait instead of results.
 // ---------------------------------------------------------------------------
 constexpr int kBarPolls = 1 << 22;  // a few seconds
 constexpr int kBarStride = 32;      // counters on cache lines of their own
@@ -1716,8 +1717,9 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
                        const int32_t *iperm) {
   bool on;
   // a small mesh in one launch (per-kernel timing keeps the separate kernels):
-  // one evaluation of 1,000 / 20,000 / 40,000 elements takes 18 / 24 / 33 us
-  // instead of 41 / 46 / 54
+  // one evaluation of 1,000 / 20,000 / 40,000 elements takes 16 / 21 / 29 us
+  // (the five launches 43 for 60,000; as seven plain launches on two streams
+  // the same meshes took 41 / 46 / 54)
   FusedLaunch fl;
   if (fused && !prof && fused_fits(m, *fused, y_ref != nullptr, &fl)) {
     ++*launches;
