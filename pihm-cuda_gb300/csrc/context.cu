@@ -17,7 +17,7 @@ namespace pihm {
 cudaError_t launch_permute(const double *src, double *dst, const int32_t *perm, int ne, int nr,
                            int to_internal, cudaStream_t st);
 cudaError_t launch_permute_ref(const double *src, double *dst, const int32_t *iperm, int ne, int nr,
-                               int to_internal, cudaStream_t st);
+                               int to_internal, const StatusOut &done, cudaStream_t st);
 }  // namespace pihm
 
 using namespace pihm;
@@ -413,12 +413,9 @@ __global__ static void k_status(const unsigned int *err, uint64_t *host, uint64_
   pihm::host_flag_set(host + 1, seq);
 }
 
-int pihm_gpu_status(pihm_gpu_ctx *c) {
-  if (!c) return PIHM_GPU_ERR_ARG;
-  const uint64_t seq = ++c->status_seq;
-  k_status<<<1, 1, 0, c->stream>>>(c->m.err, c->h_status, seq);
-  if (cudaGetLastError() != cudaSuccess || !pihm::host_flag_wait(c->h_status + 1, seq, c->stream))
-    return PIHM_GPU_ERR_CUDA;
+// the status in the error word that a kernel hands over with seq
+static int status_at(pihm_gpu_ctx *c, uint64_t seq) {
+  if (!pihm::host_flag_wait(c->h_status + 1, seq, c->stream)) return PIHM_GPU_ERR_CUDA;
   const unsigned int err = (unsigned int)c->h_status[0];
   if (err) {
     cudaMemsetAsync(c->m.err, 0, sizeof(unsigned int), c->stream);
@@ -428,6 +425,13 @@ int pihm_gpu_status(pihm_gpu_ctx *c) {
     return err & kErrWait ? PIHM_GPU_ERR_CUDA : PIHM_GPU_ERR_NAN;
   }
   return PIHM_GPU_OK;
+}
+
+int pihm_gpu_status(pihm_gpu_ctx *c) {
+  if (!c) return PIHM_GPU_ERR_ARG;
+  const uint64_t seq = ++c->status_seq;
+  k_status<<<1, 1, 0, c->stream>>>(c->m.err, c->h_status, seq);
+  return cudaGetLastError() == cudaSuccess ? status_at(c, seq) : PIHM_GPU_ERR_CUDA;
 }
 
 // The copy path's staging pairs, streams and events, on first use.
@@ -473,8 +477,14 @@ static void copy_path_release(pihm_gpu_ctx *c) {
   cp = pihm_gpu_ctx::CopyPath{};
 }
 
-// The host-buffer evaluation queued on the context's stream.
-static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_host) {
+// The host-buffer evaluation queued on the context's stream.  seq: the caller
+// waits for this evaluation alone; on the direct path of a small mesh its last
+// kernel hands the error word over with *seq (left 0 otherwise).
+// 1,000 / 5,000 / 20,000 elements: 34.4 / 35.0 / 43.0 us with k_status behind
+// it, 32.5 / 32.7 / 42.2 without; from 60,000 on the blocks' fences over the
+// host link cost as much (76.7 both; 200,000: 154.3 and 156.8).
+constexpr int kStatusWithValues = 40000;
+static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_host, uint64_t *seq = nullptr) {
   const size_t bytes = sizeof(double) * c->neq;
   // direct: k_elem_prep reads y from and the reordering kernel writes ydot to
   // host memory over the host link, in reference order (contiguous on the
@@ -490,7 +500,9 @@ static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_
     cudaError_t e = launch_rhs(c->m, y_int, ydot_int, c->stream, &c->launches, c->prof, &c->fused, y_dev,
                                c->d_iperm);
     if (e == cudaSuccess) {
-      e = launch_permute_ref(ydot_int, yd_dev, c->d_iperm, c->ne, c->nr, 0, c->stream);
+      StatusOut done{};
+      if (seq && c->ne <= kStatusWithValues) done = StatusOut{c->m.err, c->m.bar + kStatusTicket, c->h_status, *seq = ++c->status_seq};
+      e = launch_permute_ref(ydot_int, yd_dev, c->d_iperm, c->ne, c->nr, 0, done, c->stream);
       c->launches++;
     }
     return e == cudaSuccess ? PIHM_GPU_OK : PIHM_GPU_ERR_CUDA;
@@ -529,16 +541,17 @@ static int rhs_host_enqueue(pihm_gpu_ctx *c, const double *y_host, double *ydot_
 
 // Everything a host-buffer evaluation queued: the derivatives' copies out
 // (after their kernels), then the error word on the context's stream.
-static int host_wait(pihm_gpu_ctx *c) {
+static int host_wait(pihm_gpu_ctx *c, uint64_t seq = 0) {
   if (c->cp.ready && cudaStreamSynchronize(c->cp.d2h) != cudaSuccess) return PIHM_GPU_ERR_CUDA;
-  return pihm_gpu_status(c);
+  return seq ? status_at(c, seq) : pihm_gpu_status(c);
 }
 
 int pihm_gpu_rhs_host(pihm_gpu_ctx *c, double t, const double *y_host, double *ydot_host) {
   (void)t;
   if (!c || !y_host || !ydot_host) return PIHM_GPU_ERR_ARG;
-  const int rc = rhs_host_enqueue(c, y_host, ydot_host);
-  return rc != PIHM_GPU_OK ? rc : host_wait(c);
+  uint64_t seq = 0;
+  const int rc = rhs_host_enqueue(c, y_host, ydot_host, &seq);
+  return rc != PIHM_GPU_OK ? rc : host_wait(c, seq);
 }
 
 int pihm_gpu_rhs_host_async(pihm_gpu_ctx *c, double t, const double *y_host, double *ydot_host) {

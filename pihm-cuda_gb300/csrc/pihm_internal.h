@@ -41,6 +41,7 @@ constexpr int32_t kBoundary = INT32_MIN;
 // Bits of an error word: a derivative came out NaN; a wait inside a kernel
 // ran out (the evaluation's results are not valid).
 constexpr unsigned kErrNan = 1u, kErrWait = 2u;
+constexpr int kStatusTicket = 144;  // the word of it that k_permute_ref counts its blocks in
 constexpr int kBarWords = 160;  // unsigned words of DevMesh::bar
 
 // Device view of one watershed, passed by value to the kernels.
@@ -262,6 +263,14 @@ struct FusedPlan {
   int blocks[2][kSizes] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 };
 cudaError_t fused_plan(FusedPlan *f);
+
+// Where a kernel leaves an error word for the host (host_flag.h: host[0], then
+// seq in host[1]); host null: nowhere.
+struct StatusOut {
+  const unsigned int *err;
+  unsigned int *ticket;
+  uint64_t *host, seq;
+};
 
 // y_ref, iperm (host-buffer evaluation of a single watershed): the state in
 // reference order, read by k_elem_prep, which fills y (internal order) from it.

@@ -49,6 +49,7 @@
 #include <cstdlib>
 
 #include "fp64_math.cuh"
+#include "host_flag.h"
 #include "pihm_internal.h"
 
 namespace pihm {
@@ -1583,8 +1584,12 @@ __global__ void __launch_bounds__(256) k_permute(const double *src, double *dst,
 // internal element index): the reference-order side is read or written
 // contiguously, which is the side in host memory when the host-buffer
 // evaluation accesses it directly.
+//
+// With a status to hand over (done.host): the last block writes the error word
+// and the sequence number behind every block's values, which saves the host
+// call a kernel of its own for it.
 __global__ void __launch_bounds__(256) k_permute_ref(const double *src, double *dst, const int32_t *RESTRICT iperm,
-                                                     int ne, int nr, int to_internal) {
+                                                     int ne, int nr, int to_internal, StatusOut done) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   const bool elem = r < ne;
   const int i = elem ? iperm[r] : 0;
@@ -1592,6 +1597,17 @@ __global__ void __launch_bounds__(256) k_permute_ref(const double *src, double *
   const long long plane = (long long)blockIdx.y * ne;
   if (elem) dst[plane + (to_internal ? i : r)] = src[plane + (to_internal ? r : i)];
   else if (blockIdx.y == 2 && r - ne < 2 * nr) dst[plane + r] = src[plane + r];
+  if (!done.host) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    if (atomicAdd(done.ticket, 1u) == gridDim.x * gridDim.y - 1) {
+      *done.ticket = 0u;
+      __threadfence_system();
+      done.host[0] = *done.err;
+      host_flag_set(done.host + 1, done.seq);
+    }
+  }
 }
 
 }  // namespace pihm
@@ -1795,9 +1811,9 @@ cudaError_t launch_permute(const double *src, double *dst, const int32_t *perm, 
 }
 
 cudaError_t launch_permute_ref(const double *src, double *dst, const int32_t *iperm, int ne, int nr,
-                               int to_internal, cudaStream_t st) {
+                               int to_internal, const StatusOut &done, cudaStream_t st) {
   if (ne + 2LL * nr == 0) return cudaSuccess;
-  return launch_after(k_permute_ref, dim3(blocks_for(ne + 2LL * nr, 256), 3), 256, st, src, dst, iperm, ne, nr, to_internal);
+  return launch_after(k_permute_ref, dim3(blocks_for(ne + 2LL * nr, 256), 3), 256, st, src, dst, iperm, ne, nr, to_internal, done);
 }
 
 }  // namespace pihm
