@@ -1366,6 +1366,9 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
 // once (R: every river block; C: edges, rivers, banks and beds).  The last
 // block through C zeroes them -- every other block has raised C, or what C
 // waits for, behind its own last wait -- so a captured launch can be replayed.
+// For the elements' wait on A that holds because the edges wait for B: without
+// an interior edge nothing would, so then (edges alone read the gradients) the
+// elements are done when they have raised A.
 // Cooperative launch makes the blocks resident together; a wait gives up after
 // kBarPolls polls, and the blocks then report kErrWait instead of results.
 // ---------------------------------------------------------------------------
@@ -1419,7 +1422,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
   __shared__ int s_ok;
   unsigned *const A = m.bar, *const B = m.bar + kBarStride, *const C = m.bar + 2 * kBarStride,
                   *const R = m.bar + 3 * kBarStride;
-  const bool grad = m.surf_mode == kDiffWave;
+  const bool grad = m.surf_mode == kDiffWave && g.edge > 0;
   const int ne = m.ne;
   int blk = blockIdx.x;
   int sy;
