@@ -49,9 +49,9 @@ struct Seq {
   double *partials;
   const double *slots;
   unsigned int *ticket;
-  double *host;                // with a sequence number: the first reduction's
-  uint64_t *host_seq;          // value and flag go to host[0..1], or (fetch >= 0)
-  uint64_t seq;                // slots 0..fetch-1 and *word behind them
+  double *host;                // with a sequence number: the reductions' values go
+  uint64_t *host_seq;          // to host[0..1], and slots 0..fetch-1 and *word
+  uint64_t seq;                // behind them
   const unsigned int *word;
   int32_t fetch;
   SeqRed red[2];
@@ -86,7 +86,10 @@ class NvQueue {
   bool take(N_Vector z, N_Vector x, N_Vector y);
   void push(const SeqOp &o);
   void push_red(const SeqRed &r);
-  int launch();
+  // Run what is queued.  back: the reductions' values come to the host with
+  // the launch, and behind them `fetch` slots (-1 none) and *word (may be
+  // null); whatever a launch hands back is its own, not the one before's.
+  int launch(bool back, int fetch = -1, const unsigned int *word = nullptr);
   Family *fam = nullptr;
   Seq q{};
 };

@@ -958,7 +958,7 @@ void NvQueue::push_red(const SeqRed &r) {
   }
 }
 
-int NvQueue::launch() {
+int NvQueue::launch(bool back, int fetch, const unsigned int *word) {
   // results that nothing reads before they are overwritten
   for (int p = 0; p < q.nops; p++) {
     const double *z = q.op[p].z;
@@ -974,19 +974,22 @@ int NvQueue::launch() {
       }
     }
   }
-  q.partials = fam->scratch.partials;
-  q.slots = fam->scratch.slots;
-  q.ticket = fam->scratch.ticket;
+  Scratch &s = fam->scratch;
+  q.partials = s.partials;
+  q.slots = s.slots;
+  q.ticket = s.ticket;
+  q.host = s.host;
+  q.host_seq = back ? s.seq_word() : nullptr;
+  q.seq = back ? ++s.seq : 0;
+  q.fetch = fetch;
+  q.word = word;
   const int r = seq_launch(q, fam->stream);
   q.nops = q.nred = 0;
   return r;
 }
 
 int NvQueue::flush() {
-  if (empty()) return 0;
-  q.host_seq = nullptr;
-  q.fetch = -1;
-  return launch();
+  return empty() ? 0 : launch(false);
 }
 
 bool NvQueue::linear_sum(double a, N_Vector x, double b, N_Vector y, N_Vector z) {
@@ -1042,11 +1045,7 @@ bool NvQueue::reduce(int op, N_Vector x, N_Vector y, double *value) {
   }
   Scratch &s = fam->scratch;
   push_red({D(x), y ? D(y) : nullptr, s.result, 0, op, 0});
-  q.host = s.host;
-  q.host_seq = s.seq_word();
-  q.seq = ++s.seq;
-  q.fetch = -1;
-  const bool ok = launch() == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  const bool ok = launch(true) == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
   *value = ok ? s.host[0] : NAN;
   return true;
 }
@@ -1064,12 +1063,7 @@ bool NvQueue::min_wsq(N_Vector m, N_Vector x, N_Vector w, double *mn, double *su
   Scratch &s = fam->scratch;
   if (m) push_red({D(m), nullptr, s.result, 0, R_MIN, 0});
   push_red({D(x), D(w), s.result, 0, R_WSQ, 0});
-  q.host = s.host;
-  q.host_seq = s.seq_word();
-  q.seq = ++s.seq;
-  q.fetch = dev_word ? 0 : -1;
-  q.word = dev_word;
-  const bool ok = launch() == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  const bool ok = launch(true, -1, dev_word) == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
   if (m) *mn = ok ? s.host[0] : NAN;
   *sum = ok ? s.host[m ? 1 : 0] : NAN;
   if (dev_word) *word_out = ok ? *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS) : ~0u;
@@ -1086,13 +1080,8 @@ bool NvQueue::fetch(N_Vector v, int count, double *out, const unsigned int *dev_
                     int *rc) {
   if (q.nred == 0 || count < 0 || count > PIHM_NV_SLOTS || !take(v, nullptr, nullptr)) return false;
   Scratch &s = fam->scratch;
-  q.host = s.host;
-  q.host_seq = s.seq_word();
-  q.seq = ++s.seq;
-  q.fetch = count;
-  q.word = dev_word;
   *rc = -2;
-  if (launch() || !pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream)) return true;
+  if (launch(true, count, dev_word) || !pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream)) return true;
   for (int i = 0; i < count; i++) out[i] = s.host[2 + i];
   if (dev_word) *word_out = *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS);
   *rc = 0;
