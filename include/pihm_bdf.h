@@ -98,7 +98,10 @@ int pihm_bdf_get_deferred_scalars(const pihm_bdf *mem);
 enum { PIHM_BDF_OPT_ELEMENTWISE = 0, PIHM_BDF_OPT_REDUCTION, PIHM_BDF_OPT_RHS, PIHM_BDF_OPT_COUNT };
 int pihm_bdf_set_op_timing(pihm_bdf *mem, int on);
 int pihm_bdf_get_op_times(const pihm_bdf *mem, double *ms, int64_t *calls);
-/* Advance to tout (CV_NORMAL): yout receives y(tout) (or y(tstop)). */
+/* Advance to tout (CV_NORMAL): yout receives y(tout) (or y(tstop)).
+ * PIHM_BDF_RHSFUNC_FAIL also when operations queued on the device vectors
+ * could not be launched (here and from pihm_bdf_init and _reinit): the
+ * vectors then do not hold what the integrator wrote to them. */
 int pihm_bdf_solve(pihm_bdf *mem, double tout, N_Vector yout, double *tret);
 int pihm_bdf_get_stats(const pihm_bdf *mem, pihm_bdf_stats *stats);
 void pihm_bdf_free(pihm_bdf *mem);

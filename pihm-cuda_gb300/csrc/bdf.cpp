@@ -295,11 +295,13 @@ struct NVectorOps {
 
 struct pihm_bdf : pihm::bdf::BdfCore<NVectorOps> {};
 
-// A call into the integrator leaves nothing queued.
+// A call into the integrator leaves nothing queued, and ends in an error when
+// queued operations were lost on the way.
 static int run(pihm_bdf *m, pihm::Task<int> task) {
   const int rc = pihm::run_sync(std::move(task));
   m->ops.flush();
-  return rc;
+  const bool lost = m->ops.queue.take_failure();
+  return lost && rc >= 0 ? PIHM_BDF_RHSFUNC_FAIL : rc;
 }
 
 extern "C" {

@@ -9,6 +9,10 @@
 // Whatever the queue does not take (a vector of another family or length, an
 // operation the caller replaced in the vector's table) makes the call return
 // false; the caller then flushes and calls the table.
+//
+// A launch that fails loses what was queued, so every value asked for from
+// then on is NAN (a fetch fails) until the caller has taken the failure
+// (take_failure), whichever launch it was.
 #pragma once
 
 #include <cstdint>
@@ -80,6 +84,12 @@ class NvQueue {
   // N_VFetchSlots_PihmGpu with the queued work ahead of it
   bool fetch(N_Vector v, int count, double *out, const unsigned int *dev_word, unsigned int *word_out, int *rc);
   int flush();
+  // whether a launch has failed since the last call
+  bool take_failure() {
+    const bool f = failed;
+    failed = false;
+    return f;
+  }
   bool empty() const { return q.nops == 0 && q.nred == 0; }
 
  private:
@@ -91,6 +101,7 @@ class NvQueue {
   // null); whatever a launch hands back is its own, not the one before's.
   int launch(bool back, int fetch = -1, const unsigned int *word = nullptr);
   Family *fam = nullptr;
+  bool failed = false;
   Seq q{};
 };
 

@@ -983,9 +983,9 @@ int NvQueue::launch(bool back, int fetch, const unsigned int *word) {
   q.seq = back ? ++s.seq : 0;
   q.fetch = fetch;
   q.word = word;
-  const int r = seq_launch(q, fam->stream);
+  if (seq_launch(q, fam->stream) || (back && !pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream))) failed = true;
   q.nops = q.nred = 0;
-  return r;
+  return failed ? -2 : 0;
 }
 
 int NvQueue::flush() {
@@ -1039,13 +1039,13 @@ bool NvQueue::reduce(int op, N_Vector x, N_Vector y, double *value) {
                    : op == R_MAXABS ? o->nvmaxnorm == N_VMaxNorm_PihmGpu
                                     : o->nvmin == N_VMin_PihmGpu;
   // with nothing queued the vector's own kernel is the shorter one
-  if (!own || empty() || !take(x, y, nullptr)) return false;
+  if (!own || (empty() && !failed) || !take(x, y, nullptr)) return false;
   if (q.nred > 0) {  // its value is the first one's
     flush();
   }
   Scratch &s = fam->scratch;
   push_red({D(x), y ? D(y) : nullptr, s.result, 0, op, 0});
-  const bool ok = launch(true) == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  const bool ok = launch(true) == 0;
   *value = ok ? s.host[0] : NAN;
   return true;
 }
@@ -1063,7 +1063,7 @@ bool NvQueue::min_wsq(N_Vector m, N_Vector x, N_Vector w, double *mn, double *su
   Scratch &s = fam->scratch;
   if (m) push_red({D(m), nullptr, s.result, 0, R_MIN, 0});
   push_red({D(x), D(w), s.result, 0, R_WSQ, 0});
-  const bool ok = launch(true, -1, dev_word) == 0 && pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream);
+  const bool ok = launch(true, -1, dev_word) == 0;
   if (m) *mn = ok ? s.host[0] : NAN;
   *sum = ok ? s.host[m ? 1 : 0] : NAN;
   if (dev_word) *word_out = ok ? *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS) : ~0u;
@@ -1078,10 +1078,10 @@ bool NvQueue::reduce_slot(int op, N_Vector x, N_Vector y, int slot) {
 
 bool NvQueue::fetch(N_Vector v, int count, double *out, const unsigned int *dev_word, unsigned int *word_out,
                     int *rc) {
-  if (q.nred == 0 || count < 0 || count > PIHM_NV_SLOTS || !take(v, nullptr, nullptr)) return false;
+  if ((q.nred == 0 && !failed) || count < 0 || count > PIHM_NV_SLOTS || !take(v, nullptr, nullptr)) return false;
   Scratch &s = fam->scratch;
   *rc = -2;
-  if (launch(true, count, dev_word) || !pihm::host_flag_wait(s.seq_word(), s.seq, fam->stream)) return true;
+  if (launch(true, count, dev_word)) return true;
   for (int i = 0; i < count; i++) out[i] = s.host[2 + i];
   if (dev_word) *word_out = *(const unsigned int *)(s.host + 2 + PIHM_NV_SLOTS);
   *rc = 0;

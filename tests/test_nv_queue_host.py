@@ -79,3 +79,32 @@ lib.pihm_bdf_solve(m, 60.0, b.y, ctypes.byref(t))
 assert word not in words()
 lib.pihm_bdf_free(m)
 """)
+
+
+@pytest.mark.parametrize("deferred", [0, 1])
+def test_a_lost_launch_ends_the_call_in_an_error(fake, deferred):
+    """Every launch of queued operations whose value nobody waits for, refused
+    in turn: the call that lost it returns an error, and the integrator
+    initialised again is usable."""
+    _child(fake, f"""
+RHS = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_double, VP, VP, VP)
+cb = RHS(lambda t, y, ydot, ud: 0)
+y = lib.N_VNew_PihmGpu(40, None)
+m = integrator(y, ctypes.cast(cb, VP), None, {deferred})
+solve = lambda: lib.pihm_bdf_solve(m, 1.0, y, ctypes.byref(t))
+fake.fake_reset()
+assert solve() == 0
+flushes = fake.fake_flushes()
+assert flushes > 2
+for k in range(flushes):
+    assert lib.pihm_bdf_init(m, ctypes.cast(cb, VP), 0.0, y) == 0
+    fake.fake_reset()
+    fake.fake_refuse(k)
+    rc = solve()
+    assert fake.fake_flushes() > k and rc < 0, (k, rc)
+    fake.fake_refuse(-1)
+    assert lib.pihm_bdf_init(m, ctypes.cast(cb, VP), 0.0, y) == 0
+    assert solve() == 0
+lib.pihm_bdf_free(m)
+lib.N_VDestroy_PihmGpu(y)
+""")
