@@ -421,11 +421,11 @@ cudaError_t launch_program(const DeviceArena &a, int nrs, int nblocks, int varia
   if (variant == kProgramSpread) {
     cfg.gridDim = dim3((unsigned)nblocks * (kThreads / 32));
     cfg.blockDim = dim3(kSpreadThreads);
-    return cudaLaunchKernelEx(&cfg, k_program<0>, a, nrs, flag, seq);
+    return launched(cudaLaunchKernelEx(&cfg, k_program<0>, a, nrs, flag, seq));
   }
-  if (variant == 0) return cudaLaunchKernelEx(&cfg, k_program<1>, a, nrs, flag, seq);
-  if (variant == 1) return cudaLaunchKernelEx(&cfg, k_program<2>, a, nrs, flag, seq);
-  return cudaLaunchKernelEx(&cfg, k_program<4>, a, nrs, flag, seq);
+  if (variant == 0) return launched(cudaLaunchKernelEx(&cfg, k_program<1>, a, nrs, flag, seq));
+  if (variant == 1) return launched(cudaLaunchKernelEx(&cfg, k_program<2>, a, nrs, flag, seq));
+  return launched(cudaLaunchKernelEx(&cfg, k_program<4>, a, nrs, flag, seq));
 }
 
 }  // namespace batch

@@ -544,7 +544,7 @@ int land_launch(LandInstance &li, int64_t t, double stepsize, const double *y_de
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cuda_rc(cudaLaunchKernelEx(&cfg, k_land_step, li.L, y_dev, ne, (int)tm.tm_mon, stepsize));
+  return cuda_rc(launched(cudaLaunchKernelEx(&cfg, k_land_step, li.L, y_dev, ne, (int)tm.tm_mon, stepsize)));
 }
 
 void land_release(LandInstance &li) {

@@ -264,6 +264,13 @@ struct FusedPlan {
 };
 cudaError_t fused_plan(FusedPlan *f);
 
+// The result of a launch through cudaLaunchKernelEx, whose failure is taken
+// here: left behind as the runtime's last error, the next call would report it.
+inline cudaError_t launched(cudaError_t e) {
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
 // Where a kernel leaves an error word for the host (host_flag.h: host[0], then
 // seq in host[1]); host null: nowhere.
 struct StatusOut {

@@ -1714,7 +1714,7 @@ static cudaError_t launch_fused(const DevMesh &m, FusedLaunch &l, const double *
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelExC(&cfg, fused_kernel(l.dense, y_ref != nullptr), args);
+  return launched(cudaLaunchKernelExC(&cfg, fused_kernel(l.dense, y_ref != nullptr), args));
 }
 
 template <class... P, class... A>
@@ -1728,7 +1728,7 @@ static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int block, cuda
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return launched(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 
 cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStream_t st,
@@ -1804,7 +1804,8 @@ cudaError_t launch_rhs(const DevMesh &m, const double *y, double *ydot, cudaStre
     after(k_bank_rows, late + (m.nbank_run > 0 ? blocks_for(m.nbank_run, 128) : 0), 128, m, ydot, (int)late);
     prof_end(prof, on, st);
   }
-  return err == cudaSuccess ? cudaGetLastError() : err;
+  const cudaError_t plain = cudaGetLastError();
+  return err == cudaSuccess ? plain : err;
 }
 
 cudaError_t launch_permute(const double *src, double *dst, const int32_t *perm, int ne, int nr,

@@ -1,7 +1,7 @@
 // A stand-in for the CUDA runtime, preloaded into a CPU process by
 // test_nv_queue_host.py: memory is the host's, kernels do nothing, and a
 // kernel that hands values to the host hands over one constant.  It records
-// the launches of the N_Vector queue and can refuse one of them.
+// the launches of the N_Vector queue and can refuse one of them, or one of all.
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -13,7 +13,7 @@
 
 namespace {
 double g_value = 1e-3;
-long g_refuse = -1, g_flushes = 0;
+long g_refuse = -1, g_flushes = 0, g_refuse_any = -1, g_launches = 0;
 int g_last = 0;
 std::vector<const unsigned int *> g_words;
 std::map<const void *, std::string> &names() {
@@ -23,6 +23,7 @@ std::map<const void *, std::string> &names() {
 
 int launch(const void *func, void **args) {
   const std::string &name = names()[func];
+  if (g_launches++ == g_refuse_any) return g_last = 999;
   double *host = nullptr;
   uint64_t *word = nullptr, seq = 0;
   if (name.find("k_seq") != std::string::npos) {
@@ -57,8 +58,10 @@ struct Dim {
 extern "C" {
 void fake_refuse(long flush) { g_refuse = flush; }
 long fake_flushes() { return g_flushes; }
+void fake_refuse_any(long launch) { g_refuse_any = launch; }
+long fake_launches() { return g_launches; }
 void fake_reset() {
-  g_flushes = 0;
+  g_flushes = g_launches = 0;
   g_words.clear();
 }
 long fake_words(uint64_t *out, long n) {
@@ -105,8 +108,8 @@ int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *) { return cu
 int cudaStreamSynchronize(void *) { return 0; }
 int cudaDeviceSynchronize() { return 0; }
 int cudaGetDevice(int *d) { return *d = 0; }
-int cudaDeviceGetAttribute(int *v, int, int) {
-  *v = 0;
+int cudaDeviceGetAttribute(int *v, int attr, int) {
+  *v = attr == 16 ? 152 : (attr == 95 ? 1 : 0);  // SMs; cooperative launch
   return 0;
 }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *, int, size_t) {
