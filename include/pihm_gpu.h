@@ -304,6 +304,10 @@ int pihm_gpu_selftest_pow_int(const double *x, const double *y, double *out, int
  * are the IEEE results bit for bit. */
 int pihm_gpu_selftest_div_sqrt_int(const double *a, const double *b, double *q, double *r,
                                    int32_t *ok, int64_t n, void *stream);
+/* Diagnostic: the land-surface step's exponential and natural logarithm,
+ * e[i] = exp(x[i]) and l[i] = log(x[i]); device arrays of length n,
+ * asynchronous on `stream`. */
+int pihm_gpu_selftest_land_exp_log(const double *x, double *e, double *l, int64_t n, void *stream);
 
 #ifdef __cplusplus
 }

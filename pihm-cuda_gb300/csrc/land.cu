@@ -7,7 +7,8 @@
 // (-fmad=false), so every product and sum rounds where the reference's C
 // rounds; divisions and square roots are IEEE.  exp, log and pow are the
 // fixed-point functions of int_math.cuh (0.502 ulp, almost always the
-// correctly rounded value the C library returns too), cos there has an
+// correctly rounded value the C library returns too) and, out of their ranges,
+// the double-double routines of fp64_math.cuh (about 0.51 ulp); cos has an
 // absolute error of 2^-60 beside its rounding; pow(x, 2) is x * x, the
 // correctly rounded square.  So the step reproduces the reference's values to
 // the last bit on nearly every element, and within a few ulps of the affected
@@ -47,18 +48,27 @@ constexpr int kLandBlock = 256;
 constexpr int kStepBlock = 128;
 
 // The elementary functions and comparisons stay off the FP64 pipe, which was
-// 74 % busy with them; the FP64 versions, for arguments out of the ranges,
-// are out of line.
-static __device__ __noinline__ double exp_slow(double x) { return exp(x); }
-static __device__ __noinline__ double log_slow(double x) { return log(x); }
+// 74 % busy with them; the versions for arguments out of the fixed-point
+// ranges are out of line: within 2^-6 of one the logarithm's own series,
+// elsewhere the double-double routines (0.51 ulp), CUDA's for what is left.
+static __device__ __noinline__ double exp_slow(double x) {
+  double r;
+  return exp_dd_checked(x, 0.0, r) ? r : exp(x);
+}
+static __device__ __noinline__ double log_slow(double x) {
+  double r, lo;
+  if (im::log_near1_i(x, false, r)) return r;
+  return log_dd_fast(x, r, lo) ? r + lo : log(x);
+}
 static __device__ __noinline__ double cos_slow(double x) { return cos(x); }
 __device__ __forceinline__ double exp_l(double x) {
   double r;
   return im::exp_i(x, r) ? r : exp_slow(x);
 }
 __device__ __forceinline__ double log_l(double x) {
+  // (the bound of log_i's 0.502 ulp ends at |log2 x| = 1/2)
   double r;
-  return im::log_i(x, kImCLn2, r) ? r : log_slow(x);
+  return im::log_i(x, kImCLn2, r) && (cmp::lt_c(x, 0.7) || cmp::gt_c(x, 1.42)) ? r : log_slow(x);
 }
 __device__ __forceinline__ double cos_l(double x) {
   double r;
@@ -67,6 +77,13 @@ __device__ __forceinline__ double cos_l(double x) {
 __device__ __forceinline__ double at_least(double x, double c) { return cmp::lt_c(x, c) ? c : x; }  // c > 0
 __device__ __forceinline__ double at_most(double x, double c) { return cmp::gt_c(x, c) ? c : x; }   // c > 0
 __device__ __forceinline__ double not_neg(double x) { return cmp::lt0(x) ? 0.0 : x; }
+
+__global__ void k_exp_log(const double *x, double *e, double *l, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  e[i] = exp_l(x[i]);
+  l[i] = log_l(x[i]);
+}
 
 // IntrplForc's bisection (src/forcing.c:503-528): the knot `middle` with
 // T[middle-1] <= t <= T[middle], or -1.  The host has checked that t lies in
@@ -601,6 +618,12 @@ int pihm_gpu_land_get(pihm_gpu_ctx *c, int field, double *out) {
   if (rc != PIHM_GPU_OK) return rc;
   for (int i = 0; i < ne; i++) out[c->h_perm[i]] = tmp[i];
   return PIHM_GPU_OK;
+}
+
+int pihm_gpu_selftest_land_exp_log(const double *x, double *e, double *l, int64_t n, void *stream) {
+  if (n <= 0 || !x || !e || !l) return -1;
+  k_exp_log<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, e, l, n);
+  return cuda_rc(cudaGetLastError());
 }
 
 }  // extern "C"
