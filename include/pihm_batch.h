@@ -121,6 +121,9 @@ int pihm_batch_set_stream(pihm_batch *b, void *stream);
  * request at once; 1 (the default) gathers every waiting watershed into each
  * evaluation.  Results do not depend on it; throughput does. */
 int pihm_batch_set_rhs_gate(pihm_batch *b, double gate);
+/* Diagnostic: pihm_gpu_set_wait_limit for the batch's evaluations; the
+ * watersheds of one that gave up fail. */
+int pihm_batch_set_wait_limit(pihm_batch *b, int polls);
 
 /* Admit a watershed; *id receives its handle.  PIHM_GPU_ERR_NOMEM: no room now. */
 int pihm_batch_add(pihm_batch *b, const pihm_batch_job *job, int32_t *id);

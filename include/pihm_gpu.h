@@ -304,6 +304,12 @@ int pihm_gpu_selftest_pow_int(const double *x, const double *y, double *out, int
  * are the IEEE results bit for bit. */
 int pihm_gpu_selftest_div_sqrt_int(const double *a, const double *b, double *q, double *r,
                                    int32_t *ok, int64_t n, void *stream);
+/* Diagnostic: how often a wait inside the one-launch evaluation of a small
+ * mesh looks at its counter before it gives up (0: not once; negative: the
+ * default, some seconds).  An evaluation that gave up makes pihm_gpu_status
+ * (and pihm_gpu_rhs_host, pihm_gpu_wait) return PIHM_GPU_ERR_CUDA; the next one
+ * starts afresh. */
+int pihm_gpu_set_wait_limit(pihm_gpu_ctx *ctx, int polls);
 /* Diagnostic: the land-surface step's exponential and natural logarithm,
  * e[i] = exp(x[i]) and l[i] = log(x[i]); device arrays of length n,
  * asynchronous on `stream`. */

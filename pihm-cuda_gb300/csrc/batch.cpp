@@ -889,6 +889,7 @@ int pihm_batch_create(const pihm_batch_limits *lim, int surf_mode, int riv_mode,
   m.bank_part = D(8 * NE);
   m.err = dalloc<unsigned int>(1, o);
   m.bar = dalloc<unsigned int>(pihm::kBarWords, o);
+  m.bar_polls = pihm::kBarPolls;
   int32_t *se = I(NE), *sr = I(NR), *sed = I(NED), *sb = I(NE);
   m.sys_elem = se;
   m.sys_riv = sr;
@@ -1017,6 +1018,12 @@ int pihm_batch_limits_for_memory(int64_t bytes, double rivers_per_elem, double e
 int pihm_batch_set_rhs_gate(pihm_batch *b, double gate) {
   if (!b || !(gate >= 0.0 && gate <= 1.0)) return PIHM_GPU_ERR_ARG;
   b->rhs_gate = gate;
+  return PIHM_GPU_OK;
+}
+
+int pihm_batch_set_wait_limit(pihm_batch *B, int polls) {
+  if (!B) return PIHM_GPU_ERR_ARG;
+  B->A.m.bar_polls = polls < 0 ? pihm::kBarPolls : polls;
   return PIHM_GPU_OK;
 }
 

@@ -212,6 +212,7 @@ int pihm_gpu_create(const pihm_gpu_mesh *g, int surf_mode, int riv_mode, double 
   c->d_stage_out = carve<double>(dp, c->neq);
   m.err = carve<unsigned int>(dp, 1);
   m.bar = carve<unsigned int>(dp, kBarWords);
+  m.bar_polls = kBarPolls;
   m.diag = 0;
   if (cudaMallocHost((void **)&c->h_status, 2 * sizeof(uint64_t)) != cudaSuccess) {
     c->h_status = nullptr;
@@ -263,6 +264,12 @@ void *pihm_gpu_get_stream(const pihm_gpu_ctx *c) { return c ? (void *)c->stream 
 int pihm_gpu_set_kernel_shape(pihm_gpu_ctx *c, int shape) {
   if (!c || shape < 0 || shape > 2) return PIHM_GPU_ERR_ARG;
   c->m.main_shape = shape;
+  return PIHM_GPU_OK;
+}
+
+int pihm_gpu_set_wait_limit(pihm_gpu_ctx *c, int polls) {
+  if (!c) return PIHM_GPU_ERR_ARG;
+  c->m.bar_polls = polls < 0 ? kBarPolls : polls;
   return PIHM_GPU_OK;
 }
 

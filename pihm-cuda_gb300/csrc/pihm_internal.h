@@ -43,6 +43,7 @@ constexpr int32_t kBoundary = INT32_MIN;
 constexpr unsigned kErrNan = 1u, kErrWait = 2u;
 constexpr int kStatusTicket = 144;  // the word of it that k_permute_ref counts its blocks in
 constexpr int kBarWords = 160;  // unsigned words of DevMesh::bar
+constexpr int kBarPolls = 1 << 22;  // DevMesh::bar_polls, a few seconds
 
 // Device view of one watershed, passed by value to the kernels.
 struct DevMesh {
@@ -113,6 +114,7 @@ struct DevMesh {
 
   unsigned int *err;  // error word: kErrNan, kErrWait
   unsigned int *bar;  // k_rhs_fused's barrier counters (null: not used)
+  int bar_polls;      // and the polls after which a wait gives up
 
   // Launch extents.  A single-watershed context evaluates every item
   // (ne_run = ne, ...); the batch engine's arena places watersheds in ranges of

@@ -1370,9 +1370,8 @@ __global__ void __launch_bounds__(128, 6) k_bank_rows(DevMesh m, double *RESTRIC
 // an interior edge nothing would, so then (edges alone read the gradients) the
 // elements are done when they have raised A.
 // Cooperative launch makes the blocks resident together; a wait gives up after
-// kBarPolls polls, and the blocks then report kErrWait instead of results.
+// m.bar_polls polls, and the blocks then report kErrWait instead of results.
 // ---------------------------------------------------------------------------
-constexpr int kBarPolls = 1 << 22;  // a few seconds
 constexpr int kBarStride = 32;      // counters on cache lines of their own
 
 __device__ __forceinline__ void bar_arrive(unsigned *cnt) {
@@ -1380,10 +1379,10 @@ __device__ __forceinline__ void bar_arrive(unsigned *cnt) {
   if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
 }
 // false when the wait ran out; the same answer in every thread of the block
-__device__ __forceinline__ bool bar_wait(unsigned *cnt, unsigned blocks, int *s_ok) {
+__device__ __forceinline__ bool bar_wait(const DevMesh &m, unsigned *cnt, unsigned blocks, int *s_ok) {
   if (threadIdx.x == 0) {
     unsigned v = 0;
-    for (int k = 0; k < kBarPolls; k++) {
+    for (int k = 0; k < m.bar_polls; k++) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
       if (v >= blocks) break;
     }
@@ -1464,7 +1463,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     const bool on = one && first < m.ne_run && !skip_item(m, m.sys_elem, first, &sy);
     GradIn in;
     if (on) in = grad_load(m, y, first);
-    if (!bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (!bar_wait(m, A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
     if (on) m.gradmag[first] = grad_value(m, in);
     for (int i = first; !one && i < m.ne_run; i += step)
       if (!skip_item(m, m.sys_elem, i, &sy)) m.gradmag[i] = grad_value(m, grad_load(m, y, i));
@@ -1475,7 +1474,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
   if (blk < g.edge) {
     // ---- edges ----
     const int first = blk * blockDim.x + threadIdx.x, step = g.edge * blockDim.x;
-    if (!bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
+    if (!bar_wait(m, A, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
     bool waited = !grad;
     // whole blocks go round together: the wait is the block's
     for (int e = first; e - (int)threadIdx.x < m.nedge_run; e += step) {
@@ -1490,7 +1489,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
       }
       if (!waited) {
         waited = true;
-        if (!bar_wait(B, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
+        if (!bar_wait(m, B, g.elem, &s_ok)) return report_wait(m, m.sys_edge, first, m.nedge_run, step);
       }
       if (wet) m.eflux_ovl[e] = hp * diff_h * rsqrt(edge_slope(m, e, i, k, diff_h)) * m.e_ovlk[e];
     }
@@ -1514,12 +1513,12 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     bar_arrive(R);
     bool ok;
     if (part == PART_CHAN) {
-      ok = bar_wait(R, g.river, &s_ok);
+      ok = bar_wait(m, R, g.river, &s_ok);
       for (int s = first; ok && s < m.nr_run; s += step)
         if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, yr, s, PART_CHAN);
     } else {
-      ok = bar_wait(A, g.elem, &s_ok);
-      if (ok && part == PART_BED) ok = bar_wait(R, g.river, &s_ok);
+      ok = bar_wait(m, A, g.elem, &s_ok);
+      if (ok && part == PART_BED) ok = bar_wait(m, R, g.river, &s_ok);
       for (int s = first; ok && s < m.nr_run; s += step)
         if (!skip_item(m, m.sys_riv, s, &sy)) river_part(m, y, s, part);
     }
@@ -1530,7 +1529,7 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     const bool on = first < m.nr_run && !skip_item(m, m.sys_riv, first, &sy);
     RiverRowsIn in;
     if (on) in = river_rows_load(m, first);
-    if (ok) ok = bar_wait(C, lateral, &s_ok);
+    if (ok) ok = bar_wait(m, C, lateral, &s_ok);
     if (!ok) return report_wait(m, m.sys_riv, first, m.nr_run, step);
     bar_leave(m.bar, per + g.col);
     if (on) river_rows_item(m, ydot, first, sy, in);
@@ -1547,19 +1546,19 @@ __global__ void __launch_bounds__(kFusedThreads, kMinBlocks)
     Column c;
     RowsIn r;
     // kFromRef: the state in internal order is the element blocks' to write
-    if (kFromRef && !met && !bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (kFromRef && !met && !bar_wait(m, A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
     if (on) {
       column_state(m, y, i, sy, c);
       rows_load(m, i, r);
     }
-    if (!kFromRef && !met && !bar_wait(A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+    if (!kFromRef && !met && !bar_wait(m, A, g.elem, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
     if (on) {
       column_surface(m, i, c);
       c.kinf_crack = crack_kinf(c, r.kinf_mat, r.kmac_a);
     }
     if (!met) {
       met = true;
-      if (!bar_wait(C, lateral, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
+      if (!bar_wait(m, C, lateral, &s_ok)) return report_wait(m, m.sys_elem, first, m.ne_run, step);
       bar_leave(m.bar, g.river / kRivParts + g.col);
       }
     if (on) column_rows<true>(m, ydot, i, sy, c, r);
