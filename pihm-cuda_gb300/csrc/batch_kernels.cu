@@ -146,13 +146,19 @@ __device__ __forceinline__ void round_end(const DeviceArena &A, int nrs, uint64_
   }
 }
 
+// A block's shared memory, one for every reduction it may run: a round's
+// watersheds are bounded by what it and the programs leave of 48 KB.
+struct BlockShared {
+  Pair a[kThreads / 32], b[kThreads / 32];
+  bool last;
+};
+
 // RED2 >= 0: a second reduction, of A.vec slots ry and rw.
 template <int kU, int RED, int RED2 = -1>
 __device__ void run_block(const DeviceArena &A, const RoundSys &R, const SysInfo &S, const Op *prog, int b, int nrs,
-                          uint64_t *flag, uint64_t seq) {
-  __shared__ Pair sh[kThreads / 32];
-  __shared__ Pair sh2[kThreads / 32];
-  __shared__ bool last;
+                          uint64_t *flag, uint64_t seq, BlockShared &bs) {
+  Pair *const sh = bs.a, *const sh2 = bs.b;
+  bool &last = bs.last;
   const long long vs = A.neq_cap;
   double *base = A.vec + S.off;
   const int nops = R.prog_len;
@@ -319,14 +325,16 @@ __global__ void __launch_bounds__(kU == 0 ? kSpreadThreads : kThreads, (kU == 0 
       case kRedMinWsq: run_warp<R_MIN, R_WSQ>(A, R, S, s_ops, vw, nrs, flag, seq); break;
       default: run_warp<-1>(A, R, S, s_ops, vw, nrs, flag, seq); break;
     }
-  } else
-  switch (R.red) {
-    case R_DOT: run_block<kU, R_DOT>(A, R, S, s_ops, b, nrs, flag, seq); break;
-    case R_MAXABS: run_block<kU, R_MAXABS>(A, R, S, s_ops, b, nrs, flag, seq); break;
-    case R_WSQ: run_block<kU, R_WSQ>(A, R, S, s_ops, b, nrs, flag, seq); break;
-    case R_MIN: run_block<kU, R_MIN>(A, R, S, s_ops, b, nrs, flag, seq); break;
-    case kRedMinWsq: run_block<kU, R_MIN, R_WSQ>(A, R, S, s_ops, b, nrs, flag, seq); break;
-    default: run_block<kU, -1>(A, R, S, s_ops, b, nrs, flag, seq); break;
+  } else {
+    __shared__ BlockShared bs;
+    switch (R.red) {
+      case R_DOT: run_block<kU, R_DOT>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+      case R_MAXABS: run_block<kU, R_MAXABS>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+      case R_WSQ: run_block<kU, R_WSQ>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+      case R_MIN: run_block<kU, R_MIN>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+      case kRedMinWsq: run_block<kU, R_MIN, R_WSQ>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+      default: run_block<kU, -1>(A, R, S, s_ops, b, nrs, flag, seq, bs); break;
+    }
   }
 }
 
