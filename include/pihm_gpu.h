@@ -167,8 +167,11 @@ int pihm_gpu_set_river_edge_ovlflow(pihm_gpu_ctx *ctx, const double *ovlflow);
  * a device error word that pihm_gpu_status reads. */
 int pihm_gpu_rhs(pihm_gpu_ctx *ctx, double t, const double *y_dev,
                  double *ydot_dev);
-/* Synchronise the context's stream and return (then clear) the error word:
- * 0 or PIHM_GPU_ERR_NAN / PIHM_GPU_ERR_CUDA. */
+/* Wait for everything queued on the context's stream so far and return (then
+ * clear) the error word: 0 or PIHM_GPU_ERR_NAN / PIHM_GPU_ERR_CUDA (a launch
+ * failed, or a wait inside an evaluation gave up).  The word comes from a kernel
+ * behind the queued work, so an event or a query behind the call can still be
+ * pending for a moment. */
 int pihm_gpu_status(pihm_gpu_ctx *ctx);
 
 /* Same evaluation from host arrays in reference order: y in, run, ydot out,
@@ -195,14 +198,15 @@ int pihm_gpu_set_host_path(pihm_gpu_ctx *ctx, int mode);
  * beside the other's kernels. */
 int pihm_gpu_rhs_host_async(pihm_gpu_ctx *ctx, double t, const double *y_host, double *ydot_host);
 /* Wait for the context's queued work: PIHM_GPU_OK, or PIHM_GPU_ERR_NAN if any
- * of its evaluations since the last status read produced a NaN. */
+ * of its evaluations since the last status read produced a NaN
+ * (PIHM_GPU_ERR_CUDA as pihm_gpu_status). */
 int pihm_gpu_wait(pihm_gpu_ctx *ctx);
 /* Whether the last pihm_gpu_rhs_host call accessed host memory directly, and
  * whether the device can access pageable host memory (either may be NULL). */
 int pihm_gpu_host_path_info(const pihm_gpu_ctx *ctx, int *last_direct, int *pageable_access);
 
-/* pihm_gpu_ode on device vectors synchronises after each evaluation to read
- * the NaN error word (the reference checks every call).  deferred = 1 skips
+/* pihm_gpu_ode on device vectors waits after each evaluation to read the NaN
+ * error word (the reference checks every call).  deferred = 1 skips
  * that; the word is then read by the next pihm_gpu_status. */
 int pihm_gpu_set_nan_check(pihm_gpu_ctx *ctx, int deferred);
 /* Post-step update on device state (internal order): ws0.surf <- y_dev[0:nelem]
@@ -271,7 +275,9 @@ int pihm_gpu_to_reference(pihm_gpu_ctx *ctx, const double *src_int_dev,
 /* Number of kernels this context has launched so far. */
 int pihm_gpu_launch_count(const pihm_gpu_ctx *ctx, int64_t *count);
 /* Bracket every later kernel launch with CUDA events on the context's
- * stream. */
+ * stream.  While on, an evaluation runs as separate kernels: a small mesh not
+ * in one launch, and the river kernels not inside the element kernels' grids.
+ * The results are the same, the times are those of these launches. */
 int pihm_gpu_set_profiling(pihm_gpu_ctx *ctx, int on);
 /* Synchronise, then return and reset the accumulated device time (ms) and
  * launch count per kernel: 0 prep, 1 gradient, 2 element, 3 river,

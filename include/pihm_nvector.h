@@ -10,7 +10,9 @@
  * norms) use a fixed two-level tree, so they are deterministic run to run and
  * differ from the serial left-to-right sum only by rounding.
  *
- * Reductions return their value to the host, which synchronises the stream.
+ * Reductions return their value to the host: the call waits until the kernel's
+ * last block has handed it over, behind everything queued on the stream before
+ * it (an event or a query behind the call can still be pending for a moment).
  *
  * Include order: when the SUNDIALS headers are used too, include them first;
  * otherwise this header declares the layout-compatible N_Vector types itself.
@@ -174,8 +176,8 @@ int N_VWrmsNormSlot_PihmGpu(N_Vector x, N_Vector w, int slot);
 int N_VLinearSumCoef_PihmGpu(const pihm_nv_coef *a, N_Vector x, const pihm_nv_coef *b, N_Vector y,
                              N_Vector z);
 /* Copy slots 0..count-1 of v's family to out[] -- and, when dev_word is not
- * null, one 32-bit device word to *word_out -- with one synchronisation of
- * v's stream.  Returns 0, -1 (bad argument) or -2 (CUDA error). */
+ * null, one 32-bit device word to *word_out -- with one wait for v's
+ * stream.  Returns 0, -1 (bad argument) or -2 (CUDA error). */
 int N_VFetchSlots_PihmGpu(N_Vector v, int count, double *out, const unsigned int *dev_word,
                           unsigned int *word_out);
 /* The stream a device vector's operations run on. */

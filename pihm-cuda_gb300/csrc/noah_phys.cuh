@@ -3,8 +3,8 @@
 // functions below name their reference and its lines): the same operations
 // in the same order, so that, with the file compiled without multiply-add
 // contraction, each element follows the reference's arithmetic; powers go
-// through pow_any (within 0.502 ulp of the exact power, as glibc's), the
-// other elementary functions are CUDA's.
+// through pow_any (within 0.502 ulp of the exact power, as glibc's), exp, log
+// and log10 through int_math.cuh, and atan is CUDA's (Real below).
 //
 // A column carries the element's parameters, forcing and state in a
 // per-thread struct (the layer arrays in local memory); the kernels in

@@ -100,11 +100,13 @@ static inline unsigned grid_for(long long n) {
 }
 
 // The kernels here are programmatic dependent launches: a block waits for the
-// kernel before it and reads nothing until then.  An iteration's sixteen
-// operations over 31,337 entries take 68 us instead of 86, over 3.06M 238
-// instead of 258.  A grid of one wave lets the next one's blocks in as it
-// starts; of more, they would hold its own blocks' places (3.06M: 262).
-constexpr unsigned kWave = 8 * 152;
+// kernel before it and reads nothing until then.  A Newton and GMRES
+// iteration's fourteen operations, four of which return a value, over 31,337
+// entries take 68 us instead of 86, over 3.06M 239 instead of 258.  A grid of
+// one wave lets the next one's blocks in as it starts (k_red: unless its value
+// stays in a slot); of more, they would hold its own blocks' places (3.06M:
+// 262).
+constexpr unsigned kWave = 8 * 152;  // 256-thread blocks that GB300's SMs hold at once
 __device__ __forceinline__ void begin_after_previous() {
   if (gridDim.x <= kWave) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -193,7 +193,7 @@ __device__ __forceinline__ int queue_slot(int *count, bool take) {
 // evaluated densely.
 // ---------------------------------------------------------------------------
 constexpr int kPrepBlock = 256;
-constexpr unsigned kPrepWave = 8 * 152;  // blocks the SMs hold at once
+constexpr unsigned kPrepWave = 8 * 152;  // blocks that GB300's SMs hold at once
 
 // SurfH and EffKh of one element (src/hydrol.c:100-134, src/lat_flow.c:248-277):
 // what needs no root or division is stored here; thin asks for
@@ -598,8 +598,10 @@ __global__ void __launch_bounds__(kPrepBlock) k_elem_prep(DevMesh m, const doubl
   int sy = 0;
   // With more blocks than the SMs hold at once (8 each), k_elem_grad's would
   // stand waiting through the last of them: its blocks come when these end.
-  // One stream pays 1 us of 147 for it (400,000 elements), four that fill the
-  // device gain 28 of 1,056.  In one wave the early start gives 4 us of 86.
+  // Eight evaluations of 400,000 elements: on four streams that fill the
+  // device 1,035 us, 1,053 with the early start; on two 1,060 and 1,055, and
+  // one evaluation with its reordering 154 and 153.  In one wave the early
+  // start gives 4 us of 86.
   const bool early = gridDim.x <= kPrepWave;
   wait_for_previous();
   if (early || (int)blockIdx.x < river_blocks) next_may_start();
